@@ -1,0 +1,286 @@
+// Recurrences over time taken sixteen rows at a time, in float on the CUDA cores.
+//
+// A state S [N key channels, P value channels] that decays channel by channel and takes outer products is, over a chunk of sixteen
+// rows, a linear map of what it was before: with the rows' own vectors multiplied once by the decays between them and the chunk's
+// borders (a kernel over all chunks side by side), what is left in time order is
+//
+//     O = X0 S + G V          E = X1 S (delta rules only)          S <- tot * S + Z0^T V - Z1^T E
+//
+// with X0, X1, Z0, Z1 [16, N] and G [16, 16] a chunk: products over sixteen rows, where the row-by-row scan has two dot products,
+// three shuffles and an update a row, each waiting for the one before.  The arithmetic is of the same order (5 N P against 4 N P
+// multiply-adds a row of a delta rule); what goes is the chain.
+//
+// A chunk of one head is one run of floats in memory ("pack"): X0 [16][D], (X1 [16][D],) Z0 [16][D], (Z1 [16][D],) G [16][20], tot [D], D = N rounded up to 64, 128 or 256, zeros (tot: ones) past N and past a sequence's last row.
+#pragma once
+
+#include <type_traits>
+
+#include "mma_tiles.cuh"
+
+#define CHUNK 16              // rows
+#define CHUNK_G 20            // floats a row of G: sixteen and a gap, so that the rows that eight threads read start in different banks
+
+__host__ __device__ constexpr int chunk_pack_floats(int D, bool delta) { return (delta ? 4 : 2) * CHUNK * D + CHUNK * CHUNK_G + D; }
+// A launch takes chunks [first, first + count) of every sequence.  Where sequence `seq`, whose rows start at row0 of the step, keeps chunk c:
+// with all of a step's chunks in one launch (segment 0) by its rows, so that sequences never meet and few places stay empty; else `segment`
+// places a sequence.
+struct ChunkSpan {
+    int first, count, segment;
+};
+__device__ __forceinline__ size_t chunk_place(const ChunkSpan& span, int row0, int seq, int c) {
+    return span.segment ? (size_t)seq * span.segment + (c - span.first) : (size_t)(row0 / CHUNK) + seq + c;
+}
+// Chunks of scratch for a step: all of them, or as many as 2^28 floats hold (a gigabyte; at least one a sequence), and then the step goes
+// segment by segment, which hands the state on through memory and so must be allowed to write it.  0: not taken.
+static inline long long chunk_capacity(long long rows, long long seqs, long long H, int pack_floats, int write_state) {
+    const long long total = rows / CHUNK + seqs + 1, most = (1ll << 28) / (H * pack_floats);
+    if (total <= most) return total;
+    return write_state ? (most > seqs ? most / seqs * seqs : seqs) : 0;
+}
+
+// Rows of X times the state, summed over the sixteen lanes of a half warp (lane `dg` of it holds key channels 4 dg + 64 m .. + 3): lane dg is left
+// with row dg.  A lane forms its I-th partial sum for row I ^ dg, so every exchange sends a register that all lanes name alike
+// (fifteen shuffles a value, no selection).  The rows come in four groups, I = i, i + 8, i + 4, i + 12 for i = 0, 2, 1, 3: a group's
+// rows are loaded while the group before is worked on.
+__host__ __device__ constexpr int chunk_row_of(int group, int k) { return (group == 0 ? 0 : group == 1 ? 2 : group == 2 ? 1 : 3) + (k & 1) * 8 + (k >> 1) * 4; }
+template <int DT> struct ChunkRows {
+    ulonglong2 x[4][DT / 4];
+    __device__ __forceinline__ void load(const float* rows, int group, int dg) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int m = 0; m < DT / 4; m++) x[k][m] = *reinterpret_cast<const ulonglong2*>(rows + (chunk_row_of(group, k) ^ dg) * (16 * DT) + 64 * m);
+    }
+    // out: the group's four rows times the state, halved twice.
+    template <int PT> __device__ __forceinline__ void times(const uint64_t (*S)[PT], float* out) const {
+        float part[4][PT];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uint64_t a[PT];
+#pragma unroll
+            for (int m = 0; m < DT / 4; m++)
+#pragma unroll
+                for (int p = 0; p < PT; p++) a[p] = fma_f32x2(x[k][m].x, S[2 * m][p], m ? a[p] : 0ull);
+#pragma unroll
+            for (int m = 0; m < DT / 4; m++)
+#pragma unroll
+                for (int p = 0; p < PT; p++) a[p] = fma_f32x2(x[k][m].y, S[2 * m + 1][p], a[p]);
+#pragma unroll
+            for (int p = 0; p < PT; p++) {
+                float lo, hi;
+                unpack_f32x2(a[p], lo, hi);
+                part[k][p] = lo + hi;
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < PT; p++) {
+            part[0][p] += __shfl_xor_sync(0xffffffffu, part[1][p], 8);
+            part[2][p] += __shfl_xor_sync(0xffffffffu, part[3][p], 8);
+        }
+#pragma unroll
+        for (int p = 0; p < PT; p++) out[p] = part[0][p] + __shfl_xor_sync(0xffffffffu, part[2][p], 4);
+    }
+};
+template <int PT> __device__ __forceinline__ void chunk_groups(const float (*g)[PT], float* out) {
+    float a[PT], b[PT];
+#pragma unroll
+    for (int p = 0; p < PT; p++) {
+        a[p] = g[0][p] + __shfl_xor_sync(0xffffffffu, g[1][p], 2);
+        b[p] = g[2][p] + __shfl_xor_sync(0xffffffffu, g[3][p], 2);
+    }
+#pragma unroll
+    for (int p = 0; p < PT; p++) out[p] = a[p] + __shfl_xor_sync(0xffffffffu, b[p], 1);
+}
+
+// A block takes (a slice of 32 value channels, head, sequence): a half warp holds the key channels of four value channels in registers, two
+// key channels to a 64-bit register (fma.rn.f32x2), for all of the sequence's rows.  A chunk's pack and its 16 x 32 values come
+// through a ring of asynchronous copies.
+#define CHUNK_THREADS 128
+#define CHUNK_STAGES 3         // chunks on their way or worked on
+template <int DL, bool DELTA>      // D = 32 DL
+__global__ void __launch_bounds__(CHUNK_THREADS)
+chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v_stride, float* __restrict__ state, const int* __restrict__ seq_rows,
+                  const int* __restrict__ seq_slot, float* __restrict__ out, int H, int N, int P, int n_slots, int write_state) {
+    constexpr int DT = 2 * DL, D = 16 * DT, PT = 4, MATS = DELTA ? 4 : 2, PACK = chunk_pack_floats(D, DELTA), V_AT = PACK, STAGE = V_AT + CHUNK * 32;
+    extern __shared__ __align__(16) float chunk_smem[];
+    const int dg = threadIdx.x & 15, pg = threadIdx.x >> 4;
+    float* mine = chunk_smem + CHUNK_STAGES * STAGE + pg * CHUNK * PT;      // what a half warp hands to itself: -E of its value channels
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(pack); PDL_FRESH(v);
+    const int seq = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * 32;
+    const int slot = seq_slot[seq];
+    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
+    if (slot < 0 || slot >= n_slots || n_rows <= 0) return;
+    const int n_chunks = min(span.first + span.count, (n_rows + CHUNK - 1) / CHUNK);
+    if (span.first >= n_chunks) return;
+    const int pv = min(32, P - p0);                                        // value channels that exist (a multiple of four)
+    // The values past the sequence's rows and past the head's channels are never copied: they stay zero.
+    for (int i = threadIdx.x; i < CHUNK_STAGES * CHUNK * 32; i += CHUNK_THREADS) chunk_smem[(i / (CHUNK * 32)) * STAGE + V_AT + i % (CHUNK * 32)] = 0.0f;
+    __syncthreads();
+    auto issue = [&](int c) {
+        const float* src = pack + (chunk_place(span, row0, seq, c) * H + h) * PACK;
+        const uint32_t dst = ad_smem(chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < PACK / 4; i += CHUNK_THREADS) cp_async16(dst + 16 * i, src + 4 * i);
+        const int rows = min(CHUNK, n_rows - c * CHUNK), t = threadIdx.x >> 3, at = 4 * (threadIdx.x & 7);
+        if (t < rows && at < pv) cp_async16(dst + 4 * (V_AT + t * 32 + at), v + (size_t)(row0 + c * CHUNK + t) * v_stride + (size_t)h * P + p0 + at);
+    };
+#pragma unroll
+    for (int i = 0; i < CHUNK_STAGES - 1; i++) {
+        if (span.first + i < n_chunks) issue(span.first + i);
+        cp_async_commit();
+    }
+    uint64_t S[DT / 2][PT];
+    const bool p_ok = pg * PT < pv;
+    float* st = state + (((size_t)slot * H + h) * P + p0 + (p_ok ? pg * PT : 0)) * N + 4 * dg;
+#pragma unroll
+    for (int m = 0; m < DT / 4; m++)
+#pragma unroll
+        for (int p = 0; p < PT; p++) {
+            const bool ok = p_ok && 4 * dg + 64 * m < N;
+            const float4 x = ok ? *reinterpret_cast<const float4*>(st + (size_t)p * N + 64 * m) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            S[2 * m][p] = pack_f32x2(x.x, x.y);
+            S[2 * m + 1][p] = pack_f32x2(x.z, x.w);
+        }
+    for (int c = span.first; c < n_chunks; c++) {
+        cp_async_wait<CHUNK_STAGES - 2>();
+        __syncthreads();          // the chunk is there for all, and all have left the one whose stage is filled next
+        if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
+        cp_async_commit();
+        const float* sx = chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE;
+        const float *x0 = sx + 4 * dg, *z0 = x0 + (DELTA ? 2 : 1) * CHUNK * D, *z1 = z0 + CHUNK * D, *g = sx + MATS * CHUNK * D, *tot = g + CHUNK * CHUNK_G;
+        const float* sv = sx + V_AT + pg * PT;
+        float vr[CHUNK][PT];      // sixteen rows of this half warp's values
+#pragma unroll
+        for (int t = 0; t < CHUNK; t++) {
+            const float4 x = *reinterpret_cast<const float4*>(sv + t * 32);
+            vr[t][0] = x.x, vr[t][1] = x.y, vr[t][2] = x.z, vr[t][3] = x.w;
+        }
+        float o[PT], of_group[4][PT];
+        ChunkRows<DT> rows_now, rows_next;
+        rows_now.load(DELTA ? x0 + CHUNK * D : x0, 0, dg);
+        if (DELTA) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                rows_next.load(i < 3 ? x0 + CHUNK * D : x0, (i + 1) & 3, dg);
+                rows_now.template times<PT>(S, of_group[i]);
+                rows_now = rows_next;
+            }
+            float e[PT];
+            chunk_groups<PT>(of_group, e);
+            __syncwarp();
+            *reinterpret_cast<float4*>(mine + dg * PT) = make_float4(-e[0], -e[1], -e[2], -e[3]);
+            __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (i < 3) rows_next.load(x0, i + 1, dg);
+            rows_now.template times<PT>(S, of_group[i]);
+            rows_now = rows_next;
+        }
+        chunk_groups<PT>(of_group, o);
+        // The rows' own part, G V: this lane's row of G against the values up to its own (later rows' are not touched: a zero of G times
+        // an infinity would be none).
+#pragma unroll
+        for (int s4 = 0; s4 < CHUNK / 4; s4++) {
+            const float4 gg = *reinterpret_cast<const float4*>(g + dg * CHUNK_G + 4 * s4);
+            const float gs[4] = {gg.x, gg.y, gg.z, gg.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int p = 0; p < PT; p++)
+                    if (4 * s4 + e <= dg) o[p] = fmaf(gs[e], vr[4 * s4 + e][p], o[p]);
+        }
+        if (p_ok && c * CHUNK + dg < n_rows)
+            *reinterpret_cast<float4*>(out + (size_t)(row0 + c * CHUNK + dg) * H * P + (size_t)h * P + p0 + pg * PT) = make_float4(o[0], o[1], o[2], o[3]);
+        // The state after the chunk.
+        float s[DT][PT];
+#pragma unroll
+        for (int m = 0; m < DT / 4; m++) {
+            const ulonglong2 t2 = *reinterpret_cast<const ulonglong2*>(tot + 4 * dg + 64 * m);
+#pragma unroll
+            for (int p = 0; p < PT; p++) {
+                unpack_f32x2(fma_f32x2(t2.x, S[2 * m][p], 0ull), s[4 * m][p], s[4 * m + 1][p]);
+                unpack_f32x2(fma_f32x2(t2.y, S[2 * m + 1][p], 0ull), s[4 * m + 2][p], s[4 * m + 3][p]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < CHUNK; r++) {
+#pragma unroll
+            for (int m = 0; m < DT / 4; m++) {
+                const float4 z = *reinterpret_cast<const float4*>(z0 + r * D + 64 * m);
+                const float zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], vr[r][p], s[4 * m + i][p]);
+            }
+        }
+        if (DELTA) {
+#pragma unroll
+            for (int r = 0; r < CHUNK; r++) {
+                const float4 e4 = *reinterpret_cast<const float4*>(mine + r * PT);
+                const float es[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+                for (int m = 0; m < DT / 4; m++) {
+                    const float4 z = *reinterpret_cast<const float4*>(z1 + r * D + 64 * m);
+                    const float zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], es[p], s[4 * m + i][p]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < DT / 2; i++)
+#pragma unroll
+            for (int p = 0; p < PT; p++) S[i][p] = pack_f32x2(s[2 * i][p], s[2 * i + 1][p]);
+    }
+    if (write_state && p_ok) {
+#pragma unroll
+        for (int m = 0; m < DT / 4; m++)
+#pragma unroll
+            for (int p = 0; p < PT; p++)
+                if (4 * dg + 64 * m < N) {
+                    float4 x;
+                    unpack_f32x2(S[2 * m][p], x.x, x.y);
+                    unpack_f32x2(S[2 * m + 1][p], x.z, x.w);
+                    *reinterpret_cast<float4*>(st + (size_t)p * N + 64 * m) = x;
+                }
+    }
+}
+
+template <int DL, bool DELTA>
+static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, const float* v, int v_stride, float* state, const int* seq_rows, const int* seq_slot,
+                                     float* out, int seqs, int H, int N, int P, int n_slots, int write_state, cudaStream_t s) {
+    constexpr size_t SMEM = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<DL, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    return bc_launch(chunk_scan_kernel<DL, DELTA>, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H,
+                     N, P, n_slots, write_state);
+}
+
+// A step's chunks through `prepare` (the kernel that fills the pack) and the scan: at once where `capacity` chunks of scratch hold them, else
+// segment by segment (at least one chunk a sequence, and the state must be written).
+static inline bool chunk_fits(long long capacity, long long rows, long long seqs, int write_state) {
+    return capacity >= rows / CHUNK + seqs + 1 || (write_state && capacity >= seqs);
+}
+template <class Prepare, class Scan>
+static cudaError_t chunk_step(long long capacity, int rows, int seqs, int max_new, Prepare prepare, Scan scan) {
+    const int most = (max_new + CHUNK - 1) / CHUNK;
+    const bool whole = capacity >= (long long)rows / CHUNK + seqs + 1;
+    const int segment = whole ? most : (int)(capacity / seqs);
+    cudaError_t e = cudaSuccess;
+    for (int at = 0; at < most && e == cudaSuccess; at += segment) {
+        const ChunkSpan span = {at, segment < most - at ? segment : most - at, whole ? 0 : segment};
+        e = prepare(span);
+        if (e == cudaSuccess) e = scan(span);
+    }
+    return e;
+}

@@ -1,0 +1,319 @@
+// The generalized delta rule on prompts, sixteen rows at a time (chunks.cuh):
+//
+//     S_t = diag(w_t) S_(t-1) - b_t (u_t^T S_(t-1)) + k_t v_t^T        o_t = S_t^T r_t          (b = a * u)
+//
+// Within a chunk let W_t be the product of its decays up to row t (W_(-1) = 1).  The removed e_t = u_t^T S_(t-1) obeys
+//
+//     e_t = U_t S + sum_(s<t) Bm_ts v_s - A_ts e_s,      U_t = u_t W_(t-1),  A_ts = sum_i u_t b_s W_(t-1) / W_s,  Bm_ts = the same with k_s,
+//
+// a unit lower triangular system whose matrix is the chunk's own: e = P S + M V with P = (1 + A)^-1 U, M = (1 + A)^-1 Bm, by forward
+// substitution.  With H_ts = sum_i r_t b_s W_t / W_s and Gm_ts with k_s (s <= t), the chunk is then
+//
+//     X1 = P      X0 = r_t W_t - H P      G = Gm - H M      Z1 = b_s W_15 / W_s      Z0 = k_s W_15 / W_s - M^T Z1      tot = W_15.
+//
+// A decay is at least exp(-decay_scale), so sixteen of them are divided by safely up to a decay_scale of 4 (exp(-64)).  Float throughout.
+// Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
+// of 2,048 rows, 64 heads of 64, decay rank 64: 54 + 140 + 236 us, where preparing the rows and scanning them one by one takes 172 + 614.
+// The first two are bound by their instructions; the last walks 128 chunks at 1.9 us each, one warp a scheduler, each chunk's products
+// waiting for the state of the one before (IPC 0.3 to 0.6 in every layout tried: half warps or warps a row, four or eight value channels
+// a warp, sums across lanes or through shared memory, all within 3 % of one another).  Distance from 64-bit sums: 1.8e-7 of the
+// outputs and 1.4e-7 of the state, where the scan has 1.1e-7 and 0.9e-7.
+#include "chunks.cuh"
+
+// ------------------------------------------------------------------------------------ decays
+// decay[r, c] = exp(-decay_scale * sigmoid(z + w0[c])) with z = sum_j w2t[j, c] tanh(inner[r, j]): a product of 64 rows x 128 channels a block,
+// eight rows by four channels a thread, 32 inner channels at a time.
+#define DLC_ROWS 64
+#define DLC_COLS 128
+#define DLC_K 32
+__global__ void __launch_bounds__(256)
+delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __restrict__ w2t, const float* __restrict__ w0, float* __restrict__ decay, int rows, int HD,
+                   int inner, float decay_scale) {
+    __shared__ __align__(16) float th[DLC_K][DLC_ROWS + 4];
+    __shared__ __align__(16) float wt[DLC_K][DLC_COLS];
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(proj);
+    const int row0 = blockIdx.y * DLC_ROWS, c0 = blockIdx.x * DLC_COLS;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;             // channels 4 tx .., rows 8 ty ..
+    uint64_t z[8][2] = {};
+    for (int j0 = 0; j0 < inner; j0 += DLC_K) {
+        float raw[DLC_K * DLC_ROWS / 256];
+#pragma unroll
+        for (int e = 0; e < DLC_K * DLC_ROWS / 256; e++) {
+            const int i = threadIdx.x + 256 * e, r = i / DLC_K, j = i % DLC_K;
+            raw[e] = row0 + r < rows && j0 + j < inner ? proj[(size_t)(row0 + r) * stride + inner_at + j0 + j] : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < DLC_K * DLC_COLS / 256; e++) {
+            const int i = threadIdx.x + 256 * e, j = i / DLC_COLS, c = i % DLC_COLS;
+            wt[j][c] = j0 + j < inner && c0 + c < HD ? w2t[(size_t)(j0 + j) * HD + c0 + c] : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < DLC_K * DLC_ROWS / 256; e++) {
+            const int i = threadIdx.x + 256 * e;
+            th[i % DLC_K][i / DLC_K] = tanhf(raw[e]);
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int j = 0; j < DLC_K; j++) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&wt[j][4 * tx]);
+            const float4 ta = *reinterpret_cast<const float4*>(&th[j][8 * ty]), tb = *reinterpret_cast<const float4*>(&th[j][8 * ty + 4]);
+            const float t[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const uint64_t t2 = pack_f32x2(t[r], t[r]);
+                z[r][0] = fma_f32x2(w.x, t2, z[r][0]);
+                z[r][1] = fma_f32x2(w.y, t2, z[r][1]);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const int row = row0 + 8 * ty + r;
+        if (row >= rows) break;
+        float v[4];
+        unpack_f32x2(z[r][0], v[0], v[1]);
+        unpack_f32x2(z[r][1], v[2], v[3]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int c = c0 + 4 * tx + e;
+            if (c < HD) decay[(size_t)row * HD + c] = expf(-decay_scale * (1.0f / (1.0f + expf(-(v[e] + w0[c])))));
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------- packs
+#define DLC_D 64
+#define DLC_YP 36             // floats a channel of the 32 rows [r W; u W] and [b / W; k / W]: a gap against bank conflicts
+#define DLC_RUN 4             // chunks a block takes one after another, the next one's rows on their way
+
+// A block takes chunks of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen columns through the
+// same substitutions.
+__global__ void __launch_bounds__(DLC_D + 32, 4)
+delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
+                    const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int n_slots) {
+    constexpr int PACK = chunk_pack_floats(DLC_D, true), THREADS = DLC_D + 32, ROW_SET = CHUNK * DLC_D;
+    extern __shared__ __align__(16) float delta_smem[];
+    float (*in)[4][CHUNK][DLC_D] = reinterpret_cast<float (*)[4][CHUNK][DLC_D]>(delta_smem);            // two stages of decays, r, k, a
+    float *Y = delta_smem + 2 * 4 * ROW_SET, *X = Y + DLC_D * DLC_YP;
+    float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm; Bm becomes M
+    __shared__ float part[2][CHUNK];
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(proj); PDL_FRESH(decay);
+    const int h = blockIdx.y, seq = blockIdx.z, HD = H * D;
+    const int slot = seq_slot[seq];
+    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
+    const int c_first = span.first + blockIdx.x * DLC_RUN;
+    const int c_end = min(min(c_first + DLC_RUN, span.first + span.count), (n_rows + CHUNK - 1) / CHUNK);
+    if (slot < 0 || slot >= n_slots || c_first >= c_end) return;
+    const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
+    const bool channel = d < DLC_D, mine = d < D;
+    const float bias = mine ? a_bias[h * D + d] : 0.0f;
+    // What no copy reaches (rows past the sequence, channels past the head) is never used: it may hold anything.
+    auto issue = [&](int c) {
+        const int rows = min(CHUNK, n_rows - c * CHUNK), quads = D / 4;
+        const size_t first = (size_t)(row0 + c * CHUNK);
+        const uint32_t dst = ad_smem(&in[(c - c_first) & 1][0][0][0]);
+        for (int i = threadIdx.x; i < rows * quads; i += THREADS) {
+            const int t = i / quads, at = 4 * (i - t * quads);
+            const float* pr = proj + (first + t) * stride + h * D + at;
+            const uint32_t to = dst + 4 * (t * DLC_D + at);
+            cp_async16(to, decay + (first + t) * HD + h * D + at);
+            cp_async16(to + 4 * ROW_SET, pr);
+            cp_async16(to + 8 * ROW_SET, pr + HD);
+            cp_async16(to + 12 * ROW_SET, pr + 4 * HD);
+        }
+    };
+    issue(c_first);
+    cp_async_commit();
+    for (int c = c_first; c < c_end; c++) {
+        if (c + 1 < c_end) issue(c + 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const int rows = min(CHUNK, n_rows - c * CHUNK);
+        const float (*sw)[DLC_D] = in[(c - c_first) & 1][0], (*sr)[DLC_D] = in[(c - c_first) & 1][1], (*sk)[DLC_D] = in[(c - c_first) & 1][2],
+                    (*sa)[DLC_D] = in[(c - c_first) & 1][3];
+        if (channel) {
+            // Sixteen sums over a warp's channels, halved among its lanes: lane L (of sixteen) is left with row L.
+            float kk[CHUNK];
+#pragma unroll
+            for (int t = 0; t < CHUNK; t++) {
+                const float k = mine && t < rows ? sk[t][d] : 0.0f;
+                kk[t] = k * k;
+                kk[t] += __shfl_xor_sync(0xffffffffu, kk[t], 16);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int i = 0; i < o; i++) {
+                    const float keep = up ? kk[i + o] : kk[i], send = up ? kk[i] : kk[i + o];
+                    kk[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            if (lane < CHUNK) part[warp][lane] = kk[0];
+        }
+        __syncthreads();
+        float* dst = pack + (chunk_place(span, row0, seq, c) * H + h) * PACK;
+        float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
+        float total = 1.0f;
+        if (channel) {
+            float run = 1.0f, xb[4], xk[4];
+#pragma unroll
+            for (int t = 0; t < CHUNK; t++) {
+                const bool ok = mine && t < rows;
+                const float k = ok ? sk[t][d] : 0.0f;
+                const float rate = 1.0f / (1.0f + expf(-((ok ? sa[t][d] : 0.0f) + bias)));
+                const float u = ok ? k / sqrtf(part[0][t] + part[1][t] + key_eps) : 0.0f;      // zero in rows and channels that do not exist
+                U[t] = u * run;
+                run *= ok ? sw[t][d] : 1.0f;
+                own[t] = (ok ? sr[t][d] : 0.0f) * run;
+                const float over = 1.0f / run;
+                xb[t & 3] = rate * u * over;
+                xk[t & 3] = k * over;
+                if ((t & 3) == 3) {
+                    float *y = Y + d * DLC_YP + t - 3, *x = X + d * DLC_YP + t - 3;
+                    *reinterpret_cast<float4*>(y) = make_float4(own[t - 3], own[t - 2], own[t - 1], own[t]);
+                    *reinterpret_cast<float4*>(y + CHUNK) = make_float4(U[t - 3], U[t - 2], U[t - 1], U[t]);
+                    *reinterpret_cast<float4*>(x) = make_float4(xb[0], xb[1], xb[2], xb[3]);
+                    *reinterpret_cast<float4*>(x + CHUNK) = make_float4(xk[0], xk[1], xk[2], xk[3]);
+                }
+            }
+            total = run;
+        }
+        __syncthreads();
+        // [r W; u W] [b / W; k / W]^T over the channels: 32 x 32 sums, 4 x 4 a thread; those above the diagonals are left out.
+        if (channel) {
+            const int ty = d >> 3, tx = d & 7;
+            uint64_t acc[4][2] = {};
+#pragma unroll 8
+            for (int i = 0; i < DLC_D; i++) {
+                const float4 yy = *reinterpret_cast<const float4*>(Y + i * DLC_YP + 4 * ty);
+                const ulonglong2 xx = *reinterpret_cast<const ulonglong2*>(X + i * DLC_YP + 4 * tx);
+                const float ys[4] = {yy.x, yy.y, yy.z, yy.w};
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const uint64_t y2 = pack_f32x2(ys[a], ys[a]);
+                    acc[a][0] = fma_f32x2(y2, xx.x, acc[a][0]);
+                    acc[a][1] = fma_f32x2(y2, xx.y, acc[a][1]);
+                }
+            }
+            const int which = (ty >= 4 ? 0 : 2) + (tx >= 4 ? 1 : 0), t0 = 4 * (ty & 3), s0 = 4 * (tx & 3);
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    float lo, hi;
+                    unpack_f32x2(acc[a][e], lo, hi);
+                    const int t = t0 + a, s = s0 + 2 * e, most = ty >= 4 ? t - 1 : t;      // s < t in A and Bm, or s <= t
+                    lower[which][t][s] = s <= most ? lo : 0.0f;
+                    lower[which][t][s + 1] = s + 1 <= most ? hi : 0.0f;
+                }
+        }
+        __syncthreads();
+        // The substitutions: columns of U (a channel each) and of Bm alike, and own_t - sum_s H_ts x_s of the solved ones.
+        if (!channel) {
+#pragma unroll
+            for (int t = 0; t < CHUNK; t++) {
+                U[t] = lower[1][t][lane & 15];
+                own[t] = lower[3][t][lane & 15];
+            }
+        }
+#pragma unroll
+        for (int t = 1; t < CHUNK; t++)
+#pragma unroll
+            for (int s = 0; s < t; s++) U[t] = fmaf(-lower[0][t][s], U[s], U[t]);
+#pragma unroll
+        for (int t = 0; t < CHUNK; t++)
+#pragma unroll
+            for (int s = 0; s <= t; s++) own[t] = fmaf(-lower[2][t][s], U[s], own[t]);
+        __syncwarp();
+        if (!channel) {
+            if (lane < CHUNK) {
+#pragma unroll
+                for (int t = 0; t < CHUNK; t++) {
+                    lower[1][t][lane] = U[t];
+                    dst[4 * CHUNK * DLC_D + t * CHUNK_G + lane] = own[t];
+                }
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < CHUNK; t++) {
+                dst[t * DLC_D + d] = own[t];
+                dst[(CHUNK + t) * DLC_D + d] = U[t];
+            }
+        }
+        __syncthreads();
+        if (channel) {
+            float z0[CHUNK];
+#pragma unroll
+            for (int s = 0; s < CHUNK; s++) z0[s] = X[d * DLC_YP + CHUNK + s] * total;
+#pragma unroll
+            for (int t = 0; t < CHUNK; t++) {
+                const float z1 = X[d * DLC_YP + t] * total;
+                dst[(3 * CHUNK + t) * DLC_D + d] = z1;
+#pragma unroll
+                for (int s = 0; s < t; s++) z0[s] = fmaf(-lower[1][t][s], z1, z0[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < CHUNK; s++) dst[(2 * CHUNK + s) * DLC_D + d] = z0[s];
+            dst[4 * CHUNK * DLC_D + CHUNK * CHUNK_G + d] = total;
+        }
+        __syncthreads();          // the next chunk writes Y, X and the triangles
+    }
+}
+#define DLC_SMEM ((2 * 4 * CHUNK * DLC_D + 2 * DLC_D * DLC_YP + 4 * CHUNK * CHUNK_G) * sizeof(float))
+
+// Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not).
+extern "C" long long bc_delta_chunked_scratch(int rows, int seqs, int H, int D, int inner, float decay_scale, int write_state) {
+    if (D <= 0 || D > DLC_D || D % 4 || inner <= 0 || H <= 0 || H > 65535 || seqs <= 0 || seqs > 65535 || !(decay_scale >= 0.0f && decay_scale <= 4.0f)) return 0;
+    const int pack = chunk_pack_floats(DLC_D, true);
+    return chunk_capacity(rows, seqs, H, pack, write_state) * H * pack;
+}
+
+// proj, w2t, w0, a_bias as for bc_delta_prepare; state, seq_rows, seq_slot, out as for bc_delta_scan; decay: scratch [rows, H D]; pack: scratch of
+// pack_floats floats, bc_delta_chunked_scratch of them for the fewest launches; max_new: the most rows that a sequence brings.
+extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t, const float* w0, const float* a_bias, float* decay, float* pack, long long pack_floats, float* state,
+                                const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int H, int D, int inner, float decay_scale,
+                                float key_eps, int n_slots, int write_state, cudaStream_t s) {
+    BC_CHECK_ARG(rows >= 0 && seqs >= 0 && max_new >= 0, "delta_chunked: bad sizes rows=%d seqs=%d max_new=%d", rows, seqs, max_new);
+    if (rows == 0 || seqs == 0 || max_new == 0) return BC_OK;
+    BC_CHECK_ARG(bc_delta_chunked_scratch(rows, seqs, H, D, inner, decay_scale, write_state) > 0,
+                 "delta_chunked: %d heads of %d, inner %d, decay_scale %g are outside what the kernels take", H, D, inner, (double)decay_scale);
+    BC_CHECK_ARG(stride >= 5 * H * D + inner, "delta_chunked: a row of %d values cannot hold five projections of %d and %d more", stride, H * D, inner);
+    BC_CHECK_ARG((rows + DLC_ROWS - 1) / DLC_ROWS <= 65535, "delta_chunked: %d rows are too many", rows);
+    BC_CHECK_ARG(stride % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)decay % 16 == 0 && (uintptr_t)pack % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0,
+                 "delta_chunked: rows, state and scratch must start on 16-byte borders");
+    const long long capacity = pack_floats / ((long long)H * chunk_pack_floats(DLC_D, true));
+    BC_CHECK_ARG(chunk_fits(capacity, rows, seqs, write_state), "delta_chunked: scratch of %lld floats is too small", pack_floats);
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(delta_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DLC_SMEM);
+        if (e != cudaSuccess) {
+            bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
+            return (int)e;
+        }
+        configured = true;
+    }
+    cudaError_t e = bc_launch(delta_decay_kernel, dim3((H * D + DLC_COLS - 1) / DLC_COLS, (rows + DLC_ROWS - 1) / DLC_ROWS), dim3(256), 0, s, proj, stride, 5 * H * D, w2t,
+                              w0, decay, rows, H * D, inner, decay_scale);
+    if (e == cudaSuccess)
+        e = chunk_step(
+            capacity, rows, seqs, max_new,
+            [&](const ChunkSpan& span) {
+                return bc_launch(delta_chunks_kernel, dim3((span.count + DLC_RUN - 1) / DLC_RUN, H, seqs), dim3(DLC_D + 32), DLC_SMEM, s, span, proj, stride, decay, a_bias, seq_rows, seq_slot, pack, H, D,
+                                 key_eps, n_slots);
+            },
+            [&](const ChunkSpan& span) {
+                return chunk_scan_launch<DLC_D / 32, true>(span, pack, proj + 2 * H * D, stride, state, seq_rows, seq_slot, out, seqs, H, D, D, n_slots, write_state, s);
+            });
+    if (e != cudaSuccess) {
+        bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    BC_LAUNCH_STATUS();
+}

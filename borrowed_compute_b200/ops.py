@@ -155,7 +155,7 @@ def _bounds_paged(who: str, rows: int, row_pos: torch.Tensor, row_slot: torch.Te
 
 
 launches = 0   # kernels launched through this module since import (a captured graph replays them uncounted)
-_KERNELS_PER_CALL = {"bc_argmax": 2, "bc_moe_plan": 3, "bc_moe_route_f32": 2, "bc_moe_route_bf16": 2}   # launchers that start more than one kernel
+_KERNELS_PER_CALL = {"bc_argmax": 2, "bc_moe_plan": 3, "bc_moe_route_f32": 2, "bc_moe_route_bf16": 2, "bc_delta_chunked": 3, "bc_gla_chunked": 2}   # launchers that start more than one kernel
 
 
 # Timing of single launches, for engine.profile.StepProfile: while `timeline` is a list every
@@ -168,7 +168,7 @@ _CLASS_OF = {
     "bc_attention_rows": "attention", "bc_attention_decode": "attention", "bc_attention_prefill": "attention",
     "bc_short_conv": "short convolution", "bc_norm_pair": "norm", "bc_delta_split": "low-rank split", "bc_delta": "delta rule",
     "bc_hyper": "streams + norm", "bc_diff": "attention", "bc_polynorm": "activation", "bc_qkv_prepare": "rotary + append",
-    "bc_linear_scan": "recurrence", "bc_ssd_prepare": "recurrence set-up", "bc_gla_decay": "recurrence set-up", "bc_gated_norm": "gated norm",
+    "bc_linear_scan": "recurrence", "bc_ssd_prepare": "recurrence set-up", "bc_gla_decay": "recurrence set-up", "bc_gla_chunked": "recurrence", "bc_gated_norm": "gated norm",
     "bc_moe_product": "expert product", "bc_gemm_tc_grouped": "expert product", "bc_moe_route": "routing", "bc_moe_plan": "expert sort",
     "bc_moe_gather": "expert gather", "bc_moe_combine": "expert sum", "bc_softcap": "softcap", "bc_reentry": "re-entry",
     "bc_argmax": "sampling", "bc_sample": "sampling", "bc_gemm": "product", "bc_random": "random weights",
@@ -751,6 +751,45 @@ def delta_scan(proj: torch.Tensor, decay: torch.Tensor, unit: torch.Tensor, remo
           _c_int(1 if write_state else 0), _stream())
 
 
+def _chunk_scratch(name: str, *args) -> int:
+    """Floats of scratch that a chunked recurrence asks for (0: it does not take these sizes)."""
+    f = getattr(lib(), name)
+    f.restype = ctypes.c_longlong
+    return int(f(*args))
+
+
+def delta_chunked_scratch(rows: int, seqs: int, heads: int, head_dim: int, inner: int, decay_scale: float, write_state: bool = True) -> int:
+    """Floats of scratch that ``delta_chunked`` takes for ``rows`` rows of ``seqs`` sequences; 0 where ``delta_scan`` has to serve (heads
+    above 64 channels or not a multiple of four, rows of the projection off a 16-byte border, decays below exp(-4))."""
+    if (5 * heads * head_dim + inner) % 4:
+        return 0
+    return _chunk_scratch("bc_delta_chunked_scratch", _c_int(rows), _c_int(seqs), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale),
+                          _c_int(1 if write_state else 0))
+
+
+def delta_chunked(proj: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bias: torch.Tensor, decay: torch.Tensor, pack: torch.Tensor,
+                  state: torch.Tensor, seq_rows: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, seqs: int, max_new: int, heads: int,
+                  head_dim: int, decay_scale: float, key_eps: float, write_state: bool = True) -> None:
+    """``delta_prepare`` and ``delta_scan`` with the rows of a sequence taken sixteen at a time: the same recurrence in float32, its sums in
+    another order.  ``decay``: scratch like ``out``; ``pack``: scratch of ``delta_chunked_scratch`` floats (with fewer, down to a
+    chunk a sequence, the step goes in segments)."""
+    for t, name in ((proj, "proj"), (w2t, "w2t"), (w0, "w0"), (a_bias, "a_bias"), (decay, "decay"), (pack, "pack"), (state, "state"), (out, "out")):
+        _need(t, name, torch.float32)
+    _need(seq_rows, "seq_rows", torch.int32)
+    _need(seq_slot, "seq_slot", torch.int32)
+    rows, stride = proj.shape
+    HD, inner = heads * head_dim, w2t.shape[0]
+    if w2t.shape[1] != HD or w0.numel() != HD or a_bias.numel() != HD or stride != 5 * HD + inner:
+        raise KernelError(f"delta_chunked: proj {tuple(proj.shape)}, w2t {tuple(w2t.shape)} do not fit {heads} heads of {head_dim}")
+    if tuple(state.shape[1:]) != (heads, head_dim, head_dim) or tuple(out.shape) != (rows, HD) or decay.shape != out.shape:
+        raise KernelError(f"delta_chunked: state {tuple(state.shape)}, decay {tuple(decay.shape)} or out {tuple(out.shape)} do not fit {heads} heads of {head_dim}")
+    _bounds("delta_chunked: seq_slot", seq_slot, state.shape[0], seqs, lowest=-1)
+    _bounds("delta_chunked: seq_rows", seq_rows, rows + 1, seqs + 1)
+    _call(_fn("bc_delta_chunked"), _ptr(proj), _c_int(stride), _ptr(w2t), _ptr(w0), _ptr(a_bias), _ptr(decay), _ptr(pack), ctypes.c_longlong(pack.numel()), _ptr(state), _ptr(seq_rows),
+          _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale), _c_float(key_eps),
+          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
+
+
 def delta_finish(o: torch.Tensor, proj: torch.Tensor, gate_offset: int, weight: torch.Tensor, out: torch.Tensor, heads: int, head_dim: int,
                  eps: float) -> None:
     """out = o / rms(o over each head) * weight * sigmoid(gate), the gate at columns gate_offset .. of ``proj``."""
@@ -985,6 +1024,39 @@ def gla_decay(proj: torch.Tensor, inner_at: int, w2t: torch.Tensor, bias: torch.
         raise KernelError(f"gla_decay: proj {tuple(proj.shape)}, w2t {tuple(w2t.shape)}, decay {tuple(decay.shape)} do not fit")
     _call(_fn("bc_gla_decay"), _ptr(proj), _c_int(proj.shape[1]), _c_int(inner_at), _ptr(w2t), _ptr(bias), _ptr(decay), _c_int(rows), _c_int(W),
           _c_int(rank), _c_float(tau), _stream())
+
+
+def gla_chunked_scratch(proj: torch.Tensor, v_at: int, seqs: int, heads: int, key_dim: int, value_dim: int, rank: int, write_state: bool = True) -> int:
+    """Floats of scratch that ``gla_chunked`` takes for these rows; 0 where ``gla_decay`` and ``linear_scan`` have to serve (channels that are not
+    multiples of four, rows or values off a 16-byte border)."""
+    if proj.shape[1] % 4 or v_at % 4 or proj.data_ptr() % 16:
+        return 0
+    return _chunk_scratch("bc_gla_chunked_scratch", _c_int(proj.shape[0]), _c_int(seqs), _c_int(heads), _c_int(key_dim), _c_int(value_dim), _c_int(rank),
+                          _c_int(1 if write_state else 0))
+
+
+def gla_chunked(proj: torch.Tensor, q_at: int, k_at: int, v_at: int, inner_at: int, w2t: torch.Tensor, bias: torch.Tensor, tau: float, out_scale: float,
+                pack: torch.Tensor, state: torch.Tensor, seq_rows: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, seqs: int, max_new: int, heads: int,
+                key_dim: int, value_dim: int, write_state: bool = True) -> None:
+    """``gla_decay`` and ``linear_scan`` (a decay a key channel, k as it is, nothing skipped) with the rows of a sequence taken sixteen at a time:
+    the same recurrence in float32, its sums in another order.  q, k, v and the decays' inner vector are columns of ``proj``; ``pack``: scratch of
+    ``gla_chunked_scratch`` floats (with fewer, down to a chunk a sequence, the step goes in segments)."""
+    for t, name in ((proj, "proj"), (w2t, "w2t"), (bias, "bias"), (pack, "pack"), (state, "state"), (out, "out")):
+        _need(t, name, torch.float32)
+    _need(seq_rows, "seq_rows", torch.int32)
+    _need(seq_slot, "seq_slot", torch.int32)
+    rows, stride = proj.shape
+    H, N, P, rank = heads, key_dim, value_dim, w2t.shape[0]
+    if tuple(w2t.shape) != (rank, H * N) or bias.numel() != H * N or tuple(state.shape[1:]) != (H, P, N) or tuple(out.shape) != (rows, H * P):
+        raise KernelError(f"gla_chunked: w2t {tuple(w2t.shape)}, state {tuple(state.shape)} or out {tuple(out.shape)} do not fit {H} heads of {N} x {P}")
+    for at, width in ((q_at, H * N), (k_at, H * N), (v_at, H * P), (inner_at, rank)):
+        if at < 0 or at + width > stride:
+            raise KernelError(f"gla_chunked: proj {tuple(proj.shape)} has no {width} columns from {at} on")
+    _bounds("gla_chunked: seq_slot", seq_slot, state.shape[0], seqs, lowest=-1)
+    _bounds("gla_chunked: seq_rows", seq_rows, rows + 1, seqs + 1)
+    _call(_fn("bc_gla_chunked"), _ptr(proj), _c_int(stride), _c_int(q_at), _c_int(k_at), _c_int(v_at), _c_int(inner_at), _ptr(w2t), _ptr(bias), _c_int(rank), _c_float(tau),
+          _c_float(out_scale), _ptr(pack), ctypes.c_longlong(pack.numel()), _ptr(state), _ptr(seq_rows), _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(H), _c_int(N), _c_int(P),
+          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
 
 
 def gated_norm(y: torch.Tensor, gate: torch.Tensor, gate_at: int, weight: torch.Tensor, out: torch.Tensor, parts: int, eps: float,

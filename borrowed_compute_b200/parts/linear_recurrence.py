@@ -33,6 +33,11 @@ from . import products
 from .base import MIXERS, Mixer, RunMemory, Runtime, StateNeed, StepContext, TensorSpec
 
 
+# Steps in which a sequence brings at least this many rows take them sixteen at a time (bfloat16 engines: the float32 path keeps the
+# row-by-row scan, whose sums are the same however a prompt is cut).
+CHUNKED_ROWS = 16
+
+
 @MIXERS.register("gated_linear_attention")
 class GatedLinearAttention(Mixer):
     def __init__(self, hidden_size: int, heads: int, head_dim: int, value_dim: int, decay_rank: int, tau: float, norm_eps: float,
@@ -72,12 +77,20 @@ class GatedLinearAttention(Mixer):
         hd, hp, dev = H * D, H * P, x.device
         proj = torch.empty((rows, self.w_in.shape[0]), dtype=torch.float32, device=dev)
         products.linear(x, self.w_in, proj, products.EPI_STORE_F32, "recurrence projections")
-        decay = torch.empty((rows, hd), dtype=torch.float32, device=dev)
-        ops.gla_decay(proj, 2 * hd + 2 * hp, self.a2_t, self.a2_b, decay, self.tau)
         # The recurrence writes the rows of live sequences only; the norm after it skips the others (rows of no sequence).
         o = torch.empty((rows, hp), dtype=torch.float32, device=dev)
-        ops.linear_scan(proj, 0, 1, proj, hd, 1, proj, 2 * hd, decay, 0, True, None, 0, None, float(D) ** -0.5, mem.state, ctx.seq_rows,
-                        ctx.seq_slot, o, ctx.seqs, H, D, P, write_state=mem.writes)
+        scratch = 0
+        if x.dtype == torch.bfloat16 and ctx.max_new >= CHUNKED_ROWS:
+            scratch = ops.gla_chunked_scratch(proj, 2 * hd, ctx.seqs, H, D, P, self.decay_rank, mem.writes)
+        if scratch:
+            pack = torch.empty((scratch,), dtype=torch.float32, device=dev)
+            ops.gla_chunked(proj, 0, hd, 2 * hd, 2 * hd + 2 * hp, self.a2_t, self.a2_b, self.tau, float(D) ** -0.5, pack, mem.state, ctx.seq_rows,
+                            ctx.seq_slot, o, ctx.seqs, ctx.max_new, H, D, P, write_state=mem.writes)
+        else:
+            decay = torch.empty((rows, hd), dtype=torch.float32, device=dev)
+            ops.gla_decay(proj, 2 * hd + 2 * hp, self.a2_t, self.a2_b, decay, self.tau)
+            ops.linear_scan(proj, 0, 1, proj, hd, 1, proj, 2 * hd, decay, 0, True, None, 0, None, float(D) ** -0.5, mem.state, ctx.seq_rows,
+                            ctx.seq_slot, o, ctx.seqs, H, D, P, write_state=mem.writes)
         y = torch.empty((rows, hp), dtype=x.dtype, device=dev)
         ops.gated_norm(o, proj, 2 * hd + hp, self.norm_weight, y, H, self.norm_eps, gate_first=False, factor=self.out_scale, row_slot=ctx.row_slot)
         products.linear(y, self.w_o, residual, products.EPI_ADD_F32, "output product")
