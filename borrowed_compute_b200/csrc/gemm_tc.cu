@@ -976,12 +976,14 @@ extern "C" int bc_gemm_tc_act_bf16(const void* X, const void* W, void* out, int 
 // ------------------------------------------------------------ the product over groups of rows
 // Many weight matrices of one shape ([experts, rows, K], one after another) and activation rows sorted by the
 // matrix each of them meets: a table written on the device ([0]: tiles; then, a tile, matrix, first row, rows)
-// cuts the sorted rows into tiles that lie in one matrix each.  Block (x, y) multiplies weight tile x of the
-// matrix of table tile y with that tile's rows: the one-block kernel above without the splits, with its tile's
-// place read from the table.  The table comes from the kernels before, so nothing is asked for ahead of the
-// wait for them; the grid covers the most tiles the table can hold and blocks past its count leave at once.
-// A tile's box of rows may reach into the next matrix's rows (or past the last row, where TMA fills zeros):
-// those columns are computed and never written.
+// cuts the sorted rows into tiles that lie in one matrix each.  A piece of work is a weight tile of the matrix of a table
+// tile with that tile's rows; at many rows a block on every SM takes every grid-th piece, all weight tiles of a table tile
+// one after another, at few rows a block takes one.  The loader runs ahead over the pieces' k-steps, and where two accumulators' columns fit TMEM (all but the
+// widest gated tile) a piece is written out while the next one is multiplied.  The table comes from the kernels before, so
+// nothing is asked for ahead of the wait for them.  The MMA's N is the tile's rows rounded up to sixteen, and only the
+// boxes of 64 rows that hold some are loaded; columns past the tile's rows (the next matrix's, or zeros past the last)
+// are computed and never written.
+// (A block a piece, its N always the tile's: 196 + 121 us for 12,288 rows of 64 matrices of 2 x 1,408 x 2,048 and 2,048 x 1,408; now 172 + 93 us.)
 struct TcGroupParams {
     void* out;              // bf16 [rows, N] (SwiGLU) or float [rows, N]
     const int* table;
@@ -991,6 +993,9 @@ struct TcGroupParams {
     float glu_limit, glu_alpha;   // SwiGLU: as in TcParams
 };
 
+// Rows a box of the activations' map holds.
+__host__ __device__ constexpr int tcg_box(int bn) { return bn < 64 ? bn : 64; }
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(tc_threads(BN), 1)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcGroupParams p) {
@@ -998,34 +1003,29 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     constexpr int B_BYTES = BN * TC_BK * 2;
     constexpr int N_ACC = EPI == EPI_SWIGLU ? 2 : 1;
     constexpr int STAGE_BYTES = N_ACC * A_BYTES + B_BYTES;
-    constexpr int TMEM_COLS = N_ACC * BN < 32 ? 32 : N_ACC * BN;
+    constexpr int ACC_COLS = N_ACC * BN;
+    constexpr int BUFFERS = 2 * ACC_COLS <= 512 ? 2 : 1;
+    constexpr int TMEM_COLS = BUFFERS * ACC_COLS < 32 ? 32 : BUFFERS * ACC_COLS;
     constexpr int HALVES = (tc_threads(BN) - 64) / 128;
+    constexpr int BOX = tcg_box(BN);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * 16 + 1];
+    __shared__ __align__(8) uint64_t bars[2 * 16 + 4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int gave_up;
 
-    pdl_wait();                                   // the table, the rows and the output belong to the kernels before
-    const int* table = p.table;
-    PDL_FRESH(table);
-    const int tile = blockIdx.y;
-    if (tile >= table[0]) return;                 // the whole block, before anything is set up
-    const int matrix = table[1 + 3 * tile], t0 = table[2 + 3 * tile], t_count = table[3 + 3 * tile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int stages = p.stages;
-    const int n0 = blockIdx.x * TC_BM;
-    const int w_row = matrix * p.matrix_rows + n0, w_row2 = w_row + p.N;
     const int k_iters = (p.K + TC_BK - 1) / TC_BK;
-    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[16]), acc_bar = smem_u32(&bars[32]);
-
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[16]), acc_full0 = smem_u32(&bars[32]), acc_empty0 = smem_u32(&bars[34]);
     if (threadIdx.x == 0) {
-        gave_up = 0;
         for (int s = 0; s < stages; s++) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
         }
-        mbar_init(acc_bar, 1);
+        for (int b = 0; b < BUFFERS; b++) {
+            mbar_init(acc_full0 + 8 * b, 1);
+            mbar_init(acc_empty0 + 8 * b, 4 * HALVES);        // the epilogue warps
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
@@ -1034,84 +1034,127 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     pdl_launch_dependents();
+    pdl_wait();                                   // the table, the rows and the output belong to the kernels before
+    const int* table = p.table;
+    PDL_FRESH(table);
+    const int n_tiles = (p.N + TC_BM - 1) / TC_BM;
+    const int pieces = table[0] * n_tiles;
+    // Piece number -> weight tile, matrix, first row, rows.
+    auto piece_at = [&](int piece, int& n0, int& matrix, int& t0, int& t_count) {
+        const int tile = piece / n_tiles;
+        n0 = (piece - tile * n_tiles) * TC_BM;
+        matrix = table[1 + 3 * tile], t0 = table[2 + 3 * tile], t_count = table[3 + 3 * tile];
+    };
 
     if (warp == 0) {
         if (lane == 0) {
             const uint64_t stream_once = l2_evict_first_policy();
-            for (int i = 0; i < k_iters; i++) {
-                const int s = i % stages;
-                if (i >= stages && !mbar_wait(empty0 + 8 * s, ((i / stages) & 1) ^ 1, 1)) {
-                    *reinterpret_cast<volatile int*>(&gave_up) = 1;
-                    break;
+            bool ok = true;
+            int it = 0;
+            for (int piece = blockIdx.x; piece < pieces && ok; piece += gridDim.x) {
+                int n0, matrix, t0, t_count;
+                piece_at(piece, n0, matrix, t0, t_count);
+                const int w_row = matrix * p.matrix_rows + n0, w_row2 = w_row + p.N;
+                const int boxes = (t_count + BOX - 1) / BOX;
+                const uint32_t bytes = N_ACC * A_BYTES + boxes * BOX * TC_BK * 2;
+                for (int i = 0; i < k_iters; i++, it++) {
+                    const int s = it % stages;
+                    if (it >= stages && !(ok = mbar_wait(empty0 + 8 * s, ((it / stages) & 1) ^ 1, 1))) break;
+                    const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+                    mbar_expect_tx(full0 + 8 * s, bytes);
+                    const int k = i * TC_BK;
+                    if (BN <= 32) {                       // few rows a matrix: its weights are read once
+                        tma_load_2d_hint(a, &map_w, full0 + 8 * s, k, w_row, stream_once);
+                        if (N_ACC == 2) tma_load_2d_hint(a + A_BYTES, &map_w, full0 + 8 * s, k, w_row2, stream_once);
+                    } else {
+                        tma_load_2d(a, &map_w, full0 + 8 * s, k, w_row);
+                        if (N_ACC == 2) tma_load_2d(a + A_BYTES, &map_w, full0 + 8 * s, k, w_row2);
+                    }
+                    for (int b = 0; b < boxes; b++) tma_load_2d(a + N_ACC * A_BYTES + b * BOX * TC_BK * 2, &map_x, full0 + 8 * s, k, t0 + b * BOX);
                 }
-                const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
-                mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
-                const int k = i * TC_BK;
-                if (BN <= 32) {                       // few rows a matrix: its weights are read once
-                    tma_load_2d_hint(a, &map_w, full0 + 8 * s, k, w_row, stream_once);
-                    if (N_ACC == 2) tma_load_2d_hint(a + A_BYTES, &map_w, full0 + 8 * s, k, w_row2, stream_once);
-                } else {
-                    tma_load_2d(a, &map_w, full0 + 8 * s, k, w_row);
-                    if (N_ACC == 2) tma_load_2d(a + A_BYTES, &map_w, full0 + 8 * s, k, w_row2);
-                }
-                tma_load_2d(a + N_ACC * A_BYTES, &map_x, full0 + 8 * s, k, t0);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(BN);
             bool ok = true;
-            for (int i = 0; i < k_iters && ok; i++) {
-                const int s = i % stages;
-                ok = mbar_wait(full0 + 8 * s, (i / stages) & 1, 2);
-                if (!ok) break;
+            int it = 0, n = 0;
+            for (int piece = blockIdx.x; piece < pieces && ok; piece += gridDim.x, n++) {
+                const int buffer = n % BUFFERS;
+                // The epilogue warps must have read this accumulator's last piece out of TMEM.
+                if (n >= BUFFERS && !(ok = mbar_wait(acc_empty0 + 8 * buffer, ((n / BUFFERS) & 1) ^ 1, 4))) break;
                 tc_fence_after();
-                const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
-                const uint64_t da = smem_desc(a), db = smem_desc(a + N_ACC * A_BYTES);
+                int n0, matrix, t0, t_count;
+                piece_at(piece, n0, matrix, t0, t_count);
+                const uint32_t idesc = instr_desc((t_count + 15) & ~15), acc_at = tmem + buffer * ACC_COLS;
+                for (int i = 0; i < k_iters; i++, it++) {
+                    const int s = it % stages;
+                    if (!(ok = mbar_wait(full0 + 8 * s, (it / stages) & 1, 2))) break;
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+                    const uint64_t da = smem_desc(a), du = smem_desc(a + A_BYTES), db = smem_desc(a + N_ACC * A_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < TC_BK / 16; kk++) {
-                    const uint32_t acc = (i | kk) != 0;
-                    mma_bf16(tmem, da + 2 * kk, db + 2 * kk, idesc, acc);
-                    if (N_ACC == 2) mma_bf16(tmem + BN, smem_desc(a + A_BYTES) + 2 * kk, db + 2 * kk, idesc, acc);
+                    for (int kk = 0; kk < TC_BK / 16; kk++) {
+                        const uint32_t acc = (i | kk) != 0;
+                        mma_bf16(acc_at, da + 2 * kk, db + 2 * kk, idesc, acc);
+                        if (N_ACC == 2) mma_bf16(acc_at + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
+                    }
+                    mma_commit(empty0 + 8 * s);
                 }
-                mma_commit(empty0 + 8 * s);
+                if (ok) mma_commit(acc_full0 + 8 * buffer);
             }
-            if (!ok) {
-                *reinterpret_cast<volatile int*>(&gave_up) = 1;
-                __threadfence_block();
-            }
-            mma_commit(acc_bar);   // also after a wait that ran out: the epilogue warps must not be left waiting
         }
     } else {
-        // Epilogue: this warp reads TMEM lanes 32 q .. 32 q + 31, i.e. outputs n0 + 32 q + lane, and half of the rows' columns.
+        // Epilogue: this warp reads TMEM lanes 32 q .. 32 q + 31, i.e. outputs n0 + 32 q + lane, and every other run of sixteen columns where two
+        // warps share a quarter.
         const int q = warp & 3, half = (warp - 2) >> 2;
-        const int n = n0 + 32 * q + lane;
         bool ok = true;
-        if (lane == 0) ok = mbar_wait(acc_bar, 0, 3) && *reinterpret_cast<volatile int*>(&gave_up) == 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        tc_fence_after();
-        const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16);
-        if (ok) {
-            constexpr int MINE = BN / HALVES;
-            const int first = half * MINE;
-#pragma unroll 1
-            for (int cc = first; cc < first + MINE && cc < t_count; cc += 16) {
-                uint32_t v[16], u[16];
+        int n = 0;
+        for (int piece = blockIdx.x; piece < pieces; piece += gridDim.x, n++) {
+            const int buffer = n % BUFFERS;
+            int n0, matrix, t0, t_count;
+            piece_at(piece, n0, matrix, t0, t_count);
+            const int out_n = n0 + 32 * q + lane;
+            if (lane == 0) ok = mbar_wait(acc_full0 + 8 * buffer, (n / BUFFERS) & 1, 3);
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t taddr = tmem + buffer * ACC_COLS + ((uint32_t)(32 * q) << 16);
+            // Sixteen columns at a time, the next ones on their way while these are written.
+            uint32_t va[16], vb[16], ua[16], ub[16];
+            auto fetch = [&](uint32_t* v, uint32_t* u, int cc) {
                 tmem_load16(taddr + cc, v);
                 if (EPI == EPI_SWIGLU) tmem_load16(taddr + BN + cc, u);
-                tmem_load_wait();
-                if (n >= p.N) continue;
+            };
+            auto emit = [&](const uint32_t* v, const uint32_t* u, int cc) {
+                if (out_n >= p.N) return;
                 float r[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) r[j] = EPI == EPI_SWIGLU ? glu_mul(__uint_as_float(v[j]), __uint_as_float(u[j]), p.glu_limit, p.glu_alpha) : epi_plain<EPI>(__uint_as_float(v[j]));
+                const size_t o = (size_t)(t0 + cc) * p.N + out_n;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     if (cc + j >= t_count) break;
-                    const size_t at = (size_t)(t0 + cc + j) * p.N + n;
+                    const size_t at = o + (size_t)j * p.N;
                     if (EPI == EPI_SWIGLU || EPI == EPI_RELU2) ((bf16*)p.out)[at] = __float2bfloat16_rn(r[j]);
                     else ((float*)p.out)[at] = r[j];
                 }
+            };
+            constexpr int STEP = 16 * HALVES;
+            int cc = 16 * half;
+            if (cc < t_count) fetch(va, ua, cc);
+            for (; cc < t_count; cc += 2 * STEP) {
+                tmem_load_wait();
+                if (cc + STEP < t_count) fetch(vb, ub, cc + STEP);
+                emit(va, ua, cc);
+                if (cc + STEP < t_count) {
+                    tmem_load_wait();
+                    if (cc + 2 * STEP < t_count) fetch(va, ua, cc + 2 * STEP);
+                    emit(vb, ub, cc + STEP);
+                }
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty0 + 8 * buffer);
         }
     }
     tc_fence_before();
@@ -1126,13 +1169,13 @@ template <int BN, int EPI>
 static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupParams p, int max_tiles, cudaStream_t s) {
     constexpr int N_ACC = EPI == EPI_SWIGLU ? 2 : 1;
     constexpr int STAGE_BYTES = N_ACC * TC_BM * TC_BK * 2 + BN * TC_BK * 2;
-    const int k_iters = (p.K + TC_BK - 1) / TC_BK;
     int stages = (TC_SMEM_LIMIT - 1024) / STAGE_BYTES;
     if (stages > 12) stages = 12;
-    // Few rows a matrix: the product streams weights, and two blocks on an SM keep more loads in flight than one.
+    // Few rows a matrix: the product streams weights; a block a piece and two on an SM, which come and go as they end, share the bytes out better
+    // than a fixed number of pieces an SM (174 + 86 against 181 + 94 us for 256 rows of 32 matrices).
     const int half_stages = (TC_SMEM_LIMIT / 2 - 2048) / STAGE_BYTES;
-    if (BN <= 64 && half_stages >= 4 && stages > half_stages) stages = half_stages;
-    if (stages > k_iters) stages = k_iters < 2 ? 2 : k_iters;
+    const bool stream = BN <= 64 && half_stages >= 3;
+    if (stream && stages > half_stages) stages = half_stages;
     p.stages = stages;
     const int smem = stages * STAGE_BYTES + 1024;
     static bool configured = false;
@@ -1144,8 +1187,9 @@ static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupP
         }
         configured = true;
     }
-    dim3 grid((p.N + TC_BM - 1) / TC_BM, max_tiles);
-    cudaError_t e = bc_launch(gemm_tc_grouped_kernel<BN, EPI>, grid, dim3(tc_threads(BN)), (size_t)smem, s, mw, mx, p);
+    const long long pieces = (long long)((p.N + TC_BM - 1) / TC_BM) * max_tiles;      // at most: the table says how many
+    const int blocks = stream || pieces < bc_sm_count() ? (int)pieces : bc_sm_count();
+    cudaError_t e = bc_launch(gemm_tc_grouped_kernel<BN, EPI>, dim3(blocks), dim3(tc_threads(BN)), (size_t)smem, s, mw, mx, p);
     if (e != cudaSuccess) {
         bc_set_error("gemm_tc_grouped: launch failed: %s", cudaGetErrorString(e));
         return (int)e;
@@ -1164,12 +1208,13 @@ extern "C" int bc_gemm_tc_grouped_bf16(const void* X, const void* W, void* out, 
     BC_CHECK_ARG(max_tiles > 0 && max_tiles <= 65535, "gemm_tc_grouped: %d tiles are too many", max_tiles);
     BC_CHECK_ARG(gated >= 0 && gated <= 2, "gemm_tc_grouped: unknown kind of product %d", gated);
     BC_CHECK_ARG((long long)matrices * (gated == 1 ? 2 : 1) * N < 2147483647ll, "gemm_tc_grouped: too many weight rows");
+    BC_CHECK_ARG((long long)max_tiles * ((N + TC_BM - 1) / TC_BM) < 2147483647ll - 1024, "gemm_tc_grouped: too many tiles of %d outputs", N);
     if (rows == 0) return BC_OK;
     CUtensorMap mw, mx;
     const int matrix_rows = (gated == 1 ? 2 : 1) * N;
     int st = weight_map(&mw, W, matrices * matrix_rows, K);
     if (st != BC_OK) return st;
-    st = make_map(&mx, X, rows, K, tile_rows);
+    st = make_map(&mx, X, rows, K, tcg_box(tile_rows));
     if (st != BC_OK) return st;
     TcGroupParams p;
     p.out = out;
