@@ -194,7 +194,9 @@ class LatentAttention(Mixer):
         pages, widest, ints = seen_pages(ctx, self.window, dev)
         qh = torch.empty((rows, H * KP), dtype=dt, device=dev)
         ops.latent_heads(q, cos_sin, ctx.row_pos, qh, H, D, ROT)
-        found = torch.zeros((rows, H * VP), dtype=dt, device=dev)      # rows of no sequence are left as they are by the kernels
+        # Rows of no sequence are left as they are by the kernels: cleared ahead where the step has any.
+        every = ctx.host_seq_rows[ctx.seqs] == rows and min(ctx.host_seq_slot) >= 0
+        found = (torch.empty if every and pages else torch.zeros)((rows, H * VP), dtype=dt, device=dev)
         if pages:
             S = pages * ops.PAGE
             seen_c = torch.empty((S, R), dtype=dt, device=dev)
