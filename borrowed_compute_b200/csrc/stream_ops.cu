@@ -41,20 +41,38 @@ extern "C" int bc_scale_f32(float* scores, long long n, float factor, cudaStream
     BC_LAUNCH_STATUS();
 }
 
-__global__ void add_bias_kernel(float* __restrict__ x, const float* __restrict__ b, int E, size_t n) {
+// A block takes 1,024 neighbouring columns of eight rows; four columns a thread, sixteen bytes a move, the bias read once (an element a thread
+// and a 64-bit remainder each: 30 us for 2,048 x 4,096 floats, against 10 us of bytes).
+#define BIAS_ROWS 8
+__global__ void __launch_bounds__(256) add_bias_kernel(float* x, const float* __restrict__ b, int rows, int E) {
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(x);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] += b[i % E];
+    const int c = blockIdx.x * 1024 + 4 * threadIdx.x, row0 = blockIdx.y * BIAS_ROWS;
+    if (c >= E) return;
+    if (E % 4 == 0 && ((uintptr_t)x | (uintptr_t)b) % 16 == 0) {
+        const float4 v = *reinterpret_cast<const float4*>(b + c);
+        float4 y[BIAS_ROWS];
+#pragma unroll
+        for (int r = 0; r < BIAS_ROWS; r++)
+            if (row0 + r < rows) y[r] = *reinterpret_cast<const float4*>(x + (size_t)(row0 + r) * E + c);
+#pragma unroll
+        for (int r = 0; r < BIAS_ROWS; r++)
+            if (row0 + r < rows) *reinterpret_cast<float4*>(x + (size_t)(row0 + r) * E + c) = make_float4(y[r].x + v.x, y[r].y + v.y, y[r].z + v.z, y[r].w + v.w);
+        return;
+    }
+    for (int r = row0; r < min(rows, row0 + BIAS_ROWS); r++)
+        for (int e = 0; e < 4 && c + e < E; e++) x[(size_t)r * E + c + e] += b[c + e];
 }
 
 // x: [rows, E] float; b: [E] float.
 extern "C" int bc_add_bias_f32(float* x, const float* b, int rows, int E, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && E > 0, "add_bias: bad sizes rows=%d E=%d", rows, E);
-    const long long n = (long long)rows * E;
-    if (n == 0) return BC_OK;
-    const long long blocks = (n + 255) / 256;
-    bc_launch(add_bias_kernel, dim3((unsigned)(blocks < 65535 * 16 ? blocks : 65535 * 16)), dim3(256), 0, s, x, b, E, (size_t)n);
+    // More rows than a grid's second dimension holds go in turns.
+    for (int at = 0; at < rows; at += 65535 * BIAS_ROWS) {
+        const int n = rows - at < 65535 * BIAS_ROWS ? rows - at : 65535 * BIAS_ROWS;
+        bc_launch(add_bias_kernel, dim3((E + 1023) / 1024, (n + BIAS_ROWS - 1) / BIAS_ROWS), dim3(256), 0, s, x + (size_t)at * E, b, n, E);
+    }
     BC_LAUNCH_STATUS();
 }
 
