@@ -103,6 +103,62 @@ talk_prepare_kernel(const float* proj, int P, int g_at, const float* __restrict_
     }
 }
 
+// The same where a head is at most 32 lanes of four neighbouring dimensions and rows start on 16-byte borders: a warp a head, its values in
+// registers from the load to the last store, the partner of a turned dimension out of another lane; a query head's warp takes its gate along.
+// (A block a row whose warps took heads one after another, four bytes a move: 91 us for 2,048 rows of 32 + 8 heads of 128, against 26 us of
+// bytes; now 29.)
+__device__ __forceinline__ void ta_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void ta_store4(bf16* p, float4 v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
+template <class T>
+__global__ void __launch_bounds__(256)
+talk_prepare_wide_kernel(const float* proj, int P, int g_at, const float* __restrict__ bias, const float* __restrict__ cos_sin, int table_positions,
+                         const int* __restrict__ row_pos, const int* __restrict__ row_slot, const int* __restrict__ page_table, int max_pages, int n_pages,
+                         T* __restrict__ q_out, T* k_cache, T* v_cache, float* __restrict__ gate, int H, int G, int D, int rot, float eps, int write_cache) {
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(proj);
+    const int r = blockIdx.x, lane = threadIdx.x & 31, head = blockIdx.y * 8 + (threadIdx.x >> 5), d = 4 * lane;
+    if (head >= H + G) return;
+    const bool is_q = head < H, mine = d < D;
+    const float* x = proj + (size_t)r * P;
+    const int slot = row_slot[r], pos = row_pos[r];
+    size_t at = 0;
+    if (!is_q) {
+        int page = -1;
+        if (slot >= 0 && pos >= 0 && pos / BC_PAGE < max_pages) page = page_table[(size_t)slot * max_pages + pos / BC_PAGE];
+        if (!write_cache || page < 0 || page >= n_pages) return;
+        at = (((size_t)page * G + (head - H)) * BC_PAGE + pos % BC_PAGE) * D + d;
+    }
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v = mine ? *reinterpret_cast<const float4*>(x + (size_t)head * D + d) : none;       // the keys follow the queries in the projection
+    if (is_q && mine) {
+        const float4 z = *reinterpret_cast<const float4*>(x + g_at + (size_t)head * D + d);
+        *reinterpret_cast<float4*>(gate + ((size_t)r * H + head) * D + d) =
+            make_float4(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)), 1.0f / (1.0f + expf(-z.z)), 1.0f / (1.0f + expf(-z.w)));
+    }
+    if (bias != nullptr && mine) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + (size_t)head * D + d);
+        v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    }
+    if (!is_q && mine) ta_store4(v_cache + at, v);          // the values are the keys as projected
+    const int half = rot / 2;
+    if (rot > 0 && cos_sin != nullptr && pos >= 0 && pos < table_positions) {      // (the same for the whole block)
+        const bool low = d < half, turned = d < rot;
+        const int other = turned ? (low ? lane + half / 4 : lane - half / 4) : lane;
+        const float4 o = make_float4(__shfl_sync(0xffffffffu, v.x, other), __shfl_sync(0xffffffffu, v.y, other), __shfl_sync(0xffffffffu, v.z, other),
+                                     __shfl_sync(0xffffffffu, v.w, other));
+        if (turned) {
+            const float* cs = cos_sin + ((size_t)pos * half + (low ? d : d - half)) * 2;
+            const float4 a = *reinterpret_cast<const float4*>(cs), b = *reinterpret_cast<const float4*>(cs + 4);      // (cos, sin) of four pairs
+            v = low ? make_float4(v.x * a.x - o.x * a.y, v.y * a.z - o.y * a.w, v.z * b.x - o.z * b.y, v.w * b.z - o.w * b.w)
+                    : make_float4(v.x * a.x + o.x * a.y, v.y * a.z + o.y * a.w, v.z * b.x + o.z * b.y, v.w * b.z + o.w * b.w);
+        }
+    }
+    const float ss = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
+    const float f = 1.0f / sqrtf(ss / (float)D + eps);
+    if (mine) ta_store4(is_q ? q_out + ((size_t)r * H + head) * D + d : k_cache + at, make_float4(v.x * f, v.y * f, v.z * f, v.w * f));
+}
+
 // --------------------------------------------------------------------------------------- rows
 // One block a row; HPW heads a warp (warp w takes heads w, w + warps, ..); NJ value dimensions a lane (D <= 32 NJ).
 // q: [rows, H, D]; k_cache, v_cache: [pages, G, BC_PAGE, D]; gate: [rows, H D] float; out: [rows, H D].
@@ -515,6 +571,314 @@ talk_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
     }
 }
 
+// The same for sixteen heads a block (16 or 32 heads in all) whose keys of a tile take up 32 KB (heads of 128 on four kv heads a
+// block, of 64 on eight): a warp a head, as above, for both products and the softmax, but the mix goes by rows.  What bounded the kernel
+// above is the mix's reads: every warp reads all heads' raw scores for its one head, 8,700 reads of 128 bytes a tile of 32 heads, counted.  Here
+// warp w mixes eight heads of two rows, a lane one position of each: a raw score that is read serves eight heads (two 4-byte reads and
+// two uniform 16-byte reads of the mix's column for sixteen multiply-adds, two heads an instruction), about 2,000.  The mixed scores go back
+// to the warp of their head through the place of the tile's keys, which nobody reads any more.  The sums keep their order.
+//
+// The cluster's two barriers a tile (all heads' raw scores are there; nobody reads them any more) are split into arrival and wait, and what
+// needs neither stands between: the product with the tile before's values, and the next tile's scores.  Keys of the next tile are
+// asked for as soon as the mixed scores of the tile before have left their place, its values one barrier later.
+// One prompt of 2,048, 32 heads of 128 on 8, window 1,024: 557 us, with the kernel above 769.
+#define TM_PAGES_KEPT 256
+template <int CL> struct HeadsBarrier {
+    __device__ __forceinline__ void arrive() const {
+        if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    __device__ __forceinline__ void wait() const {
+        if (CL > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        else __syncthreads();
+    }
+};
+
+template <int D, int CL>
+__global__ void __launch_bounds__(512)
+talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const int* __restrict__ page_table, const int* __restrict__ seq_rows,
+                  const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const float* gate, const float* __restrict__ temp,
+                  const float* __restrict__ talk, bf16* __restrict__ out, int H, int G, int max_pages, int n_pages, int window, int keep_first, float scale,
+                  float cap, float* __restrict__ scratch, int splits) {
+    constexpr int CHUNKS = D / 8, KD = D / 16, ND = D / 8, HL = 16;
+    constexpr int HEAD_BYTES = TT_KEYS * D * 2;            // one kv head's 32 positions
+    extern __shared__ __align__(128) uint8_t tt_smem[];
+    __shared__ int page_kept[TM_PAGES_KEPT];               // the pages of the block's first tiles, fetched once (-1: none)
+    const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    const int GL = G / CL, h_first = rank * HL, g_first = rank * GL;
+    const int plane = GL * HEAD_BYTES;                     // a tile's keys of this block's kv heads; their values follow
+    float* raw = reinterpret_cast<float*>(tt_smem + (size_t)4 * plane);               // [H][16][TT_RS]: all heads' raw scores
+    float* mix = raw + (size_t)H * TT_ROWS * TT_RS;        // [H][16]: column m of the rows of the mix that make this block's heads
+    float* raw_of[CL];                                     // every block's copy of the raw scores, as this block writes them
+#pragma unroll
+    for (int c = 0; c < CL; c++) raw_of[c] = CL > 1 ? cg::this_cluster().map_shared_rank(raw, c) : raw;
+    const HeadsBarrier<CL> heads;
+
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(q); PDL_FRESH(k_cache); PDL_FRESH(v_cache); PDL_FRESH(gate);
+    const int sq = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gq = lane >> 2, tq = lane & 3, j4 = lane >> 3, r8 = lane & 7;
+    const int slot = seq_slot[sq];
+    const int row0 = seq_rows[sq], n_new = seq_rows[sq + 1] - row0;
+    const int n_tiles_q = (n_new + TT_ROWS - 1) / TT_ROWS;
+    const int q_tile = n_tiles_q - 1 - (int)blockIdx.x / CL;    // the last rows see the most: they go first
+    if (slot < 0 || q_tile < 0) return;                    // (the same for every block of a cluster)
+    const int start = seq_start[sq];
+    const int tok0 = q_tile * TT_ROWS, tok_end = min(n_new, tok0 + TT_ROWS);
+    const int* pages = page_table + (size_t)slot * max_pages;
+    const int group = H / G;
+    const int last_pos = start + n_new - 1;                // the last position the sequence holds after this step
+
+    for (int i = threadIdx.x; i < HL * H; i += 512) mix[i] = talk[(size_t)(h_first + i % HL) * H + i / HL];
+    auto first_seen = [&](int p) { return window > 0 && p + 1 > window ? p + 1 - window : 0; };
+    int pos[2], lo[2];
+    bool live[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int tok = tok0 + gq + 8 * i;
+        live[i] = tok < n_new;
+        pos[i] = start + tok;
+        lo[i] = first_seen(pos[i]);
+    }
+    // The block's tiles of positions: [0, kept) and [win_begin, win_end], as one stretch where they meet; with several splits its share of them.
+    const int p_first = start + tok0, p_last = start + tok_end - 1;
+    int kept = (min(keep_first, first_seen(p_last)) + TT_KEYS - 1) / TT_KEYS;
+    const int win_begin = first_seen(p_first) / TT_KEYS, win_end = p_last / TT_KEYS;
+    if (kept >= win_begin) kept = win_begin;
+    const int all_tiles = kept + (win_end - win_begin + 1);
+    const int per_split = (all_tiles + splits - 1) / splits;
+    const int tile_first = (int)blockIdx.z * per_split;
+    const int n_tiles = max(0, min(all_tiles, tile_first + per_split) - tile_first);      // (the same for every block of a cluster)
+    auto tile_at = [&](int k) { k += tile_first; return k < kept ? k : win_begin + (k - kept); };
+    auto page_of = [&](int it) {
+        const int pi = tile_at(it) / 2;
+        const int page = pi < max_pages ? pages[pi] : -1;
+        return page >= 0 && page < n_pages ? page : -1;
+    };
+    for (int i = threadIdx.x; i < min(n_tiles, TM_PAGES_KEPT); i += 512) page_kept[i] = page_of(i);
+    __syncthreads();
+    auto page_at = [&](int it) { return it < TM_PAGES_KEPT ? page_kept[it] : page_of(it); };
+    // Plane `which` of tile number `it` (0 keys, 1 values) into its stage.  A tile without a page is not fetched: its scores are masked whatever
+    // the stage holds, and its values are not multiplied.
+    auto load_plane = [&](int it, int which) {
+        const int tile = tile_at(it), page = page_at(it);
+        if (page < 0) return;
+        const uint32_t to = ad_smem(tt_smem + (size_t)((it & 1) * 2 + which) * plane);
+        const bf16* cache = which ? v_cache : k_cache;
+        constexpr int PER_HEAD = TT_KEYS * CHUNKS;
+        for (int i = threadIdx.x; i < GL * PER_HEAD; i += 512) {
+            const int g = i / PER_HEAD, rest = i - g * PER_HEAD, row = rest / CHUNKS, c = rest - row * CHUNKS;
+            cp_async16(to + g * HEAD_BYTES + tile_offset<D>(row, c), cache + (((size_t)page * G + g_first + g) * BC_PAGE + (tile & 1) * TT_KEYS + row) * D + c * 8);
+        }
+    };
+
+    const int h = h_first + warp, kv_bytes = (h / group - g_first) * HEAD_BYTES;       // this warp's head
+    uint32_t qf[KD][4], pf[2][4];
+    float o[ND][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, corr[2] = {1.0f, 1.0f};
+    const float factor = scale * temp[h];
+#pragma unroll
+    for (int kd = 0; kd < KD; kd++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const bf16* qr = q + ((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * D + kd * 16 + 2 * tq;
+            qf[kd][i] = live[i] ? *reinterpret_cast<const uint32_t*>(qr) : 0u;
+            qf[kd][i + 2] = live[i] ? *reinterpret_cast<const uint32_t*>(qr + 8) : 0u;
+        }
+#pragma unroll
+    for (int nd = 0; nd < ND; nd++) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.0f;
+    const float two_over_cap = cap > 0.0f ? 2.0f / cap : 0.0f;
+    const float LOG2E = 1.4426950408889634f;
+
+    float s[4][4];
+    auto scores = [&](int it) {                            // this head's raw scores of tile `it`, bounded
+        const uint32_t kh = ad_smem(tt_smem + (size_t)(it & 1) * 2 * plane) + kv_bytes;
+#pragma unroll
+        for (int nb = 0; nb < 4; nb++) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.0f;
+#pragma unroll
+        for (int kd = 0; kd < KD; kd++)
+#pragma unroll
+            for (int np = 0; np < 2; np++) {
+                uint32_t b0, b1, b2, b3;
+                ldmatrix_x4(kh + tile_offset<D>(np * 16 + (j4 >> 1) * 8 + r8, kd * 2 + (j4 & 1)), b0, b1, b2, b3);
+                mma_16816(s[2 * np], qf[kd], b0, b1);
+                mma_16816(s[2 * np + 1], qf[kd], b2, b3);
+            }
+#pragma unroll
+        for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[nb][e] *= factor;
+                if (cap > 0.0f) s[nb][e] = tt_bound(s[nb][e], cap, two_over_cap);
+            }
+    };
+    auto hand_out = [&]() {                                // to every block of the cluster
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const float4 v = make_float4(s[2 * half][2 * i], s[2 * half][2 * i + 1], s[2 * half + 1][2 * i], s[2 * half + 1][2 * i + 1]);
+#pragma unroll
+                for (int c = 0; c < CL; c++) *reinterpret_cast<float4*>(raw_of[c] + (size_t)h * TT_ROWS * TT_RS + (gq + 8 * i) * TT_RS + tq * 8 + half * 4) = v;
+            }
+    };
+    auto weigh = [&](int it) {                             // the product with the values of tile `it`
+        if (page_at(it) < 0) return;
+        const uint32_t vh = ad_smem(tt_smem + (size_t)((it & 1) * 2 + 1) * plane) + kv_bytes;
+#pragma unroll
+        for (int nd = 0; nd < ND; nd++) o[nd][0] *= corr[0], o[nd][1] *= corr[0], o[nd][2] *= corr[1], o[nd][3] *= corr[1];
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+            for (int nd = 0; nd < ND; nd += 2) {
+                uint32_t b0, b1, b2, b3;
+                ldmatrix_x4_trans(vh + tile_offset<D>(kk * 16 + (j4 & 1) * 8 + r8, nd + (j4 >> 1)), b0, b1, b2, b3);
+                mma_16816(o[nd], pf[kk], b0, b1);
+                mma_16816(o[nd + 1], pf[kk], b2, b3);
+            }
+    };
+
+    if (n_tiles > 0) {
+        load_plane(0, 0);
+        load_plane(0, 1);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    if (CL > 1) cg::this_cluster().sync();                 // every block is there before its memory is written to
+    else __syncthreads();
+    if (n_tiles > 0) {
+        scores(0);
+        hand_out();
+    }
+    for (int it = 0; it < n_tiles; it++) {
+        heads.arrive();
+        if (it > 0) weigh(it - 1);
+        heads.wait();                                      // every head's raw scores are there; the mixed ones of the tile before have been read
+        if (it + 1 < n_tiles) load_plane(it + 1, 0);
+        cp_async_commit();
+        uint64_t acc[2][4] = {};                           // heads hb .. hb + 7 of rows ra, ra + 1 at the lane's position
+        const int ra = warp & ~1, hb = 8 * (warp & 1);
+        {
+            const float* rm = raw + ra * TT_RS + lane;
+            const float* cm = mix + hb;
+#pragma unroll 4
+            for (int mm = 0; mm < H; mm++) {
+                const float x0 = rm[(size_t)mm * TT_ROWS * TT_RS], x1 = rm[(size_t)mm * TT_ROWS * TT_RS + TT_RS];
+                const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(cm + mm * HL), cb = *reinterpret_cast<const ulonglong2*>(cm + mm * HL + 4);
+                const uint64_t xx0 = pack_f32x2(x0, x0), xx1 = pack_f32x2(x1, x1);
+                acc[0][0] = fma_f32x2(ca.x, xx0, acc[0][0]);
+                acc[0][1] = fma_f32x2(ca.y, xx0, acc[0][1]);
+                acc[0][2] = fma_f32x2(cb.x, xx0, acc[0][2]);
+                acc[0][3] = fma_f32x2(cb.y, xx0, acc[0][3]);
+                acc[1][0] = fma_f32x2(ca.x, xx1, acc[1][0]);
+                acc[1][1] = fma_f32x2(ca.y, xx1, acc[1][1]);
+                acc[1][2] = fma_f32x2(cb.x, xx1, acc[1][2]);
+                acc[1][3] = fma_f32x2(cb.y, xx1, acc[1][3]);
+            }
+        }
+        heads.arrive();                                    // (this thread reads no raw score of this tile any more)
+        // [head][row][32] over the tile's keys; odd rows have their groups of four swapped, so that the reads below meet no bank twice.
+        float* mixed = reinterpret_cast<float*>(tt_smem + (size_t)(it & 1) * 2 * plane);
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                float a, b;
+                unpack_f32x2(acc[r][k], a, b);
+                float* to = mixed + ((hb + 2 * k) * TT_ROWS + ra + r) * 32 + (lane ^ (r << 2));
+                to[0] = a;
+                to[TT_ROWS * 32] = b;
+            }
+        cp_async_wait<0>();
+        __syncthreads();                                   // the mixed scores, this tile's values and the next one's keys are there; the values before have been used
+        if (it + 1 < n_tiles) load_plane(it + 1, 1);
+        cp_async_commit();
+        const int tile = tile_at(it);
+        const bool page_ok = page_at(it) >= 0;
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const float4 v = *reinterpret_cast<const float4*>(mixed + (warp * TT_ROWS + gq + 8 * i) * 32 + ((tq * 8 + half * 4) ^ ((gq & 1) << 2)));
+                s[2 * half][2 * i] = v.x, s[2 * half][2 * i + 1] = v.y, s[2 * half + 1][2 * i] = v.z, s[2 * half + 1][2 * i + 1] = v.w;
+            }
+        float tmax[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int i = e >> 1;
+                const int t = tile * TT_KEYS + nb * 8 + 2 * tq + (e & 1);
+                const bool seen = page_ok && live[i] && t <= pos[i] && (t >= lo[i] || t < keep_first);
+                s[nb][e] = seen ? s[nb][e] * LOG2E : -INFINITY;
+                tmax[i] = fmaxf(tmax[i], s[nb][e]);
+            }
+        float base[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 1));
+            tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 2));
+            const float mn = fmaxf(m[i], tmax[i]);
+            corr[i] = mn == -INFINITY ? 1.0f : fast_exp2(m[i] - mn);
+            base[i] = mn == -INFINITY ? 0.0f : mn;
+            m[i] = mn;
+        }
+        float psum[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[nb][e] = fast_exp2(s[nb][e] - base[e >> 1]);
+                psum[e >> 1] += s[nb][e];
+            }
+        l[0] = l[0] * corr[0] + psum[0];
+        l[1] = l[1] * corr[1] + psum[1];
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+            pf[kk][0] = pack_bf16(s[2 * kk][0], s[2 * kk][1]), pf[kk][1] = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
+            pf[kk][2] = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]), pf[kk][3] = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+        }
+        if (page_ok && tile == last_pos / TT_KEYS && last_pos % TT_KEYS != TT_KEYS - 1) {
+            // What lies past the sequence's last position belongs to nobody (a sequence that held the page before may have left
+            // not-a-numbers there, and 0 x NaN is NaN in the product with the values): those value rows are cleared in the copy.
+            const int first = last_pos % TT_KEYS + 1;
+            uint8_t* values = tt_smem + (size_t)((it & 1) * 2 + 1) * plane;
+            for (int i = threadIdx.x; i < GL * (TT_KEYS - first) * CHUNKS; i += 512) {
+                const int g = i / ((TT_KEYS - first) * CHUNKS), rest = i - g * (TT_KEYS - first) * CHUNKS;
+                *reinterpret_cast<uint4*>(values + g * HEAD_BYTES + tile_offset<D>(first + rest / CHUNKS, rest % CHUNKS)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            __syncthreads();
+        }
+        if (it + 1 < n_tiles) scores(it + 1);
+        heads.wait();                                      // nobody reads the raw scores any more: the next tile's may take their place
+        if (it + 1 < n_tiles) hand_out();
+    }
+    if (n_tiles > 0) weigh(n_tiles - 1);
+    cp_async_wait<0>();
+    if (CL > 1) cg::this_cluster().sync();                 // no block leaves while another may still write raw scores into its memory
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        float sum = l[i];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (!live[i]) continue;
+        if (splits > 1) {
+            float* part = scratch + (((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * splits + blockIdx.z) * (D + 2);
+            if (tq == 0) part[0] = m[i], part[1] = sum;
+#pragma unroll
+            for (int nd = 0; nd < ND; nd++) *reinterpret_cast<float2*>(part + 2 + nd * 8 + 2 * tq) = make_float2(o[nd][2 * i], o[nd][2 * i + 1]);
+            continue;
+        }
+        const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+        const size_t at = ((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * D + 2 * tq;
+#pragma unroll
+        for (int nd = 0; nd < ND; nd++) {
+            const float2 gv = *reinterpret_cast<const float2*>(gate + at + nd * 8);
+            *reinterpret_cast<uint32_t*>(out + at + nd * 8) = pack_bf16(o[nd][2 * i] * inv * gv.x, o[nd][2 * i + 1] * inv * gv.y);
+        }
+    }
+}
+
 // One block a (row, head): the splits' maxima (in powers of two), sums and products in the order of the splits, then the gate.
 __global__ void __launch_bounds__(128)
 talk_merge_kernel(const float* scratch, const int* __restrict__ row_slot, const float* gate, bf16* __restrict__ out, int H, int D, int splits) {
@@ -594,6 +958,33 @@ static int tiles_go(const void* q, const void* k_cache, const void* v_cache, con
     const int warps = (H / CL + HPW - 1) / HPW;
     const dim3 grid(((max_new + TT_ROWS - 1) / TT_ROWS) * CL, seqs, splits);
     cudaError_t e;
+    if constexpr (HPW == 1 && CL <= 2 && (D == 64 || D == 128)) {
+        // Sixteen heads a block whose mixed scores (32 KB) fit the place of a tile's keys: the mix by rows.  (Of 64 heads the raw scores leave no
+        // room for two stages.)  One prompt of 2,048, 32 heads of 128 on 8, window 1,024: 557 us by rows, 769 by heads.
+        if (H == 16 * CL && (G / CL) * D >= 512 && stages == 2) {
+            static bool raised = false;
+            if (!raised) {
+                e = cudaFuncSetAttribute(talk_mixed_kernel<D, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+                if (e != cudaSuccess) {
+                    bc_set_error("talk_tiles: cannot set shared memory: %s", cudaGetErrorString(e));
+                    return (int)e;
+                }
+                raised = true;
+            }
+            e = CL > 1 ? bc_launch_clustered(talk_mixed_kernel<D, CL>, grid, dim3(512), smem, s, dim3(CL, 1, 1), (const bf16*)q, (const bf16*)k_cache,
+                                             (const bf16*)v_cache, page_table, seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out, H, G, max_pages, n_pages,
+                                             window, keep_first, scale, cap, scratch, splits)
+                       : bc_launch(talk_mixed_kernel<D, CL>, grid, dim3(512), smem, s, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, page_table,
+                                   seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out, H, G, max_pages, n_pages, window, keep_first, scale, cap, scratch,
+                                   splits);
+            if (e != cudaSuccess) {
+                bc_set_error("talk_tiles: %s", cudaGetErrorString(e));
+                return (int)e;
+            }
+            if (splits > 1) bc_launch(talk_merge_kernel, dim3(rows, H), dim3(128), 0, s, (const float*)scratch, row_slot, gate, (bf16*)out, H, D, splits);
+            BC_LAUNCH_STATUS();
+        }
+    }
     if (CL > 1)
         e = bc_launch_clustered(talk_tiles_kernel<D, HPW, CL>, grid, dim3(32 * warps), smem, s, dim3(CL, 1, 1), (const bf16*)q, (const bf16*)k_cache,
                                 (const bf16*)v_cache, page_table, seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out, H, G, max_pages, n_pages,
@@ -660,6 +1051,13 @@ static int prepare(const float* proj, int rows, int P, int g_at, const float* bi
     BC_CHECK_ARG((H + G) * D <= P && g_at >= 0 && g_at + H * D <= P, "talk_prepare: the parts do not fit a row of %d", P);
     if (rows == 0) return BC_OK;
     const int heads = H + G;
+    // By the sizes alone (and the borders that they put the rows on).
+    if (D % 4 == 0 && D <= 128 && rot % 8 == 0 && P % 4 == 0 && g_at % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)bias % 16 == 0 && (uintptr_t)cos_sin % 16 == 0 &&
+        (uintptr_t)q_out % 16 == 0 && (uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0 && (uintptr_t)gate % 16 == 0) {
+        bc_launch(talk_prepare_wide_kernel<T>, dim3(rows, (heads + 7) / 8), dim3(256), 0, s, proj, P, g_at, bias, cos_sin, table_positions, row_pos, row_slot,
+                  page_table, max_pages, n_pages, (T*)q_out, (T*)k_cache, (T*)v_cache, gate, H, G, D, rot, eps, write_cache);
+        BC_LAUNCH_STATUS();
+    }
     const int threads = heads >= 8 ? 256 : heads >= 4 ? 128 : 64;      // by the row's heads alone
     bc_launch(talk_prepare_kernel<T>, dim3(rows), dim3(threads), 0, s, proj, P, g_at, bias, cos_sin, table_positions, row_pos, row_slot, page_table,
               max_pages, n_pages, (T*)q_out, (T*)k_cache, (T*)v_cache, gate, H, G, D, rot, eps, write_cache);
