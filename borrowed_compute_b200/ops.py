@@ -71,7 +71,9 @@ def set_gemm_tc_pair_tokens(n: int) -> None:
 
 
 def _stream() -> _c_void_p:
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream().cuda_stream without the Stream object around it, asked for anew at every launch: several
+    # microseconds of Python a launch, more than most kernels of a small step run for.
+    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
