@@ -571,47 +571,40 @@ talk_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
     }
 }
 
-// The same for sixteen heads a block (16 or 32 heads in all) whose keys of a tile take up 32 KB (heads of 128 on four kv heads a
-// block, of 64 on eight): a warp a head, as above, for both products and the softmax, but the mix goes by rows.  What bounded the kernel
-// above is the mix's reads: every warp reads all heads' raw scores for its one head, 8,700 reads of 128 bytes a tile of 32 heads, counted.  Here
-// warp w mixes eight heads of two rows, a lane one position of each: a raw score that is read serves eight heads (two 4-byte reads and
-// two uniform 16-byte reads of the mix's column for sixteen multiply-adds, two heads an instruction), about 2,000.  The mixed scores go back
-// to the warp of their head through the place of the tile's keys, which nobody reads any more.  The sums keep their order.
+// The same for sixteen heads of sixteen rows (PAIR 1) or thirty-two of eight (PAIR 2), whose keys of a position take up PAIR KB (heads of 128 on four
+// or eight kv heads, of 64 on eight or sixteen), a block of sixteen warps, but the mix goes by rows.  A warp's sixteen rows of a product are one
+// head's, or eight rows each of two neighbouring heads, which share a kv head.  What bounded the kernel above is the mix's reads: every warp
+// reads all heads' raw scores for its one head, 8,700 reads of 128 bytes a tile of 32 heads, counted.  Here a warp mixes eight heads of two rows,
+// a lane one position of each: a raw score that is read serves eight heads (two 4-byte reads and two uniform 16-byte reads of the mix's column
+// for sixteen multiply-adds, two heads an instruction), about 2,000.  The sums keep their order.
 //
-// The cluster's two barriers a tile (all heads' raw scores are there; nobody reads them any more) are split into arrival and wait, and what
-// needs neither stands between: the product with the tile before's values, and the next tile's scores.  Keys of the next tile are
-// asked for as soon as the mixed scores of the tile before have left their place, its values one barrier later.
-// One prompt of 2,048, 32 heads of 128 on 8, window 1,024: 557 us, with the kernel above 769.
+// Two barriers a tile: (A) all raw scores of a tile are there, its keys and the values before have been used; (B) the mixed scores are there,
+// the raw ones have been read.  The next keys and this tile's values arrive between them, while the mix runs, so one stage of each suffices.
+// (Thirty-two heads as a cluster of two blocks of sixteen rows handed every raw score to the other block's memory: the release of those stores, twice
+// a tile, and the registers of their addresses left a scheduler idle 62 % of the time.)
+// One prompt of 2,048, window 1,024, 32 heads of 128 on 8: 392 us; as a cluster 569, with the kernel above 769.  Of 64 on 16: 304, as a cluster 391.
+// 8 rows that see 4,000 positions: 73, as a cluster 159.  Sixteen heads of 128 on 4, one prompt: 200, with two stages and the cluster's order 236.
 #define TM_PAGES_KEPT 256
-template <int CL> struct HeadsBarrier {
-    __device__ __forceinline__ void arrive() const {
-        if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    }
-    __device__ __forceinline__ void wait() const {
-        if (CL > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        else __syncthreads();
-    }
-};
-
-template <int D, int CL>
-__global__ void __launch_bounds__(512)
-talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const int* __restrict__ page_table, const int* __restrict__ seq_rows,
+#define TP_WARPS 16
+// Steps of 16 values of the queries that lie in shared memory instead of registers (which the two products and the mix of heads of 128 use up).
+__host__ __device__ constexpr int tp_q_kept(int D) { return D == 128 ? 3 : 0; }
+__host__ __device__ constexpr size_t tp_smem_bytes(int D, int PAIR) {
+    return (size_t)PAIR * (2 * TT_KEYS * 1024 + TP_WARPS * (16 / PAIR) * (TT_RS + TT_KEYS) * 4 + PAIR * TP_WARPS * TP_WARPS * 4) + (size_t)tp_q_kept(D) * TP_WARPS * 32 * 16;
+}
+template <int D, int PAIR>
+__global__ void __launch_bounds__(32 * TP_WARPS)
+talk_by_rows_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const int* __restrict__ page_table, const int* __restrict__ seq_rows,
                   const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const float* gate, const float* __restrict__ temp,
-                  const float* __restrict__ talk, bf16* __restrict__ out, int H, int G, int max_pages, int n_pages, int window, int keep_first, float scale,
-                  float cap, float* __restrict__ scratch, int splits) {
-    constexpr int CHUNKS = D / 8, KD = D / 16, ND = D / 8, HL = 16;
-    constexpr int HEAD_BYTES = TT_KEYS * D * 2;            // one kv head's 32 positions
-    extern __shared__ __align__(128) uint8_t tt_smem[];
+                  const float* __restrict__ talk, bf16* __restrict__ out, int max_pages, int n_pages, int window, int keep_first, float scale, float cap,
+                  float* __restrict__ scratch, int splits) {
+    constexpr int CHUNKS = D / 8, KD = D / 16, ND = D / 8, H = PAIR * TP_WARPS, G = PAIR * 512 / D, ROWS = 16 / PAIR, Q_KEPT = tp_q_kept(D);
+    constexpr int HEAD_BYTES = TT_KEYS * D * 2, PLANE = G * HEAD_BYTES;
+    extern __shared__ __align__(128) uint8_t tt_smem[];    // a tile's keys, its values ..
     __shared__ int page_kept[TM_PAGES_KEPT];               // the pages of the block's first tiles, fetched once (-1: none)
-    const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
-    const int GL = G / CL, h_first = rank * HL, g_first = rank * GL;
-    const int plane = GL * HEAD_BYTES;                     // a tile's keys of this block's kv heads; their values follow
-    float* raw = reinterpret_cast<float*>(tt_smem + (size_t)4 * plane);               // [H][16][TT_RS]: all heads' raw scores
-    float* mix = raw + (size_t)H * TT_ROWS * TT_RS;        // [H][16]: column m of the rows of the mix that make this block's heads
-    float* raw_of[CL];                                     // every block's copy of the raw scores, as this block writes them
-#pragma unroll
-    for (int c = 0; c < CL; c++) raw_of[c] = CL > 1 ? cg::this_cluster().map_shared_rank(raw, c) : raw;
-    const HeadsBarrier<CL> heads;
+    float* raw = reinterpret_cast<float*>(tt_smem + 2 * PLANE);      // .. [H][ROWS][TT_RS]: all heads' raw scores
+    float* mixed = raw + H * ROWS * TT_RS;                 // [H][ROWS][32]
+    float* mix = mixed + H * ROWS * TT_KEYS;               // [H][H]: column m of the mix
+    uint4* q_kept = reinterpret_cast<uint4*>(mix + H * H) + threadIdx.x;              // [Q_KEPT][512]
 
     pdl_launch_dependents_if_resident();
     pdl_wait();
@@ -621,24 +614,26 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
     const int gq = lane >> 2, tq = lane & 3, j4 = lane >> 3, r8 = lane & 7;
     const int slot = seq_slot[sq];
     const int row0 = seq_rows[sq], n_new = seq_rows[sq + 1] - row0;
-    const int n_tiles_q = (n_new + TT_ROWS - 1) / TT_ROWS;
-    const int q_tile = n_tiles_q - 1 - (int)blockIdx.x / CL;    // the last rows see the most: they go first
-    if (slot < 0 || q_tile < 0) return;                    // (the same for every block of a cluster)
+    const int n_tiles_q = (n_new + ROWS - 1) / ROWS;
+    const int q_tile = n_tiles_q - 1 - (int)blockIdx.x;    // the last rows see the most: they go first
+    if (slot < 0 || q_tile < 0) return;
     const int start = seq_start[sq];
-    const int tok0 = q_tile * TT_ROWS, tok_end = min(n_new, tok0 + TT_ROWS);
+    const int tok0 = q_tile * ROWS, tok_end = min(n_new, tok0 + ROWS);
     const int* pages = page_table + (size_t)slot * max_pages;
-    const int group = H / G;
     const int last_pos = start + n_new - 1;                // the last position the sequence holds after this step
 
-    for (int i = threadIdx.x; i < HL * H; i += 512) mix[i] = talk[(size_t)(h_first + i % HL) * H + i / HL];
+    for (int i = threadIdx.x; i < H * H; i += 512) mix[i] = talk[(i % H) * H + i / H];
     auto first_seen = [&](int p) { return window > 0 && p + 1 > window ? p + 1 - window : 0; };
+    // This warp's products' upper and lower eight rows: rows gq and gq + 8 of one head, or row gq of two.
+    const int h = PAIR * warp, down = PAIR == 1 ? 8 : 0;
+    auto head_of = [&](int i) { return PAIR == 1 ? h : h + i; };
+    auto row_of = [&](int i) { return gq + i * down; };
     int pos[2], lo[2];
     bool live[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-        const int tok = tok0 + gq + 8 * i;
-        live[i] = tok < n_new;
-        pos[i] = start + tok;
+        live[i] = tok0 + row_of(i) < n_new;
+        pos[i] = start + tok0 + row_of(i);
         lo[i] = first_seen(pos[i]);
     }
     // The block's tiles of positions: [0, kept) and [win_begin, win_end], as one stretch where they meet; with several splits its share of them.
@@ -649,7 +644,7 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
     const int all_tiles = kept + (win_end - win_begin + 1);
     const int per_split = (all_tiles + splits - 1) / splits;
     const int tile_first = (int)blockIdx.z * per_split;
-    const int n_tiles = max(0, min(all_tiles, tile_first + per_split) - tile_first);      // (the same for every block of a cluster)
+    const int n_tiles = max(0, min(all_tiles, tile_first + per_split) - tile_first);
     auto tile_at = [&](int k) { k += tile_first; return k < kept ? k : win_begin + (k - kept); };
     auto page_of = [&](int it) {
         const int pi = tile_at(it) / 2;
@@ -659,112 +654,92 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
     for (int i = threadIdx.x; i < min(n_tiles, TM_PAGES_KEPT); i += 512) page_kept[i] = page_of(i);
     __syncthreads();
     auto page_at = [&](int it) { return it < TM_PAGES_KEPT ? page_kept[it] : page_of(it); };
-    // Plane `which` of tile number `it` (0 keys, 1 values) into its stage.  A tile without a page is not fetched: its scores are masked whatever
-    // the stage holds, and its values are not multiplied.
-    auto load_plane = [&](int it, int which) {
-        const int tile = tile_at(it), page = page_at(it);
+    // The keys or the values of tile number `it`.  A tile without a page is not fetched: its scores are masked whatever lies there, and its values
+    // are not multiplied.  A page's kv heads lie one after another.
+    auto load_plane = [&](int it, const bf16* cache, uint8_t* to) {
+        const int page = page_at(it);
         if (page < 0) return;
-        const uint32_t to = ad_smem(tt_smem + (size_t)((it & 1) * 2 + which) * plane);
-        const bf16* cache = which ? v_cache : k_cache;
+        const bf16* from = cache + ((size_t)page * G * BC_PAGE + (tile_at(it) & 1) * TT_KEYS) * D;
         constexpr int PER_HEAD = TT_KEYS * CHUNKS;
-        for (int i = threadIdx.x; i < GL * PER_HEAD; i += 512) {
-            const int g = i / PER_HEAD, rest = i - g * PER_HEAD, row = rest / CHUNKS, c = rest - row * CHUNKS;
-            cp_async16(to + g * HEAD_BYTES + tile_offset<D>(row, c), cache + (((size_t)page * G + g_first + g) * BC_PAGE + (tile & 1) * TT_KEYS + row) * D + c * 8);
+#pragma unroll
+        for (int u = 0; u < G * PER_HEAD / 512; u++) {
+            const int i = threadIdx.x + 512 * u, g = i / PER_HEAD, row = i % PER_HEAD / CHUNKS, c = i % CHUNKS;
+            cp_async16(ad_smem(to) + g * HEAD_BYTES + tile_offset<D>(row, c), from + (g * BC_PAGE + row) * D + c * 8);
         }
     };
-
-    const int h = h_first + warp, kv_bytes = (h / group - g_first) * HEAD_BYTES;       // this warp's head
-    uint32_t qf[KD][4], pf[2][4];
-    float o[ND][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, corr[2] = {1.0f, 1.0f};
-    const float factor = scale * temp[h];
+    uint8_t *keys = tt_smem, *values = tt_smem + PLANE;
+    const int kv_bytes = h / (H / G) * HEAD_BYTES;
+    uint32_t qf[KD][4], pf[2][4];                          // (the first Q_KEPT of qf go to shared memory)
+    float o[ND][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+    const float factor[2] = {scale * temp[head_of(0)], scale * temp[head_of(1)]};
 #pragma unroll
     for (int kd = 0; kd < KD; kd++)
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const bf16* qr = q + ((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * D + kd * 16 + 2 * tq;
+            const bf16* qr = q + ((size_t)(row0 + tok0 + row_of(i)) * H + head_of(i)) * D + kd * 16 + 2 * tq;
             qf[kd][i] = live[i] ? *reinterpret_cast<const uint32_t*>(qr) : 0u;
             qf[kd][i + 2] = live[i] ? *reinterpret_cast<const uint32_t*>(qr + 8) : 0u;
         }
+#pragma unroll
+    for (int kd = 0; kd < Q_KEPT; kd++) q_kept[kd * 512] = make_uint4(qf[kd][0], qf[kd][1], qf[kd][2], qf[kd][3]);
 #pragma unroll
     for (int nd = 0; nd < ND; nd++) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.0f;
     const float two_over_cap = cap > 0.0f ? 2.0f / cap : 0.0f;
     const float LOG2E = 1.4426950408889634f;
 
-    float s[4][4];
-    auto scores = [&](int it) {                            // this head's raw scores of tile `it`, bounded
-        const uint32_t kh = ad_smem(tt_smem + (size_t)(it & 1) * 2 * plane) + kv_bytes;
+    auto scores = [&]() {                                  // the raw scores of the keys that are there, bounded, to where all can read them
+        float s[4][4];
 #pragma unroll
         for (int nb = 0; nb < 4; nb++) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.0f;
 #pragma unroll
-        for (int kd = 0; kd < KD; kd++)
+        for (int kd = 0; kd < KD; kd++) {
+            uint32_t a[4] = {qf[kd][0], qf[kd][1], qf[kd][2], qf[kd][3]};
+            if (kd < Q_KEPT) {
+                const uint4 v = q_kept[kd * 512];
+                a[0] = v.x, a[1] = v.y, a[2] = v.z, a[3] = v.w;
+            }
 #pragma unroll
             for (int np = 0; np < 2; np++) {
                 uint32_t b0, b1, b2, b3;
-                ldmatrix_x4(kh + tile_offset<D>(np * 16 + (j4 >> 1) * 8 + r8, kd * 2 + (j4 & 1)), b0, b1, b2, b3);
-                mma_16816(s[2 * np], qf[kd], b0, b1);
-                mma_16816(s[2 * np + 1], qf[kd], b2, b3);
+                ldmatrix_x4(ad_smem(keys) + kv_bytes + tile_offset<D>(np * 16 + (j4 >> 1) * 8 + r8, kd * 2 + (j4 & 1)), b0, b1, b2, b3);
+                mma_16816(s[2 * np], a, b0, b1);
+                mma_16816(s[2 * np + 1], a, b2, b3);
             }
+        }
 #pragma unroll
         for (int nb = 0; nb < 4; nb++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                s[nb][e] *= factor;
+                s[nb][e] *= factor[e >> 1];
                 if (cap > 0.0f) s[nb][e] = tt_bound(s[nb][e], cap, two_over_cap);
             }
-    };
-    auto hand_out = [&]() {                                // to every block of the cluster
 #pragma unroll
         for (int i = 0; i < 2; i++)
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const float4 v = make_float4(s[2 * half][2 * i], s[2 * half][2 * i + 1], s[2 * half + 1][2 * i], s[2 * half + 1][2 * i + 1]);
-#pragma unroll
-                for (int c = 0; c < CL; c++) *reinterpret_cast<float4*>(raw_of[c] + (size_t)h * TT_ROWS * TT_RS + (gq + 8 * i) * TT_RS + tq * 8 + half * 4) = v;
-            }
-    };
-    auto weigh = [&](int it) {                             // the product with the values of tile `it`
-        if (page_at(it) < 0) return;
-        const uint32_t vh = ad_smem(tt_smem + (size_t)((it & 1) * 2 + 1) * plane) + kv_bytes;
-#pragma unroll
-        for (int nd = 0; nd < ND; nd++) o[nd][0] *= corr[0], o[nd][1] *= corr[0], o[nd][2] *= corr[1], o[nd][3] *= corr[1];
-#pragma unroll
-        for (int kk = 0; kk < 2; kk++)
-#pragma unroll
-            for (int nd = 0; nd < ND; nd += 2) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(vh + tile_offset<D>(kk * 16 + (j4 & 1) * 8 + r8, nd + (j4 >> 1)), b0, b1, b2, b3);
-                mma_16816(o[nd], pf[kk], b0, b1);
-                mma_16816(o[nd + 1], pf[kk], b2, b3);
-            }
+            for (int half = 0; half < 2; half++)
+                *reinterpret_cast<float4*>(raw + (head_of(i) * ROWS + row_of(i)) * TT_RS + tq * 8 + half * 4) =
+                    make_float4(s[2 * half][2 * i], s[2 * half][2 * i + 1], s[2 * half + 1][2 * i], s[2 * half + 1][2 * i + 1]);
     };
 
-    if (n_tiles > 0) {
-        load_plane(0, 0);
-        load_plane(0, 1);
-    }
+    if (n_tiles > 0) load_plane(0, k_cache, keys);
     cp_async_commit();
     cp_async_wait<0>();
-    if (CL > 1) cg::this_cluster().sync();                 // every block is there before its memory is written to
-    else __syncthreads();
-    if (n_tiles > 0) {
-        scores(0);
-        hand_out();
-    }
+    __syncthreads();
+    if (n_tiles > 0) scores();
     for (int it = 0; it < n_tiles; it++) {
-        heads.arrive();
-        if (it > 0) weigh(it - 1);
-        heads.wait();                                      // every head's raw scores are there; the mixed ones of the tile before have been read
-        if (it + 1 < n_tiles) load_plane(it + 1, 0);
+        __syncthreads();                                   // (A)
+        if (it + 1 < n_tiles) load_plane(it + 1, k_cache, keys);
+        load_plane(it, v_cache, values);
         cp_async_commit();
-        uint64_t acc[2][4] = {};                           // heads hb .. hb + 7 of rows ra, ra + 1 at the lane's position
-        const int ra = warp & ~1, hb = 8 * (warp & 1);
         {
+            uint64_t acc[2][4] = {};                       // heads hb .. hb + 7 of rows ra, ra + 1 at the lane's position
+            const int ra = 2 * (warp / (2 * PAIR)), hb = 8 * (warp % (2 * PAIR));
             const float* rm = raw + ra * TT_RS + lane;
             const float* cm = mix + hb;
 #pragma unroll 4
             for (int mm = 0; mm < H; mm++) {
-                const float x0 = rm[(size_t)mm * TT_ROWS * TT_RS], x1 = rm[(size_t)mm * TT_ROWS * TT_RS + TT_RS];
-                const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(cm + mm * HL), cb = *reinterpret_cast<const ulonglong2*>(cm + mm * HL + 4);
+                const float x0 = rm[mm * ROWS * TT_RS], x1 = rm[mm * ROWS * TT_RS + TT_RS];
+                const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(cm + mm * H), cb = *reinterpret_cast<const ulonglong2*>(cm + mm * H + 4);
                 const uint64_t xx0 = pack_f32x2(x0, x0), xx1 = pack_f32x2(x1, x1);
                 acc[0][0] = fma_f32x2(ca.x, xx0, acc[0][0]);
                 acc[0][1] = fma_f32x2(ca.y, xx0, acc[0][1]);
@@ -775,31 +750,28 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
                 acc[1][2] = fma_f32x2(cb.x, xx1, acc[1][2]);
                 acc[1][3] = fma_f32x2(cb.y, xx1, acc[1][3]);
             }
+            // Odd rows have their groups of four swapped, so that the reads below meet no bank twice.
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    float a, b;
+                    unpack_f32x2(acc[r][k], a, b);
+                    float* to = mixed + ((hb + 2 * k) * ROWS + ra + r) * TT_KEYS + (lane ^ (r << 2));
+                    to[0] = a;
+                    to[ROWS * TT_KEYS] = b;
+                }
         }
-        heads.arrive();                                    // (this thread reads no raw score of this tile any more)
-        // [head][row][32] over the tile's keys; odd rows have their groups of four swapped, so that the reads below meet no bank twice.
-        float* mixed = reinterpret_cast<float*>(tt_smem + (size_t)(it & 1) * 2 * plane);
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                float a, b;
-                unpack_f32x2(acc[r][k], a, b);
-                float* to = mixed + ((hb + 2 * k) * TT_ROWS + ra + r) * 32 + (lane ^ (r << 2));
-                to[0] = a;
-                to[TT_ROWS * 32] = b;
-            }
         cp_async_wait<0>();
-        __syncthreads();                                   // the mixed scores, this tile's values and the next one's keys are there; the values before have been used
-        if (it + 1 < n_tiles) load_plane(it + 1, 1);
-        cp_async_commit();
+        __syncthreads();                                   // (B)
         const int tile = tile_at(it);
         const bool page_ok = page_at(it) >= 0;
+        float s[4][4];
 #pragma unroll
         for (int i = 0; i < 2; i++)
 #pragma unroll
             for (int half = 0; half < 2; half++) {
-                const float4 v = *reinterpret_cast<const float4*>(mixed + (warp * TT_ROWS + gq + 8 * i) * 32 + ((tq * 8 + half * 4) ^ ((gq & 1) << 2)));
+                const float4 v = *reinterpret_cast<const float4*>(mixed + (head_of(i) * ROWS + row_of(i)) * TT_KEYS + ((tq * 8 + half * 4) ^ ((gq & 1) << 2)));
                 s[2 * half][2 * i] = v.x, s[2 * half][2 * i + 1] = v.y, s[2 * half + 1][2 * i] = v.z, s[2 * half + 1][2 * i + 1] = v.w;
             }
         float tmax[2] = {-INFINITY, -INFINITY};
@@ -807,13 +779,12 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
         for (int nb = 0; nb < 4; nb++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const int i = e >> 1;
-                const int t = tile * TT_KEYS + nb * 8 + 2 * tq + (e & 1);
+                const int i = e >> 1, t = tile * TT_KEYS + nb * 8 + 2 * tq + (e & 1);
                 const bool seen = page_ok && live[i] && t <= pos[i] && (t >= lo[i] || t < keep_first);
                 s[nb][e] = seen ? s[nb][e] * LOG2E : -INFINITY;
                 tmax[i] = fmaxf(tmax[i], s[nb][e]);
             }
-        float base[2];
+        float corr[2], base[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 1));
@@ -842,35 +813,43 @@ talk_mixed_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, const
             // What lies past the sequence's last position belongs to nobody (a sequence that held the page before may have left
             // not-a-numbers there, and 0 x NaN is NaN in the product with the values): those value rows are cleared in the copy.
             const int first = last_pos % TT_KEYS + 1;
-            uint8_t* values = tt_smem + (size_t)((it & 1) * 2 + 1) * plane;
-            for (int i = threadIdx.x; i < GL * (TT_KEYS - first) * CHUNKS; i += 512) {
+            for (int i = threadIdx.x; i < G * (TT_KEYS - first) * CHUNKS; i += 512) {
                 const int g = i / ((TT_KEYS - first) * CHUNKS), rest = i - g * (TT_KEYS - first) * CHUNKS;
                 *reinterpret_cast<uint4*>(values + g * HEAD_BYTES + tile_offset<D>(first + rest / CHUNKS, rest % CHUNKS)) = make_uint4(0u, 0u, 0u, 0u);
             }
             __syncthreads();
         }
-        if (it + 1 < n_tiles) scores(it + 1);
-        heads.wait();                                      // nobody reads the raw scores any more: the next tile's may take their place
-        if (it + 1 < n_tiles) hand_out();
+        if (page_ok) {                                     // the product with the values
+#pragma unroll
+            for (int nd = 0; nd < ND; nd++) o[nd][0] *= corr[0], o[nd][1] *= corr[0], o[nd][2] *= corr[1], o[nd][3] *= corr[1];
+#pragma unroll
+            for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+                for (int nd = 0; nd < ND; nd += 2) {
+                    uint32_t b0, b1, b2, b3;
+                    ldmatrix_x4_trans(ad_smem(values) + kv_bytes + tile_offset<D>(kk * 16 + (j4 & 1) * 8 + r8, nd + (j4 >> 1)), b0, b1, b2, b3);
+                    mma_16816(o[nd], pf[kk], b0, b1);
+                    mma_16816(o[nd + 1], pf[kk], b2, b3);
+                }
+        }
+        if (it + 1 < n_tiles) scores();
     }
-    if (n_tiles > 0) weigh(n_tiles - 1);
-    cp_async_wait<0>();
-    if (CL > 1) cg::this_cluster().sync();                 // no block leaves while another may still write raw scores into its memory
 #pragma unroll
     for (int i = 0; i < 2; i++) {
         float sum = l[i];
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         if (!live[i]) continue;
+        const size_t row_head = (size_t)(row0 + tok0 + row_of(i)) * H + head_of(i);
         if (splits > 1) {
-            float* part = scratch + (((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * splits + blockIdx.z) * (D + 2);
+            float* part = scratch + (row_head * splits + blockIdx.z) * (D + 2);
             if (tq == 0) part[0] = m[i], part[1] = sum;
 #pragma unroll
             for (int nd = 0; nd < ND; nd++) *reinterpret_cast<float2*>(part + 2 + nd * 8 + 2 * tq) = make_float2(o[nd][2 * i], o[nd][2 * i + 1]);
             continue;
         }
         const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
-        const size_t at = ((size_t)(row0 + tok0 + gq + 8 * i) * H + h) * D + 2 * tq;
+        const size_t at = row_head * D + 2 * tq;
 #pragma unroll
         for (int nd = 0; nd < ND; nd++) {
             const float2 gv = *reinterpret_cast<const float2*>(gate + at + nd * 8);
@@ -939,6 +918,18 @@ extern "C" int bc_talk_tiles_accepts(int H, int G, int D) {
     return CL > 0 && tt_smem_bytes(H, G, D, 1, CL) <= 216 * 1024;
 }
 
+// Whether the mix goes by rows: sixteen or thirty-two heads whose keys of a position are 512 values a sixteen heads.  (Wider ones leave the mixed
+// scores no room, of other numbers a warp's sixteen rows are not whole heads or pairs: those stay with the kernel that mixes by heads.)
+static bool tp_takes(int H, int G, int D) { return (D == 64 || D == 128) && (H == TP_WARPS || H == 2 * TP_WARPS) && G * D == 32 * H; }
+
+// Blocks that the rows of a sequence with up to max_new new ones take (times the splits).
+extern "C" int bc_talk_tiles_blocks(int H, int G, int D, int max_new) {
+    int CL, HPW;
+    tt_shape(H, G, D, &CL, &HPW);
+    const int rows = tp_takes(H, G, D) ? TT_ROWS * TP_WARPS / H : TT_ROWS;
+    return (max_new + rows - 1) / rows * (tp_takes(H, G, D) || CL < 1 ? 1 : CL);
+}
+
 template <int D, int HPW, int CL>
 static int tiles_go(const void* q, const void* k_cache, const void* v_cache, const int* page_table, const int* seq_rows, const int* seq_slot,
                     const int* seq_start, const float* gate, const float* temp, const float* talk, void* out, int seqs, int max_new, int H, int G,
@@ -959,24 +950,19 @@ static int tiles_go(const void* q, const void* k_cache, const void* v_cache, con
     const dim3 grid(((max_new + TT_ROWS - 1) / TT_ROWS) * CL, seqs, splits);
     cudaError_t e;
     if constexpr (HPW == 1 && CL <= 2 && (D == 64 || D == 128)) {
-        // Sixteen heads a block whose mixed scores (32 KB) fit the place of a tile's keys: the mix by rows.  (Of 64 heads the raw scores leave no
-        // room for two stages.)  One prompt of 2,048, 32 heads of 128 on 8, window 1,024: 557 us by rows, 769 by heads.
-        if (H == 16 * CL && (G / CL) * D >= 512 && stages == 2) {
+        if (tp_takes(H, G, D)) {
             static bool raised = false;
             if (!raised) {
-                e = cudaFuncSetAttribute(talk_mixed_kernel<D, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+                e = cudaFuncSetAttribute(talk_by_rows_kernel<D, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(D, CL));
                 if (e != cudaSuccess) {
                     bc_set_error("talk_tiles: cannot set shared memory: %s", cudaGetErrorString(e));
                     return (int)e;
                 }
                 raised = true;
             }
-            e = CL > 1 ? bc_launch_clustered(talk_mixed_kernel<D, CL>, grid, dim3(512), smem, s, dim3(CL, 1, 1), (const bf16*)q, (const bf16*)k_cache,
-                                             (const bf16*)v_cache, page_table, seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out, H, G, max_pages, n_pages,
-                                             window, keep_first, scale, cap, scratch, splits)
-                       : bc_launch(talk_mixed_kernel<D, CL>, grid, dim3(512), smem, s, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, page_table,
-                                   seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out, H, G, max_pages, n_pages, window, keep_first, scale, cap, scratch,
-                                   splits);
+            e = bc_launch(talk_by_rows_kernel<D, CL>, dim3(bc_talk_tiles_blocks(H, G, D, max_new), seqs, splits), dim3(32 * TP_WARPS), tp_smem_bytes(D, CL), s,
+                          (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, page_table, seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out,
+                          max_pages, n_pages, window, keep_first, scale, cap, scratch, splits);
             if (e != cudaSuccess) {
                 bc_set_error("talk_tiles: %s", cudaGetErrorString(e));
                 return (int)e;

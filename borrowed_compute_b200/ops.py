@@ -1405,14 +1405,20 @@ def talk_tiles(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pa
           _ptr(row_slot if splits > 1 else None), _c_int(q.shape[0]), _stream())
 
 
-def talk_tiles_splits(seqs: int, heads: int, reach: int, window: int, keep_first: int) -> int:
+def talk_tiles_blocks(heads: int, kv_heads: int, head_dim: int, max_new: int) -> int:
+    """Blocks that a sequence with up to ``max_new`` new rows takes in talk_tiles, before its positions are shared out."""
+    return int(_fn("bc_talk_tiles_blocks")(_c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(max_new)))
+
+
+def talk_tiles_splits(seqs: int, heads: int, reach: int, window: int, keep_first: int, blocks_a_seq: Optional[int] = None) -> int:
     """Splits of the positions a row sees (tiles of 32) for steps of few rows a sequence, so that the blocks fill the machine ONCE (a
     block takes most of a multiprocessor's shared memory, and more than sixteen heads take two or four blocks a sequence): never
-    more than there are tiles (``reach``: a bound on the positions any row reaches; a window bounds them further)."""
+    more than there are tiles (``reach``: a bound on the positions any row reaches; a window bounds them further).
+    ``blocks_a_seq``: what talk_tiles_blocks says (default: by the heads alone)."""
     tiles = -(-max(reach, 1) // 32)
     if window > 0:
         tiles = min(tiles, -(-keep_first // 32) + (window + 30) // 32 + 1)
-    blocks = max(seqs, 1) * (1 if heads <= 16 else 2 if heads <= 32 else 4)
+    blocks = max(seqs, 1) * (blocks_a_seq or (1 if heads <= 16 else 2 if heads <= 32 else 4))
     return max(1, min(tiles, sm_count() // blocks, 64))
 
 

@@ -99,7 +99,8 @@ class TalkingAttention(Mixer):
         att = torch.empty((rows, H * D), dtype=x.dtype, device=dev)
         if self.path(ctx, x.dtype) == "tiles":
             # Few rows a sequence (single rows above all) leave few blocks: the positions are then shared out over several.
-            splits = ops.talk_tiles_splits(ctx.seqs, H, ctx.max_total, self.window, self.keep_first) if ctx.max_new <= 16 else 1
+            splits = ops.talk_tiles_splits(ctx.seqs, H, ctx.max_total, self.window, self.keep_first,
+                                           ops.talk_tiles_blocks(H, G, D, ctx.max_new)) if ctx.max_new <= 16 else 1
             ops.talk_tiles(q, mem.k_pages, mem.v_pages, mem.page_table, ctx.seq_rows, ctx.seq_slot, ctx.seq_start, gate, self.temp, self.talk, att,
                            ctx.seqs, ctx.max_new, H, G, D, self.window, self.keep_first, self.scale, self.softcap, splits=splits,
                            row_slot=ctx.row_slot)

@@ -1,5 +1,5 @@
-"""Talking attention where the mix goes by rows (sixteen heads a block, 32 KB of keys a tile), and the kernel that prepares its operands a
-warp a head: rows and positions around their tiles of 16 and 32, windows and kept first positions around a tile's borders, pages that
+"""Talking attention where the mix goes by rows (sixteen heads of sixteen rows or thirty-two of eight a block), and the kernel that prepares its operands a
+warp a head: rows and positions around their tiles of 8, 16 and 32, windows and kept first positions around a tile's borders, pages that
 are not held, numbers that are none in positions of no sequence, positions shared out over several blocks.
 
 Tolerance of the attention: a weight is rounded to bf16 (2^-9 of it) before it meets the values and the result once more, so a result is
