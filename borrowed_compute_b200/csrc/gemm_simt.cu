@@ -280,9 +280,10 @@ __global__ void __launch_bounds__(128) gemm_simt_short_kernel(const T* X, const 
 
 template <class T, int EPI, bool VEC>
 static cudaError_t launch_vec(const T* X, const T* W, T* oa, float* of, int M, int N, int K, float a, float b, int cols, cudaStream_t s) {
-    // Short sums of few outputs: a tile of 64 x 128 a block would be four blocks or fewer an eighth of the device, each a chain of K / 16 turns
-    // (4 rows of K 64 to 176: 8 to 10 us in tiles, 5 here; from 65,536 outputs of K 512 on the tiles fill 8 SMs or more and read W a fraction as often).
-    if (K <= SHORT_K && (long long)M * N <= 1 << 16) {
+    // Short sums of few outputs.  Up to 262,144 of them the short kernel is the quicker or as quick: 128 x 1,024 at K 512 33 against 43 us in tiles,
+    // 512 x 256 at K 176 16 against 20, 2,048 x 128 at K 64 10 against 12 (caches cold); past that the tiles: 300 x 1,000 at K 256 27 against 29,
+    // 1,000 x 1,000 at K 64 12 against 14.
+    if (K <= SHORT_K && (long long)M * N <= 1 << 18) {
         const int k_row = (K + 7) / 8 * 8 + 4;                    // an odd number of 16-byte pieces
         const size_t smem = (size_t)((EPI == EPI_SWIGLU ? 64 : 32) + 16) * k_row * sizeof(float);      // at most 165 KB
         if (smem > 48 * 1024) {                                   // asked for at every such call: the attribute belongs to the current device
@@ -293,8 +294,11 @@ static cudaError_t launch_vec(const T* X, const T* W, T* oa, float* of, int M, i
     }
     const int splits = simt_splits(EPI == EPI_SWIGLU ? 2 * N : N, K), piece = simt_piece(K, splits);
     const int out_cols = EPI == EPI_SWIGLU ? SIMT_COLS / 2 : SIMT_COLS;
-    const int bm = M <= 32 ? 16 : 64;
-    const dim3 grid((N + out_cols - 1) / out_cols, (M + bm - 1) / bm, splits);
+    // Tiles of 16 rows for few rows, and as long as these are 8/3 blocks an SM at most: 48 rows of [2048, 8192] (384 blocks) 90 us against 125 in tiles of
+    // 64, 128 rows of [512, 1024] (64 blocks) 37 against 53; 96 rows of [2048, 2048] (384) 49 in either; 64 rows of [8192, 2048] (512) 110 against 92.
+    const int cols_grid = (N + out_cols - 1) / out_cols;
+    const int bm = M <= 32 || (long long)cols_grid * splits * ((M + 15) / 16) * 3 <= 8 * bc_sm_count() ? 16 : 64;
+    const dim3 grid(cols_grid, (M + bm - 1) / bm, splits);
     auto go = [&](auto kernel) {
         return splits > 1 ? bc_launch_clustered(kernel, grid, dim3(128), 0, s, dim3(1, 1, splits), X, W, oa, of, M, N, K, piece, a, b, cols)
                           : bc_launch(kernel, grid, dim3(128), 0, s, X, W, oa, of, M, N, K, piece, a, b, cols);

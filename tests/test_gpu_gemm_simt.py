@@ -14,10 +14,10 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [
-    (1, 1, 1), (5, 33, 7), (17, 31, 144), (16, 64, 176), (128, 512, 512), (3, 70, 511),        # short sums; 128 x 512 outputs are the most they take
-    (129, 512, 512), (33, 2050, 40),                                                          # one more, in tiles
+    (1, 1, 1), (5, 33, 7), (17, 31, 144), (16, 64, 176), (128, 512, 512), (3, 70, 511), (512, 512, 512), (2048, 128, 64),   # short sums; 262,144 outputs are the most they take
+    (513, 512, 512), (129, 2050, 40),                                                         # one more, in tiles
     (1, 40, 1030), (32, 129, 1030), (33, 129, 1030), (65, 64, 2051), (70, 127, 4100),         # two, four and eight pieces
-    (300, 130, 1024)])
+    (300, 130, 1024), (48, 2048, 2048), (96, 2048, 2048), (128, 512, 1024)])
 def test_products_around_the_edges_of_their_kernels(dtype, M, N, K):
     from borrowed_compute_b200 import ops
 
@@ -44,7 +44,7 @@ def test_products_around_the_edges_of_their_kernels(dtype, M, N, K):
     assert ((glu.double() - act * up).abs() <= 1.1 * bound[:, :N] * up.abs() + bound[:, N:] * act.abs() + bound[:, :N] * bound[:, N:]
             + unit * (act * up).abs() + 1e-30).all()
     # A row alone, and a few of them, give the bits that they give among all.
-    for rows in (slice(M - 1, M), slice(0, min(M, 20))):
+    for rows in (slice(M - 1, M), slice(0, min(M, 20)), slice(0, min(M, 60))):
         few = torch.empty((rows.stop - rows.start, N), device="cuda")
         ops.gemm_simt(x[rows].contiguous(), wn, few, ops.EPI_STORE_F32)
         assert torch.equal(few, out[rows])
