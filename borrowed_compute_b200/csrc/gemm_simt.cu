@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128) gemm_simt_kernel(const T* X, const T* __r
     float *As = tiles, *Bs = tiles + 2 * BK * A_ROW;
     pdl_launch_dependents();
     pdl_wait();
-    PDL_FRESH(X); PDL_FRESH(out_act); PDL_FRESH(out_f32);
+    PDL_FRESH(X); PDL_FRESH(W); PDL_FRESH(out_act); PDL_FRESH(out_f32);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * (EPI == EPI_SWIGLU ? HALF_N : SIMT_COLS);
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int k_begin = blockIdx.z * piece, k_end = min(K, k_begin + piece);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128) gemm_simt_kernel(const T* X, const T* __r
 }
 
 // Short K (at most 512) and few outputs, where a launch is all latency: a lane a weight row, a warp four rows of X.  All of the block's weights
-// and rows are asked for at once, into shared memory (the weights before the wait for the kernel before), and summed up from there; what
+// and rows are asked for at once, into shared memory, and summed up from there; what
 // the result is added to is asked for with them.  (A whole 64 x 64 tile a block behind two barriers every sixteen k: 8 to 10 us a launch at
 // K 64 to 176; straight from global memory 8; now 4.6 to 5.)
 #define SHORT_K 512
@@ -234,10 +234,11 @@ __global__ void __launch_bounds__(128) gemm_simt_short_kernel(const T* X, const 
             }
         }
     };
+    // The weights too are read behind the wait: a caller's w may be what the kernel before has just written.
+    pdl_wait();
+    PDL_FRESH(X); PDL_FRESH(W); PDL_FRESH(out_act); PDL_FRESH(out_f32);
     stage(ws, W, n0, 32, N);
     if (EPI == EPI_SWIGLU) stage(ws + 32 * k_row, W + (size_t)N * K, n0, 32, N);
-    pdl_wait();
-    PDL_FRESH(X); PDL_FRESH(out_act); PDL_FRESH(out_f32);
     stage(xs, X, r0, min(16, M - r0), M);
     const int n = n0 + lane, m0 = r0 + 4 * warp;
     float old[4] = {};

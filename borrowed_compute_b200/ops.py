@@ -346,7 +346,8 @@ def _act_numbers(who: str, epilogue: int, act: Optional[Tuple[float, float]], co
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, act: Optional[Tuple[float, float]] = None,
               cols: Optional[int] = None) -> None:
-    """out = x @ w.T on the CUDA cores with float accumulation in ascending k.
+    """out = x @ w.T on the CUDA cores with float accumulation, k ascending in one piece or in up to eight that are added in order.
+    Both operands are read after the kernels before this launch have ended.
     EPI_STORE: out in x's type; EPI_STORE_F32: float32; EPI_ADD_F32: out += (float32);
     EPI_SWIGLU: w stacks gate rows on up rows, out[:, j] = silu(g_j) * u_j in x's type;
     EPI_RELU2: out = max(sum, 0)^2 in x's type, squared in float and rounded once;

@@ -60,3 +60,21 @@ def test_an_infinity_stays_in_its_row():
         ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
         assert torch.isinf(out[2]).all() and torch.isnan(out[3]).all()
         assert (out[[0, 1, 4]] == K).all() and np.isfinite(out[4:].cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("epilogue", ["store", "glu"])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (16, 512, 512), (70, 130, 520)])
+def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K, epilogue):
+    """Kernels may start while the one before still runs; no operand is read before that one's end.  Sums of ones: exact."""
+    from borrowed_compute_b200 import ops
+
+    glu = epilogue == "glu"
+    x, w = torch.full((M, K), 2.0 ** -10, device="cuda"), torch.ones((2 * N if glu else N, K), device="cuda")
+    outs = [torch.empty((M, N), device="cuda") for _ in range(12)]
+    for out in outs:
+        ops.scale_scores(w, 2.0)
+        ops.gemm_simt(x, w, out, ops.EPI_SWIGLU if glu else ops.EPI_STORE_F32)
+    for i, out in enumerate(outs):
+        s = K * 2.0 ** (i + 1 - 10)
+        want = s * s / (1.0 + np.exp(-s)) if glu else s
+        assert ((out.double() - want).abs() <= (2.0 ** -20 if glu else 0.0) * want).all(), i
