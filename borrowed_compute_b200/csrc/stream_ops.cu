@@ -41,38 +41,52 @@ extern "C" int bc_scale_f32(float* scores, long long n, float factor, cudaStream
     BC_LAUNCH_STATUS();
 }
 
-// A block takes 1,024 neighbouring columns of eight rows; four columns a thread, sixteen bytes a move, the bias read once (an element a thread
-// and a 64-bit remainder each: 30 us for 2,048 x 4,096 floats, against 10 us of bytes).
+// A block's 256 threads lie `across` (a power of two) to a row's columns, V columns a thread, and take BIAS_ROWS rows each, all asked for together;
+// the bias is read once.  V = 4 (sixteen bytes a move) where the rows allow it.  (An element a thread and a 64-bit remainder each: 30 us
+// for 2,048 x 4,096 floats, against 10 us of bytes; now 13.  All 256 threads along one row, four columns each whatever the alignment, left narrow rows
+// with few threads and let unaligned ones touch every line four times: with the launch 63 us for 500,000 x 16 and 33 for 2,048 x 1,023, an
+// element a thread 41 and 22, now 23 and 17.)
 #define BIAS_ROWS 8
-__global__ void __launch_bounds__(256) add_bias_kernel(float* x, const float* __restrict__ b, int rows, int E) {
+template <int V>
+__global__ void __launch_bounds__(256) add_bias_kernel(float* x, const float* __restrict__ b, int rows, int E, int across, int col_blocks) {
     pdl_launch_dependents_if_resident();
     pdl_wait();
-    PDL_FRESH(x);
-    const int c = blockIdx.x * 1024 + 4 * threadIdx.x, row0 = blockIdx.y * BIAS_ROWS;
+    PDL_FRESH(x); PDL_FRESH(b);
+    const int down = 256 / across, ty = threadIdx.x / across;
+    const unsigned row_block = blockIdx.x / col_blocks;
+    const long long c = (long long)(blockIdx.x - row_block * col_blocks) * across * V + V * (threadIdx.x % across), row0 = (long long)row_block * down * BIAS_ROWS + ty;
     if (c >= E) return;
-    if (E % 4 == 0 && ((uintptr_t)x | (uintptr_t)b) % 16 == 0) {
-        const float4 v = *reinterpret_cast<const float4*>(b + c);
-        float4 y[BIAS_ROWS];
+    float v[V], y[BIAS_ROWS][V];
+    auto load = [](const float* from, float* to) {
+        if constexpr (V == 4) {
+            const float4 u = *reinterpret_cast<const float4*>(from);
+            to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+        } else to[0] = *from;
+    };
+    load(b + c, v);
 #pragma unroll
-        for (int r = 0; r < BIAS_ROWS; r++)
-            if (row0 + r < rows) y[r] = *reinterpret_cast<const float4*>(x + (size_t)(row0 + r) * E + c);
+    for (int r = 0; r < BIAS_ROWS; r++)
+        if (row0 + r * down < rows) load(x + (size_t)(row0 + r * down) * E + c, y[r]);
 #pragma unroll
-        for (int r = 0; r < BIAS_ROWS; r++)
-            if (row0 + r < rows) *reinterpret_cast<float4*>(x + (size_t)(row0 + r) * E + c) = make_float4(y[r].x + v.x, y[r].y + v.y, y[r].z + v.z, y[r].w + v.w);
-        return;
-    }
-    for (int r = row0; r < min(rows, row0 + BIAS_ROWS); r++)
-        for (int e = 0; e < 4 && c + e < E; e++) x[(size_t)r * E + c + e] += b[c + e];
+    for (int r = 0; r < BIAS_ROWS; r++)
+        if (row0 + r * down < rows) {
+            float* to = x + (size_t)(row0 + r * down) * E + c;
+            if constexpr (V == 4) *reinterpret_cast<float4*>(to) = make_float4(y[r][0] + v[0], y[r][1] + v[1], y[r][2] + v[2], y[r][3] + v[3]);
+            else *to = y[r][0] + v[0];
+        }
 }
 
 // x: [rows, E] float; b: [E] float.
 extern "C" int bc_add_bias_f32(float* x, const float* b, int rows, int E, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && E > 0, "add_bias: bad sizes rows=%d E=%d", rows, E);
-    // More rows than a grid's second dimension holds go in turns.
-    for (int at = 0; at < rows; at += 65535 * BIAS_ROWS) {
-        const int n = rows - at < 65535 * BIAS_ROWS ? rows - at : 65535 * BIAS_ROWS;
-        bc_launch(add_bias_kernel, dim3((E + 1023) / 1024, (n + BIAS_ROWS - 1) / BIAS_ROWS), dim3(256), 0, s, x + (size_t)at * E, b, n, E);
-    }
+    if (rows == 0) return BC_OK;
+    const int V = E % 4 == 0 && ((uintptr_t)x | (uintptr_t)b) % 16 == 0 ? 4 : 1;
+    int across = 1;
+    while (across < 256 && across * V < E) across *= 2;
+    const long long rows_a_block = (long long)BIAS_ROWS * (256 / across), col_blocks = ((long long)E + across * V - 1) / (across * V);
+    const long long blocks = (rows + rows_a_block - 1) / rows_a_block * col_blocks;       // (a block for every 2,048 floats or so: memory ends long before a grid does)
+    BC_CHECK_ARG(blocks <= 2147483647ll, "add_bias: %d rows of %d are too many", rows, E);
+    bc_launch(V == 4 ? add_bias_kernel<4> : add_bias_kernel<1>, dim3((unsigned)blocks), dim3(256), 0, s, x, b, rows, E, across, (int)col_blocks);
     BC_LAUNCH_STATUS();
 }
 

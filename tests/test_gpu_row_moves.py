@@ -69,7 +69,8 @@ def test_gathered_pages(R, rot):
             assert (held == 0 or torch.equal(rows[:held], src[page, :held])) and (rows[held:] == 0).all(), p
 
 
-@pytest.mark.parametrize("rows,E", [(1, 1), (7, 3), (8, 4), (9, 1024), (17, 1028), (300, 4096), (5, 1027)])
+@pytest.mark.parametrize("rows,E", [(1, 1), (7, 3), (8, 4), (9, 1024), (17, 1028), (300, 4096), (5, 1027), (2049, 1), (3000, 5), (1025, 8), (70, 130), (3, 256), (2, 257),
+                                    (524299, 3)])
 def test_bias_added_to_rows(rows, E):
     from borrowed_compute_b200 import ops
 
@@ -81,3 +82,34 @@ def test_bias_added_to_rows(rows, E):
         ops.add_bias(mine, b)
         assert torch.equal(mine, x + b)
         assert (held[:shift] == 4.0).all() and (held[shift + x.numel():] == 4.0).all()
+
+
+def test_bias_added_to_as_many_rows_as_an_int_counts():
+    from borrowed_compute_b200 import ops
+
+    x = torch.zeros((2 ** 31 - 1, 1), device=DEV)
+    ops.add_bias(x, torch.ones(1, device=DEV))
+    low, high = torch.aminmax(x)
+    assert low == 1.0 and high == 1.0
+
+
+def test_bias_of_rows_that_no_tile_divides_is_added_as_fast_as_the_others():
+    """Narrow and unaligned rows take no longer than an element a thread takes (an elementwise product over the same bytes, three times over)."""
+    from borrowed_compute_b200 import ops
+
+    def micros(run):
+        times = []
+        for _ in range(12):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(10):
+                run()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end) * 100.0)
+        return sorted(times)[3]
+
+    for rows, E in ((500000, 16), (500000, 13), (20480, 1023)):
+        x, b = torch.zeros((rows, E), device=DEV), torch.ones(E, device=DEV)
+        mine, plain = micros(lambda: ops.add_bias(x, b)), micros(lambda: ops.scale_scores(x, 1.0))
+        assert mine <= 2.0 * plain, (rows, E, mine, plain)
