@@ -596,14 +596,9 @@ static int launch_as(const CUtensorMap& mk, const CUtensorMap& mv, const void* q
     constexpr int STAGE_BYTES = 64 * (D + DV) * 2;
     constexpr int MERGE_BYTES = (2 * 4 * 16 + 4 * 16 * DV + 16 * DV + 32) * 4;
     constexpr int SMEM = (AD_STAGES * STAGE_BYTES > MERGE_BYTES ? AD_STAGES * STAGE_BYTES : MERGE_BYTES) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<D, DV, TMA, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("attention_decode: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<attention_decode_kernel<D, DV, TMA, BIAS>>(SMEM); e != cudaSuccess) {
+        bc_set_error("attention_decode: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     dim3 grid(n_splits, G, rows);
     // Up to eight splits (the portable cluster size) exchange their results through
@@ -613,10 +608,13 @@ static int launch_as(const CUtensorMap& mk, const CUtensorMap& mv, const void* q
     if (n_splits == 16 && fr.allow_cluster && g_ad_cluster16 && (long long)rows * G * 16 <= bc_sm_count()) {
         // One cluster of sixteen, where every block has an SM to itself (with more blocks than SMs two clusters of
         // eight place better: measured).  Sixteen blocks a cluster is more than every device must offer: asked for
-        // once, and taken only if the device can place one.
-        static int sixteen = -1;
-        if (sixteen < 0) {
-            sixteen = 0;
+        // once a device, and taken only if it can place one.
+        static std::atomic<int> placed[BC_KNOWN_DEVICES];      // 0: not asked yet; 1: no; 2: yes
+        int device = 0;
+        const bool known = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < BC_KNOWN_DEVICES;
+        int sixteen = known ? placed[device].load() : 1;
+        if (sixteen == 0) {
+            sixteen = 1;
             if (cudaFuncSetAttribute(attention_decode_kernel<D, DV, TMA, BIAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(16, 1, 1);
@@ -629,11 +627,12 @@ static int launch_as(const CUtensorMap& mk, const CUtensorMap& mv, const void* q
                 cfg.attrs = attr;
                 cfg.numAttrs = 1;
                 int fit = 0;
-                if (cudaOccupancyMaxActiveClusters(&fit, attention_decode_kernel<D, DV, TMA, BIAS>, &cfg) == cudaSuccess && fit > 0) sixteen = 1;
+                if (cudaOccupancyMaxActiveClusters(&fit, attention_decode_kernel<D, DV, TMA, BIAS>, &cfg) == cudaSuccess && fit > 0) sixteen = 2;
             }
             (void)cudaGetLastError();
+            placed[device].store(sixteen);
         }
-        if (sixteen == 1) csize = 16;
+        if (sixteen == 2) csize = 16;
     }
     if (n_splits > 8 && csize < n_splits && !(scratch && counters)) csize = 1;
     const bool clustered = n_splits > 1 && fr.allow_cluster && csize > 1;
@@ -776,28 +775,19 @@ static __device__ __align__(256) unsigned char g_static_scratch[BC_STATIC_SCRATC
 
 #define BC_STATIC_MAX_DEVICES 64
 static void* g_static_scratch_addr[BC_STATIC_MAX_DEVICES];        // per device, null until looked up
-static unsigned g_static_configured[BC_STATIC_MAX_DEVICES];       // per device, bit D / 16: that head size's kernel is set up
 static std::mutex g_static_mutex;
 
 template <int D>
 static int launch_static(float* scratch, int* counters, const void* q, int q_stride, const void* k_cache, const void* v_cache,
                          const int* page_table, const int* row_pos, const int* row_slot, void* out, int rows, int H, int G, int max_pages,
-                         int n_pages, int window, float scale, int n_splits, int device, cudaStream_t s) {
+                         int n_pages, int window, float scale, int n_splits, cudaStream_t s) {
     constexpr int TILE_BYTES = 64 * D * 2;
     constexpr int MERGE_BYTES = (2 * 4 * 16 + 4 * 16 * D + 16 * D + 32) * 4;
     constexpr int SMEM = (AD_STAGES * 2 * TILE_BYTES > MERGE_BYTES ? AD_STAGES * 2 * TILE_BYTES : MERGE_BYTES) + 1024;
     const CUtensorMap none = {};   // this entry point fetches pages by cp.async: it needs no tensor maps
-    {
-        // First call for this head size on this device: let the kernel use the shared memory it needs.
-        std::lock_guard<std::mutex> lock(g_static_mutex);
-        if (!(g_static_configured[device] & (1u << (D / 16)))) {
-            cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<D, D, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-            if (e != cudaSuccess) {
-                bc_set_error("attention_decode_static: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-                return (int)e;
-            }
-            g_static_configured[device] |= 1u << (D / 16);
-        }
+    if (cudaError_t e = bc_allow_shared<attention_decode_kernel<D, D, false, false>>(SMEM); e != cudaSuccess) {
+        bc_set_error("attention_decode_static: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     bc_launch(attention_decode_kernel<D, D, false, false>, dim3(n_splits, G, rows), dim3(AD_THREADS), (size_t)SMEM, s, none, none, (const bf16*)q, q_stride,
               (const bf16*)k_cache, (const bf16*)v_cache, page_table, row_pos, row_slot, (bf16*)out, scratch, counters, H, G, max_pages,
@@ -857,7 +847,7 @@ extern "C" int bc_attention_decode_static_bf16(const void* q, int q_stride, cons
         }
     }
 #define ADS_CASE(DD) \
-    case DD: return launch_static<DD>(scratch, counters, q, q_stride, k_cache, v_cache, page_table, row_pos, row_slot, out, rows, heads, kv_heads, max_pages, n_pages, window, scale, n_splits, device, stream);
+    case DD: return launch_static<DD>(scratch, counters, q, q_stride, k_cache, v_cache, page_table, row_pos, row_slot, out, rows, heads, kv_heads, max_pages, n_pages, window, scale, n_splits, stream);
     switch (head_dim) {
         ADS_CASE(16) ADS_CASE(32) ADS_CASE(48) ADS_CASE(64) ADS_CASE(80) ADS_CASE(96) ADS_CASE(112) ADS_CASE(128)
     }

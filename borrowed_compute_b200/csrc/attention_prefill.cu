@@ -258,14 +258,9 @@ static int launch(const void* q, int q_stride, const void* k_cache, const void* 
                   const int* seq_slot, const int* seq_start, void* out, int seqs, int max_new, int H, int G, int max_pages, int n_pages,
                   int window, int chunk, float scale, int sink, const float* sink_values, float out_scale, const float* bias, int bias_reach, cudaStream_t s) {
     constexpr int SMEM = AP_STAGES * 64 * (D + DV) * 2;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("attention_prefill: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<attention_prefill_kernel<D, DV>>(SMEM); e != cudaSuccess) {
+        bc_set_error("attention_prefill: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     const int tokens_per_tile = AP_ROWS / (H / G);
     dim3 grid(G, (max_new + tokens_per_tile - 1) / tokens_per_tile, seqs);

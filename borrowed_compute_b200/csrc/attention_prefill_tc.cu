@@ -506,14 +506,9 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
     constexpr int STAGES = APT_STAGES(D, NT), PB = APT_PB(D, NT);
     constexpr int SMEM = DB * NT * APT_ROWS * 128 + NT * PB * APT_ROWS * 128 + STAGES * 2 * DB * BC_PAGE * 128 + 1024;
     static_assert(SMEM <= APT_SMEM_LIMIT, "the ring does not fit");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<D, DV, NT, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("attention_prefill_tc: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<attention_prefill_tc_kernel<D, DV, NT, BIAS>>(SMEM); e != cudaSuccess) {
+        bc_set_error("attention_prefill_tc: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     const int tokens_per_block = NT * APT_ROWS / (H / G);
     dim3 grid(G, (max_new + tokens_per_block - 1) / tokens_per_block, seqs);

@@ -256,12 +256,7 @@ template <int DL, bool DELTA>
 static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, const float* v, int v_stride, float* state, const int* seq_rows, const int* seq_slot,
                                      float* out, int seqs, int H, int N, int P, int n_slots, int write_state, cudaStream_t s) {
     constexpr size_t SMEM = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<DL, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    if (cudaError_t e = bc_allow_shared<chunk_scan_kernel<DL, DELTA>>(SMEM); e != cudaSuccess) return e;
     return bc_launch(chunk_scan_kernel<DL, DELTA>, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H,
                      N, P, n_slots, write_state);
 }

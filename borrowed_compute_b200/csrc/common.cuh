@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_limits.h"
+
 // Every exported launcher returns 0 on success, a cudaError_t if the launch failed, or one
 // of the library's own codes below.  bc_last_error() gives the text.
 #define BC_OK 0
@@ -109,6 +111,16 @@ static inline cudaError_t bc_launch_clustered(void (*kernel)(KArgs...), dim3 gri
     cfg.attrs = attr;
     cfg.numAttrs = g_bc_pdl ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Lets Kernel use `bytes` of dynamic shared memory on the current device, to which the attribute belongs.
+template <auto Kernel>
+static inline cudaError_t bc_allow_shared(size_t bytes) {
+    static BcDeviceLimits limits;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)limits.at_least(device, (int)bytes, [](int value) { return (int)cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, value); });
 }
 
 __device__ __forceinline__ float to_f32(float v) { return v; }

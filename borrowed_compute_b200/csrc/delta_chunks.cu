@@ -290,14 +290,9 @@ extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t,
                  "delta_chunked: rows, state and scratch must start on 16-byte borders");
     const long long capacity = pack_floats / ((long long)H * chunk_pack_floats(DLC_D, true));
     BC_CHECK_ARG(chunk_fits(capacity, rows, seqs, write_state), "delta_chunked: scratch of %lld floats is too small", pack_floats);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(delta_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DLC_SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<delta_chunks_kernel>(DLC_SMEM); e != cudaSuccess) {
+        bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
+        return (int)e;
     }
     cudaError_t e = bc_launch(delta_decay_kernel, dim3((H * D + DLC_COLS - 1) / DLC_COLS, (rows + DLC_ROWS - 1) / DLC_ROWS), dim3(256), 0, s, proj, stride, 5 * H * D, w2t,
                               w0, decay, rows, H * D, inner, decay_scale);

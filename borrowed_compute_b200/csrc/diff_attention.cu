@@ -475,14 +475,9 @@ static int tiles_launch(const void* q, const void* k_cache, const void* v_cache,
     constexpr int STAGES = WM == 1 && 3 * STAGE <= 110 * 1024 ? 3 : 2;      // few rows: more bytes on their way
     constexpr int SMEM = STAGES * STAGE;
     static_assert(SMEM >= WM * 32 * (VP / 8) * 4 * 4, "the maps meet in the page buffers");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(diff_tiles_kernel<DP, VP, WM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("diff_tiles: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<diff_tiles_kernel<DP, VP, WM, STAGES>>(SMEM); e != cudaSuccess) {
+        bc_set_error("diff_tiles: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     const int tokens_per_tile = 16 * WM / (H / G);
     dim3 grid(G, (max_new + tokens_per_tile - 1) / tokens_per_tile, seqs * splits);

@@ -364,14 +364,9 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
                   float eps, float factor, cudaStream_t s) {
     constexpr int SMEM = DT_Q_BYTES(D) + DT_STAGES(D, DV) * DT_STAGE_BYTES(D, DV) + 1024;
     static_assert(SMEM + 4096 <= DT_SMEM_LIMIT + 1024, "the ring does not fit");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(diff_attention_tc_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) {
-            bc_set_error("diff_attention_tc: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<diff_attention_tc_kernel<D, DV>>(SMEM); e != cudaSuccess) {
+        bc_set_error("diff_attention_tc: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));
+        return (int)e;
     }
     const int tokens = DT_ROWS / (H / G);
     dim3 grid(G, (max_new + tokens - 1) / tokens, seqs);

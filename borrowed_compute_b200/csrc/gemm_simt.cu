@@ -287,10 +287,8 @@ static cudaError_t launch_vec(const T* X, const T* W, T* oa, float* of, int M, i
     if (K <= SHORT_K && (long long)M * N <= 1 << 18) {
         const int k_row = (K + 7) / 8 * 8 + 4;                    // an odd number of 16-byte pieces
         const size_t smem = (size_t)((EPI == EPI_SWIGLU ? 64 : 32) + 16) * k_row * sizeof(float);      // at most 165 KB
-        if (smem > 48 * 1024) {                                   // asked for at every such call: the attribute belongs to the current device
-            cudaError_t e = cudaFuncSetAttribute(gemm_simt_short_kernel<T, EPI, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 168 * 1024);
-            if (e != cudaSuccess) return e;
-        }
+        if (smem > 48 * 1024)
+            if (cudaError_t e = bc_allow_shared<gemm_simt_short_kernel<T, EPI, VEC>>(168 * 1024); e != cudaSuccess) return e;
         return bc_launch(gemm_simt_short_kernel<T, EPI, VEC>, dim3((N + 31) / 32, (M + 15) / 16), dim3(128), smem, s, X, W, oa, of, M, N, K, k_row, a, b, cols);
     }
     const int splits = simt_splits(EPI == EPI_SWIGLU ? 2 * N : N, K), piece = simt_piece(K, splits);

@@ -733,14 +733,9 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, TcParams p, int 
     if (stages > p.k_iters_per_split) stages = p.k_iters_per_split < 2 ? 2 : p.k_iters_per_split;
     p.stages = stages;
     const int smem = stages * STAGE_BYTES + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, EPI, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
-        if (e != cudaSuccess) {
-            bc_set_error("gemm_tc: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<gemm_tc_kernel<BN, EPI, STACK>>(TC_SMEM_LIMIT); e != cudaSuccess) {
+        bc_set_error("gemm_tc: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
+        return (int)e;
     }
     constexpr int ROWS = TWO_TILES ? 2 * TC_BM : TC_BM;   // output rows a block
     p.n_tiles = (p.N + ROWS - 1) / ROWS;
@@ -779,20 +774,11 @@ static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcParams p,
     p.clustered = 0;
     p.k_iters_per_split = k_iters;
     const int smem = stages * STAGE_BYTES + 1024;
-    static bool configured = false;
-    static int pairs_on_device = 0;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
-        if (e != cudaSuccess) {
-            bc_set_error("gemm_tc: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
-            return (int)e;
-        }
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        pairs_on_device = sms / 2 > 0 ? sms / 2 : 1;
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<gemm_tc_pair_kernel<EPI>>(TC_SMEM_LIMIT); e != cudaSuccess) {
+        bc_set_error("gemm_tc: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
+        return (int)e;
     }
+    const int pairs_on_device = bc_sm_count() / 2 > 0 ? bc_sm_count() / 2 : 1;
     const int rows = EPI == EPI_SWIGLU ? 2 * TC_BM : 4 * TC_BM;   // outputs a pair
     p.n_tiles = (p.N + rows - 1) / rows;
     // Tokens a tile: whole tiles are lost when the tile count is just over a multiple of the
@@ -1178,14 +1164,9 @@ static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupP
     if (stream && stages > half_stages) stages = half_stages;
     p.stages = stages;
     const int smem = stages * STAGE_BYTES + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_grouped_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT);
-        if (e != cudaSuccess) {
-            bc_set_error("gemm_tc_grouped: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<gemm_tc_grouped_kernel<BN, EPI>>(TC_SMEM_LIMIT); e != cudaSuccess) {
+        bc_set_error("gemm_tc_grouped: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
+        return (int)e;
     }
     const long long pieces = (long long)((p.N + TC_BM - 1) / TC_BM) * max_tiles;      // at most: the table says how many
     const int blocks = stream || pieces < bc_sm_count() ? (int)pieces : bc_sm_count();

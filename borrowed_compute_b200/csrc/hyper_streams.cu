@@ -154,11 +154,7 @@ static int hyper_step(float* x, float* y, const float* scale, const float* mix, 
     cudaError_t e = cudaSuccess;
 #define HS_GO(SS, V)                                                                                                                          \
     do {                                                                                                                                      \
-        static bool configured = false;                                                                                                       \
-        if (!configured) {                                                                                                                    \
-            e = cudaFuncSetAttribute(hyper_step_kernel<SS, V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4);                    \
-            configured = e == cudaSuccess;                                                                                                    \
-        }                                                                                                                                     \
+        e = bc_allow_shared<hyper_step_kernel<SS, V, T>>(32768 * 4);                                                                          \
         if (e == cudaSuccess)                                                                                                                 \
             e = bc_launch(hyper_step_kernel<SS, V, T>, dim3(rows), dim3(hs_threads(E)), smem, s, x, y, scale, mix, out_w, in_w, w, gather, (T*)h, S, \
                           E, x_rows, eps);                                                                                                    \

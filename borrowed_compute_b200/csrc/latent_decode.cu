@@ -336,14 +336,9 @@ static int decode_launch(const void* a, const void* c_pages, const void* r_pages
                          float* scratch, int rows, int H, int R, int ROT, int max_pages, int n_pages, int window, float scale, int splits, const float* sink,
                          cudaStream_t s) {
     const size_t smem = ld_smem_bytes(R, ROT);
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<MAXP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            bc_set_error("latent_decode: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = smem;
+    if (cudaError_t e = bc_allow_shared<latent_decode_kernel<MAXP>>(smem); e != cudaSuccess) {
+        bc_set_error("latent_decode: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
+        return (int)e;
     }
     const int groups = (H + LD_HEADS - 1) / LD_HEADS;
     cudaError_t e = bc_launch(latent_decode_kernel<MAXP>, dim3(rows, groups, splits), dim3(LD_THREADS), smem, s, (const bf16*)a, (const bf16*)c_pages,

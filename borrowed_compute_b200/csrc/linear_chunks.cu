@@ -127,14 +127,9 @@ template <int D>
 static int gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_at, int inner_at, const float* w2t, const float* b, int rank, float inv_tau, float f,
                        float* pack, long long pack_floats, float* state, const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int H, int N, int P,
                        int n_slots, int write_state, cudaStream_t s) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gla_chunks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        if (e != cudaSuccess) {
-            bc_set_error("gla_chunked: %s", cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = true;
+    if (cudaError_t e = bc_allow_shared<gla_chunks_kernel<D>>(64 * 1024); e != cudaSuccess) {
+        bc_set_error("gla_chunked: %s", cudaGetErrorString(e));
+        return (int)e;
     }
     const cudaError_t e = chunk_step(
         pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, max_new,

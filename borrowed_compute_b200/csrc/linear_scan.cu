@@ -187,12 +187,7 @@ static cudaError_t scan_launch_one(dim3 grid, size_t smem, cudaStream_t s, const
                                    int k_rep, const float* v, int v_stride, const float* decay, int d_stride, const float* kscale, int c_stride,
                                    const float* skip, float out_scale, float* state, const int* seq_rows, const int* seq_slot, float* out, int H,
                                    int N, int P, int R, int n_slots, int write_state) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(linear_scan_kernel<NJ, VD, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    if (cudaError_t e = bc_allow_shared<linear_scan_kernel<NJ, VD, VEC>>(100 * 1024); e != cudaSuccess) return e;
     return bc_launch(linear_scan_kernel<NJ, VD, VEC>, grid, dim3(128), smem, s, q, q_stride, q_rep, k, k_stride, k_rep, v, v_stride, decay, d_stride,
                      kscale, c_stride, skip, out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state);
 }

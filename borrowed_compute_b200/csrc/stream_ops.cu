@@ -43,7 +43,7 @@ extern "C" int bc_scale_f32(float* scores, long long n, float factor, cudaStream
 
 // A block's 256 threads lie `across` (a power of two) to a row's columns, V columns a thread, and take BIAS_ROWS rows each, all asked for together;
 // the bias is read once.  V = 4 (sixteen bytes a move) where the rows allow it.  (An element a thread and a 64-bit remainder each: 30 us
-// for 2,048 x 4,096 floats, against 10 us of bytes; now 13.  All 256 threads along one row, four columns each whatever the alignment, left narrow rows
+// for 2,048 x 4,096 floats, 45 cold with the launch; now 23 so.  All 256 threads along one row, four columns each whatever the alignment, left narrow rows
 // with few threads and let unaligned ones touch every line four times: with the launch 63 us for 500,000 x 16 and 33 for 2,048 x 1,023, an
 // element a thread 41 and 22, now 23 and 17.)
 #define BIAS_ROWS 8

@@ -937,28 +937,19 @@ static int tiles_go(const void* q, const void* k_cache, const void* v_cache, con
                     int rows, cudaStream_t s) {
     const int stages = tt_smem_bytes(H, G, D, 2, CL) <= 216 * 1024 ? 2 : 1;
     const size_t smem = tt_smem_bytes(H, G, D, stages, CL);
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(talk_tiles_kernel<D, HPW, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            bc_set_error("talk_tiles: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = smem;
+    if (cudaError_t e = bc_allow_shared<talk_tiles_kernel<D, HPW, CL>>(smem); e != cudaSuccess) {
+        bc_set_error("talk_tiles: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
+        return (int)e;
     }
     const int warps = (H / CL + HPW - 1) / HPW;
     const dim3 grid(((max_new + TT_ROWS - 1) / TT_ROWS) * CL, seqs, splits);
     cudaError_t e;
     if constexpr (HPW == 1 && CL <= 2 && (D == 64 || D == 128)) {
         if (tp_takes(H, G, D)) {
-            static bool raised = false;
-            if (!raised) {
-                e = cudaFuncSetAttribute(talk_by_rows_kernel<D, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(D, CL));
-                if (e != cudaSuccess) {
-                    bc_set_error("talk_tiles: cannot set shared memory: %s", cudaGetErrorString(e));
-                    return (int)e;
-                }
-                raised = true;
+            e = bc_allow_shared<talk_by_rows_kernel<D, CL>>(tp_smem_bytes(D, CL));
+            if (e != cudaSuccess) {
+                bc_set_error("talk_tiles: cannot set shared memory: %s", cudaGetErrorString(e));
+                return (int)e;
             }
             e = bc_launch(talk_by_rows_kernel<D, CL>, dim3(bc_talk_tiles_blocks(H, G, D, max_new), seqs, splits), dim3(32 * TP_WARPS), tp_smem_bytes(D, CL), s,
                           (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, page_table, seq_rows, seq_slot, seq_start, gate, temp, talk, (bf16*)out,
@@ -1070,14 +1061,9 @@ static int rows_go(const void* q, const void* k_cache, const void* v_cache, cons
                    int window, int keep_first, float scale, float cap, cudaStream_t s) {
     const int warps = (H + HPW - 1) / HPW;
     const size_t smem = ((size_t)H * D + (size_t)H * 32 + (size_t)H * H) * sizeof(float);
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(talk_rows_kernel<T, NJ, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            bc_set_error("talk_rows: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
-            return (int)e;
-        }
-        configured = smem;
+    if (cudaError_t e = bc_allow_shared<talk_rows_kernel<T, NJ, HPW>>(smem); e != cudaSuccess) {
+        bc_set_error("talk_rows: cannot set shared memory to %zu: %s", smem, cudaGetErrorString(e));
+        return (int)e;
     }
     bc_launch(talk_rows_kernel<T, NJ, HPW>, dim3(rows), dim3(32 * warps), smem, s, (const T*)q, (const T*)k_cache, (const T*)v_cache, page_table, row_pos,
               row_slot, gate, temp, talk, (T*)out, H, G, D, max_pages, n_pages, window, keep_first, scale, cap);
