@@ -28,7 +28,7 @@ NVCC_FLAGS = ARCH_FLAGS + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPI
 # More flags for a build of one's own (say -DBC_TC_TRACE for time stamps inside the product kernels); such a build
 # has another stamp than the plain one, so give it a folder of its own with BC_B200_BUILD_DIR.
 NVCC_FLAGS += os.environ.get("BC_B200_NVCC_EXTRA", "").split()
-ABI_VERSION = 1
+ABI_VERSION = 2
 
 _lib: Optional[ctypes.CDLL] = None
 

@@ -21,19 +21,50 @@
 #define CHUNK_G 20            // floats a row of G: sixteen and a gap, so that the rows that eight threads read start in different banks
 
 __host__ __device__ constexpr int chunk_pack_floats(int D, bool delta) { return (delta ? 4 : 2) * CHUNK * D + CHUNK * CHUNK_G + D; }
-// A launch takes chunks [first, first + count) of every sequence.  Where sequence `seq`, whose rows start at row0 of the step, keeps chunk c:
-// with all of a step's chunks in one launch (segment 0) by its rows, so that sequences never meet and few places stay empty; else `segment`
-// places a sequence.
+// A launch takes chunks [first, first + count) of every sequence of at least min_rows rows.  Where sequence `seq`, whose rows start at row0 of the
+// step, keeps chunk c: with all of a step's chunks in one launch (segment 0) by its rows, so that sequences never meet and few places stay
+// empty; else `segment` places a sequence.  By its rows: one place more a sequence for its last, partial chunk; or, crowded (many sequences beside
+// few rows, none of the ones taken shorter than a chunk), two places every sixteen rows.
 struct ChunkSpan {
-    int first, count, segment;
+    int first, count, segment, crowded, min_rows;
 };
+__device__ __forceinline__ int chunk_first_place(const ChunkSpan& span, int row0, int seq) { return span.crowded ? row0 / CHUNK * 2 : row0 / CHUNK + seq; }
 __device__ __forceinline__ size_t chunk_place(const ChunkSpan& span, int row0, int seq, int c) {
-    return span.segment ? (size_t)seq * span.segment + (c - span.first) : (size_t)(row0 / CHUNK) + seq + c;
+    return span.segment ? (size_t)seq * span.segment + (c - span.first) : (size_t)(chunk_first_place(span, row0, seq) + c);
+}
+// The chunk at a place: its first row of the step and how many it has (0: none, or one of a sequence that is not taken).  The kernel that fills the
+// packs goes by places, not by the longest sequence times all of them: a prompt beside many single rows leaves few blocks without work.
+struct ChunkAt {
+    int row, rows;
+};
+__device__ __forceinline__ ChunkAt chunk_at(const ChunkSpan& span, int place, const int* seq_rows, const int* seq_slot, int seqs, int n_slots) {
+    int seq = 0, c;
+    if (span.segment) {
+        seq = place / span.segment;
+        c = place - seq * span.segment;
+        if (seq >= seqs || c >= span.count) return {0, 0};
+        c += span.first;
+    } else {
+        int end = seqs;                        // the last sequence whose places begin here or before
+        while (end - seq > 1) {
+            const int mid = (seq + end) / 2;
+            if (chunk_first_place(span, seq_rows[mid], mid) <= place) seq = mid;
+            else end = mid;
+        }
+        c = place - chunk_first_place(span, seq_rows[seq], seq);
+    }
+    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0, slot = seq_slot[seq];
+    if (c < 0 || c * CHUNK >= n_rows || n_rows < span.min_rows || slot < 0 || slot >= n_slots) return {0, 0};
+    return {row0 + c * CHUNK, min(CHUNK, n_rows - c * CHUNK)};
+}
+static inline bool chunk_crowded(long long rows, long long seqs, int min_rows) { return min_rows >= CHUNK && rows / CHUNK + 1 < seqs; }
+static inline long long chunk_places(long long rows, long long seqs, int min_rows) {
+    return chunk_crowded(rows, seqs, min_rows) ? 2 * (rows / CHUNK) + 2 : rows / CHUNK + seqs + 1;
 }
 // Chunks of scratch for a step: all of them, or as many as 2^28 floats hold (a gigabyte; at least one a sequence), and then the step goes
 // segment by segment, which hands the state on through memory and so must be allowed to write it.  0: not taken.
-static inline long long chunk_capacity(long long rows, long long seqs, long long H, int pack_floats, int write_state) {
-    const long long total = rows / CHUNK + seqs + 1, most = (1ll << 28) / (H * pack_floats);
+static inline long long chunk_capacity(long long rows, long long seqs, int min_rows, long long H, int pack_floats, int write_state) {
+    const long long total = chunk_places(rows, seqs, min_rows), most = (1ll << 28) / (H * pack_floats);
     if (total <= most) return total;
     return write_state ? (most > seqs ? most / seqs * seqs : seqs) : 0;
 }
@@ -111,7 +142,7 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
     const int seq = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * 32;
     const int slot = seq_slot[seq];
     const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
-    if (slot < 0 || slot >= n_slots || n_rows <= 0) return;
+    if (slot < 0 || slot >= n_slots || n_rows <= 0 || n_rows < span.min_rows) return;
     const int n_chunks = min(span.first + span.count, (n_rows + CHUNK - 1) / CHUNK);
     if (span.first >= n_chunks) return;
     const int pv = min(32, P - p0);                                        // value channels that exist (a multiple of four)
@@ -263,18 +294,20 @@ static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, c
 
 // A step's chunks through `prepare` (the kernel that fills the pack) and the scan: at once where `capacity` chunks of scratch hold them, else
 // segment by segment (at least one chunk a sequence, and the state must be written).
-static inline bool chunk_fits(long long capacity, long long rows, long long seqs, int write_state) {
-    return capacity >= rows / CHUNK + seqs + 1 || (write_state && capacity >= seqs);
+static inline bool chunk_fits(long long capacity, long long rows, long long seqs, int min_rows, int write_state) {
+    return capacity >= chunk_places(rows, seqs, min_rows) || (write_state && capacity >= seqs);
 }
+// prepare(span, places): the kernel over the places that the span's chunks lie at; scan(span).
 template <class Prepare, class Scan>
-static cudaError_t chunk_step(long long capacity, int rows, int seqs, int max_new, Prepare prepare, Scan scan) {
+static cudaError_t chunk_step(long long capacity, int rows, int seqs, int max_new, int min_rows, Prepare prepare, Scan scan) {
     const int most = (max_new + CHUNK - 1) / CHUNK;
-    const bool whole = capacity >= (long long)rows / CHUNK + seqs + 1;
-    const int segment = whole ? most : (int)(capacity / seqs);
+    const long long all = chunk_places(rows, seqs, min_rows);
+    const bool whole = capacity >= all;
+    const int segment = whole ? most : (int)(capacity / seqs < most ? capacity / seqs : most);
     cudaError_t e = cudaSuccess;
     for (int at = 0; at < most && e == cudaSuccess; at += segment) {
-        const ChunkSpan span = {at, segment < most - at ? segment : most - at, whole ? 0 : segment};
-        e = prepare(span);
+        const ChunkSpan span = {at, segment < most - at ? segment : most - at, whole ? 0 : segment, whole && chunk_crowded(rows, seqs, min_rows), min_rows};
+        e = prepare(span, whole ? all : (long long)seqs * segment);
         if (e == cudaSuccess) e = scan(span);
     }
     return e;

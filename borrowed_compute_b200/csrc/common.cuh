@@ -129,6 +129,20 @@ template <class T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// Whether one of the rows row0 .. row0 + n - 1 belongs to a sequence of fewer than `below` rows (sequence s owns rows seq_rows[s] .. seq_rows[s + 1]):
+// what a kernel over rows asks where long sequences go another way.
+__device__ __forceinline__ bool rows_of_short_sequences(const int* seq_rows, int seqs, int below, int row0, int n) {
+    int s = 0, end = seqs;                     // the last sequence that starts at row0 or before
+    while (end - s > 1) {
+        const int mid = (s + end) / 2;
+        if (seq_rows[mid] <= row0) s = mid;
+        else end = mid;
+    }
+    for (; s < seqs && seq_rows[s] < row0 + n; s++)
+        if (seq_rows[s + 1] > row0 && seq_rows[s + 1] - seq_rows[s] < below) return true;
+    return false;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

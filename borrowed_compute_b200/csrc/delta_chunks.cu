@@ -87,36 +87,47 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
 // ------------------------------------------------------------------------------------- packs
 #define DLC_D 64
 #define DLC_YP 36             // floats a channel of the 32 rows [r W; u W] and [b / W; k / W]: a gap against bank conflicts
-#define DLC_RUN 4             // chunks a block takes one after another, the next one's rows on their way
+#define DLC_RUN 4             // places of chunks a block takes one after another, the next one's rows on their way
 
-// A block takes chunks of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen columns through the
-// same substitutions.
+// A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
+// columns through the same substitutions.
 __global__ void __launch_bounds__(DLC_D + 32, 4)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
-                    const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int n_slots) {
+                    const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
     constexpr int PACK = chunk_pack_floats(DLC_D, true), THREADS = DLC_D + 32, ROW_SET = CHUNK * DLC_D;
     extern __shared__ __align__(16) float delta_smem[];
     float (*in)[4][CHUNK][DLC_D] = reinterpret_cast<float (*)[4][CHUNK][DLC_D]>(delta_smem);            // two stages of decays, r, k, a
     float *Y = delta_smem + 2 * 4 * ROW_SET, *X = Y + DLC_D * DLC_YP;
     float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm; Bm becomes M
     __shared__ float part[2][CHUNK];
+    __shared__ ChunkAt todo[DLC_RUN];
+    __shared__ int todo_place[DLC_RUN], n_todo;
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(proj); PDL_FRESH(decay);
-    const int h = blockIdx.y, seq = blockIdx.z, HD = H * D;
-    const int slot = seq_slot[seq];
-    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
-    const int c_first = span.first + blockIdx.x * DLC_RUN;
-    const int c_end = min(min(c_first + DLC_RUN, span.first + span.count), (n_rows + CHUNK - 1) / CHUNK);
-    if (slot < 0 || slot >= n_slots || c_first >= c_end) return;
+    const int h = blockIdx.y, HD = H * D;
     const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
+    if (warp == 0) {                                       // the chunks there are, one after another
+        const int place = blockIdx.x * run + lane;
+        const ChunkAt at = lane < run && place < places ? chunk_at(span, place, seq_rows, seq_slot, seqs, n_slots) : ChunkAt{0, 0};
+        const unsigned there = __ballot_sync(0xffffffffu, at.rows > 0);
+        if (at.rows > 0) {
+            const int i = __popc(there & ((1u << lane) - 1u));
+            todo[i] = at;
+            todo_place[i] = place;
+        }
+        if (lane == 0) n_todo = __popc(there);
+    }
+    __syncthreads();
+    const int n = n_todo;
+    if (n == 0) return;
     const bool channel = d < DLC_D, mine = d < D;
     const float bias = mine ? a_bias[h * D + d] : 0.0f;
     // What no copy reaches (rows past the sequence, channels past the head) is never used: it may hold anything.
     auto issue = [&](int c) {
-        const int rows = min(CHUNK, n_rows - c * CHUNK), quads = D / 4;
-        const size_t first = (size_t)(row0 + c * CHUNK);
-        const uint32_t dst = ad_smem(&in[(c - c_first) & 1][0][0][0]);
+        const int rows = todo[c].rows, quads = D / 4;
+        const size_t first = (size_t)todo[c].row;
+        const uint32_t dst = ad_smem(&in[c & 1][0][0][0]);
         for (int i = threadIdx.x; i < rows * quads; i += THREADS) {
             const int t = i / quads, at = 4 * (i - t * quads);
             const float* pr = proj + (first + t) * stride + h * D + at;
@@ -127,16 +138,15 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             cp_async16(to + 12 * ROW_SET, pr + 4 * HD);
         }
     };
-    issue(c_first);
+    issue(0);
     cp_async_commit();
-    for (int c = c_first; c < c_end; c++) {
-        if (c + 1 < c_end) issue(c + 1);
+    for (int c = 0; c < n; c++) {
+        if (c + 1 < n) issue(c + 1);
         cp_async_commit();
         cp_async_wait<1>();
         __syncthreads();
-        const int rows = min(CHUNK, n_rows - c * CHUNK);
-        const float (*sw)[DLC_D] = in[(c - c_first) & 1][0], (*sr)[DLC_D] = in[(c - c_first) & 1][1], (*sk)[DLC_D] = in[(c - c_first) & 1][2],
-                    (*sa)[DLC_D] = in[(c - c_first) & 1][3];
+        const int rows = todo[c].rows;
+        const float (*sw)[DLC_D] = in[c & 1][0], (*sr)[DLC_D] = in[c & 1][1], (*sk)[DLC_D] = in[c & 1][2], (*sa)[DLC_D] = in[c & 1][3];
         if (channel) {
             // Sixteen sums over a warp's channels, halved among its lanes: lane L (of sixteen) is left with row L.
             float kk[CHUNK];
@@ -158,7 +168,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             if (lane < CHUNK) part[warp][lane] = kk[0];
         }
         __syncthreads();
-        float* dst = pack + (chunk_place(span, row0, seq, c) * H + h) * PACK;
+        float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
         float total = 1.0f;
         if (channel) {
@@ -268,28 +278,30 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
 }
 #define DLC_SMEM ((2 * 4 * CHUNK * DLC_D + 2 * DLC_D * DLC_YP + 4 * CHUNK * CHUNK_G) * sizeof(float))
 
-// Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not).
-extern "C" long long bc_delta_chunked_scratch(int rows, int seqs, int H, int D, int inner, float decay_scale, int write_state) {
+// Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not), of which those of
+// fewer than min_rows rows are left alone.
+extern "C" long long bc_delta_chunked_scratch(int rows, int seqs, int min_rows, int H, int D, int inner, float decay_scale, int write_state) {
     if (D <= 0 || D > DLC_D || D % 4 || inner <= 0 || H <= 0 || H > 65535 || seqs <= 0 || seqs > 65535 || !(decay_scale >= 0.0f && decay_scale <= 4.0f)) return 0;
     const int pack = chunk_pack_floats(DLC_D, true);
-    return chunk_capacity(rows, seqs, H, pack, write_state) * H * pack;
+    return chunk_capacity(rows, seqs, min_rows, H, pack, write_state) * H * pack;
 }
 
 // proj, w2t, w0, a_bias as for bc_delta_prepare; state, seq_rows, seq_slot, out as for bc_delta_scan; decay: scratch [rows, H D]; pack: scratch of
-// pack_floats floats, bc_delta_chunked_scratch of them for the fewest launches; max_new: the most rows that a sequence brings.
+// pack_floats floats, bc_delta_chunked_scratch of them for the fewest launches; max_new: the most rows that a sequence brings; min_rows: sequences of
+// fewer rows are left alone, their states and their rows of out.
 extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t, const float* w0, const float* a_bias, float* decay, float* pack, long long pack_floats, float* state,
-                                const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int H, int D, int inner, float decay_scale,
-                                float key_eps, int n_slots, int write_state, cudaStream_t s) {
+                                const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int min_rows, int H, int D, int inner,
+                                float decay_scale, float key_eps, int n_slots, int write_state, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && seqs >= 0 && max_new >= 0, "delta_chunked: bad sizes rows=%d seqs=%d max_new=%d", rows, seqs, max_new);
     if (rows == 0 || seqs == 0 || max_new == 0) return BC_OK;
-    BC_CHECK_ARG(bc_delta_chunked_scratch(rows, seqs, H, D, inner, decay_scale, write_state) > 0,
+    BC_CHECK_ARG(bc_delta_chunked_scratch(rows, seqs, min_rows, H, D, inner, decay_scale, write_state) > 0,
                  "delta_chunked: %d heads of %d, inner %d, decay_scale %g are outside what the kernels take", H, D, inner, (double)decay_scale);
     BC_CHECK_ARG(stride >= 5 * H * D + inner, "delta_chunked: a row of %d values cannot hold five projections of %d and %d more", stride, H * D, inner);
     BC_CHECK_ARG((rows + DLC_ROWS - 1) / DLC_ROWS <= 65535, "delta_chunked: %d rows are too many", rows);
     BC_CHECK_ARG(stride % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)decay % 16 == 0 && (uintptr_t)pack % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0,
                  "delta_chunked: rows, state and scratch must start on 16-byte borders");
     const long long capacity = pack_floats / ((long long)H * chunk_pack_floats(DLC_D, true));
-    BC_CHECK_ARG(chunk_fits(capacity, rows, seqs, write_state), "delta_chunked: scratch of %lld floats is too small", pack_floats);
+    BC_CHECK_ARG(chunk_fits(capacity, rows, seqs, min_rows, write_state), "delta_chunked: scratch of %lld floats is too small", pack_floats);
     if (cudaError_t e = bc_allow_shared<delta_chunks_kernel>(DLC_SMEM); e != cudaSuccess) {
         bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
         return (int)e;
@@ -298,10 +310,13 @@ extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t,
                               w0, decay, rows, H * D, inner, decay_scale);
     if (e == cudaSuccess)
         e = chunk_step(
-            capacity, rows, seqs, max_new,
-            [&](const ChunkSpan& span) {
-                return bc_launch(delta_chunks_kernel, dim3((span.count + DLC_RUN - 1) / DLC_RUN, H, seqs), dim3(DLC_D + 32), DLC_SMEM, s, span, proj, stride, decay, a_bias, seq_rows, seq_slot, pack, H, D,
-                                 key_eps, n_slots);
+            capacity, rows, seqs, max_new, min_rows,
+            [&](const ChunkSpan& span, long long places) {
+                // Four chunks a block hide the loads of the next one (128 chunks of 64 heads: 232 us one a block, 143 four); where that leaves
+                // places on the SMs empty, one (with the rest of a call, 64 heads: 4 sequences of 64 rows 92 us four a block, 83 one; 8 heads: one of 64 rows 67 and 47).
+                const int run = (places + DLC_RUN - 1) / DLC_RUN * H >= 4 * bc_sm_count() ? DLC_RUN : 1;
+                return bc_launch(delta_chunks_kernel, dim3((unsigned)((places + run - 1) / run), H), dim3(DLC_D + 32), DLC_SMEM, s, span, proj, stride, decay, a_bias, seq_rows, seq_slot, pack, H, D,
+                                 key_eps, seqs, n_slots, run, (int)places);
             },
             [&](const ChunkSpan& span) {
                 return chunk_scan_launch<DLC_D / 32, true>(span, pack, proj + 2 * H * D, stride, state, seq_rows, seq_slot, out, seqs, H, D, D, n_slots, write_state, s);

@@ -99,7 +99,7 @@ template <int R> __device__ __forceinline__ void load_staged(const float* vec, i
 __global__ void delta_prepare_kernel(const float* __restrict__ proj, int stride, const float* __restrict__ w2t, const float* __restrict__ w0,
                                      const float* __restrict__ a_bias, float* __restrict__ decay, float* __restrict__ unit,
                                      float* __restrict__ removal, float* __restrict__ dots, int rows, int H, int D, int inner,
-                                     float decay_scale, float key_eps) {
+                                     float decay_scale, float key_eps, const int* __restrict__ seq_rows, int seqs, int below) {
     extern __shared__ float th[];        // tanh of the inner projection, [DP_ROWS][inner]
     __shared__ float scratch[32];
     pdl_launch_dependents_if_resident();
@@ -107,6 +107,7 @@ __global__ void delta_prepare_kernel(const float* __restrict__ proj, int stride,
     PDL_FRESH(proj);
     const int row0 = blockIdx.x * DP_ROWS, head = blockIdx.y, HD = H * D;
     const int n = min(DP_ROWS, rows - row0);
+    if (below > 0 && !rows_of_short_sequences(seq_rows, seqs, below, row0, n)) return;      // (the same for the whole block)
     for (int e = threadIdx.x; e < n * inner; e += blockDim.x) th[e] = tanhf(proj[(size_t)(row0 + e / inner) * stride + 5 * HD + e % inner]);
     __syncthreads();
     const int d = threadIdx.x, c = head * D + d;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(DR_LANES * DR_COLS)
 delta_scan_kernel(const float* __restrict__ proj, int stride, const float* __restrict__ decay, const float* __restrict__ unit,
                   const float* __restrict__ removal, const float* __restrict__ dots, float* __restrict__ state,
                   const int* __restrict__ seq_rows, const int* __restrict__ seq_slot, float* __restrict__ out, int H, int D, int n_slots,
-                  int write_state) {
+                  int write_state, int below) {
     constexpr int DP = DR_LANES * R;
     constexpr int VEC = DR_STEPS * DP;                              // one staged vector: [DR_STEPS][DP]
     constexpr int BUF = 5 * VEC + DR_STEPS * DR_BLOCK_COLS + DR_STEPS * 2;
@@ -175,7 +176,7 @@ delta_scan_kernel(const float* __restrict__ proj, int stride, const float* __res
     const int sq = blockIdx.x, head = blockIdx.y, HD = H * D;
     const int slot = seq_slot[sq];
     const int row0 = seq_rows[sq], n_new = seq_rows[sq + 1] - row0;
-    if (slot < 0 || slot >= n_slots || n_new <= 0) return;
+    if (slot < 0 || slot >= n_slots || n_new <= 0 || (below > 0 && n_new >= below)) return;
     const int lane = threadIdx.x % DR_LANES, col = threadIdx.x / DR_LANES;
     const int j0 = blockIdx.z * DR_BLOCK_COLS + col;                // this thread's value channels: j0 and j0 + DR_COLS
     // Channels past the head's width are never copied to: they stay zero.
@@ -445,30 +446,31 @@ extern "C" int bc_delta_step_bf16(const float* proj, int stride, const float* w2
 static int threads_for(int D) { return ((D + 31) / 32) * 32; }
 
 extern "C" int bc_delta_prepare(const float* proj, int stride, const float* w2t, const float* w0, const float* a_bias, float* decay, float* unit,
-                                float* removal, float* dots, int rows, int H, int D, int inner, float decay_scale, float key_eps,
-                                cudaStream_t s) {
+                                float* removal, float* dots, int rows, int H, int D, int inner, float decay_scale, float key_eps, const int* seq_rows,
+                                int seqs, int below, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && H > 0 && H <= 65535 && D > 0 && D <= 1024 && inner > 0 && inner <= 1024,
                  "delta_prepare: bad sizes rows=%d H=%d D=%d inner=%d (an inner width of at most 1024)", rows, H, D, inner);
     BC_CHECK_ARG(stride >= 5 * H * D + inner, "delta_prepare: a row of %d values cannot hold five projections of %d and %d more", stride, H * D, inner);
-    if (rows == 0) return BC_OK;
+    BC_CHECK_ARG(below <= 0 || (seq_rows != nullptr && seqs >= 0), "delta_prepare: which rows are of sequences below %d needs the sequences", below);
+    if (rows == 0 || (below > 0 && seqs == 0)) return BC_OK;
     bc_launch(delta_prepare_kernel, dim3((rows + DP_ROWS - 1) / DP_ROWS, H), dim3(threads_for(D)), (size_t)DP_ROWS * inner * sizeof(float), s, proj,
-              stride, w2t, w0, a_bias, decay, unit, removal, dots, rows, H, D, inner, decay_scale, key_eps);
+              stride, w2t, w0, a_bias, decay, unit, removal, dots, rows, H, D, inner, decay_scale, key_eps, seq_rows, seqs, below);
     BC_LAUNCH_STATUS();
 }
 
 // state: [n_slots, H, D, D] float, value channel before key channel.  Sequence s owns rows seq_rows[s] .. seq_rows[s + 1] and lives in
 // slot seq_slot[s] (negative: skipped, its rows of `out` are left untouched).  write_state 0 leaves
-// the state as it was.
+// the state as it was.  below > 0: sequences of at least so many rows are skipped too (bc_delta_prepare then prepares the others' rows alone).
 extern "C" int bc_delta_scan(const float* proj, int stride, const float* decay, const float* unit, const float* removal, const float* dots,
                              float* state, const int* seq_rows, const int* seq_slot, float* out, int seqs, int H, int D, int n_slots,
-                             int write_state, cudaStream_t s) {
+                             int write_state, int below, cudaStream_t s) {
     BC_CHECK_ARG(seqs >= 0 && seqs <= 2147483647 && H > 0 && H <= 65535 && D > 0 && D <= DR_MAX_D,
                  "delta_scan: bad sizes seqs=%d H=%d D=%d (a head of at most %d)", seqs, H, D, DR_MAX_D);
     if (seqs == 0) return BC_OK;
     const dim3 grid(seqs, H, (D + DR_BLOCK_COLS - 1) / DR_BLOCK_COLS), block(DR_LANES * DR_COLS);
 #define DR_CASE(R, STEPS)                                                                                                                      \
     bc_launch(delta_scan_kernel<R, STEPS>, grid, block, 0, s, proj, stride, decay, unit, removal, dots, state, seq_rows, seq_slot, out, H, D, \
-              n_slots, write_state)
+              n_slots, write_state, below)
     if (D <= 16) DR_CASE(2, 16);
     else if (D <= 32) DR_CASE(4, 16);
     else if (D <= 64) DR_CASE(8, 16);

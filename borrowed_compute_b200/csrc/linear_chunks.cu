@@ -20,26 +20,25 @@ template <int I, class F> __device__ __forceinline__ void glc_each(F&& f) {
     }
 }
 
-// A block takes a chunk of one head, a thread a key channel: decays as gla_decay_kernel works them out, then the 136 products of a
+// A block takes the chunk at a place, of one head, a thread a key channel: decays as gla_decay_kernel works them out, then the 136 products of a
 // pair of rows, each a running product of k_s with the decays after it.  The sums over channels: 32 pairs at a time are halved
 // among a warp's lanes, the warps' sums meet in shared memory.
 template <int D>
 __global__ void __launch_bounds__(D)
 gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at, int k_at, int inner_at, const float* __restrict__ w2t, const float* __restrict__ b,
                   int rank, const int* __restrict__ seq_rows, const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int N, float inv_tau, float f,
-                  int n_slots) {
+                  int seqs, int n_slots) {
     constexpr int WARPS = D / 32, PACK = chunk_pack_floats(D, false);
     extern __shared__ __align__(16) float inner[];           // [rank][16]
     __shared__ float part[WARPS][160];
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(proj);
-    const int c = span.first + blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
-    const int slot = seq_slot[seq];
-    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
-    const int rows = min(CHUNK, n_rows - c * CHUNK);
-    if (slot < 0 || slot >= n_slots || rows <= 0) return;
-    const float* p = proj + (size_t)(row0 + c * CHUNK) * stride;
+    const int h = blockIdx.y;
+    const ChunkAt at = chunk_at(span, blockIdx.x, seq_rows, seq_slot, seqs, n_slots);
+    const int rows = at.rows;
+    if (rows <= 0) return;
+    const float* p = proj + (size_t)at.row * stride;
     for (int i = threadIdx.x; i < rank * CHUNK; i += D) {
         const int t = i / rank, j = i - t * rank;
         inner[j * CHUNK + t] = t < rows ? p[(size_t)t * stride + inner_at + j] : 0.0f;
@@ -68,7 +67,7 @@ gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at,
         const float sp = fmaxf(m, 0.0f) + log1pf(expf(-fabsf(m)));
         a[t] = mine && t < rows ? expf(-sp * inv_tau) : 1.0f;
     }
-    float* dst = pack + (chunk_place(span, row0, seq, c) * H + h) * PACK;
+    float* dst = pack + ((size_t)blockIdx.x * H + h) * PACK;
     float run = 1.0f;
 #pragma unroll
     for (int t = 0; t < CHUNK; t++) {
@@ -125,17 +124,17 @@ gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at,
 
 template <int D>
 static int gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_at, int inner_at, const float* w2t, const float* b, int rank, float inv_tau, float f,
-                       float* pack, long long pack_floats, float* state, const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int H, int N, int P,
-                       int n_slots, int write_state, cudaStream_t s) {
+                       float* pack, long long pack_floats, float* state, const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int min_rows, int H, int N,
+                       int P, int n_slots, int write_state, cudaStream_t s) {
     if (cudaError_t e = bc_allow_shared<gla_chunks_kernel<D>>(64 * 1024); e != cudaSuccess) {
         bc_set_error("gla_chunked: %s", cudaGetErrorString(e));
         return (int)e;
     }
     const cudaError_t e = chunk_step(
-        pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, max_new,
-        [&](const ChunkSpan& span) {
-            return bc_launch(gla_chunks_kernel<D>, dim3(span.count, H, seqs), dim3(D), (size_t)rank * CHUNK * sizeof(float), s, span, proj, stride, q_at, k_at, inner_at,
-                             w2t, b, rank, seq_rows, seq_slot, pack, H, N, inv_tau, f, n_slots);
+        pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, max_new, min_rows,
+        [&](const ChunkSpan& span, long long places) {
+            return bc_launch(gla_chunks_kernel<D>, dim3((unsigned)places, H), dim3(D), (size_t)rank * CHUNK * sizeof(float), s, span, proj, stride, q_at, k_at, inner_at,
+                             w2t, b, rank, seq_rows, seq_slot, pack, H, N, inv_tau, f, seqs, n_slots);
         },
         [&](const ChunkSpan& span) {
             return chunk_scan_launch<D / 32, false>(span, pack, proj + v_at, stride, state, seq_rows, seq_slot, out, seqs, H, N, P, n_slots, write_state, s);
@@ -150,28 +149,29 @@ static int gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_
 static int glc_width(int N) { return N <= 64 ? 64 : N <= 128 ? 128 : 256; }
 
 // Whether gated linear attention of N key and P value channels a head runs in chunks, and the floats of scratch that `rows` rows of `seqs`
-// sequences take (0: it does not).
-extern "C" long long bc_gla_chunked_scratch(int rows, int seqs, int H, int N, int P, int rank, int write_state) {
+// sequences take (0: it does not), of which those of fewer than min_rows rows are left alone.
+extern "C" long long bc_gla_chunked_scratch(int rows, int seqs, int min_rows, int H, int N, int P, int rank, int write_state) {
     if (N <= 0 || N > 256 || N % 4 || P <= 0 || P % 4 || rank <= 0 || rank > 1024 || H <= 0 || H > 65535 || seqs <= 0 || seqs > 65535) return 0;
     const int pack = chunk_pack_floats(glc_width(N), false);
-    return chunk_capacity(rows, seqs, H, pack, write_state) * H * pack;
+    return chunk_capacity(rows, seqs, min_rows, H, pack, write_state) * H * pack;
 }
 
 // proj: [rows, stride] float with q and k (N values a head), v (P values a head) and the decay's inner vector (`rank` values) at columns q_at, k_at,
 // v_at and inner_at; w2t: [rank, H N]; b: [H N]; pack: scratch of pack_floats floats, bc_gla_chunked_scratch of them for the fewest launches; state: [slots, H, P, N]; out: [rows, H P].  Sequence i
-// owns rows seq_rows[i] .. seq_rows[i + 1], at most max_new, and lives in slot seq_slot[i] (negative: skipped, its rows of out untouched).
+// owns rows seq_rows[i] .. seq_rows[i + 1], at most max_new, and lives in slot seq_slot[i] (negative, or fewer than min_rows rows: skipped, its rows
+// of out untouched).
 extern "C" int bc_gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_at, int inner_at, const float* w2t, const float* b, int rank, float tau,
-                              float f, float* pack, long long pack_floats, float* state, const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int H, int N,
-                              int P, int n_slots, int write_state, cudaStream_t s) {
+                              float f, float* pack, long long pack_floats, float* state, const int* seq_rows, const int* seq_slot, float* out, int rows, int seqs, int max_new, int min_rows, int H,
+                              int N, int P, int n_slots, int write_state, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && seqs >= 0 && max_new >= 0 && tau > 0.0f, "gla_chunked: bad sizes rows=%d seqs=%d max_new=%d tau=%g", rows, seqs, max_new, (double)tau);
     if (rows == 0 || seqs == 0 || max_new == 0) return BC_OK;
-    BC_CHECK_ARG(bc_gla_chunked_scratch(rows, seqs, H, N, P, rank, write_state) > 0, "gla_chunked: %d heads of %d x %d channels, rank %d, are outside what the kernels take",
+    BC_CHECK_ARG(bc_gla_chunked_scratch(rows, seqs, min_rows, H, N, P, rank, write_state) > 0, "gla_chunked: %d heads of %d x %d channels, rank %d, are outside what the kernels take",
                  H, N, P, rank);
     BC_CHECK_ARG(stride % 4 == 0 && v_at % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)pack % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0,
                  "gla_chunked: rows, values, state and scratch must start on 16-byte borders");
     const int D = glc_width(N);
-    BC_CHECK_ARG(chunk_fits(pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, write_state), "gla_chunked: scratch of %lld floats is too small", pack_floats);
-#define GLC(DD) gla_chunked<DD>(proj, stride, q_at, k_at, v_at, inner_at, w2t, b, rank, 1.0f / tau, f, pack, pack_floats, state, seq_rows, seq_slot, out, rows, seqs, max_new, H, N, P, n_slots, write_state, s)
+    BC_CHECK_ARG(chunk_fits(pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, min_rows, write_state), "gla_chunked: scratch of %lld floats is too small", pack_floats);
+#define GLC(DD) gla_chunked<DD>(proj, stride, q_at, k_at, v_at, inner_at, w2t, b, rank, 1.0f / tau, f, pack, pack_floats, state, seq_rows, seq_slot, out, rows, seqs, max_new, min_rows, H, N, P, n_slots, write_state, s)
     return D == 64 ? GLC(64) : D == 128 ? GLC(128) : GLC(256);
 #undef GLC
 }

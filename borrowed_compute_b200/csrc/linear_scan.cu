@@ -46,7 +46,7 @@ linear_scan_kernel(const float* __restrict__ q, int q_stride, int q_rep, const f
                    const float* __restrict__ v, int v_stride, const float* __restrict__ decay, int d_stride,
                    const float* __restrict__ kscale, int c_stride, const float* __restrict__ skip, float out_scale,
                    float* __restrict__ state, const int* __restrict__ seq_rows, const int* __restrict__ seq_slot, float* __restrict__ out,
-                   int H, int N, int P, int R, int n_slots, int write_state) {
+                   int H, int N, int P, int R, int n_slots, int write_state, int below) {
     extern __shared__ __align__(16) float staged[];
     pdl_launch_dependents_if_resident();
     pdl_wait();
@@ -54,7 +54,7 @@ linear_scan_kernel(const float* __restrict__ q, int q_stride, int q_rep, const f
     const int sidx = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * SCAN_PT;
     const int slot = seq_slot[sidx];
     const int row0 = seq_rows[sidx], n_rows = seq_rows[sidx + 1] - row0;
-    if (slot < 0 || slot >= n_slots || n_rows <= 0) return;
+    if (slot < 0 || slot >= n_slots || n_rows <= 0 || (below > 0 && n_rows >= below)) return;
     const int tn = threadIdx.x % SCAN_NT, pl = threadIdx.x / SCAN_NT;         // 8 x 16 threads
     const int pa = p0 + pl, pb = p0 + 16 + pl;
     const bool live_a = pa < P, live_b = pb < P;
@@ -186,22 +186,22 @@ template <int NJ, bool VD, bool VEC>
 static cudaError_t scan_launch_one(dim3 grid, size_t smem, cudaStream_t s, const float* q, int q_stride, int q_rep, const float* k, int k_stride,
                                    int k_rep, const float* v, int v_stride, const float* decay, int d_stride, const float* kscale, int c_stride,
                                    const float* skip, float out_scale, float* state, const int* seq_rows, const int* seq_slot, float* out, int H,
-                                   int N, int P, int R, int n_slots, int write_state) {
+                                   int N, int P, int R, int n_slots, int write_state, int below) {
     if (cudaError_t e = bc_allow_shared<linear_scan_kernel<NJ, VD, VEC>>(100 * 1024); e != cudaSuccess) return e;
     return bc_launch(linear_scan_kernel<NJ, VD, VEC>, grid, dim3(128), smem, s, q, q_stride, q_rep, k, k_stride, k_rep, v, v_stride, decay, d_stride,
-                     kscale, c_stride, skip, out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state);
+                     kscale, c_stride, skip, out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state, below);
 }
 
 template <bool VD, bool VEC>
 static int scan_launch(int NJ, dim3 grid, size_t smem, cudaStream_t s, const float* q, int q_stride, int q_rep, const float* k, int k_stride,
                        int k_rep, const float* v, int v_stride, const float* decay, int d_stride, const float* kscale, int c_stride,
                        const float* skip, float out_scale, float* state, const int* seq_rows, const int* seq_slot, float* out, int H, int N,
-                       int P, int R, int n_slots, int write_state) {
+                       int P, int R, int n_slots, int write_state, int below) {
     cudaError_t e = cudaSuccess;
 #define SCAN_CASE(J)                                                                                                                         \
     case J:                                                                                                                                  \
         e = scan_launch_one<J, VD, VEC>(grid, smem, s, q, q_stride, q_rep, k, k_stride, k_rep, v, v_stride, decay, d_stride, kscale, c_stride, \
-                                        skip, out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state);                  \
+                                        skip, out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state, below);           \
         break;
     switch (NJ) {
         SCAN_CASE(1) SCAN_CASE(2) SCAN_CASE(4) SCAN_CASE(8) SCAN_CASE(12) SCAN_CASE(16) SCAN_CASE(24) SCAN_CASE(32)
@@ -217,11 +217,12 @@ static int scan_launch(int NJ, dim3 grid, size_t smem, cudaStream_t s, const flo
 // q, k: row r's vector for head h at base + r * stride + (h / rep) * N (rep heads share one); v: at v + r * v_stride + h * P;
 // decay: N values a head at decay + r * d_stride + h * N (vector_decay) or one at decay + r * d_stride + h; kscale (may be null):
 // one factor a head on the key at kscale + r * c_stride + h; skip (may be null): [H].  state: [slots, H, P, N]; out: [rows, H P].
-// Sequence i owns rows seq_rows[i] .. seq_rows[i + 1] and lives in slot seq_slot[i] (negative: skipped, its rows of out untouched).
+// Sequence i owns rows seq_rows[i] .. seq_rows[i + 1] and lives in slot seq_slot[i] (negative: skipped, its rows of out untouched; below > 0: so are
+// sequences of at least so many rows).
 extern "C" int bc_linear_scan(const float* q, int q_stride, int q_rep, const float* k, int k_stride, int k_rep, const float* v, int v_stride,
                               const float* decay, int d_stride, int vector_decay, const float* kscale, int c_stride, const float* skip,
                               float out_scale, float* state, const int* seq_rows, const int* seq_slot, float* out, int seqs, int H, int N, int P,
-                              int n_slots, int write_state, cudaStream_t s) {
+                              int n_slots, int write_state, int below, cudaStream_t s) {
     BC_CHECK_ARG(seqs >= 0 && seqs <= 65535 && H > 0 && H <= 65535 && P > 0, "linear_scan: bad sizes seqs=%d H=%d P=%d", seqs, H, P);
     BC_CHECK_ARG(N > 0 && N <= SCAN_MAX_N, "linear_scan: %d key channels are outside 1 to %d", N, SCAN_MAX_N);
     BC_CHECK_ARG(q_rep > 0 && k_rep > 0, "linear_scan: bad sharing of q (%d) or k (%d)", q_rep, k_rep);
@@ -239,7 +240,7 @@ extern "C" int bc_linear_scan(const float* q, int q_stride, int q_rep, const flo
     dim3 grid((P + SCAN_PT - 1) / SCAN_PT, H, seqs);
 #define SCAN_GO(VD, VEC)                                                                                                                    \
     return scan_launch<VD, VEC>(nj, grid, smem, s, q, q_stride, q_rep, k, k_stride, k_rep, v, v_stride, decay, d_stride, kscale, c_stride, skip, \
-                                out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state)
+                                out_scale, state, seq_rows, seq_slot, out, H, N, P, R, n_slots, write_state, below)
     if (vector_decay) {
         if (vec) SCAN_GO(true, true);
         SCAN_GO(true, false);
@@ -348,12 +349,13 @@ extern "C" int bc_ssd_prepare(const float* proj, int stride, int conv_at, int dt
 // so that no logarithm of a rounded sigmoid is taken.  One block a row; the inner vector is staged in shared memory.
 __global__ void __launch_bounds__(256)
 gla_decay_kernel(const float* __restrict__ proj, int stride, int inner_at, const float* __restrict__ w2t, const float* __restrict__ b,
-                 float* __restrict__ decay, int W, int rank, float inv_tau) {
+                 float* __restrict__ decay, int W, int rank, float inv_tau, const int* __restrict__ seq_rows, int seqs, int below) {
     extern __shared__ float inner[];
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(proj);
     const int r = blockIdx.x;
+    if (below > 0 && !rows_of_short_sequences(seq_rows, seqs, below, r, 1)) return;
     for (int i = threadIdx.x; i < rank; i += blockDim.x) inner[i] = proj[(size_t)r * stride + inner_at + i];
     __syncthreads();
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
@@ -366,13 +368,15 @@ gla_decay_kernel(const float* __restrict__ proj, int stride, int inner_at, const
     }
 }
 
-// proj: [rows, stride] float with the inner projection's `rank` values at column inner_at; w2t: [rank, W]; b: [W]; decay: [rows, W].
+// proj: [rows, stride] float with the inner projection's `rank` values at column inner_at; w2t: [rank, W]; b: [W]; decay: [rows, W].  below > 0:
+// rows of sequences of at least so many rows are left out.
 extern "C" int bc_gla_decay(const float* proj, int stride, int inner_at, const float* w2t, const float* b, float* decay, int rows, int W, int rank,
-                            float tau, cudaStream_t s) {
+                            float tau, const int* seq_rows, int seqs, int below, cudaStream_t s) {
     BC_CHECK_ARG(rows >= 0 && W > 0 && rank > 0 && rank <= 8192 && tau > 0.0f, "gla_decay: bad sizes rows=%d W=%d rank=%d tau=%g", rows, W, rank, (double)tau);
-    if (rows == 0) return BC_OK;
+    BC_CHECK_ARG(below <= 0 || (seq_rows != nullptr && seqs >= 0), "gla_decay: which rows are of sequences below %d needs the sequences", below);
+    if (rows == 0 || (below > 0 && seqs == 0)) return BC_OK;
     bc_launch(gla_decay_kernel, dim3(rows), dim3(W >= 1024 ? 256 : 128), (size_t)rank * sizeof(float), s, proj, stride, inner_at, w2t, b, decay, W,
-              rank, 1.0f / tau);
+              rank, 1.0f / tau, seq_rows, seqs, below);
     BC_LAUNCH_STATUS();
 }
 

@@ -21,7 +21,7 @@ extern "C" int bc_get_pdl() { return g_bc_pdl; }
 extern "C" const char* bc_last_error() { return g_error; }
 
 // Bumped when an exported signature changes, so a stale build is never called.
-extern "C" int bc_abi_version() { return 1; }
+extern "C" int bc_abi_version() { return 2; }
 
 extern "C" int bc_page_size() { return BC_PAGE; }
 

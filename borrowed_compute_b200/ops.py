@@ -718,11 +718,13 @@ def norm_pair(x: torch.Tensor, w1: torch.Tensor, w2: Optional[torch.Tensor], out
 
 
 def delta_prepare(proj: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bias: torch.Tensor, decay: torch.Tensor, unit: torch.Tensor,
-                  removal: torch.Tensor, dots: torch.Tensor, heads: int, head_dim: int, decay_scale: float, key_eps: float) -> None:
+                  removal: torch.Tensor, dots: torch.Tensor, heads: int, head_dim: int, decay_scale: float, key_eps: float,
+                  seq_rows: Optional[torch.Tensor] = None, seqs: int = 0, below: int = 0) -> None:
     """From the fused projection [rows, 5 H D + inner] (r, k, v, gate, a, decay's inner projection; float32): per key
     channel the decay exp(-decay_scale * sigmoid(w2 tanh(inner) + w0)), the key over its length, the removal
     rate sigmoid(a + a_bias) times that unit key, and per head the dot products r.(removal) and r.k.
-    ``w2t`` is w2 transposed, [inner, H D]."""
+    ``w2t`` is w2 transposed, [inner, H D].  With ``below`` only rows of sequences (``seq_rows``, ``seqs`` of them) that bring
+    fewer than so many are sure to be prepared."""
     rows, stride = proj.shape
     HD = heads * head_dim
     inner = w2t.shape[0]
@@ -732,15 +734,29 @@ def delta_prepare(proj: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bia
         raise KernelError(f"delta_prepare: proj {tuple(proj.shape)}, w2t {tuple(w2t.shape)} do not fit {heads} heads of {head_dim}")
     if any(tuple(t.shape) != (rows, HD) for t in (decay, unit, removal)) or tuple(dots.shape) != (rows, heads, 2):
         raise KernelError("delta_prepare: outputs must be [rows, H D] and dots [rows, H, 2]")
+    _need_sequences("delta_prepare", seq_rows, seqs, rows, below)
     _call(_fn("bc_delta_prepare"), _ptr(proj), _c_int(stride), _ptr(w2t), _ptr(w0), _ptr(a_bias), _ptr(decay), _ptr(unit), _ptr(removal),
-          _ptr(dots), _c_int(rows), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale), _c_float(key_eps), _stream())
+          _ptr(dots), _c_int(rows), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale), _c_float(key_eps),
+          _ptr(seq_rows), _c_int(seqs), _c_int(below), _stream())
+
+
+def _need_sequences(who: str, seq_rows: Optional[torch.Tensor], seqs: int, rows: int, below: int) -> None:
+    if below <= 0:
+        return
+    if seq_rows is None:
+        raise KernelError(f"{who}: which rows are of sequences below {below} needs the sequences")
+    _need(seq_rows, "seq_rows", torch.int32)
+    if seq_rows.numel() < seqs + 1:
+        raise KernelError(f"{who}: {seq_rows.numel()} numbers are no rows of {seqs} sequences")
+    _bounds(f"{who}: seq_rows", seq_rows, rows + 1, seqs + 1)
 
 
 def delta_scan(proj: torch.Tensor, decay: torch.Tensor, unit: torch.Tensor, removal: torch.Tensor, dots: torch.Tensor, state: torch.Tensor,
                seq_rows: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, seqs: int, heads: int, head_dim: int,
-               write_state: bool = True) -> None:
+               write_state: bool = True, below: int = 0) -> None:
     """The recurrence S <- diag(decay) S - removal (unit^T S) + k v^T, o = S^T r over every sequence's rows in
-    time order, from and into ``state`` [slots, H, D, D] float32; ``out`` [rows, H D] float32."""
+    time order, from and into ``state`` [slots, H, D, D] float32; ``out`` [rows, H D] float32.  With ``below`` sequences
+    that bring at least so many rows are left alone."""
     for t, name in ((proj, "proj"), (decay, "decay"), (unit, "unit"), (removal, "removal"), (dots, "dots"), (state, "state"), (out, "out")):
         _need(t, name, torch.float32)
     _need(seq_rows, "seq_rows", torch.int32)
@@ -751,7 +767,7 @@ def delta_scan(proj: torch.Tensor, decay: torch.Tensor, unit: torch.Tensor, remo
     _bounds("delta_scan: seq_rows", seq_rows, proj.shape[0] + 1, seqs + 1)
     _call(_fn("bc_delta_scan"), _ptr(proj), _c_int(proj.shape[1]), _ptr(decay), _ptr(unit), _ptr(removal), _ptr(dots), _ptr(state),
           _ptr(seq_rows), _ptr(seq_slot), _ptr(out), _c_int(seqs), _c_int(heads), _c_int(head_dim), _c_int(state.shape[0]),
-          _c_int(1 if write_state else 0), _stream())
+          _c_int(1 if write_state else 0), _c_int(below), _stream())
 
 
 def _chunk_scratch(name: str, *args) -> int:
@@ -761,21 +777,22 @@ def _chunk_scratch(name: str, *args) -> int:
     return int(f(*args))
 
 
-def delta_chunked_scratch(rows: int, seqs: int, heads: int, head_dim: int, inner: int, decay_scale: float, write_state: bool = True) -> int:
-    """Floats of scratch that ``delta_chunked`` takes for ``rows`` rows of ``seqs`` sequences; 0 where ``delta_scan`` has to serve (heads
+def delta_chunked_scratch(rows: int, seqs: int, heads: int, head_dim: int, inner: int, decay_scale: float, write_state: bool = True,
+                          min_rows: int = 0) -> int:
+    """Floats of scratch that ``delta_chunked`` takes for ``rows`` rows of ``seqs`` sequences, with the same ``min_rows``; 0 where ``delta_scan`` has to serve (heads
     above 64 channels or not a multiple of four, rows of the projection off a 16-byte border, decays below exp(-4))."""
     if (5 * heads * head_dim + inner) % 4:
         return 0
-    return _chunk_scratch("bc_delta_chunked_scratch", _c_int(rows), _c_int(seqs), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale),
-                          _c_int(1 if write_state else 0))
+    return _chunk_scratch("bc_delta_chunked_scratch", _c_int(rows), _c_int(seqs), _c_int(min_rows), _c_int(heads), _c_int(head_dim), _c_int(inner),
+                          _c_float(decay_scale), _c_int(1 if write_state else 0))
 
 
 def delta_chunked(proj: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bias: torch.Tensor, decay: torch.Tensor, pack: torch.Tensor,
                   state: torch.Tensor, seq_rows: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, seqs: int, max_new: int, heads: int,
-                  head_dim: int, decay_scale: float, key_eps: float, write_state: bool = True) -> None:
+                  head_dim: int, decay_scale: float, key_eps: float, write_state: bool = True, min_rows: int = 0) -> None:
     """``delta_prepare`` and ``delta_scan`` with the rows of a sequence taken sixteen at a time: the same recurrence in float32, its sums in
     another order.  ``decay``: scratch like ``out``; ``pack``: scratch of ``delta_chunked_scratch`` floats (with fewer, down to a
-    chunk a sequence, the step goes in segments)."""
+    chunk a sequence, the step goes in segments).  Sequences of fewer than ``min_rows`` rows are left alone."""
     for t, name in ((proj, "proj"), (w2t, "w2t"), (w0, "w0"), (a_bias, "a_bias"), (decay, "decay"), (pack, "pack"), (state, "state"), (out, "out")):
         _need(t, name, torch.float32)
     _need(seq_rows, "seq_rows", torch.int32)
@@ -789,8 +806,8 @@ def delta_chunked(proj: torch.Tensor, w2t: torch.Tensor, w0: torch.Tensor, a_bia
     _bounds("delta_chunked: seq_slot", seq_slot, state.shape[0], seqs, lowest=-1)
     _bounds("delta_chunked: seq_rows", seq_rows, rows + 1, seqs + 1)
     _call(_fn("bc_delta_chunked"), _ptr(proj), _c_int(stride), _ptr(w2t), _ptr(w0), _ptr(a_bias), _ptr(decay), _ptr(pack), ctypes.c_longlong(pack.numel()), _ptr(state), _ptr(seq_rows),
-          _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale), _c_float(key_eps),
-          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
+          _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(min_rows), _c_int(heads), _c_int(head_dim), _c_int(inner), _c_float(decay_scale),
+          _c_float(key_eps), _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
 
 
 def delta_finish(o: torch.Tensor, proj: torch.Tensor, gate_offset: int, weight: torch.Tensor, out: torch.Tensor, heads: int, head_dim: int,
@@ -943,11 +960,12 @@ def qkv_prepare_heads(qkv: torch.Tensor, q_weight: Optional[torch.Tensor], k_wei
 def linear_scan(q: torch.Tensor, q_at: int, q_rep: int, k: torch.Tensor, k_at: int, k_rep: int, v: torch.Tensor, v_at: int,
                 decay: torch.Tensor, decay_at: int, vector_decay: bool, kscale: Optional[torch.Tensor], kscale_at: int,
                 skip: Optional[torch.Tensor], out_scale: float, state: torch.Tensor, seq_rows: torch.Tensor, seq_slot: torch.Tensor,
-                out: torch.Tensor, seqs: int, heads: int, key_dim: int, value_dim: int, write_state: bool = True) -> None:
+                out: torch.Tensor, seqs: int, heads: int, key_dim: int, value_dim: int, write_state: bool = True, below: int = 0) -> None:
     """S_t = diag(a_t) S_(t-1) + (c_t k_t) v_t^T, o_t = out_scale * S_t^T q_t + skip * v_t for every head over every sequence's rows
     in time order, all float32.  q, k, v, decay and kscale are [rows, anything] tensors read from column ``*_at`` on: q and k hold
     ``key_dim`` values for each group of ``*_rep`` heads, v ``value_dim`` a head, decay ``key_dim`` a head (``vector_decay``) or one,
-    kscale one a head (None: 1).  A ``decay`` of a single row serves every row (constant decays).  ``state`` [slots, heads, value_dim, key_dim] (value channel by value channel), ``out`` [rows, heads * value_dim]."""
+    kscale one a head (None: 1).  A ``decay`` of a single row serves every row (constant decays).  ``state`` [slots, heads, value_dim, key_dim] (value channel by value channel), ``out`` [rows, heads * value_dim].
+    With ``below`` sequences that bring at least so many rows are left alone."""
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (decay, "decay"), (state, "state"), (out, "out")):
         _need(t, name, torch.float32)
     _need(seq_rows, "seq_rows", torch.int32)
@@ -978,7 +996,7 @@ def linear_scan(q: torch.Tensor, q_at: int, q_rep: int, k: torch.Tensor, k_at: i
           _c_int(v.shape[1]), at(decay, decay_at), _c_int(0 if decay.shape[0] == 1 else decay.shape[1]), _c_int(1 if vector_decay else 0),
           _c_void_p(0) if kscale is None else at(kscale, kscale_at), _c_int(0 if kscale is None else kscale.shape[1]), _ptr(skip),
           _c_float(out_scale), _ptr(state), _ptr(seq_rows), _ptr(seq_slot), _ptr(out), _c_int(seqs), _c_int(H), _c_int(N), _c_int(P),
-          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
+          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _c_int(below), _stream())
 
 
 SSD_MAX_TAPS = 9
@@ -1017,33 +1035,38 @@ def ssd_prepare(proj: torch.Tensor, conv_at: int, dt_at: int, weight_t: torch.Te
           _c_int(taps), _c_int(tail.shape[0]), _c_int(1 if write_tail else 0), _stream())
 
 
-def gla_decay(proj: torch.Tensor, inner_at: int, w2t: torch.Tensor, bias: torch.Tensor, decay: torch.Tensor, tau: float) -> None:
-    """decay = sigmoid(z)^(1/tau) with z = inner @ w2t + bias, inner being proj's columns inner_at .. inner_at + rank; float32."""
+def gla_decay(proj: torch.Tensor, inner_at: int, w2t: torch.Tensor, bias: torch.Tensor, decay: torch.Tensor, tau: float,
+              seq_rows: Optional[torch.Tensor] = None, seqs: int = 0, below: int = 0) -> None:
+    """decay = sigmoid(z)^(1/tau) with z = inner @ w2t + bias, inner being proj's columns inner_at .. inner_at + rank; float32.  With ``below``
+    rows of sequences (``seq_rows``, ``seqs`` of them) that bring at least so many are left out."""
     for t, name in ((proj, "proj"), (w2t, "w2t"), (bias, "bias"), (decay, "decay")):
         _need(t, name, torch.float32)
     rank, W = w2t.shape
     rows = proj.shape[0]
     if bias.numel() != W or tuple(decay.shape) != (rows, W) or inner_at + rank > proj.shape[1]:
         raise KernelError(f"gla_decay: proj {tuple(proj.shape)}, w2t {tuple(w2t.shape)}, decay {tuple(decay.shape)} do not fit")
+    _need_sequences("gla_decay", seq_rows, seqs, rows, below)
     _call(_fn("bc_gla_decay"), _ptr(proj), _c_int(proj.shape[1]), _c_int(inner_at), _ptr(w2t), _ptr(bias), _ptr(decay), _c_int(rows), _c_int(W),
-          _c_int(rank), _c_float(tau), _stream())
+          _c_int(rank), _c_float(tau), _ptr(seq_rows), _c_int(seqs), _c_int(below), _stream())
 
 
-def gla_chunked_scratch(proj: torch.Tensor, v_at: int, seqs: int, heads: int, key_dim: int, value_dim: int, rank: int, write_state: bool = True) -> int:
-    """Floats of scratch that ``gla_chunked`` takes for these rows; 0 where ``gla_decay`` and ``linear_scan`` have to serve (channels that are not
+def gla_chunked_scratch(proj: torch.Tensor, v_at: int, seqs: int, heads: int, key_dim: int, value_dim: int, rank: int, write_state: bool = True,
+                        min_rows: int = 0) -> int:
+    """Floats of scratch that ``gla_chunked`` takes for these rows, with the same ``min_rows``; 0 where ``gla_decay`` and ``linear_scan`` have to serve (channels that are not
     multiples of four, rows or values off a 16-byte border)."""
     if proj.shape[1] % 4 or v_at % 4 or proj.data_ptr() % 16:
         return 0
-    return _chunk_scratch("bc_gla_chunked_scratch", _c_int(proj.shape[0]), _c_int(seqs), _c_int(heads), _c_int(key_dim), _c_int(value_dim), _c_int(rank),
-                          _c_int(1 if write_state else 0))
+    return _chunk_scratch("bc_gla_chunked_scratch", _c_int(proj.shape[0]), _c_int(seqs), _c_int(min_rows), _c_int(heads), _c_int(key_dim), _c_int(value_dim),
+                          _c_int(rank), _c_int(1 if write_state else 0))
 
 
 def gla_chunked(proj: torch.Tensor, q_at: int, k_at: int, v_at: int, inner_at: int, w2t: torch.Tensor, bias: torch.Tensor, tau: float, out_scale: float,
                 pack: torch.Tensor, state: torch.Tensor, seq_rows: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, seqs: int, max_new: int, heads: int,
-                key_dim: int, value_dim: int, write_state: bool = True) -> None:
+                key_dim: int, value_dim: int, write_state: bool = True, min_rows: int = 0) -> None:
     """``gla_decay`` and ``linear_scan`` (a decay a key channel, k as it is, nothing skipped) with the rows of a sequence taken sixteen at a time:
     the same recurrence in float32, its sums in another order.  q, k, v and the decays' inner vector are columns of ``proj``; ``pack``: scratch of
-    ``gla_chunked_scratch`` floats (with fewer, down to a chunk a sequence, the step goes in segments)."""
+    ``gla_chunked_scratch`` floats (with fewer, down to a chunk a sequence, the step goes in segments).  Sequences of fewer than ``min_rows``
+    rows are left alone."""
     for t, name in ((proj, "proj"), (w2t, "w2t"), (bias, "bias"), (pack, "pack"), (state, "state"), (out, "out")):
         _need(t, name, torch.float32)
     _need(seq_rows, "seq_rows", torch.int32)
@@ -1058,8 +1081,8 @@ def gla_chunked(proj: torch.Tensor, q_at: int, k_at: int, v_at: int, inner_at: i
     _bounds("gla_chunked: seq_slot", seq_slot, state.shape[0], seqs, lowest=-1)
     _bounds("gla_chunked: seq_rows", seq_rows, rows + 1, seqs + 1)
     _call(_fn("bc_gla_chunked"), _ptr(proj), _c_int(stride), _c_int(q_at), _c_int(k_at), _c_int(v_at), _c_int(inner_at), _ptr(w2t), _ptr(bias), _c_int(rank), _c_float(tau),
-          _c_float(out_scale), _ptr(pack), ctypes.c_longlong(pack.numel()), _ptr(state), _ptr(seq_rows), _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(H), _c_int(N), _c_int(P),
-          _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
+          _c_float(out_scale), _ptr(pack), ctypes.c_longlong(pack.numel()), _ptr(state), _ptr(seq_rows), _ptr(seq_slot), _ptr(out), _c_int(rows), _c_int(seqs), _c_int(max_new), _c_int(min_rows), _c_int(H), _c_int(N),
+          _c_int(P), _c_int(state.shape[0]), _c_int(1 if write_state else 0), _stream())
 
 
 def gated_norm(y: torch.Tensor, gate: torch.Tensor, gate_at: int, weight: torch.Tensor, out: torch.Tensor, parts: int, eps: float,

@@ -282,6 +282,16 @@ class StepContext:
     hand_over: bool = False
     handed: Optional[Tuple[torch.Tensor, torch.Tensor]] = None
 
+    def brings_fewer(self, rows: int) -> bool:
+        """Whether some sequence brings fewer than ``rows`` rows (as far as is known: without the host copies, yes)."""
+        if len(self.host_seq_rows) <= self.seqs:
+            return True
+        key = ("brings_fewer", rows)
+        if key not in self.extras:
+            at = self.host_seq_rows
+            self.extras[key] = any(0 < at[s + 1] - at[s] < rows for s in range(self.seqs))
+        return self.extras[key]
+
 
 # ------------------------------------------------------------------------------- interfaces
 

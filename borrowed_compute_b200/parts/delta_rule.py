@@ -28,8 +28,10 @@ from . import products
 from .base import MIXERS, Mixer, RunMemory, Runtime, StateNeed, StepContext, TensorSpec
 
 
-# Steps in which a sequence brings at least this many rows take them sixteen at a time (bfloat16 engines: the float32 path keeps the
-# row-by-row scan, whose sums are the same however a prompt is cut).
+# A sequence that brings at least this many rows takes them sixteen at a time, whatever else the step holds (bfloat16 engines: there a prompt cut in
+# other portions has its sums in another order; the float32 path keeps the row-by-row scan, whose sums are the same however a prompt is cut).
+# One whole chunk: 64 heads of 64 take 85 us by rows and 78 in chunks for 16 sequences of 16 rows, 161 and 189 for 64 of 8
+# (a chunk costs the same however few of its rows there are), 68 and 76 for 16 of 8.
 CHUNKED_ROWS = 16
 split_steps = False      # tests: steps of single rows through the three kernels of a prompt step
 
@@ -82,15 +84,18 @@ class GeneralizedDelta(Mixer):
         o, decay = (torch.empty((rows, hd), dtype=f32, device=dev) for _ in range(2))
         scratch = 0
         if x.dtype == torch.bfloat16 and ctx.max_new >= CHUNKED_ROWS:
-            scratch = ops.delta_chunked_scratch(rows, ctx.seqs, H, D, self.decay_rank, self.decay_scale, mem.writes)
+            scratch = ops.delta_chunked_scratch(rows, ctx.seqs, H, D, self.decay_rank, self.decay_scale, mem.writes, min_rows=CHUNKED_ROWS)
         if scratch:
             pack = torch.empty((scratch,), dtype=f32, device=dev)
             ops.delta_chunked(proj, self.w2_t, self.w0, self.a_bias, decay, pack, mem.state, ctx.seq_rows, ctx.seq_slot, o, ctx.seqs, ctx.max_new, H, D,
-                              self.decay_scale, self.key_eps, write_state=mem.writes)
-        else:
+                              self.decay_scale, self.key_eps, write_state=mem.writes, min_rows=CHUNKED_ROWS)
+            del pack                                    # (its memory serves what comes next)
+        if not scratch or ctx.brings_fewer(CHUNKED_ROWS):
+            below = CHUNKED_ROWS if scratch else 0
             unit, removal = (torch.empty((rows, hd), dtype=f32, device=dev) for _ in range(2))
             dots = torch.empty((rows, H, 2), dtype=f32, device=dev)
-            ops.delta_prepare(proj, self.w2_t, self.w0, self.a_bias, decay, unit, removal, dots, H, D, self.decay_scale, self.key_eps)
-            ops.delta_scan(proj, decay, unit, removal, dots, mem.state, ctx.seq_rows, ctx.seq_slot, o, ctx.seqs, H, D, write_state=mem.writes)
+            ops.delta_prepare(proj, self.w2_t, self.w0, self.a_bias, decay, unit, removal, dots, H, D, self.decay_scale, self.key_eps,
+                              ctx.seq_rows, ctx.seqs, below)
+            ops.delta_scan(proj, decay, unit, removal, dots, mem.state, ctx.seq_rows, ctx.seq_slot, o, ctx.seqs, H, D, write_state=mem.writes, below=below)
         ops.delta_finish(o, proj, 3 * hd, self.norm_weight, y, H, D, self.norm_eps)
         products.linear(y, self.w_o, residual, products.EPI_ADD_F32, "output product")

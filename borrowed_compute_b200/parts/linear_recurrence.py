@@ -33,8 +33,10 @@ from . import products
 from .base import MIXERS, Mixer, RunMemory, Runtime, StateNeed, StepContext, TensorSpec
 
 
-# Steps in which a sequence brings at least this many rows take them sixteen at a time (bfloat16 engines: the float32 path keeps the
-# row-by-row scan, whose sums are the same however a prompt is cut).
+# A sequence that brings at least this many rows takes them sixteen at a time, whatever else the step holds (bfloat16 engines: there a prompt cut in
+# other portions has its sums in another order; the float32 path keeps the row-by-row scan, whose sums are the same however a prompt is cut).
+# One whole chunk: 16 heads of 128 x 256 take 84 us by rows and 53 in chunks for 16 sequences of 16 rows, 119 and 123 for
+# 64 of 4; 4 heads of 64 x 64 take 32 and 30 for 16 of 16, 30 and 28 for 16 of 4.
 CHUNKED_ROWS = 16
 
 
@@ -81,16 +83,18 @@ class GatedLinearAttention(Mixer):
         o = torch.empty((rows, hp), dtype=torch.float32, device=dev)
         scratch = 0
         if x.dtype == torch.bfloat16 and ctx.max_new >= CHUNKED_ROWS:
-            scratch = ops.gla_chunked_scratch(proj, 2 * hd, ctx.seqs, H, D, P, self.decay_rank, mem.writes)
+            scratch = ops.gla_chunked_scratch(proj, 2 * hd, ctx.seqs, H, D, P, self.decay_rank, mem.writes, min_rows=CHUNKED_ROWS)
         if scratch:
             pack = torch.empty((scratch,), dtype=torch.float32, device=dev)
             ops.gla_chunked(proj, 0, hd, 2 * hd, 2 * hd + 2 * hp, self.a2_t, self.a2_b, self.tau, float(D) ** -0.5, pack, mem.state, ctx.seq_rows,
-                            ctx.seq_slot, o, ctx.seqs, ctx.max_new, H, D, P, write_state=mem.writes)
-        else:
+                            ctx.seq_slot, o, ctx.seqs, ctx.max_new, H, D, P, write_state=mem.writes, min_rows=CHUNKED_ROWS)
+            del pack                                    # (its memory serves what comes next)
+        if not scratch or ctx.brings_fewer(CHUNKED_ROWS):
+            below = CHUNKED_ROWS if scratch else 0
             decay = torch.empty((rows, hd), dtype=torch.float32, device=dev)
-            ops.gla_decay(proj, 2 * hd + 2 * hp, self.a2_t, self.a2_b, decay, self.tau)
+            ops.gla_decay(proj, 2 * hd + 2 * hp, self.a2_t, self.a2_b, decay, self.tau, ctx.seq_rows, ctx.seqs, below)
             ops.linear_scan(proj, 0, 1, proj, hd, 1, proj, 2 * hd, decay, 0, True, None, 0, None, float(D) ** -0.5, mem.state, ctx.seq_rows,
-                            ctx.seq_slot, o, ctx.seqs, H, D, P, write_state=mem.writes)
+                            ctx.seq_slot, o, ctx.seqs, H, D, P, write_state=mem.writes, below=below)
         y = torch.empty((rows, hp), dtype=x.dtype, device=dev)
         ops.gated_norm(o, proj, 2 * hd + hp, self.norm_weight, y, H, self.norm_eps, gate_first=False, factor=self.out_scale, row_slot=ctx.row_slot)
         products.linear(y, self.w_o, residual, products.EPI_ADD_F32, "output product")

@@ -1,7 +1,8 @@
 """The recurrences that take sixteen rows at a time (csrc/delta_chunks.cu, csrc/linear_chunks.cu) against float64 sums and against the row-by-row
 scans they stand in for: sequences around the edges of a chunk, several beside one another and one of no slot, states that are not
 zero, channel counts that fill a tile and that do not, scratch for the whole step and for one chunk a sequence at a time, decays at the
-ends of their range, and an infinity that may reach later rows but no earlier one.
+ends of their range, an infinity that may reach later rows but no earlier one, and steps in which short sequences go row by row beside long
+ones in chunks.
 
 Tolerance: 32-bit sums over a chunk and a head (at most 16 + 256 terms) and their chain over a prompt that the decays forget, measured
 at 2.5e-7 of a tensor's 2-norm at most; 2e-6 is allowed, and no value may be off by 2e-5 of the largest."""
@@ -143,3 +144,131 @@ def test_an_infinity_reaches_no_earlier_row(kind):
             ops.gla_chunked(p, 0, HD, 2 * HD, 5 * HD, w2t, zero, 16.0, 0.125, pack, state, seq_rows, seq_slot, out, 1, rows, H, D, D)
     assert torch.equal(clean[:bad], poisoned[:bad])
     assert not bool(torch.isfinite(poisoned[bad:]).all(-1).any())
+
+
+MIXED = [[1, 40, 3, 16, 15, 2, 100, 1, 9], [33, 1], [1] * 40 + [16, 17] + [2] * 30 + [50, 4]]      # (the last: more sequences than places by sequence are worth)
+
+
+def delta_args(lens, seed, H=2, D=64, inner=8):
+    rnd, HD = draw(seed), H * D
+    rows, seq_rows, seq_slot = batch(lens)
+    return dict(rows=rows, H=H, D=D, HD=HD, inner=inner, seq_rows=seq_rows, seq_slot=seq_slot, seqs=len(lens), longest=max(lens), proj=1.2 * rnd(rows, 5 * HD + inner),
+                w2t=0.5 * rnd(inner, HD), w0=rnd(HD), a_b=0.5 * rnd(HD), state=0.3 * rnd(len(lens) + 1, H, D, D))
+
+
+def delta_run(a, chunks=None, below=None, pack_chunks=None, write_state=True):
+    """(outputs, states) of the chunked path over sequences of at least ``chunks`` rows, the row by row path over those below ``below``."""
+    from borrowed_compute_b200 import ops
+
+    state, out = a["state"].clone(), torch.full((a["rows"], a["HD"]), 7.0, device=DEV)
+    decay, unit, removal = (torch.full((a["rows"], a["HD"]), float("nan"), device=DEV) for _ in range(3))
+    dots = torch.full((a["rows"], a["H"], 2), float("nan"), device=DEV)
+    if chunks is not None:
+        need = ops.delta_chunked_scratch(a["rows"], a["seqs"], a["H"], a["D"], a["inner"], 0.6, write_state, min_rows=chunks)
+        assert need > 0
+        if pack_chunks is not None:
+            need = pack_chunks * a["seqs"] * a["H"] * (4 * 16 * 64 + 16 * 20 + 64)
+        pack = torch.full((need,), float("nan"), device=DEV)
+        ops.delta_chunked(a["proj"], a["w2t"], a["w0"], a["a_b"], decay, pack, state, a["seq_rows"], a["seq_slot"], out, a["seqs"], a["longest"], a["H"], a["D"],
+                          0.6, 1e-6, write_state=write_state, min_rows=chunks)
+    if below is not None:
+        ops.delta_prepare(a["proj"], a["w2t"], a["w0"], a["a_b"], decay, unit, removal, dots, a["H"], a["D"], 0.6, 1e-6, a["seq_rows"], a["seqs"], below)
+        ops.delta_scan(a["proj"], decay, unit, removal, dots, state, a["seq_rows"], a["seq_slot"], out, a["seqs"], a["H"], a["D"], write_state=write_state, below=below)
+    return out, state
+
+
+def linear_args(lens, seed, H=2, N=24, P=36, rank=8):
+    rnd, hd, hp = draw(seed), H * N, H * P
+    rows, seq_rows, seq_slot = batch(lens)
+    return dict(rows=rows, H=H, N=N, P=P, hd=hd, hp=hp, rank=rank, seq_rows=seq_rows, seq_slot=seq_slot, seqs=len(lens), longest=max(lens),
+                proj=rnd(rows, 2 * hd + 2 * hp + rank), w2t=0.5 * rnd(rank, hd), bias=rnd(hd), state=0.3 * rnd(len(lens) + 1, H, P, N))
+
+
+def linear_run(a, chunks=None, below=None, pack_chunks=None, write_state=True):
+    from borrowed_compute_b200 import ops
+
+    H, N, P, hd, hp = (a[k] for k in ("H", "N", "P", "hd", "hp"))
+    state, out, decay = a["state"].clone(), torch.full((a["rows"], hp), 7.0, device=DEV), torch.full((a["rows"], hd), float("nan"), device=DEV)
+    proj, inner_at = a["proj"], 2 * hd + 2 * hp
+    if chunks is not None:
+        need = ops.gla_chunked_scratch(proj, 2 * hd, a["seqs"], H, N, P, a["rank"], write_state, min_rows=chunks)
+        assert need > 0
+        if pack_chunks is not None:
+            need = pack_chunks * a["seqs"] * H * (2 * 16 * 64 + 16 * 20 + 64)
+        pack = torch.full((need,), float("nan"), device=DEV)
+        ops.gla_chunked(proj, 0, hd, 2 * hd, inner_at, a["w2t"], a["bias"], 16.0, 0.2, pack, state, a["seq_rows"], a["seq_slot"], out, a["seqs"], a["longest"], H, N, P,
+                        write_state=write_state, min_rows=chunks)
+    if below is not None:
+        ops.gla_decay(proj, inner_at, a["w2t"], a["bias"], decay, 16.0, a["seq_rows"], a["seqs"], below)
+        ops.linear_scan(proj, 0, 1, proj, hd, 1, proj, 2 * hd, decay, 0, True, None, 0, None, 0.2, state, a["seq_rows"], a["seq_slot"], out, a["seqs"], H, N, P,
+                        write_state=write_state, below=below)
+    return out, state
+
+
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+@pytest.mark.parametrize("lens", MIXED, ids=["few", "two", "many"])
+def test_each_sequence_goes_by_its_own_rows(lens, kind):
+    args, run = (delta_args, delta_run) if kind == "delta" else (linear_args, linear_run)
+    a = args(lens, 11)
+    chunked, scanned, nothing = run(a, chunks=0), run(a, below=10 ** 9), a["state"]
+    both, long, short = run(a, chunks=16, below=16), run(a, chunks=16), run(a, below=16)
+    small = run(a, chunks=16, below=16, pack_chunks=2)             # two chunks a sequence at a time
+    at = 0
+    for n, slot in zip(lens, a["seq_slot"].tolist()):
+        rows = slice(at, at + n)
+        at += n
+        if slot < 0:
+            assert all(bool((o[rows] == 7.0).all()) for o, _ in (both, long, short, small))
+            continue
+        want = chunked if n >= 16 else scanned
+        for got in (both, small, long if n >= 16 else short):
+            assert torch.equal(got[0][rows], want[0][rows]) and torch.equal(got[1][slot], want[1][slot]), (n, slot)
+        other = short if n >= 16 else long
+        assert bool((other[0][rows] == 7.0).all()) and torch.equal(other[1][slot], nothing[slot]), (n, slot)
+
+
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+def test_a_short_sequence_beside_a_long_one_has_the_bits_it_has_alone(kind):
+    """A part on bfloat16 rows.  Its matrices hold small whole numbers and its last one is the identity, so that the products are exact
+    however many rows share them."""
+    from borrowed_compute_b200.cache import PagedCache
+    from borrowed_compute_b200.engine import StepEntry, plan_step
+    from borrowed_compute_b200.parts import MIXERS, Runtime, StepContext
+
+    H, D, E, rank = 2, 64, 128, 8
+    part = MIXERS.get("generalized_delta")(hidden_size=E, heads=H, head_dim=D, decay_rank=rank, norm_eps=1e-5) if kind == "delta" else \
+        MIXERS.get("gated_linear_attention")(hidden_size=E, heads=H, head_dim=D, value_dim=D, decay_rank=rank, tau=16.0, norm_eps=1e-5)
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(5)
+    weights = {}
+    for name, spec in part.tensors().items():
+        t = torch.randint(-1, 2, spec.shape, generator=gen, device=DEV).float() / 8.0
+        weights[name] = torch.eye(E, device=DEV).bfloat16() if name == "o" else t if spec.role == "vector" else t.bfloat16()
+    lens = [5, 70, 1, 16, 15]
+    x = torch.randint(-1, 2, (sum(lens), E), generator=gen, device=DEV).bfloat16()
+    rt = Runtime(torch.device(DEV), torch.bfloat16, max_positions=128)
+    part.load(weights, rt)
+
+    def run(which):
+        n = [lens[i] for i in which]
+        cache = PagedCache(rt, [part.cache_need()], [part.state_need()], [None], max_tokens=64 * 2 * len(n), n_slots=len(n), max_seq=128)
+        slots = [cache.acquire() for _ in n]
+        cache.slots.reserve_many([(slot, k, k) for slot, k in zip(slots, n)])
+        cache.sync_tables()
+        plan = plan_step([StepEntry(slot, [0] * k) for slot, k in zip(slots, n)], [0] * len(n))
+        dev = lambda v: torch.from_numpy(v).to(DEV)       # noqa: E731
+        ctx = StepContext(rows=plan.rows, seqs=plan.seqs, tokens=dev(plan.tokens), row_pos=dev(plan.row_pos), row_slot=dev(plan.row_slot), seq_rows=dev(plan.seq_rows),
+                          seq_slot=dev(plan.seq_slot), seq_start=dev(plan.seq_start), max_new=plan.max_new, max_total=plan.max_total, decode=plan.decode,
+                          host_seq_rows=tuple(int(v) for v in plan.seq_rows), host_seq_slot=tuple(int(v) for v in plan.seq_slot),
+                          host_seq_start=tuple(int(v) for v in plan.seq_start))
+        at = [sum(lens[:i]) for i in which]
+        rows = torch.cat([x[a:a + k] for a, k in zip(at, n)])
+        out, mem = torch.zeros(rows.shape, device=DEV), cache.memory(0)
+        mem.state.zero_()
+        part.forward(rows, out, ctx, mem)
+        return list(out.split(n)), [mem.state[slot].clone() for slot in slots]
+
+    outs, states = run(range(len(lens)))
+    for i in range(len(lens)):
+        (out,), (state,) = run([i])
+        assert torch.equal(out, outs[i]) and torch.equal(state, states[i]), lens[i]
