@@ -146,7 +146,8 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
     const int n_chunks = min(span.first + span.count, (n_rows + CHUNK - 1) / CHUNK);
     if (span.first >= n_chunks) return;
     const int pv = min(32, P - p0);                                        // value channels that exist (a multiple of four)
-    // The values past the sequence's rows and past the head's channels are never copied: they stay zero.
+    // The values past the head's channels are never copied: they stay zero.  (Those past the sequence's last row are set to zero with its chunk,
+    // whose place may have held another's: rows of zeros in Z0, times an infinity, would be none.)
     for (int i = threadIdx.x; i < CHUNK_STAGES * CHUNK * 32; i += CHUNK_THREADS) chunk_smem[(i / (CHUNK * 32)) * STAGE + V_AT + i % (CHUNK * 32)] = 0.0f;
     __syncthreads();
     auto issue = [&](int c) {
@@ -156,6 +157,7 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
         for (int i = threadIdx.x; i < PACK / 4; i += CHUNK_THREADS) cp_async16(dst + 16 * i, src + 4 * i);
         const int rows = min(CHUNK, n_rows - c * CHUNK), t = threadIdx.x >> 3, at = 4 * (threadIdx.x & 7);
         if (t < rows && at < pv) cp_async16(dst + 4 * (V_AT + t * 32 + at), v + (size_t)(row0 + c * CHUNK + t) * v_stride + (size_t)h * P + p0 + at);
+        if (t >= rows) *reinterpret_cast<float4*>(chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE + V_AT + t * 32 + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     };
 #pragma unroll
     for (int i = 0; i < CHUNK_STAGES - 1; i++) {

@@ -272,3 +272,14 @@ def test_a_short_sequence_beside_a_long_one_has_the_bits_it_has_alone(kind):
     for i in range(len(lens)):
         (out,), (state,) = run([i])
         assert torch.equal(out, outs[i]) and torch.equal(state, states[i]), lens[i]
+
+
+def test_an_infinity_leaves_with_its_own_chunk():
+    """A last chunk of four rows takes the place of an earlier one that held an infinite value: the state keeps the sign it gave."""
+    a = linear_args([52, 1], 14)
+    a["proj"][8, 2 * a["hd"] + 3] = float("inf")                    # value channel 3 of head 0
+    (_, chunked), (_, scanned) = linear_run(a, chunks=0), linear_run(a, below=10 ** 9)
+    assert bool(torch.isinf(scanned[2, 0, 3]).all())
+    assert torch.equal(chunked[2, 0, 3], scanned[2, 0, 3])
+    chunked[2, 0, 3] = scanned[2, 0, 3] = 0.0
+    assert torch.allclose(chunked, scanned, rtol=1e-4, atol=1e-5)
