@@ -227,7 +227,8 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
         }
         if (p_ok && c * CHUNK + dg < n_rows)
             *reinterpret_cast<float4*>(out + (size_t)(row0 + c * CHUNK + dg) * H * P + (size_t)h * P + p0 + pg * PT) = make_float4(o[0], o[1], o[2], o[3]);
-        // The state after the chunk.
+        // The state after the chunk: what is removed first, then what is added (the other way round the sums carry parts that cancel: the state's
+        // distance from 64-bit sums 1.8 times as large).
         float s[DT][PT];
 #pragma unroll
         for (int m = 0; m < DT / 4; m++) {
@@ -236,18 +237,6 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
             for (int p = 0; p < PT; p++) {
                 unpack_f32x2(fma_f32x2(t2.x, S[2 * m][p], 0ull), s[4 * m][p], s[4 * m + 1][p]);
                 unpack_f32x2(fma_f32x2(t2.y, S[2 * m + 1][p], 0ull), s[4 * m + 2][p], s[4 * m + 3][p]);
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < CHUNK; r++) {
-#pragma unroll
-            for (int m = 0; m < DT / 4; m++) {
-                const float4 z = *reinterpret_cast<const float4*>(z0 + r * D + 64 * m);
-                const float zs[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], vr[r][p], s[4 * m + i][p]);
             }
         }
         if (DELTA) {
@@ -264,6 +253,18 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
 #pragma unroll
                         for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], es[p], s[4 * m + i][p]);
                 }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < CHUNK; r++) {
+#pragma unroll
+            for (int m = 0; m < DT / 4; m++) {
+                const float4 z = *reinterpret_cast<const float4*>(z0 + r * D + 64 * m);
+                const float zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], vr[r][p], s[4 * m + i][p]);
             }
         }
 #pragma unroll

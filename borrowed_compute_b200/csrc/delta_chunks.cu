@@ -11,13 +11,16 @@
 //
 //     X1 = P      X0 = r_t W_t - H P      G = Gm - H M      Z1 = b_s W_15 / W_s      Z0 = k_s W_15 / W_s - M^T Z1      tot = W_15.
 //
-// A decay is at least exp(-decay_scale), so sixteen of them are divided by safely up to a decay_scale of 4 (exp(-64)).  Float throughout.
+// A decay is at least exp(-decay_scale), so sixteen of them are divided by safely up to a decay_scale of 4 (exp(-64)).  Operands and results are
+// float; the sums over channels (A, Bm, H, Gm) and the correction of Z0 are double, and rows are decayed to a chunk's end by the products
+// of the decays after them.  With all of it in float the results were 1.1 to 1.9 times as far from 64-bit sums as the row scan's; so they
+// are 0.80 to 1.00 times as far (outputs) and 0.95 to 1.00 (state): 1.1e-7 and 0.9e-7 at a decay_scale of exp(-1/2), the scan 1.2e-7 and 1.0e-7.
 // Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
-// of 2,048 rows, 64 heads of 64, decay rank 64: 54 + 140 + 236 us, where preparing the rows and scanning them one by one takes 172 + 614.
-// The first two are bound by their instructions; the last walks 128 chunks at 1.9 us each, one warp a scheduler, each chunk's products
-// waiting for the state of the one before (IPC 0.3 to 0.6 in every layout tried: half warps or warps a row, four or eight value channels
-// a warp, sums across lanes or through shared memory, all within 3 % of one another).  Distance from 64-bit sums: 1.8e-7 of the
-// outputs and 1.4e-7 of the state, where the scan has 1.1e-7 and 0.9e-7.
+// of 2,048 rows, 64 heads of 64, decay rank 64: 485 us with the launches (421 with the packs in float), where the kernels that prepare the rows and
+// scan them one by one take 172 + 614 without.
+// The first two are bound by their instructions; the last walks 128 chunks, one warp a scheduler, each chunk's products waiting for the state of
+// the one before (half warps or warps a row, four or eight value channels a warp, sums across lanes or through shared memory: all within
+// 3 % of one another).
 #include "chunks.cuh"
 
 // ------------------------------------------------------------------------------------ decays
@@ -86,19 +89,19 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
 
 // ------------------------------------------------------------------------------------- packs
 #define DLC_D 64
-#define DLC_YP 36             // floats a channel of the 32 rows [r W; u W] and [b / W; k / W]: a gap against bank conflicts
+#define DLC_YP 34             // numbers a channel of the 32 rows [r W; u W] and [b / W; k / W]: a gap, so that 16-byte writes of eight channels meet no bank twice
 #define DLC_RUN 4             // places of chunks a block takes one after another, the next one's rows on their way
 
 // A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
 // columns through the same substitutions.
-__global__ void __launch_bounds__(DLC_D + 32, 4)
+__global__ void __launch_bounds__(DLC_D + 32, 3)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
                     const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
     constexpr int PACK = chunk_pack_floats(DLC_D, true), THREADS = DLC_D + 32, ROW_SET = CHUNK * DLC_D;
     extern __shared__ __align__(16) float delta_smem[];
     float (*in)[4][CHUNK][DLC_D] = reinterpret_cast<float (*)[4][CHUNK][DLC_D]>(delta_smem);            // two stages of decays, r, k, a
-    float *Y = delta_smem + 2 * 4 * ROW_SET, *X = Y + DLC_D * DLC_YP;
-    float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm; Bm becomes M
+    double *Y = reinterpret_cast<double*>(delta_smem + 2 * 4 * ROW_SET), *X = Y + DLC_D * DLC_YP, *M = Y;      // (M [16][16] where Y was, once that has been used)
+    float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm
     __shared__ float part[2][CHUNK];
     __shared__ ChunkAt todo[DLC_RUN];
     __shared__ int todo_place[DLC_RUN], n_todo;
@@ -170,9 +173,9 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         __syncthreads();
         float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
-        float total = 1.0f;
+        float z1[CHUNK], zk[CHUNK];               // b_t and k_t, then times the decays after row t
         if (channel) {
-            float run = 1.0f, xb[4], xk[4];
+            float run = 1.0f, xb_even = 0.0f, xk_even = 0.0f;
 #pragma unroll
             for (int t = 0; t < CHUNK; t++) {
                 const bool ok = mine && t < rows;
@@ -182,46 +185,53 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
                 U[t] = u * run;
                 run *= ok ? sw[t][d] : 1.0f;
                 own[t] = (ok ? sr[t][d] : 0.0f) * run;
-                const float over = 1.0f / run;
-                xb[t & 3] = rate * u * over;
-                xk[t & 3] = k * over;
-                if ((t & 3) == 3) {
-                    float *y = Y + d * DLC_YP + t - 3, *x = X + d * DLC_YP + t - 3;
-                    *reinterpret_cast<float4*>(y) = make_float4(own[t - 3], own[t - 2], own[t - 1], own[t]);
-                    *reinterpret_cast<float4*>(y + CHUNK) = make_float4(U[t - 3], U[t - 2], U[t - 1], U[t]);
-                    *reinterpret_cast<float4*>(x) = make_float4(xb[0], xb[1], xb[2], xb[3]);
-                    *reinterpret_cast<float4*>(x + CHUNK) = make_float4(xk[0], xk[1], xk[2], xk[3]);
+                const float over = 1.0f / run, xb = rate * u * over, xk = k * over;
+                z1[t] = rate * u;
+                zk[t] = k;
+                if (t & 1) {
+                    double *y = Y + d * DLC_YP + t - 1, *x = X + d * DLC_YP + t - 1;
+                    *reinterpret_cast<double2*>(y) = make_double2(own[t - 1], own[t]);
+                    *reinterpret_cast<double2*>(y + CHUNK) = make_double2(U[t - 1], U[t]);
+                    *reinterpret_cast<double2*>(x) = make_double2(xb_even, xb);
+                    *reinterpret_cast<double2*>(x + CHUNK) = make_double2(xk_even, xk);
                 }
+                xb_even = xb;
+                xk_even = xk;
             }
-            total = run;
+            // (From the last row back, not as the quotient of two products: the latest rows, which weigh most, then have the fewest roundings.)
+            run = 1.0f;
+#pragma unroll
+            for (int t = CHUNK - 1; t >= 0; t--) {
+                z1[t] *= run;
+                zk[t] *= run;
+                run *= mine && t < rows ? sw[t][d] : 1.0f;
+                dst[(3 * CHUNK + t) * DLC_D + d] = z1[t];
+            }
+            dst[4 * CHUNK * DLC_D + CHUNK * CHUNK_G + d] = run;
         }
         __syncthreads();
-        // [r W; u W] [b / W; k / W]^T over the channels: 32 x 32 sums, 4 x 4 a thread; those above the diagonals are left out.
+        // [r W; u W] [b / W; k / W]^T over the channels in double: 32 x 32 sums, four rows by two of b and two of k a thread; those above the
+        // diagonals are left out.
         if (channel) {
             const int ty = d >> 3, tx = d & 7;
-            uint64_t acc[4][2] = {};
-#pragma unroll 8
+            double acc[4][4] = {};
+#pragma unroll 4
             for (int i = 0; i < DLC_D; i++) {
-                const float4 yy = *reinterpret_cast<const float4*>(Y + i * DLC_YP + 4 * ty);
-                const ulonglong2 xx = *reinterpret_cast<const ulonglong2*>(X + i * DLC_YP + 4 * tx);
-                const float ys[4] = {yy.x, yy.y, yy.z, yy.w};
+                const double2 ya = *reinterpret_cast<const double2*>(Y + i * DLC_YP + 4 * ty), yb = *reinterpret_cast<const double2*>(Y + i * DLC_YP + 4 * ty + 2);
+                const double2 xb = *reinterpret_cast<const double2*>(X + i * DLC_YP + 2 * tx), xk = *reinterpret_cast<const double2*>(X + i * DLC_YP + CHUNK + 2 * tx);
+                const double ys[4] = {ya.x, ya.y, yb.x, yb.y}, xs[4] = {xb.x, xb.y, xk.x, xk.y};
 #pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const uint64_t y2 = pack_f32x2(ys[a], ys[a]);
-                    acc[a][0] = fma_f32x2(y2, xx.x, acc[a][0]);
-                    acc[a][1] = fma_f32x2(y2, xx.y, acc[a][1]);
-                }
+                for (int a = 0; a < 4; a++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[a][e] = fma(ys[a], xs[e], acc[a][e]);
             }
-            const int which = (ty >= 4 ? 0 : 2) + (tx >= 4 ? 1 : 0), t0 = 4 * (ty & 3), s0 = 4 * (tx & 3);
+            const int t0 = 4 * (ty & 3);
 #pragma unroll
             for (int a = 0; a < 4; a++)
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    float lo, hi;
-                    unpack_f32x2(acc[a][e], lo, hi);
-                    const int t = t0 + a, s = s0 + 2 * e, most = ty >= 4 ? t - 1 : t;      // s < t in A and Bm, or s <= t
-                    lower[which][t][s] = s <= most ? lo : 0.0f;
-                    lower[which][t][s + 1] = s + 1 <= most ? hi : 0.0f;
+                for (int e = 0; e < 4; e++) {
+                    const int t = t0 + a, s = 2 * tx + (e & 1), most = ty >= 4 ? t - 1 : t;      // s < t in A and Bm, or s <= t
+                    lower[(ty >= 4 ? 0 : 2) + (e >> 1)][t][s] = s <= most ? (float)acc[a][e] : 0.0f;
                 }
         }
         __syncthreads();
@@ -246,7 +256,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             if (lane < CHUNK) {
 #pragma unroll
                 for (int t = 0; t < CHUNK; t++) {
-                    lower[1][t][lane] = U[t];
+                    M[t * CHUNK + lane] = U[t];
                     dst[4 * CHUNK * DLC_D + t * CHUNK_G + lane] = own[t];
                 }
             }
@@ -259,24 +269,26 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         }
         __syncthreads();
         if (channel) {
-            float z0[CHUNK];
+            double z0[CHUNK];
 #pragma unroll
-            for (int s = 0; s < CHUNK; s++) z0[s] = X[d * DLC_YP + CHUNK + s] * total;
+            for (int s = 0; s < CHUNK; s++) z0[s] = zk[s];
 #pragma unroll
-            for (int t = 0; t < CHUNK; t++) {
-                const float z1 = X[d * DLC_YP + t] * total;
-                dst[(3 * CHUNK + t) * DLC_D + d] = z1;
+            for (int t = 1; t < CHUNK; t++) {
+                const double z = -z1[t];
 #pragma unroll
-                for (int s = 0; s < t; s++) z0[s] = fmaf(-lower[1][t][s], z1, z0[s]);
+                for (int s = 0; s < t; s += 2) {
+                    const double2 m = *reinterpret_cast<const double2*>(M + t * CHUNK + s);
+                    z0[s] = fma(m.x, z, z0[s]);
+                    if (s + 1 < t) z0[s + 1] = fma(m.y, z, z0[s + 1]);
+                }
             }
 #pragma unroll
-            for (int s = 0; s < CHUNK; s++) dst[(2 * CHUNK + s) * DLC_D + d] = z0[s];
-            dst[4 * CHUNK * DLC_D + CHUNK * CHUNK_G + d] = total;
+            for (int s = 0; s < CHUNK; s++) dst[(2 * CHUNK + s) * DLC_D + d] = (float)z0[s];
         }
         __syncthreads();          // the next chunk writes Y, X and the triangles
     }
 }
-#define DLC_SMEM ((2 * 4 * CHUNK * DLC_D + 2 * DLC_D * DLC_YP + 4 * CHUNK * CHUNK_G) * sizeof(float))
+#define DLC_SMEM ((2 * 4 * CHUNK * DLC_D + 4 * CHUNK * CHUNK_G) * sizeof(float) + 2 * DLC_D * DLC_YP * sizeof(double))
 
 // Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not), of which those of
 // fewer than min_rows rows are left alone.
@@ -312,9 +324,9 @@ extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t,
         e = chunk_step(
             capacity, rows, seqs, max_new, min_rows,
             [&](const ChunkSpan& span, long long places) {
-                // Four chunks a block hide the loads of the next one (128 chunks of 64 heads: 232 us one a block, 143 four); where that leaves
+                // Four chunks a block hide the loads of the next one (128 chunks of 64 heads, all in float: 232 us one a block, 143 four); where that leaves
                 // places on the SMs empty, one (with the rest of a call, 64 heads: 4 sequences of 64 rows 92 us four a block, 83 one; 8 heads: one of 64 rows 67 and 47).
-                const int run = (places + DLC_RUN - 1) / DLC_RUN * H >= 4 * bc_sm_count() ? DLC_RUN : 1;
+                const int run = (places + DLC_RUN - 1) / DLC_RUN * H >= 3 * bc_sm_count() ? DLC_RUN : 1;
                 return bc_launch(delta_chunks_kernel, dim3((unsigned)((places + run - 1) / run), H), dim3(DLC_D + 32), DLC_SMEM, s, span, proj, stride, decay, a_bias, seq_rows, seq_slot, pack, H, D,
                                  key_eps, seqs, n_slots, run, (int)places);
             },
