@@ -131,7 +131,7 @@ template <int PT> __device__ __forceinline__ void chunk_groups(const float (*g)[
 template <int DL, bool DELTA>      // D = 32 DL
 __global__ void __launch_bounds__(CHUNK_THREADS)
 chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v_stride, float* __restrict__ state, const int* __restrict__ seq_rows,
-                  const int* __restrict__ seq_slot, float* __restrict__ out, int H, int N, int P, int n_slots, int write_state) {
+                  const int* __restrict__ seq_slot, float* __restrict__ out, int H, int N, int P, int n_slots, int write_state, float out_scale) {
     constexpr int DT = 2 * DL, D = 16 * DT, PT = 4, MATS = DELTA ? 4 : 2, PACK = chunk_pack_floats(D, DELTA), V_AT = PACK, STAGE = V_AT + CHUNK * 32;
     extern __shared__ __align__(16) float chunk_smem[];
     const int dg = threadIdx.x & 15, pg = threadIdx.x >> 4;
@@ -214,32 +214,42 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
         }
         chunk_groups<PT>(of_group, o);
         // The rows' own part, G V: this lane's row of G against the values up to its own (later rows' are not touched: a zero of G times
-        // an infinity would be none).
+        // an infinity would be none).  Without what is removed, the first eight rows' sum is taken by itself: fewer roundings of the whole.
+        float own[PT] = {};
 #pragma unroll
         for (int s4 = 0; s4 < CHUNK / 4; s4++) {
             const float4 gg = *reinterpret_cast<const float4*>(g + dg * CHUNK_G + 4 * s4);
             const float gs[4] = {gg.x, gg.y, gg.z, gg.w};
+            if (!DELTA && s4 == 2)
+#pragma unroll
+                for (int p = 0; p < PT; p++) o[p] += own[p];
+            float* to = !DELTA && s4 < 2 ? own : o;
 #pragma unroll
             for (int e = 0; e < 4; e++)
 #pragma unroll
                 for (int p = 0; p < PT; p++)
-                    if (4 * s4 + e <= dg) o[p] = fmaf(gs[e], vr[4 * s4 + e][p], o[p]);
+                    if (4 * s4 + e <= dg) to[p] = fmaf(gs[e], vr[4 * s4 + e][p], to[p]);
         }
         if (p_ok && c * CHUNK + dg < n_rows)
-            *reinterpret_cast<float4*>(out + (size_t)(row0 + c * CHUNK + dg) * H * P + (size_t)h * P + p0 + pg * PT) = make_float4(o[0], o[1], o[2], o[3]);
-        // The state after the chunk: what is removed first, then what is added (the other way round the sums carry parts that cancel: the state's
-        // distance from 64-bit sums 1.8 times as large).
+            *reinterpret_cast<float4*>(out + (size_t)(row0 + c * CHUNK + dg) * H * P + (size_t)h * P + p0 + pg * PT) = make_float4(out_scale * o[0], out_scale * o[1], out_scale * o[2], out_scale * o[3]);
+        // The state after the chunk.  Of a delta rule: what was, less what is removed, then what is added (removed last, the sums carry parts that
+        // cancel: 1.8 times as far from 64-bit sums).  Else: twelve rows' sum from nothing, what was, the last four rows (what was first: 1.1 times
+        // as far where decays are slow; what was last: 1.2 times where they are fast).
         float s[DT][PT];
+        auto decayed = [&](bool first) {
 #pragma unroll
-        for (int m = 0; m < DT / 4; m++) {
-            const ulonglong2 t2 = *reinterpret_cast<const ulonglong2*>(tot + 4 * dg + 64 * m);
+            for (int m = 0; m < DT / 4; m++) {
+                const ulonglong2 t2 = *reinterpret_cast<const ulonglong2*>(tot + 4 * dg + 64 * m);
 #pragma unroll
-            for (int p = 0; p < PT; p++) {
-                unpack_f32x2(fma_f32x2(t2.x, S[2 * m][p], 0ull), s[4 * m][p], s[4 * m + 1][p]);
-                unpack_f32x2(fma_f32x2(t2.y, S[2 * m + 1][p], 0ull), s[4 * m + 2][p], s[4 * m + 3][p]);
+                for (int p = 0; p < PT; p++) {
+                    const uint64_t lo = first ? 0ull : pack_f32x2(s[4 * m][p], s[4 * m + 1][p]), hi = first ? 0ull : pack_f32x2(s[4 * m + 2][p], s[4 * m + 3][p]);
+                    unpack_f32x2(fma_f32x2(t2.x, S[2 * m][p], lo), s[4 * m][p], s[4 * m + 1][p]);
+                    unpack_f32x2(fma_f32x2(t2.y, S[2 * m + 1][p], hi), s[4 * m + 2][p], s[4 * m + 3][p]);
+                }
             }
-        }
+        };
         if (DELTA) {
+            decayed(true);
 #pragma unroll
             for (int r = 0; r < CHUNK; r++) {
                 const float4 e4 = *reinterpret_cast<const float4*>(mine + r * PT);
@@ -254,9 +264,15 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
                         for (int p = 0; p < PT; p++) s[4 * m + i][p] = fmaf(zs[i], es[p], s[4 * m + i][p]);
                 }
             }
+        } else {
+#pragma unroll
+            for (int i = 0; i < DT; i++)
+#pragma unroll
+                for (int p = 0; p < PT; p++) s[i][p] = 0.0f;
         }
 #pragma unroll
         for (int r = 0; r < CHUNK; r++) {
+            if (!DELTA && r == 12) decayed(false);
 #pragma unroll
             for (int m = 0; m < DT / 4; m++) {
                 const float4 z = *reinterpret_cast<const float4*>(z0 + r * D + 64 * m);
@@ -288,11 +304,11 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
 
 template <int DL, bool DELTA>
 static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, const float* v, int v_stride, float* state, const int* seq_rows, const int* seq_slot,
-                                     float* out, int seqs, int H, int N, int P, int n_slots, int write_state, cudaStream_t s) {
+                                     float* out, int seqs, int H, int N, int P, int n_slots, int write_state, float out_scale, cudaStream_t s) {
     constexpr size_t SMEM = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
     if (cudaError_t e = bc_allow_shared<chunk_scan_kernel<DL, DELTA>>(SMEM); e != cudaSuccess) return e;
     return bc_launch(chunk_scan_kernel<DL, DELTA>, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H,
-                     N, P, n_slots, write_state);
+                     N, P, n_slots, write_state, out_scale);
 }
 
 // A step's chunks through `prepare` (the kernel that fills the pack) and the scan: at once where `capacity` chunks of scratch hold them, else

@@ -2,11 +2,13 @@
 //
 //     S_t = diag(a_t) S_(t-1) + k_t v_t^T        o_t = f S_t^T q_t,        a = sigmoid(z)^(1/tau), z = W_2 inner + b
 //
-// With A(s, t) the product of the decays of rows s + 1 .. t of a chunk: X0 = f q_t A(-1, t), Z0 = k_s A(s, last), tot = A(-1, last) and
-// G_ts = f sum_i q_ti k_si A(s, t)_i for s <= t.  No decay is ever divided by, so decays of zero are as good as any.  Float throughout.
+// With A(s, t) the product of the decays of rows s + 1 .. t of a chunk: X0 = q_t A(-1, t), Z0 = k_s A(s, last), tot = A(-1, last) and
+// G_ts = sum_i q_ti k_si A(s, t)_i for s <= t; f multiplies the finished sums.  No decay is ever divided by, so decays of zero are as good as any.
+// Float throughout, but for the products of decays in X0, Z0 and tot: those are double and rounded once (a state that decays slowly is
+// multiplied by tot again and again).
 // Sequences of 400, 1,100 and 1,800 rows, 16 heads of 128 x 256: 60 + 315 us, where the decays and the scan row by row take 52 + 764.  The scan
-// in chunks is bound by the longest sequence's 113 chunks, one after another (IPC 0.6 while all sequences run).  Distance from 64-bit
-// sums as the scan's (2.4e-7 and 2.5e-7 against 2.3e-7 and 2.5e-7).
+// in chunks is bound by the longest sequence's 113 chunks, one after another.  Distance from 64-bit sums: 0.94 to 1.01 times the row scan's
+// (outputs) and 0.93 to 0.99 (state); with float products of decays and one running sum 1.00 to 1.12 times.
 #include "chunks.cuh"
 
 #define GLC_PAIRS (CHUNK * (CHUNK + 1) / 2)      // 136
@@ -26,8 +28,8 @@ template <int I, class F> __device__ __forceinline__ void glc_each(F&& f) {
 template <int D>
 __global__ void __launch_bounds__(D)
 gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at, int k_at, int inner_at, const float* __restrict__ w2t, const float* __restrict__ b,
-                  int rank, const int* __restrict__ seq_rows, const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int N, float inv_tau, float f,
-                  int seqs, int n_slots) {
+                  int rank, const int* __restrict__ seq_rows, const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int N, float inv_tau, int seqs,
+                  int n_slots) {
     constexpr int WARPS = D / 32, PACK = chunk_pack_floats(D, false);
     extern __shared__ __align__(16) float inner[];           // [rank][16]
     __shared__ float part[WARPS][160];
@@ -50,7 +52,7 @@ gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at,
 #pragma unroll
     for (int t = 0; t < CHUNK; t++) {
         const bool ok = mine && t < rows;
-        q[t] = ok ? p[(size_t)t * stride + q_at + col] * f : 0.0f;
+        q[t] = ok ? p[(size_t)t * stride + q_at + col] : 0.0f;
         k[t] = ok ? p[(size_t)t * stride + k_at + col] : 0.0f;
         a[t] = b[col];
     }
@@ -68,17 +70,17 @@ gla_chunks_kernel(const ChunkSpan span, const float* proj, int stride, int q_at,
         a[t] = mine && t < rows ? expf(-sp * inv_tau) : 1.0f;
     }
     float* dst = pack + ((size_t)blockIdx.x * H + h) * PACK;
-    float run = 1.0f;
+    double run = 1.0;
 #pragma unroll
     for (int t = 0; t < CHUNK; t++) {
         run *= a[t];
-        dst[t * D + n] = q[t] * run;
+        dst[t * D + n] = (float)(q[t] * run);
     }
-    dst[2 * CHUNK * D + CHUNK * CHUNK_G + n] = run;
-    run = 1.0f;
+    dst[2 * CHUNK * D + CHUNK * CHUNK_G + n] = (float)run;
+    run = 1.0;
 #pragma unroll
     for (int t = CHUNK - 1; t >= 0; t--) {
-        dst[(CHUNK + t) * D + n] = k[t] * run;
+        dst[(CHUNK + t) * D + n] = (float)(k[t] * run);
         run *= a[t];
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -134,10 +136,10 @@ static int gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_
         pack_floats / ((long long)H * chunk_pack_floats(D, false)), rows, seqs, max_new, min_rows,
         [&](const ChunkSpan& span, long long places) {
             return bc_launch(gla_chunks_kernel<D>, dim3((unsigned)places, H), dim3(D), (size_t)rank * CHUNK * sizeof(float), s, span, proj, stride, q_at, k_at, inner_at,
-                             w2t, b, rank, seq_rows, seq_slot, pack, H, N, inv_tau, f, seqs, n_slots);
+                             w2t, b, rank, seq_rows, seq_slot, pack, H, N, inv_tau, seqs, n_slots);
         },
         [&](const ChunkSpan& span) {
-            return chunk_scan_launch<D / 32, false>(span, pack, proj + v_at, stride, state, seq_rows, seq_slot, out, seqs, H, N, P, n_slots, write_state, s);
+            return chunk_scan_launch<D / 32, false>(span, pack, proj + v_at, stride, state, seq_rows, seq_slot, out, seqs, H, N, P, n_slots, write_state, f, s);
         });
     if (e != cudaSuccess) {
         bc_set_error("gla_chunked: %s", cudaGetErrorString(e));

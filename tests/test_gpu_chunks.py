@@ -321,3 +321,34 @@ def test_delta_chunks_are_no_further_from_64_bit_sums_than_the_scan(scale):
                 sums[way, what] = sums.get((way, what), 0.0) + value ** 2
     for what in ("outputs", "state"):
         assert sums["chunks", what] <= 1.05 ** 2 * sums["scan", what], (what, sums)
+
+
+@pytest.mark.parametrize("tau", [1.0, 16.0, 100.0])
+def test_linear_chunks_are_no_further_from_64_bit_sums_than_the_scan(tau):
+    from borrowed_compute_b200 import ops
+
+    T, H, N, P, rank = 256, 4, 128, 64, 16
+    hd, hp, f, sums = H * N, H * P, N ** -0.5, {}
+    for seed in range(4):
+        rnd = draw(200 + seed)
+        proj, w2t, bias, before = rnd(T, 2 * hd + 2 * hp + rank), rnd(rank, hd) / rank ** 0.5, rnd(hd), 0.3 * rnd(1, H, P, N)
+        p = proj.double()
+        q, k, v = f * p[:, :hd].view(T, H, N), p[:, hd:2 * hd].view(T, H, N), p[:, 2 * hd:2 * hd + hp].view(T, H, P)
+        a = torch.exp(torch.nn.functional.logsigmoid(p[:, 2 * hd + 2 * hp:] @ w2t.double() + bias.double()) / tau).view(T, H, N)
+        want, S = torch.empty(T, H, P, dtype=torch.float64, device=DEV), before[0].double().transpose(1, 2)
+        for t in range(T):
+            S = a[t][..., None] * S + k[t][..., None] * v[t][:, None]
+            want[t] = torch.bmm(q[t][:, None], S)[:, 0]
+        for way in ("scan", "chunks"):
+            state, out = before.clone(), torch.empty((T, hp), device=DEV)
+            if way == "scan":
+                decay = torch.empty((T, hd), device=DEV)
+                ops.gla_decay(proj, 2 * hd + 2 * hp, w2t, bias, decay, tau)
+                ops.linear_scan(proj, 0, 1, proj, hd, 1, proj, 2 * hd, decay, 0, True, None, 0, None, f, state, i32([0, T]), i32([0]), out, 1, H, N, P)
+            else:
+                pack = torch.empty((ops.gla_chunked_scratch(proj, 2 * hd, 1, H, N, P, rank),), device=DEV)
+                ops.gla_chunked(proj, 0, hd, 2 * hd, 2 * hd + 2 * hp, w2t, bias, tau, f, pack, state, i32([0, T]), i32([0]), out, 1, T, H, N, P)
+            for what, value in (("outputs", distance(out, want.view(T, hp))), ("state", distance(state[0], S.transpose(1, 2)))):
+                sums[way, what] = sums.get((way, what), 0.0) + value ** 2
+    for what in ("outputs", "state"):
+        assert sums["chunks", what] <= 1.05 ** 2 * sums["scan", what], (what, sums)
