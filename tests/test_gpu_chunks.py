@@ -352,3 +352,33 @@ def test_linear_chunks_are_no_further_from_64_bit_sums_than_the_scan(tau):
                 sums[way, what] = sums.get((way, what), 0.0) + value ** 2
     for what in ("outputs", "state"):
         assert sums["chunks", what] <= 1.05 ** 2 * sums["scan", what], (what, sums)
+
+
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+@pytest.mark.parametrize("pack_chunks", [None, 4, 5])
+def test_segments_of_several_chunks(kind, pack_chunks):
+    """A pack that holds four or five chunks a sequence: the same bits as with all of them at once."""
+    args, run = (delta_args, delta_run) if kind == "delta" else (linear_args, linear_run)
+    a = args([150, 64, 65, 3], 12)
+    whole, got = run(a, chunks=0), run(a, chunks=0, pack_chunks=pack_chunks)
+    assert all(torch.equal(x, y) for x, y in zip(whole, got))
+
+
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+def test_a_state_that_is_only_read(kind):
+    from borrowed_compute_b200 import ops
+
+    args, run = (delta_args, delta_run) if kind == "delta" else (linear_args, linear_run)
+    a = args([50, 17, 16, 3], 13)
+    writing, reading = run(a, chunks=16, below=16), run(a, chunks=16, below=16, write_state=False)
+    assert torch.equal(writing[0], reading[0]) and torch.equal(reading[1], a["state"]) and not torch.equal(writing[1], a["state"])
+    with pytest.raises(ops.KernelError):             # segments hand the state on through memory
+        run(a, chunks=0, pack_chunks=1, write_state=False)
+    many = 10 ** 6                                   # rows whose packs are past what a step is given
+    if kind == "delta":
+        assert ops.delta_chunked_scratch(many, 1, 64, 64, 64, 0.6, False) == 0 < ops.delta_chunked_scratch(many, 1, 64, 64, 64, 0.6, True) <= 2 ** 28
+    else:
+        proj = torch.empty((0, 64), device=DEV).expand(0, 64)
+        big = torch.empty((1, 64), device=DEV).expand(many, 64)
+        assert ops.gla_chunked_scratch(proj, 0, 1, 64, 256, 4, 4, False) > 0
+        assert ops.gla_chunked_scratch(big, 0, 1, 64, 256, 4, 4, False) == 0 < ops.gla_chunked_scratch(big, 0, 1, 64, 256, 4, 4, True) <= 2 ** 28

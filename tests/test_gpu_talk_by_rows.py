@@ -104,3 +104,45 @@ def test_operands_a_warp_a_head(dtype, H, G, D, rot, extra):
                 want_k[page, :, pos[r] % 64], want_v[page, :, pos[r] % 64] = unit[r, H:], z[r, H:]
         assert (k.double() - want_k).abs().max() <= tol * max(unit.abs().max(), 1.0)
         assert (v.double() - want_v).abs().max() <= tol * max(z.abs().max(), 1.0)
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("H,G,D", [(16, 8, 64), (32, 8, 128)])
+def test_more_tiles_than_pages_are_kept(H, G, D, splits):
+    """A block keeps the pages of its first 256 tiles of 32 positions and looks the others up: rows that see 8,300 positions without a window, a
+    page that is not held and a last page that is not full beyond them."""
+    from borrowed_compute_b200 import ops
+
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(H)
+    rnd = lambda *shape: torch.randn(*shape, generator=gen, device=DEV)       # noqa: E731
+    held, n, scale, cap = 8297, 9, 1.5 / D ** 0.5, 6.0
+    total = held + n
+    pages = -(-total // 64)
+    table = torch.randperm(pages, generator=gen, device=DEV).int()
+    k, v = rnd(pages, G, 64, D).bfloat16(), rnd(pages, G, 64, D).bfloat16()
+    for t in (k, v):
+        t[table[-1].long(), :, (total - 1) % 64 + 1:] = float("nan")
+    kk, vv = (t[table.long()].permute(1, 0, 2, 3).reshape(G, -1, D)[:, :total].double().repeat_interleave(H // G, 0) for t in (k, v))
+    gone = torch.zeros(total, dtype=torch.bool, device=DEV)
+    for page in (3, 128):
+        gone[page * 64:(page + 1) * 64] = True
+        table[page] = -1
+    # Some weight on every part: the positions past the 256th tile are as likely as the others, so a wrong page among them shows.
+    q, gate = rnd(n, H * D).bfloat16(), torch.sigmoid(rnd(n, H * D))
+    temp, talk = 1.0 + 0.2 * rnd(H), torch.eye(H, device=DEV) + 0.3 * rnd(H, H) / H ** 0.5
+    kk[:, 8192:] *= 3.0
+    k[table[129].long(), :, :] *= 3.0
+    raw = torch.einsum("rhd,hnd->hrn", q.view(n, H, D).double(), kk) * scale * temp.double()[:, None, None]
+    mixed = torch.einsum("hm,mrn->hrn", talk.double(), cap * torch.tanh(raw / cap))
+    i, j = torch.arange(held, total, device=DEV)[:, None], torch.arange(total, device=DEV)[None]
+    p = torch.softmax(mixed.masked_fill(~((j <= i) & ~gone), -float("inf")), -1)
+    ref = torch.einsum("hrn,hnd->rhd", p, vv).reshape(n, -1) * gate.double()
+    assert p[:, :, 8256:].sum(-1).mean() > 0.02
+    out = torch.full((n, H * D), 3.0, dtype=torch.bfloat16, device=DEV)
+    ops.talk_tiles(q, k, v, table[None].contiguous(), i32([0, n]), i32([0]), i32([held]), gate, temp, talk, out, 1, n, H, G, D, 0, 0, scale, cap, splits=splits,
+                   row_slot=i32([0] * n))
+    # (8,300 weights of about the same size: the largest value that a result has is far below the largest value that it is a mean of)
+    assert (out.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 1e-4
+    without = torch.einsum("hrn,hnd->rhd", torch.softmax(mixed.masked_fill(~((j <= i) & ~gone & (j < 8192)), -float("inf")), -1), vv).reshape(n, -1) * gate.double()
+    assert (without - ref).abs().max() > 4 * (2.0 ** -8 * ref.abs().max() + 1e-4)
