@@ -312,7 +312,8 @@ delta_finish_kernel(const float* o, const float* gate, int gate_stride, const fl
 // A step of one row a sequence: prepare, one step of the scan and finish in one launch, a block a (row, head)
 // with eight threads a value channel.  Every sum is taken by the same threads in the same order as in the three
 // kernels above (thread d holds channel d in the sums over a head), so a row decoded alone and the same row in a
-// prompt give the same bits.  Heads of up to 128 channels.
+// prompt that those take give the same bits.  (A bfloat16 prompt of sixteen rows or more goes by delta_chunks.cu, whose sums are in
+// another order.)  Heads of up to 128 channels.
 template <int R, class T>
 __global__ void __launch_bounds__(64 * R)
 delta_step_kernel(const float* __restrict__ proj, int stride, const float* __restrict__ w2t, const float* __restrict__ w0,

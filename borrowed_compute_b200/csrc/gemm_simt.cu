@@ -61,7 +61,7 @@ __device__ __forceinline__ void simt_emit(T* out_act, float* out_f32, int m, int
 
 // A tile of BM rows by 128 weight rows a block (SwiGLU: 64 gate rows and their 64 up rows), 128 threads, TM x TN sums each, two to an
 // instruction (fma.rn.f32x2: the roundings of fmaf).  The next sixteen k are on their way to registers while these are multiplied, into the
-// other of two buffers.  BM 64: 8 x 8 a thread, 16 LDS bytes for every eight multiply-adds; BM 16 (few rows): 4 x 4, and what counts is that
+// other of two buffers.  BM 64: 8 x 8 a thread, 64 bytes of shared memory for its 64 multiply-adds a k; BM 16 (few rows): 4 x 4, and what counts is that
 // the weights stream.  With several pieces of K the blocks of a tile are one cluster and add up through one another's shared memory.
 // (64 x 64 tiles, 4 x 4 a thread, one buffer: 720 + 763 us for 300 rows of a feed-forward of 2,048 x 8,192, 20 TFLOP/s; now
 // 557 + 311 us.)

@@ -1158,7 +1158,7 @@ static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupP
     int stages = (TC_SMEM_LIMIT - 1024) / STAGE_BYTES;
     if (stages > 12) stages = 12;
     // Few rows a matrix: the product streams weights; a block a piece and two on an SM, which come and go as they end, share the bytes out better
-    // than a fixed number of pieces an SM (174 + 86 against 181 + 94 us for 256 rows of 32 matrices).
+    // than a fixed number of pieces an SM (160 + 88 against 181 + 94 us for 256 rows of 32 matrices).
     const int half_stages = (TC_SMEM_LIMIT / 2 - 2048) / STAGE_BYTES;
     const bool stream = BN <= 64 && half_stages >= 3;
     if (stream && stages > half_stages) stages = half_stages;

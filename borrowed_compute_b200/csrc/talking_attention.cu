@@ -919,7 +919,8 @@ extern "C" int bc_talk_tiles_accepts(int H, int G, int D) {
 }
 
 // Whether the mix goes by rows: sixteen or thirty-two heads whose keys of a position are 512 values a sixteen heads.  (Wider ones leave the mixed
-// scores no room, of other numbers a warp's sixteen rows are not whole heads or pairs: those stay with the kernel that mixes by heads.)
+// scores no room, of other numbers a warp's sixteen rows are not whole heads or pairs.  Fewer kv heads would fit; the kernel has their number as a
+// constant and has not been built for them.  All those stay with the kernel that mixes by heads.)
 static bool tp_takes(int H, int G, int D) { return (D == 64 || D == 128) && (H == TP_WARPS || H == 2 * TP_WARPS) && G * D == 32 * H; }
 
 // Blocks that the rows of a sequence with up to max_new new ones take (times the splits).

@@ -1406,8 +1406,8 @@ def talk_tiles(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pa
                seq_start: torch.Tensor, gate: torch.Tensor, temp: torch.Tensor, talk: torch.Tensor, out: torch.Tensor, seqs: int, max_new: int,
                heads: int, kv_heads: int, head_dim: int, window: int, keep_first: int, scale: float, cap: float, splits: int = 1,
                row_slot: Optional[torch.Tensor] = None) -> None:
-    """What talk_rows computes, for bf16 on mma.sync tiles: a block owns sixteen rows of one sequence and all heads, so that
-    every head can mix its score out of all heads' raw scores; sequence s brings rows seq_rows[s] .. seq_rows[s + 1] and held
+    """What talk_rows computes, for bf16 on mma.sync tiles: a block (or a cluster of blocks) owns sixteen rows of one sequence, or eight of
+    thirty-two heads in one block, and all heads, so that every head can mix its score out of all heads' raw scores; sequence s brings rows seq_rows[s] .. seq_rows[s + 1] and held
     seq_start[s] positions before.  ``splits`` > 1 (steps of few rows a sequence) shares the positions a block would walk out over
     that many blocks and merges their parts in a second kernel, in the order of the splits; ``row_slot`` then marks padding rows."""
     _talk_check("talk_tiles", q, k_cache, v_cache, gate, temp, talk, out, heads, kv_heads, head_dim)
@@ -1436,9 +1436,9 @@ def talk_tiles_blocks(heads: int, kv_heads: int, head_dim: int, max_new: int) ->
 
 def talk_tiles_splits(seqs: int, heads: int, reach: int, window: int, keep_first: int, blocks_a_seq: Optional[int] = None) -> int:
     """Splits of the positions a row sees (tiles of 32) for steps of few rows a sequence, so that the blocks fill the machine ONCE (a
-    block takes most of a multiprocessor's shared memory, and more than sixteen heads take two or four blocks a sequence): never
-    more than there are tiles (``reach``: a bound on the positions any row reaches; a window bounds them further).
-    ``blocks_a_seq``: what talk_tiles_blocks says (default: by the heads alone)."""
+    block takes most of a multiprocessor's shared memory): never more than there are tiles (``reach``: a bound on the positions any row
+    reaches; a window bounds them further).  ``blocks_a_seq``: what talk_tiles_blocks says for the step's sizes (default: a cluster's two
+    or four blocks for more than sixteen heads, which is more than some sizes take)."""
     tiles = -(-max(reach, 1) // 32)
     if window > 0:
         tiles = min(tiles, -(-keep_first // 32) + (window + 30) // 32 + 1)

@@ -3,8 +3,9 @@
     S_t = diag(a_t) S_(t-1) + (c_t k_t) v_t^T          o_t = f S_t^T q_t + d v_t
 
 per head, S being [key channels, value channels], zero at a sequence's start and carried from token to
-token in the cache's per-sequence state.  Three mixers are this recurrence (``csrc/linear_scan.cu`` runs it,
-the same kernel for prompts and single rows, so that both give the same bits):
+token in the cache's per-sequence state.  Three mixers are this recurrence (``csrc/linear_scan.cu`` runs it, the same
+kernel for prompts and single rows, so that both give the same bits; gated linear attention takes bfloat16 prompts of sixteen
+rows or more in chunks, ``csrc/linear_chunks.cu``, whose sums are in another order):
 
 ``gated_linear_attention``: q, k (heads x dim) and v (heads x vdim) from h; a decay per key channel
 a = sigmoid(z)^(1/tau) with z = W_a2 (W_a1 h) + b; c = 1, d = 0, f = dim^(-1/2).  Each head's o over its root
