@@ -30,8 +30,8 @@ from .base import MIXERS, Mixer, RunMemory, Runtime, StateNeed, StepContext, Ten
 
 # A sequence that brings at least this many rows takes them sixteen at a time, whatever else the step holds (bfloat16 engines: there a prompt cut in
 # other portions has its sums in another order; the float32 path keeps the row-by-row scan, whose sums are the same however a prompt is cut).
-# One whole chunk: 64 heads of 64 take 85 us by rows and 78 in chunks for 16 sequences of 16 rows, 161 and 189 for 64 of 8
-# (a chunk costs the same however few of its rows there are), 68 and 76 for 16 of 8.
+# One whole chunk: 1, 4, 16 and 64 sequences of 16 rows, 64 heads of 64, take 61, 60, 87 and 262 us by rows and 51, 57, 100 and 253 in chunks; of 48
+# rows 84, 79, 206 and 675 against 61, 76, 194 and 618; a chunk costs the same however few of its rows there are.
 CHUNKED_ROWS = 16
 split_steps = False      # tests: steps of single rows through the three kernels of a prompt step
 

@@ -36,8 +36,8 @@ from .base import MIXERS, Mixer, RunMemory, Runtime, StateNeed, StepContext, Ten
 
 # A sequence that brings at least this many rows takes them sixteen at a time, whatever else the step holds (bfloat16 engines: there a prompt cut in
 # other portions has its sums in another order; the float32 path keeps the row-by-row scan, whose sums are the same however a prompt is cut).
-# One whole chunk: 16 heads of 128 x 256 take 84 us by rows and 53 in chunks for 16 sequences of 16 rows, 119 and 123 for
-# 64 of 4; 4 heads of 64 x 64 take 32 and 30 for 16 of 16, 30 and 28 for 16 of 4.
+# One whole chunk: 1, 4, 16 and 64 sequences of 16 rows, 16 heads of 128 x 256, take 44, 53, 85 and 211 us by rows and 33, 37, 56 and 132 in
+# chunks; 64 of 4 rows took 119 and 123.
 CHUNKED_ROWS = 16
 
 
