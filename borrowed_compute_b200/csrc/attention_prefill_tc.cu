@@ -41,19 +41,11 @@
 
 #define APT_ROWS 128        // query rows of one tile: the M of the MMAs, the lanes of TMEM
 #define APT_PAGES_KEPT 256
-// Where P (the exponentials, bf16) goes between the softmax and the product with the values:
-// into tensor memory, over the first half of the scores it came from (1, the default: the
-// product then reads its A operand out of TMEM and shared memory carries 72 KB a page less for
-// two query tiles of head size 128), or into shared memory (0, for comparison).
-#ifndef APT_P_TMEM
-#define APT_P_TMEM 1
-#endif
 #define APT_SMEM_LIMIT 232448
 #define APT_Q_BYTES(D, NT) (((D) / 64) * (NT) * APT_ROWS * 128)
 #define APT_STAGE_BYTES(D) (2 * ((D) / 64) * 64 * 128)
-#define APT_PB(D, NT) (APT_P_TMEM ? 0 : ((D) == 128 && (NT) == 2) ? 1 : 2)
 #define APT_STAGES_FIT(D, NT) ((APT_SMEM_LIMIT - 1024 - APT_Q_BYTES(D, NT)) / APT_STAGE_BYTES(D))
-#define APT_STAGES(D, NT) (!APT_P_TMEM ? 4 : APT_STAGES_FIT(D, NT) > 6 ? 6 : APT_STAGES_FIT(D, NT))
+#define APT_STAGES(D, NT) (APT_STAGES_FIT(D, NT) > 6 ? 6 : APT_STAGES_FIT(D, NT))
 #define APT_RAISE 8.0f      // the running maximum follows the true one at this distance at most
 
 // Time stamps of one block's life, for measurement builds only (-DBC_APT_TRACE; compiled out
@@ -88,10 +80,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const float* __restrict__ bias, int bias_reach) {
     constexpr int THREADS = 64 + NT * 128;
     constexpr int STAGES = APT_STAGES(D, NT);
-    // P in shared memory only (APT_P_TMEM 0): two P tiles a query tile let the softmax of page
-    // j + 1 write while the product of page j reads; with two query tiles of head size 128 shared
-    // memory has room for one only, and the softmax then waits for that product.
-    constexpr int PB = APT_PB(D, NT);
     constexpr int DB = D / 64;                         // 64-element blocks of the head size
     constexpr int DVB = DV / 64;                       // and of a head's values (a stage keeps room for DB of them)
     constexpr int ROW_BLOCK = APT_ROWS * 128;          // bytes of a [128 rows][64 elements] block
@@ -106,8 +94,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_smem = smem;
-    uint8_t* p_smem = q_smem + Q_BYTES;                // P of (tile t, buffer b) at (PB t + b) ROW_BLOCK
-    uint8_t* kv_smem = p_smem + NT * PB * ROW_BLOCK;
+    uint8_t* kv_smem = q_smem + Q_BYTES;
     __shared__ __align__(8) uint64_t bars[2 * STAGES + 1 + 6 * NT];
     __shared__ uint32_t tmem_slot;
     __shared__ int page_of[APT_PAGES_KEPT];   // the first pages this block reads, fetched once (-1: none)
@@ -115,7 +102,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     pdl_launch_dependents();
     pdl_wait();
     const int g = blockIdx.x, sq = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int group = H / G;
     const int tokens_per_block = NT * APT_ROWS / group;   // rows past tokens_per_block * group are padding
     const int slot = seq_slot[sq];
@@ -176,7 +163,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Q: one box [tokens][heads of the group][64 elements] per 64 elements of the head size.
             mbar_expect_tx(q_full, (uint32_t)(DB * tokens_per_block * group * 128));
             for (int b = 0; b < DB; b++) tma_load_3d(smem_u32(q_smem + b * NT * ROW_BLOCK), &map_q, q_full, b * 64, g * group, row0 + tok0);
@@ -199,18 +186,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = instr_desc_b(BC_PAGE, false);   // S: N = 64 positions, keys k-major
-            constexpr uint32_t idesc_o = instr_desc_b(DV, true);         // O: N = the values' width, values n-major
-            // The operand descriptors are worked out once; an address further on is the descriptor
-            // plus that many 16-byte units, so that a product costs its issuing thread an addition
-            // or two (this one thread issues every product of the block: what it spends between
-            // two of them, the tensor core waits).
-            const uint64_t q_desc0 = smem_desc(smem_u32(q_smem));
-            const uint64_t k_desc0 = smem_desc(smem_u32(kv_smem));
-            const uint64_t v_desc0 = smem_desc_mn(smem_u32(kv_smem) + DB * KV_BLOCK, KV_BLOCK);
-            auto scores = [&](int j) {   // S[t][j & 1] = Q_t K(j)^T for every query tile t
-                const uint64_t k_desc = k_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));
+        // The whole warp waits, one elected lane issues (tc_ptx.cuh): a product of N 64 costs the issuing warp 52 clocks and one of N 128 whose A lies in
+        // tensor memory 75, against 68 and 118 behind a comparison of lane numbers, more than the tensor core takes for them.
+        constexpr uint32_t idesc_s = instr_desc_b(BC_PAGE, false);   // S: N = 64 positions, keys k-major
+        constexpr uint32_t idesc_o = instr_desc_b(DV, true);         // O: N = the values' width, values n-major
+        // The operand descriptors are worked out once; an address further on is the descriptor plus that many 16-byte units.
+        const uint64_t q_desc0 = smem_desc(smem_u32(q_smem));
+        const uint64_t k_desc0 = smem_desc(smem_u32(kv_smem));
+        const uint64_t v_desc0 = smem_desc_mn(smem_u32(kv_smem) + DB * KV_BLOCK, KV_BLOCK);
+        auto scores = [&](int j) {   // S[t][j & 1] = Q_t K(j)^T for every query tile t
+            const uint64_t k_desc = k_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
 #pragma unroll
@@ -219,48 +205,45 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                                  k_desc + (uint64_t)(((kk >> 2) * KV_BLOCK >> 4) + 2 * (kk & 3)), idesc_s, kk != 0);
                     mma_commit(s_full(t, j & 1));
                 }
-            };
-            bool ok = mbar_wait(q_full, 0, 2);
-            for (int j = 0; j < 2 && j < n_tiles && ok; j++) {
-                ok = mbar_wait(kv_full0 + 8 * (j % STAGES), 0, 3);
-                if (!ok) break;
-                tc_fence_after();
-                scores(j);
             }
-            for (int j = 0; j < n_tiles && ok; j++) {
-                const uint64_t v_desc = v_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));   // 16 positions on: 2048 bytes
+            __syncwarp();
+        };
+        bool ok = mbar_wait_warp(q_full, 0, 2);
+        for (int j = 0; j < 2 && j < n_tiles && ok; j++) {
+            ok = mbar_wait_warp(kv_full0 + 8 * (j % STAGES), 0, 3);
+            if (!ok) break;
+            tc_fence_after();
+            scores(j);
+        }
+        for (int j = 0; j < n_tiles && ok; j++) {
+            const uint64_t v_desc = v_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));   // 16 positions on: 2048 bytes
 #pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    ok = ok && mbar_wait(p_full(t, j & 1), (j >> 1) & 1, 4);
-                    if (!ok) break;
-                    APT_STAMP(j, 2 * t);
-                    tc_fence_after();
-#if APT_P_TMEM
+            for (int t = 0; t < NT; t++) {
+                ok = ok && mbar_wait_warp(p_full(t, j & 1), (j >> 1) & 1, 4);
+                if (!ok) break;
+                if (lane == 0) APT_STAMP(j, 2 * t);
+                tc_fence_after();
+                if (elect_one()) {
                     // P lies over the first 32 columns of the scores it came from: 8 columns a k-step of 16 positions.
 #pragma unroll
                     for (int kk = 0; kk < BC_PAGE / 16; kk++)
                         mma_bf16_a_tmem(tmem + O_COL + t * D, tmem + (2 * t + (j & 1)) * BC_PAGE + 8 * kk, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o,
                                         (j | kk) != 0);
-#else
-                    const uint32_t p_addr = smem_u32(p_smem + (PB * t + (j & (PB - 1))) * ROW_BLOCK);
-#pragma unroll
-                    for (int kk = 0; kk < BC_PAGE / 16; kk++)
-                        mma_bf16(tmem + O_COL + t * D, smem_desc(p_addr) + 2 * kk, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (j | kk) != 0);
-#endif
                     mma_commit(o_done(t, j & 1));
-                    APT_STAMP(j, 2 * t + 1);
+                    if (t == NT - 1) mma_commit(kv_empty0 + 8 * (j % STAGES));
                 }
+                __syncwarp();
+                if (lane == 0) APT_STAMP(j, 2 * t + 1);
+            }
+            if (!ok) break;
+            if (j + 2 < n_tiles) {
+                const int s = (j + 2) % STAGES;
+                ok = mbar_wait_warp(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
                 if (!ok) break;
-                mma_commit(kv_empty0 + 8 * (j % STAGES));
-                if (j + 2 < n_tiles) {
-                    const int s = (j + 2) % STAGES;
-                    ok = mbar_wait(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
-                    if (!ok) break;
-                    APT_STAMP(j, 4);
-                    tc_fence_after();
-                    scores(j + 2);
-                    APT_STAMP(j, 5);
-                }
+                if (lane == 0) APT_STAMP(j, 4);
+                tc_fence_after();
+                scores(j + 2);
+                if (lane == 0) APT_STAMP(j, 5);
             }
         }
     } else {
@@ -283,8 +266,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         float m_used = -INFINITY, l = 0.0f;
         bool ok = true;
         for (int j = 0; j < n_tiles; j++) {
-            if (lane == 0) ok = mbar_wait(s_full(t, j & 1), (j >> 1) & 1, 6);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(s_full(t, j & 1), (j >> 1) & 1, 6);
             if (!ok) break;
             if (warp == 2 && lane == 0) APT_STAMP(j, 8);
             tc_fence_after();
@@ -346,24 +328,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 l *= corr;
             }
             if (warp == 2 && lane == 0) APT_STAMP(j, 10);
-            if (j >= (APT_P_TMEM ? 2 : PB)) {
-                // The P tile written below was last read by the product of page j - PB (with two
-                // P tiles: done long ago as a rule, the scores of page j were issued after it).
-                // Waiting for every phase in order also keeps the parities apart: a parity tells
-                // two phases apart, not more.
-                constexpr int BACK = APT_P_TMEM ? 2 : PB;   // in TMEM, P lies over the scores of the page two before: that product is long done
-                if (lane == 0) ok = mbar_wait(o_done(t, (j - BACK) & 1), ((j - BACK) >> 1) & 1, 7);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (j >= 2) {
+                // P goes over the scores just read, whose product of two pages ago is long done (they were issued after it).  Waiting for every
+                // phase in order keeps the parities apart: a parity tells two phases apart, not more.
+                ok = mbar_wait_warp(o_done(t, j & 1), ((j - 2) >> 1) & 1, 7);
                 if (!ok) break;
             }
             if (warp == 2 && lane == 0) APT_STAMP(j, 11);
             if (j > 0 && __any_sync(0xffffffffu, raise)) {
                 // Rescale this warp's rows of the accumulator, once every product issued so far is in it.
-                if (PB != 1) {
-                    if (lane == 0) ok = mbar_wait(o_done(t, (j - 1) & 1), ((j - 1) >> 1) & 1, 9);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (!ok) break;
-                }
+                ok = mbar_wait_warp(o_done(t, (j - 1) & 1), ((j - 1) >> 1) & 1, 9);
+                if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < DV; c += 16) {
@@ -382,7 +357,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             const float shift = BIAS ? page_bias - base : -base;
             const uint64_t scale2 = pack_f32x2(page_scale, page_scale), shift2 = pack_f32x2(shift, shift);
             uint64_t sums[4] = {0ull, 0ull, 0ull, 0ull};
-#if APT_P_TMEM
             // P goes back into tensor memory, two bf16 a column, over the scores just read (this
             // thread's own lane): the product reads it there as its A operand.
             const uint32_t p_addr = lane_base + (2 * t + (j & 1)) * BC_PAGE;
@@ -399,22 +373,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
                 tmem_store16(p_addr + 16 * c16, packed);
             }
-#else
-            uint8_t* p_row = p_smem + (PB * t + (j & (PB - 1))) * ROW_BLOCK + (32 * q + lane) * 128;
-#pragma unroll
-            for (int c8 = 0; c8 < 8; c8++) {
-                uint32_t packed[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float a, b;
-                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[c8 * 8 + 2 * i]), __uint_as_float(sv[c8 * 8 + 2 * i + 1])), scale2, shift2), a, b);
-                    a = fast_exp2(a), b = fast_exp2(b);
-                    sums[i] = add_f32x2(sums[i], pack_f32x2(a, b));
-                    packed[i] = pack_bf16(a, b);
-                }
-                *reinterpret_cast<uint4*>(p_row + ((c8 ^ (lane & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            }
-#endif
             {
                 float s0, s1, s2, s3;
                 unpack_f32x2(add_f32x2(sums[0], sums[1]), s0, s1);
@@ -434,20 +392,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     *reinterpret_cast<uint4*>(v_tile + (within >> 3) * KV_BLOCK + vrow * 128 + (within & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
                 }
             }
-#if APT_P_TMEM
             if (t == 0 && first_bad < BC_PAGE) fence_proxy_async();   // the cleared value rows, for the tensor core's reads
             tmem_store_wait();
-#else
-            fence_proxy_async();
-#endif
             tc_fence_before();
             mbar_arrive(p_full(t, j & 1));
             if (warp == 2 && lane == 0) APT_STAMP(j, 12);
         }
         // The output: the accumulator over this row's sum.
         if (ok) {
-            if (lane == 0) ok = mbar_wait(o_done(t, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 8);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(o_done(t, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 8);
         }
         if (ok) {
             tc_fence_after();
@@ -503,8 +456,8 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
                   const int* seq_slot, const int* seq_start, void* out, int seqs, int max_new, int H, int G, int max_pages, int n_pages,
                   int window, int chunk, float scale, int sink, const float* sink_values, float out_scale, const float* bias, int bias_reach, cudaStream_t s) {
     constexpr int DB = D / 64;
-    constexpr int STAGES = APT_STAGES(D, NT), PB = APT_PB(D, NT);
-    constexpr int SMEM = DB * NT * APT_ROWS * 128 + NT * PB * APT_ROWS * 128 + STAGES * 2 * DB * BC_PAGE * 128 + 1024;
+    constexpr int STAGES = APT_STAGES(D, NT);
+    constexpr int SMEM = DB * NT * APT_ROWS * 128 + STAGES * 2 * DB * BC_PAGE * 128 + 1024;
     static_assert(SMEM <= APT_SMEM_LIMIT, "the ring does not fit");
     if (cudaError_t e = bc_allow_shared<attention_prefill_tc_kernel<D, DV, NT, BIAS>>(SMEM); e != cudaSuccess) {
         bc_set_error("attention_prefill_tc: cannot set shared memory to %d: %s", SMEM, cudaGetErrorString(e));

@@ -56,7 +56,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     pdl_launch_dependents();
     pdl_wait();
     const int g = blockIdx.x, sq = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int group = H / G;
     const int tokens_per_block = DT_ROWS / group;      // rows past tokens_per_block * group are padding
     const int slot = seq_slot[sq];
@@ -112,7 +112,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(q_full, (uint32_t)(2 * DB * tokens_per_block * group * 128));
             for (int m = 0; m < 2; m++)
                 for (int b = 0; b < DB; b++) tma_load_3d(smem_u32(q_smem + (m * DB + b) * ROW_BLOCK), &map_q, q_full, m * D + b * 64, g * group, row0 + tok0);
@@ -134,14 +134,15 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = instr_desc_b(BC_PAGE, false);   // S: N = 64 positions, keys k-major
-            constexpr uint32_t idesc_o = instr_desc_b(DV, true);         // O: N = the values' width, values n-major
-            const uint64_t q_desc0 = smem_desc(smem_u32(q_smem));
-            const uint64_t k_desc0 = smem_desc(smem_u32(kv_smem));
-            const uint64_t v_desc0 = smem_desc_mn(smem_u32(kv_smem) + V_AT, KV_BLOCK);
-            auto scores = [&](int j) {
-                const uint64_t k_desc = k_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));
+        // The whole warp waits, one elected lane issues (see tc_ptx.cuh).
+        constexpr uint32_t idesc_s = instr_desc_b(BC_PAGE, false);   // S: N = 64 positions, keys k-major
+        constexpr uint32_t idesc_o = instr_desc_b(DV, true);         // O: N = the values' width, values n-major
+        const uint64_t q_desc0 = smem_desc(smem_u32(q_smem));
+        const uint64_t k_desc0 = smem_desc(smem_u32(kv_smem));
+        const uint64_t v_desc0 = smem_desc_mn(smem_u32(kv_smem) + V_AT, KV_BLOCK);
+        auto scores = [&](int j) {
+            const uint64_t k_desc = k_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
 #pragma unroll
@@ -150,37 +151,41 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                                  k_desc + (uint64_t)(((m * DB + (kk >> 2)) * KV_BLOCK >> 4) + 2 * (kk & 3)), idesc_s, kk != 0);
                     mma_commit(s_full(m, j & 1));
                 }
-            };
-            bool ok = mbar_wait(q_full, 0, 2);
-            for (int j = 0; j < 2 && j < n_tiles && ok; j++) {
-                ok = mbar_wait(kv_full0 + 8 * (j % STAGES), 0, 3);
+            }
+            __syncwarp();
+        };
+        bool ok = mbar_wait_warp(q_full, 0, 2);
+        for (int j = 0; j < 2 && j < n_tiles && ok; j++) {
+            ok = mbar_wait_warp(kv_full0 + 8 * (j % STAGES), 0, 3);
+            if (!ok) break;
+            tc_fence_after();
+            scores(j);
+        }
+        for (int j = 0; j < n_tiles && ok; j++) {
+            const uint64_t v_desc = v_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));   // 16 positions on: 2048 bytes
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                ok = ok && mbar_wait_warp(p_full(m, j & 1), (j >> 1) & 1, 4);
                 if (!ok) break;
                 tc_fence_after();
-                scores(j);
-            }
-            for (int j = 0; j < n_tiles && ok; j++) {
-                const uint64_t v_desc = v_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));   // 16 positions on: 2048 bytes
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    ok = ok && mbar_wait(p_full(m, j & 1), (j >> 1) & 1, 4);
-                    if (!ok) break;
-                    tc_fence_after();
+                if (elect_one()) {
                     // P lies over the first 32 columns of the scores it came from: 8 columns a k-step of 16 positions.
 #pragma unroll
                     for (int kk = 0; kk < BC_PAGE / 16; kk++)
                         mma_bf16_a_tmem(tmem + O_COL + m * DV, tmem + (2 * m + (j & 1)) * BC_PAGE + 8 * kk, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc_o,
                                         (j | kk) != 0);
                     mma_commit(o_done(m, j & 1));
+                    if (m == 1) mma_commit(kv_empty0 + 8 * (j % STAGES));
                 }
+                __syncwarp();
+            }
+            if (!ok) break;
+            if (j + 2 < n_tiles) {
+                const int s = (j + 2) % STAGES;
+                ok = mbar_wait_warp(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
                 if (!ok) break;
-                mma_commit(kv_empty0 + 8 * (j % STAGES));
-                if (j + 2 < n_tiles) {
-                    const int s = (j + 2) % STAGES;
-                    ok = mbar_wait(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
-                    if (!ok) break;
-                    tc_fence_after();
-                    scores(j + 2);
-                }
+                tc_fence_after();
+                scores(j + 2);
             }
         }
     } else {
@@ -198,8 +203,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         float m_used = -INFINITY, l = 0.0f;
         bool ok = true;
         for (int j = 0; j < n_tiles; j++) {
-            if (lane == 0) ok = mbar_wait(s_full(m, j & 1), (j >> 1) & 1, 6);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(s_full(m, j & 1), (j >> 1) & 1, 6);
             if (!ok) break;
             tc_fence_after();
             uint32_t sv[64];
@@ -239,14 +243,12 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (j >= 2) {
                 // P goes over the scores of the page two before, whose product has to be done; waiting for every phase in order keeps
                 // the parities apart.
-                if (lane == 0) ok = mbar_wait(o_done(m, j & 1), ((j - 2) >> 1) & 1, 7);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                ok = mbar_wait_warp(o_done(m, j & 1), ((j - 2) >> 1) & 1, 7);
                 if (!ok) break;
             }
             if (j > 0 && __any_sync(0xffffffffu, raise)) {
                 // Rescale this warp's rows of the accumulator, once every product issued so far is in it.
-                if (lane == 0) ok = mbar_wait(o_done(m, (j - 1) & 1), ((j - 1) >> 1) & 1, 9);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                ok = mbar_wait_warp(o_done(m, (j - 1) & 1), ((j - 1) >> 1) & 1, 9);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
@@ -299,8 +301,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             mbar_arrive(p_full(m, j & 1));
         }
         if (ok) {
-            if (lane == 0) ok = mbar_wait(o_done(m, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 8);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(o_done(m, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 8);
         }
         // Both maps' accumulators are whole once every softmax warp has seen its own: a row's sums are exchanged at the same barrier.
         row_sum[m][row] = l;

@@ -110,7 +110,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ uint32_t tmem_slot;
     __shared__ int gave_up;   // a wait of this block ran out: nothing is written, the block only tears down
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int stages = p.stages;
     const int band_blocks = TC_RASTER * p.n_tiles;
     const int band = blockIdx.x / band_blocks, in_band = blockIdx.x - band * band_blocks;
@@ -141,7 +141,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     pdl_launch_dependents();
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             TC_STAMP(1);
             // Weights are written by no kernel, so the first ring of weight tiles is asked
             // for before the wait on the preceding kernel; activations only after it.
@@ -180,25 +180,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(BN);
-            bool ok = true;
-            for (int i = 0; i < k_iters && ok; i++) {
-                const int s = i % stages;
-                ok = mbar_wait(full0 + 8 * s, (i / stages) & 1, 2);
-                if (!ok) break;
-                if (i == 0) TC_STAMP(4);
-                tc_fence_after();
-                const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
-                const uint64_t da = smem_desc(a), db = smem_desc(a + N_ACC * A_BYTES);
+        // The whole warp waits, one elected lane issues (see tc_ptx.cuh).
+        constexpr uint32_t idesc = instr_desc(BN);
+        bool ok = true;
+        for (int i = 0, s = 0, round = 0; i < k_iters; i++) {
+            ok = mbar_wait_warp(full0 + 8 * s, round & 1, 2);
+            if (!ok) break;
+            if (i == 0 && lane == 0) TC_STAMP(4);
+            tc_fence_after();
+            const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+            const uint64_t da = smem_desc(a), du = smem_desc(a + A_BYTES), db = smem_desc(a + N_ACC * A_BYTES);
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; kk++) {
                     const uint32_t acc = (i | kk) != 0;
                     mma_bf16(tmem, da + 2 * kk, db + 2 * kk, idesc, acc);
-                    if (N_ACC == 2) mma_bf16(tmem + BN, smem_desc(a + A_BYTES) + 2 * kk, db + 2 * kk, idesc, acc);
+                    if (N_ACC == 2) mma_bf16(tmem + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
                 }
                 mma_commit(empty0 + 8 * s);
             }
+            __syncwarp();
+            if (++s == stages) s = 0, round++;
+        }
+        if (elect_one()) {
             if (!ok) {
                 *reinterpret_cast<volatile int*>(&gave_up) = 1;
                 __threadfence_block();
@@ -206,6 +210,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             TC_STAMP(5);
             mma_commit(acc_bar);   // also after a wait that ran out: the epilogue warps must not be left waiting
         }
+        __syncwarp();
     } else {
         // Epilogue: this warp reads TMEM lanes 32 q .. 32 q + 31, i.e. weight rows n0 + 32 q + lane.
         const int q = warp & 3, half = (warp - 2) >> 2;
@@ -223,8 +228,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         int* counter = split ? p.counters + (size_t)tile * 4 + q : nullptr;
         bool ok = true;
         pdl_wait();   // the output, the scratch and the counters may still be in use by the preceding kernel
-        if (lane == 0) ok = mbar_wait(acc_bar, 0, 3) && *reinterpret_cast<volatile int*>(&gave_up) == 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
+        ok = mbar_wait_warp(acc_bar, 0, 3) && __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&gave_up) == 0);
         if (warp == 2 && lane == 0) TC_STAMP(6);
         tc_fence_after();
         const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16);
@@ -461,7 +465,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     __shared__ uint32_t tmem_slot;
 
     cg::cluster_group cl = cg::this_cluster();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();              // 0: the block that issues the MMAs
     const int stages = p.stages;
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -497,7 +501,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     pdl_launch_dependents();
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t pair_full0 = map_to_rank(full0, 0);   // the even block's barriers count both blocks' bytes
             // This pair's k-steps over all of its tiles, numbered through: step `it` belongs to
             // the pair's tile number it / k_iters.
@@ -542,29 +546,33 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            // The whole warp waits, one elected lane issues (see tc_ptx.cuh).
             const uint32_t idesc = instr_desc_pair(bn);
             bool ok = true;
-            int it = 0, n = 0;
+            int s = 0, round = 0, n = 0;
             for (int tile = pair; tile < total_tiles && ok; tile += n_pairs, n++) {
                 // The epilogue warps of both blocks must have read the previous tile out of TMEM.
-                if (!(ok = mbar_wait(acc_empty, (n & 1) ^ 1, 4))) break;
+                if (!(ok = mbar_wait_warp(acc_empty, (n & 1) ^ 1, 4))) break;
                 tc_fence_after();
-                for (int i = 0; i < k_iters; i++, it++) {
-                    const int s = it % stages;
-                    if (!(ok = mbar_wait(full0 + 8 * s, (it / stages) & 1, 2))) break;
+                for (int i = 0; i < k_iters; i++) {
+                    if (!(ok = mbar_wait_warp(full0 + 8 * s, round & 1, 2))) break;
                     tc_fence_after();
                     const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
                     const uint64_t da = smem_desc(a), du = smem_desc(a + TILE), db = smem_desc(a + 2 * TILE);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < TC_BK / 16; kk++) {
-                        const uint32_t acc = (i | kk) != 0;
-                        mma_bf16_pair(tmem, da + 2 * kk, db + 2 * kk, idesc, acc);
-                        mma_bf16_pair(tmem + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
+                        for (int kk = 0; kk < TC_BK / 16; kk++) {
+                            const uint32_t acc = (i | kk) != 0;
+                            mma_bf16_pair(tmem, da + 2 * kk, db + 2 * kk, idesc, acc);
+                            mma_bf16_pair(tmem + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
+                        }
+                        mma_commit_pair(empty0 + 8 * s, 3);
+                        if (i + 1 == k_iters) mma_commit_pair(acc_full, 3);
                     }
-                    mma_commit_pair(empty0 + 8 * s, 3);
+                    __syncwarp();
+                    if (++s == stages) s = 0, round++;
                 }
-                if (ok) mma_commit_pair(acc_full, 3);
             }
         }
     } else {
@@ -581,8 +589,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             int tile_n, tile_t;
             place(tile, tile_n, tile_t);
             const int t0 = tile_t * bn;
-            if (lane == 0) ok = mbar_wait(acc_full, n & 1, 3);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(acc_full, n & 1, 3);
             if (!ok) break;
             tc_fence_after();
             const int out_n = tile_n * 2 * OUT_ROWS + (int)rank * OUT_ROWS + 32 * q + lane + (EPI == EPI_SWIGLU ? 0 : TC_BM * set);
@@ -999,7 +1006,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     __shared__ __align__(8) uint64_t bars[2 * 16 + 4];
     __shared__ uint32_t tmem_slot;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int stages = p.stages;
     const int k_iters = (p.K + TC_BK - 1) / TC_BK;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[16]), acc_full0 = smem_u32(&bars[32]), acc_empty0 = smem_u32(&bars[34]);
@@ -1033,7 +1040,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint64_t stream_once = l2_evict_first_policy();
             bool ok = true;
             int it = 0;
@@ -1061,23 +1068,23 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            int it = 0, n = 0;
-            for (int piece = blockIdx.x; piece < pieces && ok; piece += gridDim.x, n++) {
-                const int buffer = n % BUFFERS;
-                // The epilogue warps must have read this accumulator's last piece out of TMEM.
-                if (n >= BUFFERS && !(ok = mbar_wait(acc_empty0 + 8 * buffer, ((n / BUFFERS) & 1) ^ 1, 4))) break;
+        // The whole warp waits, one elected lane issues (see tc_ptx.cuh).
+        bool ok = true;
+        int s = 0, round = 0, n = 0;
+        for (int piece = blockIdx.x; piece < pieces && ok; piece += gridDim.x, n++) {
+            const int buffer = n % BUFFERS;
+            // The epilogue warps must have read this accumulator's last piece out of TMEM.
+            if (n >= BUFFERS && !(ok = mbar_wait_warp(acc_empty0 + 8 * buffer, ((n / BUFFERS) & 1) ^ 1, 4))) break;
+            tc_fence_after();
+            int n0, matrix, t0, t_count;
+            piece_at(piece, n0, matrix, t0, t_count);
+            const uint32_t idesc = instr_desc((t_count + 15) & ~15), acc_at = tmem + buffer * ACC_COLS;
+            for (int i = 0; i < k_iters; i++) {
+                if (!(ok = mbar_wait_warp(full0 + 8 * s, round & 1, 2))) break;
                 tc_fence_after();
-                int n0, matrix, t0, t_count;
-                piece_at(piece, n0, matrix, t0, t_count);
-                const uint32_t idesc = instr_desc((t_count + 15) & ~15), acc_at = tmem + buffer * ACC_COLS;
-                for (int i = 0; i < k_iters; i++, it++) {
-                    const int s = it % stages;
-                    if (!(ok = mbar_wait(full0 + 8 * s, (it / stages) & 1, 2))) break;
-                    tc_fence_after();
-                    const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
-                    const uint64_t da = smem_desc(a), du = smem_desc(a + A_BYTES), db = smem_desc(a + N_ACC * A_BYTES);
+                const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+                const uint64_t da = smem_desc(a), du = smem_desc(a + A_BYTES), db = smem_desc(a + N_ACC * A_BYTES);
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < TC_BK / 16; kk++) {
                         const uint32_t acc = (i | kk) != 0;
@@ -1085,8 +1092,10 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         if (N_ACC == 2) mma_bf16(acc_at + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
                     }
                     mma_commit(empty0 + 8 * s);
+                    if (i + 1 == k_iters) mma_commit(acc_full0 + 8 * buffer);
                 }
-                if (ok) mma_commit(acc_full0 + 8 * buffer);
+                __syncwarp();
+                if (++s == stages) s = 0, round++;
             }
         }
     } else {
@@ -1100,8 +1109,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             int n0, matrix, t0, t_count;
             piece_at(piece, n0, matrix, t0, t_count);
             const int out_n = n0 + 32 * q + lane;
-            if (lane == 0) ok = mbar_wait(acc_full0 + 8 * buffer, (n / BUFFERS) & 1, 3);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            ok = mbar_wait_warp(acc_full0 + 8 * buffer, (n / BUFFERS) & 1, 3);
             if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem + buffer * ACC_COLS + ((uint32_t)(32 * q) << 16);

@@ -109,6 +109,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int cod
     }
     return true;
 }
+// The same for a whole converged warp, every lane asking for itself: 46 clocks where the phase is over, against 190 for one lane
+// that asks and tells the others (measured: the others' way around the branch and back costs more than the question).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const bool ok = mbar_wait(bar, parity, code);
+    return __all_sync(0xffffffffu, ok);
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                  "l"(map), "r"(bar), "r"(x), "r"(y)
@@ -166,6 +173,22 @@ __device__ __forceinline__ void mma_bf16_a_tmem(uint32_t d_tmem, uint32_t a_tmem
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// One lane of a converged warp, chosen by the hardware, the same at every call: what issues tensor-core products does so behind this.  Behind a
+// comparison of lane numbers a product held its issuing thread 68 clocks (118 with A in tensor memory) whatever its N; behind this one 42 at N 16,
+// 52 at N 64 and 70 at N 128 (33, 44 and 75 with A in tensor memory), chains of 64 products, measured.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok));
+    return ok != 0;
+}
+// This thread's warp, as a number that the compiler knows to be the same in all of its lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
