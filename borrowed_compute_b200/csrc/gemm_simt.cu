@@ -1,7 +1,7 @@
 // Matrix product on the CUDA cores: Y[m, n] = sum_k X[m, k] * W[n, k], float accumulation
 // in ascending k, one fused multiply-add a term.  This is the product of the true 32-bit
-// path (tensor cores would round operands to tf32) and the checked twin of the tensor-core
-// kernel for bf16 operands.  Reference: the same contraction is k_matmul,
+// path where K is short (at most 512) or the operands are not laid out for tensor copies (the others: gemm_split.cu, by the
+// matrix alone) and the checked twin of the tensor-core kernel for bf16 operands.  Reference: the same contraction is k_matmul,
 // crates/bc-infer/src/gpu/kernels.h:204-223, one warp a weight row.  An output's sum never depends on how many other rows
 // share the launch: k is walked in ascending order, in one piece or in two to eight equal ones whose sums are added in
 // ascending order (simt_splits, by the matrix alone), whichever of the kernels below takes the launch.
@@ -11,11 +11,10 @@
 // numbers; floats whose first columns are gated by their own sigmoid.
 #include <cooperative_groups.h>
 
+#include "epilogue.cuh"
 #include "mma_tiles.cuh"
 
 namespace cg = cooperative_groups;
-
-enum { EPI_STORE = 0, EPI_STORE_F32 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU = 3, EPI_RELU2 = 4, EPI_XIELU = 5, EPI_SILU_F32 = 6 };
 
 #define BK 16
 
@@ -44,27 +43,12 @@ __host__ __device__ constexpr int simt_splits(int cols, int K) {
 // k a piece: a multiple of BK.
 __host__ __device__ constexpr int simt_piece(int K, int splits) { return ((K + splits - 1) / splits + BK - 1) / BK * BK; }
 
-template <class T, int EPI>
-__device__ __forceinline__ void simt_emit(T* out_act, float* out_f32, int m, int n, int N, float v, float u, float act_a, float act_b, int act_cols) {
-    const size_t o = (size_t)m * N + n;
-    if (EPI == EPI_STORE) out_act[o] = from_f32<T>(v);
-    if (EPI == EPI_RELU2) {
-        const float z = fmaxf(v, 0.0f);
-        out_act[o] = from_f32<T>(z * z);
-    }
-    if (EPI == EPI_XIELU) out_act[o] = from_f32<T>(fmaf(0.5f, v, v > 0.0f ? act_a * v * v : act_b * (expm1f(v) - v)));
-    if (EPI == EPI_SILU_F32) out_f32[o] = n < act_cols ? v / (1.0f + expf(-v)) : v;
-    if (EPI == EPI_STORE_F32) out_f32[o] = v;
-    if (EPI == EPI_ADD_F32) out_f32[o] += v;
-    if (EPI == EPI_SWIGLU) out_act[o] = from_f32<T>(v / (1.0f + expf(-v)) * u);
-}
-
 // A tile of BM rows by 128 weight rows a block (SwiGLU: 64 gate rows and their 64 up rows), 128 threads, TM x TN sums each, two to an
 // instruction (fma.rn.f32x2: the roundings of fmaf).  The next sixteen k are on their way to registers while these are multiplied, into the
 // other of two buffers.  BM 64: 8 x 8 a thread, 64 bytes of shared memory for its 64 multiply-adds a k; BM 16 (few rows): 4 x 4, and what counts is that
 // the weights stream.  With several pieces of K the blocks of a tile are one cluster and add up through one another's shared memory.
-// (64 x 64 tiles, 4 x 4 a thread, one buffer: 720 + 763 us for 300 rows of a feed-forward of 2,048 x 8,192, 20 TFLOP/s; now
-// 557 + 311 us.)
+// (64 x 64 tiles, 4 x 4 a thread, one buffer: 720 + 763 us for 300 rows of a feed-forward of 2,048 x 8,192, 20 TFLOP/s; these 557 + 311 us.  Such
+// float products go to gemm_split.cu now.)
 #define SIMT_COLS 128
 template <class T, int EPI, bool VEC, int BM>
 __global__ void __launch_bounds__(128) gemm_simt_kernel(const T* X, const T* __restrict__ W, T* out_act, float* out_f32, int M, int N, int K, int piece, float act_a,
@@ -321,11 +305,15 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
 
 // X [M, K] and W [N, K] (for SwiGLU: W [2N, K], gate rows then up rows) in the operand
 // type; `out` is [M, N] in the operand type (store, SwiGLU) or float (store_f32, add_f32).
+extern "C" int bc_gemm_split_takes(const void* X, const void* W, int cols, int K);
+extern "C" int bc_gemm_split_f32(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, cudaStream_t s);
+
 template <class T>
 static int dispatch(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, cudaStream_t s) {
     BC_CHECK_ARG(M >= 0 && N > 0 && K > 0, "gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
     BC_CHECK_ARG((M + 63) / 64 <= 65535, "gemm_simt: %d rows are more than 65535 tiles of 64", M);
     if (M == 0) return BC_OK;
+    if (sizeof(T) == 4 && bc_gemm_split_takes(X, W, epilogue == EPI_SWIGLU ? 2 * N : N, K)) return bc_gemm_split_f32(X, W, out, M, N, K, epilogue, a, b, cols, s);
     switch (epilogue) {
         case EPI_STORE: return launch<T, EPI_STORE>(X, W, out, M, N, K, a, b, cols, s);
         case EPI_STORE_F32: return launch<T, EPI_STORE_F32>(X, W, out, M, N, K, a, b, cols, s);

@@ -6,8 +6,8 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "epilogue.cuh"
 
-enum { EPI_STORE = 0, EPI_STORE_F32 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU = 3, EPI_RELU2 = 4, EPI_XIELU = 5, EPI_SILU_F32 = 6 };
 // Which epilogues store the activation type, and which store floats.
 #define EPI_TO_BF16(E) ((E) == EPI_STORE || (E) == EPI_SWIGLU || (E) == EPI_RELU2 || (E) == EPI_XIELU)
 #define EPI_TO_F32(E) ((E) == EPI_STORE_F32 || (E) == EPI_SILU_F32)

@@ -346,7 +346,8 @@ def _act_numbers(who: str, epilogue: int, act: Optional[Tuple[float, float]], co
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, act: Optional[Tuple[float, float]] = None,
               cols: Optional[int] = None) -> None:
-    """out = x @ w.T on the CUDA cores with float accumulation, k ascending in one piece or in up to eight that are added in order.
+    """out = x @ w.T with float accumulation, k ascending in one piece or in up to eight that are added in order: on the CUDA cores, or,
+    for float32 sums of more than 512 products, on the tensor cores with every operand whole, as three bfloat16 parts (csrc/gemm_split.cu).
     Both operands are read after the kernels before this launch have ended.
     EPI_STORE: out in x's type; EPI_STORE_F32: float32; EPI_ADD_F32: out += (float32);
     EPI_SWIGLU: w stacks gate rows on up rows, out[:, j] = silu(g_j) * u_j in x's type;
@@ -491,7 +492,7 @@ def gemm_tc_status(reset: bool = True) -> int:
 def set_wait_cycles(cycles: int = 0) -> None:
     """The most clocks a bounded wait inside the tensor-core kernels may take before it gives
     up and records its status (0: back to the default, about a second)."""
-    for unit in ("gemm_tc", "attention_prefill_tc", "attention_decode", "diff_attention_tc"):
+    for unit in ("gemm_tc", "attention_prefill_tc", "attention_decode", "diff_attention_tc", "gemm_split"):
         st = _fn(f"bc_{unit}_set_wait_cycles")(ctypes.c_longlong(int(cycles)))
         if st != 0:
             raise KernelError(f"setting the wait limit of {unit} failed ({st})")
@@ -506,7 +507,7 @@ def gemm_tc_test_starve_next_launch() -> None:
 # ------------------------------------------------------------ errors that reach the caller
 
 _STATUS_UNITS = ("the tensor-core product (gemm_tc)", "the tcgen05 prompt attention (attention_prefill_tc)", "the decode attention (attention_decode)",
-                 "the tcgen05 differential attention (diff_attention_tc)")
+                 "the tcgen05 differential attention (diff_attention_tc)", "the true 32-bit product (gemm_split)")
 _WAITS = {
     0: {1: "the loader's wait for a free stage", 2: "the wait for a stage's operands", 3: "the epilogue's wait for the accumulator",
         4: "the wait for the epilogue to hand the accumulator back"},
@@ -517,6 +518,8 @@ _WAITS = {
     3: {1: "the loader's wait for a free stage", 2: "the wait for the queries", 3: "the wait for the first pages", 4: "the wait for P",
         5: "the wait for a page", 6: "the softmax's wait for scores", 7: "the wait for a product that frees P", 8: "the wait for the last product",
         9: "the wait before a rescale"},
+    4: {1: "the wait for a raw tile", 2: "the wait for products that free operands", 3: "the wait for a stretch's sums", 4: "the loader's wait for a free stage",
+        5: "the wait for the sums to be taken out", 6: "the wait for operands"},
 }
 _bound_devices = set()
 

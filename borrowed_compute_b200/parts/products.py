@@ -1,7 +1,8 @@
 """The one place that decides which kernel multiplies matrices.
 
 ``linear(x, w, out, epilogue)`` computes ``x @ w.T`` with float accumulation.  On the
-32-bit path it is the CUDA-core kernel (tensor cores would round operands to tf32).  For
+32-bit path ``ops.gemm_simt`` chooses: every operand whole as three bfloat16 parts on the tensor
+cores, or, for short sums, the CUDA-core kernel; never tf32.  For
 bfloat16 it is the tcgen05 tensor-core kernel; the CUDA-core kernel on the same operands is
 its checked twin and can be forced for a test with ``force_simt``.
 """

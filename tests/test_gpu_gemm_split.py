@@ -1,0 +1,106 @@
+"""The true 32-bit product on the tensor cores: tiles of 128 weight rows and up to 128 rows of x, chunks of 32 k, sums taken out every 64,
+one piece of K or a cluster of two to eight.
+
+Tolerance, in units of sum |x w|: the products of parts that are left out, at most 2^-22 + 2^-24; a stretch of 64 k is four truncated additions, 4 x 2^-23;
+its sums are added in float, one rounding a stretch and one a piece; the smaller products are at most 2^-6 of the whole and truncated 5 K / 16 times."""
+
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def bound(K):
+    return 2.0 ** -22 + 2.0 ** -24 + 4 * 2.0 ** -23 + (K / 64 + 8 + 3) * 2.0 ** -24 + 5 * K / 16 * 2.0 ** -29
+
+
+def operands(M, N, K, seed=0):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N + K + seed)
+    return torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") / K ** 0.5
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 1, 516), (16, 64, 516), (17, 65, 544), (128, 128, 548), (129, 127, 576), (112, 129, 600), (257, 192, 640),       # tiles, a chunk's and a stretch's ends
+    (33, 128, 1024), (5, 130, 1028), (140, 64, 2052), (20, 200, 4100), (130, 128, 8196)])                                # two, four and eight pieces
+def test_products_around_the_edges_of_tiles_stretches_and_pieces(M, N, K):
+    from borrowed_compute_b200 import ops
+
+    x, w = operands(M, 2 * N, K)
+    full, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    wn = w[:N].contiguous()
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_simt(x, wn, out, ops.EPI_STORE_F32)
+    off = bound(K) * size
+    assert ((out.double() - full[:, :N]).abs() <= off[:, :N]).all()
+    base = torch.randn(M, N, device="cuda")
+    acc = base.clone()
+    ops.gemm_simt(x, wn, acc, ops.EPI_ADD_F32)
+    ref = base.double() + full[:, :N]
+    assert ((acc.double() - ref).abs() <= off[:, :N] + 2.0 ** -23 * ref.abs()).all()
+    glu = torch.empty((M, N), device="cuda")
+    ops.gemm_simt(x, w, glu, ops.EPI_SWIGLU)
+    gate, up = full[:, :N], full[:, N:]
+    act = gate * torch.sigmoid(gate)                                      # |silu'| <= 1.1; a few roundings of the quotient
+    assert ((glu.double() - act * up).abs() <= 1.1 * off[:, :N] * up.abs() + off[:, N:] * act.abs() + off[:, :N] * off[:, N:] + 2.0 ** -21 * (act * up).abs()).all()
+    for rows in (slice(M - 1, M), slice(0, min(M, 20)), slice(0, min(M, 60))):      # the same bits alone, among a few and among all
+        few = torch.empty((rows.stop - rows.start, N), device="cuda")
+        ops.gemm_simt(x[rows].contiguous(), wn, few, ops.EPI_STORE_F32)
+        assert torch.equal(few, out[rows])
+
+
+def test_no_further_from_64_bits_than_one_multiply_add_after_another():
+    from borrowed_compute_b200 import ops
+
+    for M, N, K in ((7, 128, 1024), (300, 256, 2048)):
+        x, w = operands(M, N, K, 1)
+        full = x.double() @ w.double().T
+        out = torch.empty((M, N), device="cuda")
+        ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+        plain = torch.zeros((M, N), device="cuda")
+        for k in range(K):
+            plain = torch.addcmul(plain, x[:, k:k + 1], w[:, k])
+        assert (out.double() - full).norm() <= (plain.double() - full).norm()
+
+
+def test_numbers_at_the_ends_of_the_range():
+    """Infinities and not-a-numbers reach every output of their row and column and no other; the largest floats and small ones keep their bits."""
+    from borrowed_compute_b200 import ops
+
+    M, N, K = 40, 140, 1032
+    inf, biggest = float("inf"), 3.4028234663852886e38
+    x, w = torch.ones((M, K), device="cuda"), torch.ones((N, K), device="cuda")
+    x[2, K - 1], x[3, 0], x[5, 7], w[9, 40] = inf, float("nan"), -inf, inf
+    x[4, 1:] = 0.0
+    x[4, 0], w[:, 0] = biggest, 1.0
+    x[6], x[7, :] = 2.0 ** -100 * (1 + 2.0 ** -23), 0.0
+    out = torch.empty((M, N), device="cuda")
+    ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+    others = [n for n in range(N) if n != 9]
+    assert (out[2] == inf).all() and out[3].isnan().all() and (out[5][others] == -inf).all() and out[5, 9].isnan()
+    assert (out[4][others] == biggest).all() and out[4, 9].isnan()
+    assert (out[[0, 1, 8]][:, others] == K).all() and (out[[0, 1, 8], 9] == inf).all()
+    assert ((out[6][others].double() / (K * 2.0 ** -100 * (1 + 2.0 ** -23)) - 1).abs() <= bound(K)).all() and (out[7][others] == 0).all()
+    # A payload below bfloat16's bits is still not a number.
+    odd = torch.full((1, K), 1.0, device="cuda")
+    odd.view(torch.int32)[0, 3] = 0x7F800001
+    got = torch.empty((1, N), device="cuda")
+    ops.gemm_simt(odd, w, got, ops.EPI_STORE_F32)
+    assert got.isnan().all()
+
+
+def test_operands_that_tensor_copies_cannot_take_go_the_other_way():
+    """K no multiple of four, or operands off their 16 bytes: the CUDA-core kernel, as before."""
+    from borrowed_compute_b200 import ops
+
+    for K, shift in ((1030, 0), (1032, 1)):
+        x, w = operands(9, 70, K)
+        room = torch.empty(9 * K + 4, device="cuda")
+        moved = room[shift:shift + 9 * K].view(9, K)
+        moved.copy_(x)
+        out = torch.empty((9, 70), device="cuda")
+        ops.gemm_simt(moved, w, out, ops.EPI_STORE_F32)
+        size = x.double().abs() @ w.double().abs().T
+        assert ((out.double() - x.double() @ w.double().T).abs() <= (K + 4) * 2.0 ** -24 * size).all()
