@@ -21,6 +21,15 @@
 //     operand is read out of tensor memory, into a TMEM accumulator that stays there for the
 //     whole block.  Values are the n-major B operand ([position][d] with d contiguous),
 //     exactly as TMA wrote the page.  Shared memory holds Q and the ring of pages, nothing else.
+//   - The two tiles of a block take turns: the exponential unit (16 a clock and SM, 512 clocks a warp and page) is what a page of softmax
+//     mostly waits for, and two warps of an SM sub-partition that both stand in it leave it idle when both read scores and look for
+//     maxima.  A warp asks for its turn before its exponentials and gives it on near their end; products go tile by tile, P V and at once the
+//     scores that take P's place.
+//     One prompt of 16,384, 32 heads of 128 on 8 kv heads, us: 1,762 (without turns 1,863; turns and both tiles' products together 1,797 to 1,803; before that
+//     1,967).  A page of two tiles takes 1,710 clocks: products 1,432 (52 each for N 64, 75 for P V: shared memory and issue), exponentials 1,024, a warp by itself 600 clocks
+//     of scores and maxima, 650 to 900 of exponentials, 180 between pages.  No faster, each built and timed: two pages a step with one buffer of scores
+//     (1,841; with the second page's maximum between the first's exponentials and P handed over by pages 1,776 to 1,823), a row split over two threads (2,414),
+//     the next page's scores read during this one's exponentials (1,877 to 1,919).
 //   - A table of biases by distance (common.cuh; BIAS) is added to the scores on their way to the exponentials: by the element in
 //     pages near a warp's rows (the lanes of a warp are consecutive rows, so their entries lie side by side), as one number a
 //     row where every distance of the page is past the table's reach.
@@ -46,14 +55,14 @@
 #define APT_STAGE_BYTES(D) (2 * ((D) / 64) * 64 * 128)
 #define APT_STAGES_FIT(D, NT) ((APT_SMEM_LIMIT - 1024 - APT_Q_BYTES(D, NT)) / APT_STAGE_BYTES(D))
 #define APT_STAGES(D, NT) (APT_STAGES_FIT(D, NT) > 6 ? 6 : APT_STAGES_FIT(D, NT))
+#define APT_LET_GO 24       // of a page's 32 pairs of exponentials, how many a warp makes before the other tile's may begin (16 to 31: the same time)
 #define APT_RAISE 8.0f      // the running maximum follows the true one at this distance at most
 
 // Time stamps of one block's life, for measurement builds only (-DBC_APT_TRACE; compiled out
 // otherwise): the block (0, trace_y, 0) writes clock64() values, [page][what], what 0-7 by the
 // MMA thread (0 P of tile 0 seen, 1 its product issued, 2 P of tile 1 seen, 3 its product issued,
 // 4 the page after next seen, 5 its scores issued), 8-15 by the first softmax warp of tile 0
-// (8 scores seen, 9 read out of TMEM, 10 maximum known, 11 the product before seen, 12 P written
-// and handed over).
+// (8 scores seen, 9 read out of TMEM, 10 maximum known, 12 P written and handed over).
 #ifdef BC_APT_TRACE
 __device__ long long* g_apt_trace = nullptr;
 __device__ int g_apt_trace_y = 0;
@@ -95,7 +104,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_smem = smem;
     uint8_t* kv_smem = q_smem + Q_BYTES;
-    __shared__ __align__(8) uint64_t bars[2 * STAGES + 1 + 6 * NT];
+    __shared__ __align__(8) uint64_t bars[2 * STAGES + 1 + 6 * NT + (NT == 2 ? 8 : 0)];
     __shared__ uint32_t tmem_slot;
     __shared__ int page_of[APT_PAGES_KEPT];   // the first pages this block reads, fetched once (-1: none)
 
@@ -129,7 +138,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     auto s_full = [&](int t, int b) { return smem_u32(&bars[2 * STAGES + 1 + 6 * t + b]); };
     auto p_full = [&](int t, int b) { return smem_u32(&bars[2 * STAGES + 1 + 6 * t + 2 + b]); };
     auto o_done = [&](int t, int b) { return smem_u32(&bars[2 * STAGES + 1 + 6 * t + 4 + b]); };
+    // Two tiles: whose turn it is to exponentiate, for the two warps (one a tile) that share an SM sub-partition.
+    auto turn = [&](int t, int q) { return smem_u32(&bars[2 * STAGES + 1 + 6 * NT + 4 * t + q]); };
     if (threadIdx.x == 0) {
+        for (int i = 0; NT == 2 && i < 8; i++) mbar_init(turn(0, i), 1);
         for (int s = 0; s < STAGES; s++) {
             mbar_init(kv_full0 + 8 * s, 1);
             mbar_init(kv_empty0 + 8 * s, 1);
@@ -194,17 +206,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const uint64_t q_desc0 = smem_desc(smem_u32(q_smem));
         const uint64_t k_desc0 = smem_desc(smem_u32(kv_smem));
         const uint64_t v_desc0 = smem_desc_mn(smem_u32(kv_smem) + DB * KV_BLOCK, KV_BLOCK);
-        auto scores = [&](int j) {   // S[t][j & 1] = Q_t K(j)^T for every query tile t
+        auto scores = [&](int t, int j) {   // S[t][j & 1] = Q_t K(j)^T
             const uint64_t k_desc = k_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));
             if (elect_one()) {
 #pragma unroll
-                for (int t = 0; t < NT; t++) {
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; kk++)
-                        mma_bf16(tmem + (2 * t + (j & 1)) * BC_PAGE, q_desc0 + (uint64_t)((((kk >> 2) * NT + t) * ROW_BLOCK >> 4) + 2 * (kk & 3)),
-                                 k_desc + (uint64_t)(((kk >> 2) * KV_BLOCK >> 4) + 2 * (kk & 3)), idesc_s, kk != 0);
-                    mma_commit(s_full(t, j & 1));
-                }
+                for (int kk = 0; kk < D / 16; kk++)
+                    mma_bf16(tmem + (2 * t + (j & 1)) * BC_PAGE, q_desc0 + (uint64_t)((((kk >> 2) * NT + t) * ROW_BLOCK >> 4) + 2 * (kk & 3)),
+                             k_desc + (uint64_t)(((kk >> 2) * KV_BLOCK >> 4) + 2 * (kk & 3)), idesc_s, kk != 0);
+                mma_commit(s_full(t, j & 1));
             }
             __syncwarp();
         };
@@ -213,7 +222,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             ok = mbar_wait_warp(kv_full0 + 8 * (j % STAGES), 0, 3);
             if (!ok) break;
             tc_fence_after();
-            scores(j);
+            for (int t = 0; t < NT; t++) scores(t, j);
         }
         for (int j = 0; j < n_tiles && ok; j++) {
             const uint64_t v_desc = v_desc0 + (uint64_t)((j % STAGES) * (STAGE_BYTES >> 4));   // 16 positions on: 2048 bytes
@@ -234,17 +243,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
                 __syncwarp();
                 if (lane == 0) APT_STAMP(j, 2 * t + 1);
+                // This tile's scores of the page after next take the place of those that P was made of.
+                if (j + 2 < n_tiles) {
+                    const int s = (j + 2) % STAGES;
+                    if (t == 0) ok = mbar_wait_warp(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
+                    if (!ok) break;
+                    tc_fence_after();
+                    scores(t, j + 2);
+                }
             }
             if (!ok) break;
-            if (j + 2 < n_tiles) {
-                const int s = (j + 2) % STAGES;
-                ok = mbar_wait_warp(kv_full0 + 8 * s, ((j + 2) / STAGES) & 1, 5);
-                if (!ok) break;
-                if (lane == 0) APT_STAMP(j, 4);
-                tc_fence_after();
-                scores(j + 2);
-                if (lane == 0) APT_STAMP(j, 5);
-            }
         }
     } else {
         // Softmax: warps 2-5 own query tile 0, warps 6-9 tile 1; this thread owns row 32 q + lane
@@ -328,13 +336,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 l *= corr;
             }
             if (warp == 2 && lane == 0) APT_STAMP(j, 10);
-            if (j >= 2) {
-                // P goes over the scores just read, whose product of two pages ago is long done (they were issued after it).  Waiting for every
-                // phase in order keeps the parities apart: a parity tells two phases apart, not more.
-                ok = mbar_wait_warp(o_done(t, j & 1), ((j - 2) >> 1) & 1, 7);
-                if (!ok) break;
-            }
-            if (warp == 2 && lane == 0) APT_STAMP(j, 11);
             if (j > 0 && __any_sync(0xffffffffu, raise)) {
                 // Rescale this warp's rows of the accumulator, once every product issued so far is in it.
                 ok = mbar_wait_warp(o_done(t, (j - 1) & 1), ((j - 1) >> 1) & 1, 9);
@@ -350,6 +351,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     tmem_store16(o_addr + c, ov);
                 }
                 tmem_store_wait();
+            }
+            if (NT == 2 && (t == 1 || j > 0)) {
+                ok = mbar_wait_warp(turn(t, q), t ? j & 1 : (j - 1) & 1, 10);
+                if (!ok) break;
             }
             const float base = m_used == -INFINITY ? 0.0f : m_used;
             // Scores scaled and shifted two at a time (fma.rn.f32x2: the same roundings as fmaf),
@@ -368,6 +373,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     float a, b;
                     unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[c16 * 32 + 2 * i]), __uint_as_float(sv[c16 * 32 + 2 * i + 1])), scale2, shift2), a, b);
                     a = fast_exp2(a), b = fast_exp2(b);
+                    if (NT == 2 && 16 * c16 + i == APT_LET_GO && lane == 0) mbar_arrive(turn(t ^ 1, q));
                     sums[i & 3] = add_f32x2(sums[i & 3], pack_f32x2(a, b));
                     packed[i] = pack_bf16(a, b);
                 }

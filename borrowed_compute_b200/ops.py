@@ -513,7 +513,7 @@ _WAITS = {
         4: "the wait for the epilogue to hand the accumulator back"},
     1: {1: "the loader's wait for a free stage", 2: "the wait for the queries", 3: "the wait for the first pages", 4: "the wait for P",
         5: "the wait for a page", 6: "the softmax's wait for scores", 7: "the wait for a product that frees P", 8: "the wait for the last product",
-        9: "the wait before a rescale"},
+        9: "the wait before a rescale", 10: "the wait for the other tile's exponentials"},
     2: {1: "the wait for a page of keys and values"},
     3: {1: "the loader's wait for a free stage", 2: "the wait for the queries", 3: "the wait for the first pages", 4: "the wait for P",
         5: "the wait for a page", 6: "the softmax's wait for scores", 7: "the wait for a product that frees P", 8: "the wait for the last product",
