@@ -16,8 +16,7 @@
 // of the decays after them.  With all of it in float the results were 1.1 to 1.9 times as far from 64-bit sums as the row scan's; so they
 // are 0.80 to 1.00 times as far (outputs) and 0.95 to 1.00 (state): 1.1e-7 and 0.9e-7 at a decay_scale of exp(-1/2), the scan 1.2e-7 and 1.0e-7.
 // Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
-// of 2,048 rows, 64 heads of 64, decay rank 64: 485 us with the launches (421 with the packs in float), where the kernels that prepare the rows and
-// scan them one by one take 172 + 614 without.
+// of 2,048 rows, 64 heads of 64, decay rank 64: 450 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
 // The first two are bound by their instructions; the last walks 128 chunks, one warp a scheduler, each chunk's products waiting for the state of
 // the one before (half warps or warps a row, four or eight value channels a warp, sums across lanes or through shared memory: all within
 // 3 % of one another).
@@ -93,16 +92,17 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
 #define DLC_RUN 4             // places of chunks a block takes one after another, the next one's rows on their way
 
 // A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
-// columns through the same substitutions.
-__global__ void __launch_bounds__(DLC_D + 32, 3)
+// columns through the same substitutions.  Chains of dependent steps, so what counts is how many blocks an SM holds: one stage of rows, refilled as soon as
+// they are in registers, leaves room for four (two stages: three; with them and a square root a channel instead of a row 488 us the whole call, now 450).
+__global__ void __launch_bounds__(DLC_D + 32, 4)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
                     const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
     constexpr int PACK = chunk_pack_floats(DLC_D, true), THREADS = DLC_D + 32, ROW_SET = CHUNK * DLC_D;
     extern __shared__ __align__(16) float delta_smem[];
-    float (*in)[4][CHUNK][DLC_D] = reinterpret_cast<float (*)[4][CHUNK][DLC_D]>(delta_smem);            // two stages of decays, r, k, a
-    double *Y = reinterpret_cast<double*>(delta_smem + 2 * 4 * ROW_SET), *X = Y + DLC_D * DLC_YP, *M = Y;      // (M [16][16] where Y was, once that has been used)
+    float (*in)[CHUNK][DLC_D] = reinterpret_cast<float (*)[CHUNK][DLC_D]>(delta_smem);                  // a chunk's decays, r, k, a
+    double *Y = reinterpret_cast<double*>(delta_smem + 4 * ROW_SET), *X = Y + DLC_D * DLC_YP, *M = Y;      // (M [16][16] where Y was, once that has been used)
     float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm
-    __shared__ float part[2][CHUNK];
+    __shared__ float part[2][CHUNK], norm[CHUNK];
     __shared__ ChunkAt todo[DLC_RUN];
     __shared__ int todo_place[DLC_RUN], n_todo;
     pdl_launch_dependents_if_resident();
@@ -130,7 +130,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
     auto issue = [&](int c) {
         const int rows = todo[c].rows, quads = D / 4;
         const size_t first = (size_t)todo[c].row;
-        const uint32_t dst = ad_smem(&in[c & 1][0][0][0]);
+        const uint32_t dst = ad_smem(&in[0][0][0]);
         for (int i = threadIdx.x; i < rows * quads; i += THREADS) {
             const int t = i / quads, at = 4 * (i - t * quads);
             const float* pr = proj + (first + t) * stride + h * D + at;
@@ -143,13 +143,11 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
     };
     issue(0);
     cp_async_commit();
+    const float (*sw)[DLC_D] = in[0], (*sr)[DLC_D] = in[1], (*sk)[DLC_D] = in[2], (*sa)[DLC_D] = in[3];
     for (int c = 0; c < n; c++) {
-        if (c + 1 < n) issue(c + 1);
-        cp_async_commit();
-        cp_async_wait<1>();
+        cp_async_wait<0>();
         __syncthreads();
         const int rows = todo[c].rows;
-        const float (*sw)[DLC_D] = in[c & 1][0], (*sr)[DLC_D] = in[c & 1][1], (*sk)[DLC_D] = in[c & 1][2], (*sa)[DLC_D] = in[c & 1][3];
         if (channel) {
             // Sixteen sums over a warp's channels, halved among its lanes: lane L (of sixteen) is left with row L.
             float kk[CHUNK];
@@ -171,6 +169,8 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             if (lane < CHUNK) part[warp][lane] = kk[0];
         }
         __syncthreads();
+        if (d < CHUNK) norm[d] = sqrtf(part[0][d] + part[1][d] + key_eps);      // once a row, not once a channel
+        __syncthreads();
         float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
         float z1[CHUNK], zk[CHUNK];               // b_t and k_t, then times the decays after row t
@@ -181,7 +181,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
                 const bool ok = mine && t < rows;
                 const float k = ok ? sk[t][d] : 0.0f;
                 const float rate = 1.0f / (1.0f + expf(-((ok ? sa[t][d] : 0.0f) + bias)));
-                const float u = ok ? k / sqrtf(part[0][t] + part[1][t] + key_eps) : 0.0f;      // zero in rows and channels that do not exist
+                const float u = ok ? k / norm[t] : 0.0f;      // zero in rows and channels that do not exist
                 U[t] = u * run;
                 run *= ok ? sw[t][d] : 1.0f;
                 own[t] = (ok ? sr[t][d] : 0.0f) * run;
@@ -210,6 +210,8 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             dst[4 * CHUNK * DLC_D + CHUNK * CHUNK_G + d] = run;
         }
         __syncthreads();
+        if (c + 1 < n) issue(c + 1);              // these rows are in registers and in Y and X: the next ones may take their place
+        cp_async_commit();
         // [r W; u W] [b / W; k / W]^T over the channels in double: 32 x 32 sums, four rows by two of b and two of k a thread; those above the
         // diagonals are left out.
         if (channel) {
@@ -288,7 +290,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         __syncthreads();          // the next chunk writes Y, X and the triangles
     }
 }
-#define DLC_SMEM ((2 * 4 * CHUNK * DLC_D + 4 * CHUNK * CHUNK_G) * sizeof(float) + 2 * DLC_D * DLC_YP * sizeof(double))
+#define DLC_SMEM ((4 * CHUNK * DLC_D + 4 * CHUNK * CHUNK_G) * sizeof(float) + 2 * DLC_D * DLC_YP * sizeof(double))
 
 // Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not), of which those of
 // fewer than min_rows rows are left alone.
