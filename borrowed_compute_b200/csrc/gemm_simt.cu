@@ -305,15 +305,11 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
 
 // X [M, K] and W [N, K] (for SwiGLU: W [2N, K], gate rows then up rows) in the operand
 // type; `out` is [M, N] in the operand type (store, SwiGLU) or float (store_f32, add_f32).
-extern "C" int bc_gemm_split_takes(const void* X, const void* W, int cols, int K);
-extern "C" int bc_gemm_split_f32(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, cudaStream_t s);
-
 template <class T>
 static int dispatch(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, cudaStream_t s) {
     BC_CHECK_ARG(M >= 0 && N > 0 && K > 0, "gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
     BC_CHECK_ARG((M + 63) / 64 <= 65535, "gemm_simt: %d rows are more than 65535 tiles of 64", M);
     if (M == 0) return BC_OK;
-    if (sizeof(T) == 4 && bc_gemm_split_takes(X, W, epilogue == EPI_SWIGLU ? 2 * N : N, K)) return bc_gemm_split_f32(X, W, out, M, N, K, epilogue, a, b, cols, s);
     switch (epilogue) {
         case EPI_STORE: return launch<T, EPI_STORE>(X, W, out, M, N, K, a, b, cols, s);
         case EPI_STORE_F32: return launch<T, EPI_STORE_F32>(X, W, out, M, N, K, a, b, cols, s);

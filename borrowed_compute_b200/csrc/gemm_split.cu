@@ -10,17 +10,24 @@
 // Operands below 2^-110 lose their last bits (bfloat16 ends at 2^-133).
 // An operand that is infinite or not a number has no m and l: where the sum of h h is either, it is the result by itself.
 //
-// What bounds it: six tensor-core products a multiply-add, 32 k of 128 weight rows by N tokens in 6 N clocks of an SM, beside the
-// conversions (285 clocks a warp for 32 rows of 32 k) and shared memory (B operands, raw tiles and planes).  To keep shared memory free the weights' triples
-// go to tensor memory (the MMA's A operand), only the tokens' to shared memory.
-// Times, caches cold, this kernel against gemm_simt.cu's: 300 rows of a feed-forward of 2,048 x 8,192 157 + 126 us against 544 + 303; 3 rows 50 + 53 against 126 + 78;
-// 2,000 x 4,096 x 4,096 481 against 1,574; one row of 2 x 14,336 x 4,096 168 against 260, of 4,096 x 14,336 80 against 219; 5 x 64 x 2,048 19 against 35.
+// Two ways, the same sums in the same order and so the same bits:
 //
-// Warps: 0-3 split the weights, a row a thread, into tensor memory; 4-7 the tokens, into shared memory; 8-15 take D1 out and write the
-// result; 16 asks for raw tiles (TMA, 32 floats of a row, 128-byte swizzle); 17 issues the products.  Every wait is bounded.
+//   rows   Every block splits its weights, into tensor memory (the MMA's A operand, so that shared memory is free for the other), and its tokens, into
+//          shared memory.  What bounds it: six tensor-core products a multiply-add, 32 k (a chunk) of 128 weight rows by N tokens in some 1,000 clocks of an SM
+//          at N 112, and the rounds of wait, split, store and fence of its warps, 1,425 clocks a chunk.
+//   few    Up to a tile of rows, where weights are what there is to read: a kernel splits the tokens once, into planes of bfloat16 in scratch memory; they
+//          come by TMA as they are multiplied and all sixteen warps split weights.  742 clocks a chunk at one token, most of them the weights' way from memory.
+//          With more rows the planes' six bytes instead of four a value through the L2, in every block, cost more than the splits: 300 rows of 16,384 x 2,048
+//          173 us against 158, 2,000 of 4,096 x 4,096 529 against 481; 130 of 1,024 x 2,816 34 against 31; 64 of 16,384 x 2,048 48 against 54, 128 of 512 x 1,024 21 against 27.
+//
+// Times, caches cold, against gemm_simt.cu's: 300 rows of a feed-forward of 2,048 x 8,192 157 + 126 us, 544 + 303; 3 rows 44 + 44, 126 + 78;
+// 2,000 x 4,096 x 4,096 481, 1,574; one row of 2 x 14,336 x 4,096 126, 260, of 4,096 x 14,336 64, 219; 5 x 64 x 2,048 15, 35.
+// (Tried for many rows, none faster: sixteen warps that split and take sums out, three and four buffers of triples, two thirds of the products, 80 and 96 tokens a tile.)
+//
+// Every wait is bounded.
 //
 // An output's sum depends on its own rows and the matrix's sizes alone: the pieces of K are the matrix's (split_pieces), added in
-// ascending order through the shared memory of a cluster, and every launch of a matrix that this kernel takes goes here, one row or many.
+// ascending order through the shared memory of a cluster, and every launch of a matrix that these kernels take goes here, one row or many.
 #include <cooperative_groups.h>
 
 #include "mma_tiles.cuh"
@@ -34,14 +41,20 @@ namespace cg = cooperative_groups;
 #define SPL_BN 128               // tokens a tile at most
 #define SPL_W_BYTES (TC_BM * SPL_K * 4)
 #define SPL_STAGES 8
-#define SPL_D2 256               // tensor memory: D1 at 0 and 128, D2, then two buffers of the weights' triples, 16 columns a part
+#define SPL_FEW 112              // rows at most that go the second way, in one tile
+#define SPL_X_STAGES 4           // stages of 64 k of their planes on their way at most
+#define SPL_D2 256               // tensor memory of the first way: D1 at 0 and 128, D2, then two buffers of the weights' triples, 16 columns a part
 #define SPL_A 384
+
+// The second way: D1 (two of bn columns), D2, then the triples' buffers, three at 112 tokens, four below.
+#define SPL_A_COLS 48
+__host__ __device__ constexpr int split_buffers(int bn) { return (512 - 3 * bn) / SPL_A_COLS > 4 ? 4 : (512 - 3 * bn) / SPL_A_COLS; }
 
 struct SplitParams {
     float* out;
     int M, N, K;
     int second_row;              // SwiGLU: the matrix row where the up rows start
-    int bn, stages, piece;
+    int bn, stages, x_stages, piece;
     float act_a, act_b;
     int act_cols;
 };
@@ -62,6 +75,38 @@ __device__ __forceinline__ void split4(const float4 v, uint32_t* h, uint32_t* m,
     two(v.z, v.w, h[1], m[1], l[1]);
 }
 
+// The end of both: the sums of the pieces of K, in ascending order out of the cluster's blocks, and the epilogue.
+template <int EPI>
+__device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, const int* gave_up, int t0, int n0) {
+    constexpr int HALF_N = TC_BM / 2, OUT_COLS = EPI == EPI_SWIGLU ? HALF_N : TC_BM;
+    const int S = gridDim.z;
+    __syncwarp();
+    tc_fence_before();
+    if (S > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    if (dealloc) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+    if (!*reinterpret_cast<const volatile int*>(gave_up)) {
+        const int rows = min(p.bn, p.M - t0);
+        for (int e = blockIdx.z * SPL_THREADS + threadIdx.x; e < rows * OUT_COLS; e += S * SPL_THREADS) {
+            const int r = e / OUT_COLS, c = e % OUT_COLS, n = n0 + c;
+            if (n >= p.N) continue;
+            float v = 0.0f, u = 0.0f;
+            for (int z = 0; z < S; z++) {
+                const float* theirs = S > 1 ? cg::this_cluster().map_shared_rank(tile, z) : tile;
+                v = z ? v + theirs[r * TC_BM + c] : theirs[r * TC_BM + c];
+                if (EPI == EPI_SWIGLU) u = z ? u + theirs[r * TC_BM + HALF_N + c] : theirs[r * TC_BM + HALF_N + c];
+            }
+            simt_emit<float, EPI>(p.out, p.out, t0 + r, n, p.N, v, u, p.act_a, p.act_b, p.act_cols);
+        }
+    }
+    if (S > 1) cg::this_cluster().sync();      // no block leaves while a peer still reads its shared memory
+}
+
+// Warps: 0-3 split the weights, a row a thread, 4-7 the tokens; 8-15 take D1 out and write the result; 16 asks for raw tiles (TMA, 32 floats of a row, 128-byte
+// swizzle); 17 issues the products.
 template <int EPI>
 __global__ void __launch_bounds__(SPL_THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SplitParams p) {
@@ -233,30 +278,216 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
     }
     if (!ok) *reinterpret_cast<volatile int*>(&gave_up) = 1;
-    const int S = gridDim.z;
-    __syncwarp();
-    tc_fence_before();
-    if (S > 1) cg::this_cluster().sync();
-    else __syncthreads();
-    if (warp == 17) {
-        tc_fence_after();
-        tmem_dealloc(tmem, 512);
+    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, t0, n0);
+}
+
+// planes[part][row][k_row] = the parts of x[row][k], four k a thread.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* x, bf16* __restrict__ planes, int rows, int K, int k_row) {
+    pdl_wait();                        // before the next kernel may start: it reads its weights at once
+    pdl_launch_dependents();
+    PDL_FRESH(x);
+    const int quads = K / 4;
+    const size_t part = (size_t)rows * k_row;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < (long long)rows * quads; i += 256ll * gridDim.x) {
+        const int r = (int)(i / quads), k = 4 * (int)(i - (long long)r * quads);
+        uint32_t h[2], m[2], l[2];
+        split4(*reinterpret_cast<const float4*>(x + (size_t)r * K + k), h, m, l);
+        bf16* to = planes + (size_t)r * k_row + k;
+        *reinterpret_cast<uint2*>(to) = make_uint2(h[0], h[1]);
+        *reinterpret_cast<uint2*>(to + part) = make_uint2(m[0], m[1]);
+        *reinterpret_cast<uint2*>(to + 2 * part) = make_uint2(l[0], l[1]);
     }
-    if (!*reinterpret_cast<volatile int*>(&gave_up)) {
-        const int rows = min(bn, p.M - t0);
-        for (int e = blockIdx.z * SPL_THREADS + threadIdx.x; e < rows * OUT_COLS; e += S * SPL_THREADS) {
-            const int r = e / OUT_COLS, c = e % OUT_COLS, n = n0 + c;
-            if (n >= p.N) continue;
-            float v = 0.0f, u = 0.0f;
-            for (int z = 0; z < S; z++) {
-                const float* theirs = S > 1 ? cg::this_cluster().map_shared_rank(tile, z) : tile;
-                v = z ? v + theirs[r * TC_BM + c] : theirs[r * TC_BM + c];
-                if (EPI == EPI_SWIGLU) u = z ? u + theirs[r * TC_BM + HALF_N + c] : theirs[r * TC_BM + HALF_N + c];
+}
+
+// Warps: 0-15 split the weights of every fourth chunk, four warps a chunk, a row a thread, and take D1 out, a share of the columns each; 16 asks for tiles; 17
+// issues the products.
+template <int EPI>
+__global__ void __launch_bounds__(SPL_THREADS, 1)
+gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SplitParams p) {
+    constexpr int HALF_N = TC_BM / 2;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t bars[2 * SPL_STAGES + 2 * SPL_X_STAGES + 4 + 4 + 2 + 2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int gave_up;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const int bn = p.bn, stages = p.stages, x_stages = p.x_stages;
+    const int buffers = split_buffers(bn), d2_at = 2 * bn, a_at = 3 * bn;
+    const int plane = bn * 128;                              // bn rows of 64 k of one part; stages of three behind the ring of weights
+    uint8_t* planes = smem + stages * SPL_W_BYTES;
+    const int t0 = blockIdx.x * bn, n0 = blockIdx.y * (EPI == EPI_SWIGLU ? HALF_N : TC_BM);
+    const int k_begin = blockIdx.z * p.piece, k_end = min(p.K, k_begin + p.piece);
+    const int chunks = (k_end - k_begin + SPL_K - 1) / SPL_K, periods = (chunks + 1) / 2;
+    const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * SPL_STAGES, x_full = w_empty + 8 * SPL_STAGES, x_empty = x_full + 8 * SPL_X_STAGES,
+                   ready = x_empty + 8 * SPL_X_STAGES, done = ready + 32, d1_full = done + 32, d1_empty = d1_full + 16;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        for (int i = 0; i < SPL_STAGES; i++) {
+            mbar_init(w_full + 8 * i, 1);
+            mbar_init(w_empty + 8 * i, 4);
+        }
+        for (int i = 0; i < SPL_X_STAGES; i++) {
+            mbar_init(x_full + 8 * i, 1);
+            mbar_init(x_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < 4; i++) {
+            mbar_init(ready + 8 * i, 4);
+            mbar_init(done + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(d1_full + 8 * i, 1);
+            mbar_init(d1_empty + 8 * i, 16);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 17) tmem_alloc(smem_u32(&tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    float* tile = reinterpret_cast<float*>(smem);        // [bn][128]: the result, over the ring of weights once that is drained
+    bool ok = true;
+    auto wait = [&](uint32_t bar, int phase, int code) { return ok = mbar_wait_warp(bar, phase & 1, code); };   // the whole warp
+    pdl_launch_dependents();
+    if (warp < 16) {
+        // Chunk j is four warps' (j % 4): out of ring stage j % stages into tensor memory buffer j % buffers, free when the products of chunk j - buffers
+        // are done.  After its chunk every warp takes its share of the stretches (two chunks each) before out of D1.
+        const int q = warp & 3, part = warp >> 2;
+        const int row = 32 * q + lane;
+        const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16);
+        uint64_t acc[2][8] = {};                             // token columns 16 part .. and 64 + 16 part ..
+        int taken = 0;
+        auto take_out_before = [&](int end) {
+            for (; taken < end; taken++) {
+                const int b = taken & 1;
+                if (!wait(d1_full + 8 * b, taken >> 1, 3)) return;
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    if (64 * c + 16 * part >= bn) break;
+                    uint32_t v[16];
+                    tmem_load16(lanes + bn * b + 64 * c + 16 * part, v);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int e = 0; e < 8; e++) acc[c][e] = add_f32x2(acc[c][e], pack_f32x2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(d1_empty + 8 * b);
             }
-            simt_emit<float, EPI>(p.out, p.out, t0 + r, n, p.N, v, u, p.act_a, p.act_b, p.act_cols);
+        };
+        for (int j = part, s = part % stages, round = part / stages, buffer = part % buffers; j < chunks; j += 4) {
+            if (!wait(w_full + 8 * s, round, 1)) break;
+            const uint8_t* src = smem + s * SPL_W_BYTES + row * 128;
+            uint32_t h[16], m[16], l[16];
+            float4 v[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) v[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
+#pragma unroll
+            for (int c = 0; c < 8; c++) split4(v[c], h + 2 * c, m + 2 * c, l + 2 * c);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(w_empty + 8 * s);
+            if ((s += 4) >= stages) s -= stages, round++;
+            if (j >= buffers && !wait(done + 8 * ((j - buffers) & 3), (j - buffers) >> 2, 2)) break;
+            tc_fence_after();
+            const uint32_t to = lanes + a_at + buffer * SPL_A_COLS;
+            tmem_store16(to, h);
+            tmem_store16(to + 16, m);
+            tmem_store16(to + 32, l);
+            tmem_store_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ready + 8 * (j & 3));
+            if ((buffer += 4 % buffers) >= buffers) buffer -= buffers;
+            take_out_before(j / 2);       // all but the stretch under way: the products of the next one but one wait for this one's sums
+            if (!ok) break;
+        }
+        if (ok) take_out_before(periods);
+        if (ok) {
+            // D1's last sums came after the last product, D2's with them.  No tile is on its way and none is read any more.
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                if (64 * c + 16 * part >= bn) break;
+                uint32_t v[16];
+                tmem_load16(lanes + d2_at + 64 * c + 16 * part, v);
+                tmem_load_wait();
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    float a0, a1;
+                    unpack_f32x2(acc[c][e], a0, a1);
+                    float* to = tile + (64 * c + 16 * part + 2 * e) * TC_BM + 32 * q + lane;
+                    to[0] = fabsf(a0) < INFINITY ? a0 + __uint_as_float(v[2 * e]) : a0;
+                    to[TC_BM] = fabsf(a1) < INFINITY ? a1 + __uint_as_float(v[2 * e + 1]) : a1;
+                }
+            }
+        }
+    } else if (warp == 16) {
+        if (elect_one()) {
+            const int second = EPI == EPI_SWIGLU ? p.second_row + n0 : n0 + HALF_N;
+            auto load_w = [&](int j, int s) {
+                const uint32_t dst = smem_u32(smem + s * SPL_W_BYTES), bar = w_full + 8 * s;
+                mbar_expect_tx(bar, SPL_W_BYTES);
+                tma_load_2d(dst, &map_w, bar, k_begin + j * SPL_K, n0);
+                tma_load_2d(dst + SPL_W_BYTES / 2, &map_w, bar, k_begin + j * SPL_K, second);
+            };
+            // The kernel before is the one that split the tokens, and it waited for all before it: the weights are there.
+            const int ahead = min(stages, chunks);
+            for (int j = 0; j < ahead; j++) load_w(j, j);
+            pdl_wait();
+            for (int j = 0, s = 0, round = 0, xs = 0, x_round = 0; j < chunks; j++) {
+                if (!(j & 1)) {
+                    if (x_round && !(ok = mbar_wait(x_empty + 8 * xs, (x_round - 1) & 1, 4))) break;
+                    const uint32_t dst = smem_u32(planes + xs * 3 * plane), bar = x_full + 8 * xs;
+                    mbar_expect_tx(bar, (uint32_t)(3 * plane));
+                    for (int i = 0; i < 3; i++) tma_load_3d(dst + i * plane, &map_x, bar, k_begin + j * SPL_K, t0, i);
+                    if (++xs == x_stages) xs = 0, x_round++;
+                }
+                if (round) {
+                    if (!(ok = mbar_wait(w_empty + 8 * s, (round - 1) & 1, 4))) break;
+                    load_w(j, s);
+                }
+                if (++s == stages) s = 0, round++;
+            }
+        }
+    } else {
+        const uint32_t idesc = instr_desc(bn);
+        const uint64_t b_desc = smem_desc(smem_u32(planes));
+        const uint32_t part = (uint32_t)plane >> 4;
+        for (int j = 0, buffer = 0, xs = 0, x_round = 0; j < chunks; j++) {
+            const int b = (j >> 1) & 1;
+            const bool last = (j & 1) || j + 1 == chunks;     // of its stretch and its stage of tokens
+            if (!(j & 1)) {
+                if (!wait(x_full + 8 * xs, x_round, 6)) break;
+                if (j >= 4 && !wait(d1_empty + 8 * b, (j >> 2) - 1, 5)) break;
+            }
+            if (!wait(ready + 8 * (j & 3), j >> 2, 6)) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < SPL_K / 16; kk++) {
+                    const uint32_t a = tmem + a_at + buffer * SPL_A_COLS + 8 * kk;
+                    const uint64_t h = b_desc + (uint64_t)(xs * 3 * part + (j & 1) * 4 + 2 * kk), m = h + part, l = m + part;
+                    mma_bf16_a_tmem(tmem + bn * b, a, h, idesc, (j & 1) | kk);
+                    mma_bf16_a_tmem(tmem + d2_at, a + 16, h, idesc, j | kk);
+                    mma_bf16_a_tmem(tmem + d2_at, a, m, idesc, 1);
+                    mma_bf16_a_tmem(tmem + d2_at, a + 16, m, idesc, 1);
+                    mma_bf16_a_tmem(tmem + d2_at, a + 32, h, idesc, 1);
+                    mma_bf16_a_tmem(tmem + d2_at, a, l, idesc, 1);
+                }
+                mma_commit(done + 8 * (j & 3));
+                if (last) {
+                    mma_commit(x_empty + 8 * xs);
+                    mma_commit(d1_full + 8 * b);
+                }
+            }
+            __syncwarp();
+            if (last && ++xs == x_stages) xs = 0, x_round++;
+            if (++buffer == buffers) buffer = 0;
         }
     }
-    if (S > 1) cg::this_cluster().sync();      // no block leaves while a peer still reads its shared memory
+    pdl_wait();       // the output may still be in use by a kernel before
+    if (!ok) *reinterpret_cast<volatile int*>(&gave_up) = 1;
+    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, t0, n0);
 }
 
 // -------------------------------------------------------------------------------- the host
@@ -269,6 +500,18 @@ static int float_map(CUtensorMap* map, const void* base, int rows, int K, int bo
                                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         bc_set_error("gemm_split: cuTensorMapEncodeTiled failed (%d) for a [%d, %d] matrix, box %d x %d", (int)r, rows, K, box_rows, SPL_K);
+        return BC_ERR_DRIVER;
+    }
+    return BC_OK;
+}
+
+static int planes_map(CUtensorMap* map, const void* base, int rows, int K, int k_row, int bn) {
+    cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)k_row * 2, (cuuint64_t)k_row * 2 * rows};
+    cuuint32_t box[3] = {2 * SPL_K, (cuuint32_t)bn, 1}, elem[3] = {1, 1, 1};
+    const CUresult r = bc_encode_tiled_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        bc_set_error("gemm_split: cuTensorMapEncodeTiled failed (%d) for planes of [%d, %d], box %d x %d", (int)r, rows, K, bn, 2 * SPL_K);
         return BC_ERR_DRIVER;
     }
     return BC_OK;
@@ -287,31 +530,42 @@ extern "C" int bc_gemm_split_takes(const void* X, const void* W, int cols, int K
     return K > 512 && K % 4 == 0 && (uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0 && (long long)cols <= 65535ll * 64 && bc_encode_tiled_fn() != nullptr;
 }
 
+static int split_k_row(int K) { return (K + 7) / 8 * 8; }
+// Bytes of scratch: three planes of the rows that go the second way.
+extern "C" long long bc_gemm_split_scratch(int M, int K) { return M <= SPL_FEW ? 6ll * M * split_k_row(K) : 0; }
+
 template <int EPI>
-static int launch(const void* X, const void* W, void* out, int M, int N, int K, float a, float b, int cols, cudaStream_t s) {
+static int launch(const void* X, const void* W, void* out, int M, int N, int K, float a, float b, int cols, void* scratch, cudaStream_t s) {
     const int w_rows = EPI == EPI_SWIGLU ? 2 * N : N, out_cols = EPI == EPI_SWIGLU ? TC_BM / 2 : TC_BM;
+    const bool few = M <= SPL_FEW;
     SplitParams p = {};
     p.out = (float*)out, p.M = M, p.N = N, p.K = K, p.second_row = N, p.act_a = a, p.act_b = b, p.act_cols = cols;
     const int t_tiles = (M + SPL_BN - 1) / SPL_BN;
     p.bn = ((M + t_tiles - 1) / t_tiles + 15) / 16 * 16;
     const int splits = split_pieces(w_rows, K);
-    p.piece = ((K + splits - 1) / splits + SPL_K - 1) / SPL_K * SPL_K;
-    const int stage = SPL_W_BYTES + p.bn * 128;
-    p.stages = (TC_SMEM_LIMIT - 1024 - 6 * p.bn * 128) / stage;
+    p.piece = ((K + splits - 1) / splits + 2 * SPL_K - 1) / (2 * SPL_K) * (2 * SPL_K);
+    // A ring of chunks, both operands' raw tiles or the weights' alone, and stages of 64 k of the tokens' planes.
+    p.x_stages = !few || p.bn > 64 ? 2 : SPL_X_STAGES;
+    const int stage = SPL_W_BYTES + (few ? 0 : p.bn * 128), planes = p.x_stages * 3 * p.bn * 128;
+    p.stages = (TC_SMEM_LIMIT - 1024 - planes) / stage;
     if (p.stages > SPL_STAGES) p.stages = SPL_STAGES;
-    const int smem = p.stages * stage + 6 * p.bn * 128 + 1024;
+    const int smem = p.stages * stage + planes + 1024;
     CUtensorMap mw, mx;
     int st = float_map(&mw, W, w_rows, K, TC_BM / 2);
-    if (st == BC_OK) st = float_map(&mx, X, M, K, p.bn);
+    if (st == BC_OK) st = few ? planes_map(&mx, scratch, M, K, split_k_row(K), p.bn) : float_map(&mx, X, M, K, p.bn);
     if (st != BC_OK) return st;
-    if (cudaError_t e = bc_allow_shared<gemm_split_kernel<EPI>>(TC_SMEM_LIMIT); e != cudaSuccess) {
-        bc_set_error("gemm_split: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
-        return (int)e;
+    cudaError_t e = few ? bc_allow_shared<gemm_split_few_kernel<EPI>>(TC_SMEM_LIMIT) : bc_allow_shared<gemm_split_kernel<EPI>>(TC_SMEM_LIMIT);
+    if (e == cudaSuccess && few) {
+        const int quads = M * (K / 4), most = 8 * bc_sm_count();
+        e = bc_launch(split_rows_kernel, dim3((quads + 255) / 256 < most ? (quads + 255) / 256 : most), dim3(256), 0, s, (const float*)X, (bf16*)scratch, M, K, split_k_row(K));
     }
     // Token tiles fastest: the blocks that read the same weights run side by side.
     const dim3 grid((M + p.bn - 1) / p.bn, (N + out_cols - 1) / out_cols, splits);
-    const cudaError_t e = splits > 1 ? bc_launch_clustered(gemm_split_kernel<EPI>, grid, dim3(SPL_THREADS), (size_t)smem, s, dim3(1, 1, splits), mw, mx, p)
-                                     : bc_launch(gemm_split_kernel<EPI>, grid, dim3(SPL_THREADS), (size_t)smem, s, mw, mx, p);
+    auto go = [&](auto kernel) {
+        return splits > 1 ? bc_launch_clustered(kernel, grid, dim3(SPL_THREADS), (size_t)smem, s, dim3(1, 1, splits), mw, mx, p)
+                          : bc_launch(kernel, grid, dim3(SPL_THREADS), (size_t)smem, s, mw, mx, p);
+    };
+    if (e == cudaSuccess) e = few ? go(gemm_split_few_kernel<EPI>) : go(gemm_split_kernel<EPI>);
     if (e != cudaSuccess) {
         bc_set_error("gemm_split: launch failed: %s", cudaGetErrorString(e));
         return (int)e;
@@ -319,16 +573,20 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
     BC_LAUNCH_STATUS();
 }
 
-// The interface of gemm_simt's float product, for what bc_gemm_split_takes.
-extern "C" int bc_gemm_split_f32(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, cudaStream_t s) {
+// gemm_simt's float product for what bc_gemm_split_takes, with bc_gemm_split_scratch(M, K) bytes of scratch (on a 16-byte border).
+extern "C" int bc_gemm_split_f32(const void* X, const void* W, void* out, int M, int N, int K, int epilogue, float a, float b, int cols, void* scratch, cudaStream_t s) {
+    BC_CHECK_ARG(M >= 0 && N > 0 && K > 0, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
+    BC_CHECK_ARG(bc_gemm_split_takes(X, W, epilogue == EPI_SWIGLU ? 2 * N : N, K), "gemm_split: K=%d must be more than 512 and a multiple of four, the operands on 16-byte borders", K);
+    if (M == 0) return BC_OK;
+    BC_CHECK_ARG(M > SPL_FEW || (scratch != nullptr && (uintptr_t)scratch % 16 == 0), "gemm_split: %d rows take scratch on a 16-byte border", M);
     switch (epilogue) {
-        case EPI_STORE: return launch<EPI_STORE>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_STORE_F32: return launch<EPI_STORE_F32>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_ADD_F32: return launch<EPI_ADD_F32>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_SWIGLU: return launch<EPI_SWIGLU>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_RELU2: return launch<EPI_RELU2>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_XIELU: return launch<EPI_XIELU>(X, W, out, M, N, K, a, b, cols, s);
-        case EPI_SILU_F32: return launch<EPI_SILU_F32>(X, W, out, M, N, K, a, b, cols, s);
+        case EPI_STORE: return launch<EPI_STORE>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_STORE_F32: return launch<EPI_STORE_F32>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_ADD_F32: return launch<EPI_ADD_F32>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_SWIGLU: return launch<EPI_SWIGLU>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_RELU2: return launch<EPI_RELU2>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_XIELU: return launch<EPI_XIELU>(X, W, out, M, N, K, a, b, cols, scratch, s);
+        case EPI_SILU_F32: return launch<EPI_SILU_F32>(X, W, out, M, N, K, a, b, cols, scratch, s);
     }
     bc_set_error("gemm_split: unknown epilogue %d", epilogue);
     return BC_ERR_ARG;

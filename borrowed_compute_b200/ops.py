@@ -344,6 +344,15 @@ def _act_numbers(who: str, epilogue: int, act: Optional[Tuple[float, float]], co
     return (0.0, 0.0, int(cols)) if act is None else (float(act[0]), float(act[1]), 0)
 
 
+SPLIT_FEW = 112     # rows at most whose parts the float32 product on the tensor cores keeps in scratch memory (csrc/gemm_split.cu)
+
+
+def _split_scratch(M: int, K: int) -> int:
+    f = getattr(lib(), "bc_gemm_split_scratch")
+    f.restype = ctypes.c_longlong
+    return int(f(_c_int(M), _c_int(K)))
+
+
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, act: Optional[Tuple[float, float]] = None,
               cols: Optional[int] = None) -> None:
     """out = x @ w.T with float accumulation, k ascending in one piece or in up to eight that are added in order: on the CUDA cores, or,
@@ -365,6 +374,16 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int
     if tuple(out.shape) != (M, N):
         raise KernelError(f"gemm: out is {tuple(out.shape)}, wanted {(M, N)}")
     numbers = _act_numbers("gemm_simt", epilogue, act, cols)
+    if x.dtype == torch.float32 and K > 512 and _fn("bc_gemm_split_takes")(_ptr(x), _ptr(w), _c_int(n_w), _c_int(K)):
+        a, b, n_cols = numbers or (0.0, 0.0, 0)
+        scratch = None
+        if M <= SPLIT_FEW:
+            global launches
+            launches += 1                                  # the kernel that fills the scratch memory
+            scratch = torch.empty(_split_scratch(M, K), dtype=torch.uint8, device=x.device)
+        _call(_fn("bc_gemm_split_f32"), _ptr(x), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _c_int(epilogue), _c_float(a), _c_float(b), _c_int(n_cols),
+              _ptr(scratch), _stream())
+        return
     if numbers is not None:
         a, b, n_cols = numbers
         _call(_fn("bc_gemm_simt_act_" + _suffix(x.dtype)), _ptr(x), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _c_int(epilogue), _c_float(a),
@@ -518,7 +537,7 @@ _WAITS = {
     3: {1: "the loader's wait for a free stage", 2: "the wait for the queries", 3: "the wait for the first pages", 4: "the wait for P",
         5: "the wait for a page", 6: "the softmax's wait for scores", 7: "the wait for a product that frees P", 8: "the wait for the last product",
         9: "the wait before a rescale"},
-    4: {1: "the wait for a raw tile", 2: "the wait for products that free operands", 3: "the wait for a stretch's sums", 4: "the loader's wait for a free stage",
+    4: {1: "the wait for a tile", 2: "the wait for products that free operands", 3: "the wait for a stretch's sums", 4: "the loader's wait for a free stage",
         5: "the wait for the sums to be taken out", 6: "the wait for operands"},
 }
 _bound_devices = set()
