@@ -989,6 +989,44 @@ struct TcGroupParams {
 // Rows a box of the activations' map holds.
 __host__ __device__ constexpr int tcg_box(int bn) { return bn < 64 ? bn : 64; }
 
+// What a warp writes of a piece: output out_n a lane, every HALVES-th run of sixteen of the piece's rows.
+template <int EPI, int BN, int HALVES>
+__device__ __forceinline__ void grouped_emit(const TcGroupParams& p, uint32_t taddr, int out_n, int t0, int t_count, int half) {
+    // Sixteen columns at a time, the next ones on their way while these are written.
+    uint32_t va[16], vb[16], ua[16], ub[16];
+    auto fetch = [&](uint32_t* v, uint32_t* u, int cc) {
+        tmem_load16(taddr + cc, v);
+        if (EPI == EPI_SWIGLU) tmem_load16(taddr + BN + cc, u);
+    };
+    auto emit = [&](const uint32_t* v, const uint32_t* u, int cc) {
+        if (out_n >= p.N) return;
+        float r[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) r[j] = EPI == EPI_SWIGLU ? glu_mul(__uint_as_float(v[j]), __uint_as_float(u[j]), p.glu_limit, p.glu_alpha) : epi_plain<EPI>(__uint_as_float(v[j]));
+        const size_t o = (size_t)(t0 + cc) * p.N + out_n;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            if (cc + j >= t_count) break;
+            const size_t at = o + (size_t)j * p.N;
+            if (EPI == EPI_SWIGLU || EPI == EPI_RELU2) ((bf16*)p.out)[at] = __float2bfloat16_rn(r[j]);
+            else ((float*)p.out)[at] = r[j];
+        }
+    };
+    constexpr int STEP = 16 * HALVES;
+    int cc = 16 * half;
+    if (cc < t_count) fetch(va, ua, cc);
+    for (; cc < t_count; cc += 2 * STEP) {
+        tmem_load_wait();
+        if (cc + STEP < t_count) fetch(vb, ub, cc + STEP);
+        emit(va, ua, cc);
+        if (cc + STEP < t_count) {
+            tmem_load_wait();
+            if (cc + 2 * STEP < t_count) fetch(va, ua, cc + 2 * STEP);
+            emit(vb, ub, cc + STEP);
+        }
+    }
+}
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(tc_threads(BN), 1)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcGroupParams p) {
@@ -1113,39 +1151,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem + buffer * ACC_COLS + ((uint32_t)(32 * q) << 16);
-            // Sixteen columns at a time, the next ones on their way while these are written.
-            uint32_t va[16], vb[16], ua[16], ub[16];
-            auto fetch = [&](uint32_t* v, uint32_t* u, int cc) {
-                tmem_load16(taddr + cc, v);
-                if (EPI == EPI_SWIGLU) tmem_load16(taddr + BN + cc, u);
-            };
-            auto emit = [&](const uint32_t* v, const uint32_t* u, int cc) {
-                if (out_n >= p.N) return;
-                float r[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++) r[j] = EPI == EPI_SWIGLU ? glu_mul(__uint_as_float(v[j]), __uint_as_float(u[j]), p.glu_limit, p.glu_alpha) : epi_plain<EPI>(__uint_as_float(v[j]));
-                const size_t o = (size_t)(t0 + cc) * p.N + out_n;
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    if (cc + j >= t_count) break;
-                    const size_t at = o + (size_t)j * p.N;
-                    if (EPI == EPI_SWIGLU || EPI == EPI_RELU2) ((bf16*)p.out)[at] = __float2bfloat16_rn(r[j]);
-                    else ((float*)p.out)[at] = r[j];
-                }
-            };
-            constexpr int STEP = 16 * HALVES;
-            int cc = 16 * half;
-            if (cc < t_count) fetch(va, ua, cc);
-            for (; cc < t_count; cc += 2 * STEP) {
-                tmem_load_wait();
-                if (cc + STEP < t_count) fetch(vb, ub, cc + STEP);
-                emit(va, ua, cc);
-                if (cc + STEP < t_count) {
-                    tmem_load_wait();
-                    if (cc + 2 * STEP < t_count) fetch(va, ua, cc + 2 * STEP);
-                    emit(vb, ub, cc + STEP);
-                }
-            }
+            grouped_emit<EPI, BN, HALVES>(p, taddr, out_n, t0, t_count, half);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty0 + 8 * buffer);
@@ -1156,6 +1162,141 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
+// The same on pairs of SMs (cta_group::2) where matrices meet many rows: the two blocks of a pair take neighbouring weight tiles and half of the table tile's
+// rows each, and the tensor cores of both read both halves.  What bounds the product at such rows is the way of the operands from the L2 to the SMs, some
+// 7.5 TB/s for all kernels of this file: a block's k-step of 64 is 44 KB instead of 56 (gated, 192 rows), 28 instead of 40 (not gated).
+// Pairs against one block a piece, caches cold, us: not gated, 12,288 rows of 64 matrices of 2,048 x 1,408 82 against 93, 24,576 rows 128 and 155,
+// 16,384 rows of 32 of 4,096 x 2,048 222 and 255; gated, 16,384 rows of 32 of 2 x 2,048 x 4,096 497 and 523, 3,000 of 8 of 2 x 4,096 x 4,096 206 and 212, but 24,576 rows of 64 of
+// 2 x 1,408 x 2,048, eleven weight tiles, 304 and 280.
+template <int EPI>
+__global__ void __launch_bounds__(TCP_THREADS, 1)
+gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcGroupParams p) {
+    constexpr int TILE = TC_BM * TC_BK * 2;               // 16 KB: 128 rows of 64 k
+    constexpr int N_ACC = EPI == EPI_SWIGLU ? 2 : 1;      // weight tiles a block: gate and up rows of its 128 outputs, or 128 outputs
+    constexpr int STAGE_BYTES = (N_ACC + 1) * TILE;       // and its half of the rows, at most 128
+    constexpr int BN = 256, BUFFERS = 2 / N_ACC, BOX = 64;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t bars[2 * 16 + 4];
+    __shared__ uint32_t tmem_slot;
+
+    cg::cluster_group cl = cg::this_cluster();
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();              // 0: the block that issues the products
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int stages = p.stages;
+    const int k_iters = (p.K + TC_BK - 1) / TC_BK;
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[16]), acc_full0 = smem_u32(&bars[32]), acc_empty0 = smem_u32(&bars[34]);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; s++) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int b = 0; b < BUFFERS; b++) {
+            mbar_init(acc_full0 + 8 * b, 1);
+            mbar_init(acc_empty0 + 8 * b, 16);            // the eight epilogue warps of both blocks
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(&tmem_slot), 512);
+    tc_fence_before();
+    cl.sync();   // both blocks' barriers and TMEM exist before either signals or writes the other's
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();                                   // the table, the rows and the output belong to the kernels before
+    const int* table = p.table;
+    PDL_FRESH(table);
+    const int n_tiles = (p.N + 2 * TC_BM - 1) / (2 * TC_BM);
+    const int pieces = table[0] * n_tiles;
+    // Piece number -> this block's first output, matrix, first row, rows, the rows rounded up to what the pair multiplies.
+    auto piece_at = [&](int piece, int& n0, int& matrix, int& t0, int& t_count, int& bn) {
+        const int tile = piece / n_tiles;
+        n0 = (2 * (piece - tile * n_tiles) + (int)rank) * TC_BM;
+        matrix = table[1 + 3 * tile], t0 = table[2 + 3 * tile], t_count = table[3 + 3 * tile];
+        bn = (t_count + 31) & ~31;
+    };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            const uint32_t pair_full0 = map_to_rank(full0, 0);   // the even block's barriers count both blocks' bytes
+            bool ok = true;
+            int s = 0, round = 0;
+            for (int piece = pair; piece < pieces && ok; piece += n_pairs) {
+                int n0, matrix, t0, t_count, bn;
+                piece_at(piece, n0, matrix, t0, t_count, bn);
+                const int w_row = matrix * p.matrix_rows + n0, x_row = t0 + (int)rank * (bn / 2);
+                const int boxes = (bn / 2 + BOX - 1) / BOX;
+                const uint32_t bytes = N_ACC * TILE + boxes * BOX * TC_BK * 2;
+                for (int i = 0; i < k_iters; i++) {
+                    if (round && !(ok = mbar_wait(empty0 + 8 * s, (round - 1) & 1, 1))) break;
+                    const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), bar = pair_full0 + 8 * s;
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * bytes);
+                    const int k = i * TC_BK;
+                    tma_load_2d_pair(a, &map_w, bar, k, w_row);
+                    if (N_ACC == 2) tma_load_2d_pair(a + TILE, &map_w, bar, k, w_row + p.N);
+                    for (int b = 0; b < boxes; b++) tma_load_2d_pair(a + N_ACC * TILE + b * BOX * TC_BK * 2, &map_x, bar, k, x_row + b * BOX);
+                    if (++s == stages) s = 0, round++;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            bool ok = true;
+            int s = 0, round = 0, n = 0;
+            for (int piece = pair; piece < pieces && ok; piece += n_pairs, n++) {
+                const int buffer = n % BUFFERS;
+                // The epilogue warps of both blocks must have read this accumulator's last piece out of TMEM.
+                if (n >= BUFFERS && !(ok = mbar_wait_warp(acc_empty0 + 8 * buffer, ((n / BUFFERS) & 1) ^ 1, 4))) break;
+                tc_fence_after();
+                int n0, matrix, t0, t_count, bn;
+                piece_at(piece, n0, matrix, t0, t_count, bn);
+                const uint32_t idesc = instr_desc_pair(bn), acc_at = tmem + buffer * BN;
+                for (int i = 0; i < k_iters; i++) {
+                    if (!(ok = mbar_wait_warp(full0 + 8 * s, round & 1, 2))) break;
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+                    const uint64_t da = smem_desc(a), du = smem_desc(a + TILE), db = smem_desc(a + N_ACC * TILE);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < TC_BK / 16; kk++) {
+                            const uint32_t acc = (i | kk) != 0;
+                            mma_bf16_pair(acc_at, da + 2 * kk, db + 2 * kk, idesc, acc);
+                            if (N_ACC == 2) mma_bf16_pair(acc_at + BN, du + 2 * kk, db + 2 * kk, idesc, acc);
+                        }
+                        mma_commit_pair(empty0 + 8 * s, 3);
+                        if (i + 1 == k_iters) mma_commit_pair(acc_full0 + 8 * buffer, 3);
+                    }
+                    __syncwarp();
+                    if (++s == stages) s = 0, round++;
+                }
+            }
+        }
+    } else {
+        // Epilogue, in both blocks: lanes 32 q .. 32 q + 31 of this SM's tensor memory, every other run of sixteen columns a warp.
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        int n = 0;
+        for (int piece = pair; piece < pieces; piece += n_pairs, n++) {
+            const int buffer = n % BUFFERS;
+            int n0, matrix, t0, t_count, bn;
+            piece_at(piece, n0, matrix, t0, t_count, bn);
+            if (!mbar_wait_warp(acc_full0 + 8 * buffer, (n / BUFFERS) & 1, 3)) break;
+            tc_fence_after();
+            grouped_emit<EPI, BN, 2>(p, tmem + buffer * BN + ((uint32_t)(32 * q) << 16), n0 + 32 * q + lane, t0, t_count, half);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_rank(acc_empty0 + 8 * buffer, 0));
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cl.sync();   // neither block leaves, or frees TMEM, while the pair's products or arrivals may still touch it
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem, 512);
     }
 }
 
@@ -1179,6 +1320,26 @@ static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupP
     const long long pieces = (long long)((p.N + TC_BM - 1) / TC_BM) * max_tiles;      // at most: the table says how many
     const int blocks = stream || pieces < bc_sm_count() ? (int)pieces : bc_sm_count();
     cudaError_t e = bc_launch(gemm_tc_grouped_kernel<BN, EPI>, dim3(blocks), dim3(tc_threads(BN)), (size_t)smem, s, mw, mx, p);
+    if (e != cudaSuccess) {
+        bc_set_error("gemm_tc_grouped: launch failed: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    BC_LAUNCH_STATUS();
+}
+
+template <int EPI>
+static int launch_grouped_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcGroupParams p, int max_tiles, cudaStream_t s) {
+    constexpr int STAGE_BYTES = ((EPI == EPI_SWIGLU ? 2 : 1) + 1) * TC_BM * TC_BK * 2;
+    p.stages = (TC_SMEM_LIMIT - 1024) / STAGE_BYTES;
+    const int smem = p.stages * STAGE_BYTES + 1024;
+    if (cudaError_t e = bc_allow_shared<gemm_tc_grouped_pair_kernel<EPI>>(TC_SMEM_LIMIT); e != cudaSuccess) {
+        bc_set_error("gemm_tc_grouped: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    const long long pieces = (long long)((p.N + 2 * TC_BM - 1) / (2 * TC_BM)) * max_tiles;      // at most: the table says how many
+    const int pairs_on_device = bc_sm_count() / 2 > 0 ? bc_sm_count() / 2 : 1;
+    const int pairs = pieces < pairs_on_device ? (int)pieces : pairs_on_device;
+    cudaError_t e = bc_launch_clustered(gemm_tc_grouped_pair_kernel<EPI>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)smem, s, dim3(2, 1, 1), mw, mx, p);
     if (e != cudaSuccess) {
         bc_set_error("gemm_tc_grouped: launch failed: %s", cudaGetErrorString(e));
         return (int)e;
@@ -1214,6 +1375,11 @@ extern "C" int bc_gemm_tc_grouped_bf16(const void* X, const void* W, void* out, 
     p.stages = 0;
     p.glu_limit = glu_limit;
     p.glu_alpha = glu_alpha;
+    // Pairs where matrices meet more than 128 rows on average and an even number of weight tiles leaves no block of a pair without outputs.
+    if (tile_rows == 256 && (N + TC_BM - 1) / TC_BM % 2 == 0 && g_tc_pair)
+        return gated == 1 ? launch_grouped_pair<EPI_SWIGLU>(mw, mx, p, max_tiles, s)
+               : gated == 2 ? launch_grouped_pair<EPI_RELU2>(mw, mx, p, max_tiles, s)
+                            : launch_grouped_pair<EPI_STORE_F32>(mw, mx, p, max_tiles, s);
 #define GROUPED(BN)                                                                         \
     case BN:                                                                                \
         return gated == 1 ? launch_grouped<BN, EPI_SWIGLU>(mw, mx, p, max_tiles, s)                \
