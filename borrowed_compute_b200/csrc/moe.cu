@@ -18,7 +18,7 @@
 // Every sum of a row runs in an order that the sizes alone fix, and no two blocks add into one place: a row's result is the
 // same bits in any batch and at every repeat.  The products here run on the CUDA cores in float (the true 32-bit path, and
 // the checked twin of the tensor-core grouped product).
-#include "common.cuh"
+#include "mma_tiles.cuh"
 
 #define MOE_BM 32
 #define MOE_BN 64
@@ -75,6 +75,76 @@ moe_logits_kernel(const T* __restrict__ h, const float* __restrict__ router, flo
         const float v = warp_sum(z[i]);
         if (lane == 0 && r0 + i < rows) logits[(size_t)(r0 + i) * E + e] = v;
     }
+}
+
+// The same sums where rows are many: sixteen rows by sixteen experts a block, four by eight a warp, both operands through shared memory 256 k at a time,
+// the next ones on their way.  A lane's share of a row's sum and the order of the shares are those of the kernel above, so are the bits.
+// What bounds that one at many rows are its reads (two 16-byte loads for eight multiply-adds); here twelve serve 128.
+// Logits and choice, us, that kernel and this: bfloat16, K 2,048, 64 experts: 4,096 rows 81 and 54, 2,048 48 and 34, 500 24 and 17, 256 17 and 17, 64 17 and 17; 64 rows of
+// 32 experts, K 4,096 26 and 24; 600 of 17, K 1,000 17 and 13; but of 8 experts, half a tile, 9,000 rows 36 and 38, 2,048, K 4,096 24 and 26.
+#define RT_ROWS 16
+#define RT_EXPERTS 16
+#define RT_K 256
+template <class T> __host__ __device__ constexpr size_t route_tile_smem() { return 2 * RT_K * (RT_ROWS * sizeof(T) + RT_EXPERTS * sizeof(float)); }
+template <class T>
+__global__ void __launch_bounds__(256)
+moe_logits_tile_kernel(const T* h, const float* __restrict__ router, float* __restrict__ logits, int rows, int E, int K) {
+    extern __shared__ __align__(16) uint8_t route_smem[];
+    float (*ws)[RT_EXPERTS][RT_K] = reinterpret_cast<float (*)[RT_EXPERTS][RT_K]>(route_smem);                                 // two stages each
+    T (*xs)[RT_ROWS][RT_K] = reinterpret_cast<T (*)[RT_ROWS][RT_K]>(route_smem + 2 * RT_EXPERTS * RT_K * sizeof(float));
+    pdl_launch_dependents_if_resident();
+    pdl_wait();
+    PDL_FRESH(h);
+    const int r0 = blockIdx.x * RT_ROWS, e0 = blockIdx.y * RT_EXPERTS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wr = 4 * (warp & 3), we = 8 * (warp >> 2);
+    auto issue = [&](int k0, int stage) {                       // what lies past K is neither copied nor read
+        constexpr int X_PIECES = RT_K * sizeof(T) / 16, W_PIECES = RT_K * sizeof(float) / 16;
+#pragma unroll
+        for (int u = 0; u < RT_ROWS * X_PIECES / 256; u++) {
+            const int i = threadIdx.x + 256 * u, r = i / X_PIECES, k = i % X_PIECES * (16 / (int)sizeof(T));
+            if (k0 + k < K) cp_async16(ad_smem(&xs[stage][r][k]), h + (size_t)min(r0 + r, rows - 1) * K + k0 + k);
+        }
+#pragma unroll
+        for (int u = 0; u < RT_EXPERTS * W_PIECES / 256; u++) {
+            const int i = threadIdx.x + 256 * u, e = i / W_PIECES, k = i % W_PIECES * 4;
+            if (k0 + k < K) cp_async16(ad_smem(&ws[stage][e][k]), router + (size_t)min(e0 + e, E - 1) * K + k0 + k);
+        }
+    };
+    float z[32] = {};                                           // row i, expert e of the warp: 8 i + e
+    issue(0, 0);
+    cp_async_commit();
+    for (int k0 = 0, stage = 0; k0 < K; k0 += RT_K, stage ^= 1) {
+        if (k0 + RT_K < K) issue(k0 + RT_K, stage ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RT_K; k += 128) {
+            if (k0 + k + 4 * lane >= K) break;
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = route_load4(&xs[stage][wr + i][k + 4 * lane]);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float4 b = route_load4(&ws[stage][we + e][k + 4 * lane]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) z[8 * i + e] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, z[8 * i + e]))));
+            }
+        }
+        __syncthreads();                                        // all have left the stage that is filled next
+    }
+    // Thirty-two sums over the lanes, halved among them in the order of a sum of each by itself: lane L is left with number L.
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? z[i + o] : z[i], send = up ? z[i] : z[i + o];
+            z[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    const int r = r0 + wr + (lane >> 3), e = e0 + we + (lane & 7);
+    if (r < rows && e < E) logits[(size_t)r * E + e] = z[0];
 }
 
 // One warp a row: the `top` largest logits (the lower index wins a tie) and their scores.  CORRECTED: the largest scores plus
@@ -609,6 +679,9 @@ moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ choice, 
 }
 
 // ------------------------------------------------------------------------------------ launchers
+static int g_route_tiles = -1;     // for measurements and tests: 0 never, 1 always; else where there are a tile's experts
+extern "C" void bc_moe_set_route_tiles(int n) { g_route_tiles = n; }
+
 template <class T>
 static int route(const void* h, const float* router, const int* row_slot, float* logits, int* choice, float* weight, int rows, int E, int K, int top,
                  int softmax, int renorm, float factor, const float* correction, int n_groups, int keep, cudaStream_t s) {
@@ -617,7 +690,16 @@ static int route(const void* h, const float* router, const int* row_slot, float*
     if (rows == 0) return BC_OK;
     const int groups = (E + ROUTE_EXPERTS - 1) / ROUTE_EXPERTS;
     BC_CHECK_ARG(groups <= 65535, "moe_route: too many experts (%d)", E);
-    bc_launch(moe_logits_kernel<T>, dim3((rows + ROUTE_ROWS - 1) / ROUTE_ROWS, groups), dim3(32 * ROUTE_EXPERTS), 0, s, (const T*)h, router, logits, rows, E, K);
+    const dim3 tiles((rows + RT_ROWS - 1) / RT_ROWS, (E + RT_EXPERTS - 1) / RT_EXPERTS);
+    if ((g_route_tiles < 0 ? E >= RT_EXPERTS : g_route_tiles != 0) && K % (16 / sizeof(T)) == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)router % 16 == 0) {
+        if (cudaError_t e = bc_allow_shared<moe_logits_tile_kernel<T>>(route_tile_smem<T>()); e != cudaSuccess) {
+            bc_set_error("moe_route: %s", cudaGetErrorString(e));
+            return (int)e;
+        }
+        bc_launch(moe_logits_tile_kernel<T>, tiles, dim3(256), route_tile_smem<T>(), s, (const T*)h, router, logits, rows, E, K);
+    } else {
+        bc_launch(moe_logits_kernel<T>, dim3((rows + ROUTE_ROWS - 1) / ROUTE_ROWS, groups), dim3(32 * ROUTE_EXPERTS), 0, s, (const T*)h, router, logits, rows, E, K);
+    }
     if (correction != nullptr || keep < n_groups)
         bc_launch(moe_choose_kernel<true>, dim3((rows + 3) / 4), dim3(128), (size_t)4 * (E + n_groups) * sizeof(float), s, (const float*)logits, row_slot,
                   choice, weight, rows, E, top, softmax, renorm, factor, correction, n_groups, keep);
