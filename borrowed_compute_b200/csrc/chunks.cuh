@@ -128,6 +128,7 @@ template <int PT> __device__ __forceinline__ void chunk_groups(const float (*g)[
 // through a ring of asynchronous copies.
 #define CHUNK_THREADS 128
 #define CHUNK_STAGES 3         // chunks on their way or worked on
+#define CHUNK_ALONE (120 * 1024)      // bytes of shared memory of which an SM holds one block's
 template <int DL, bool DELTA>      // D = 32 DL
 __global__ void __launch_bounds__(CHUNK_THREADS)
 chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v_stride, float* __restrict__ state, const int* __restrict__ seq_rows,
@@ -304,8 +305,14 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
 
 template <int DL, bool DELTA>
 static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, const float* v, int v_stride, float* state, const int* seq_rows, const int* seq_slot,
-                                     float* out, int seqs, int H, int N, int P, int n_slots, int write_state, float out_scale, cudaStream_t s) {
-    constexpr size_t SMEM = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
+                                     float* out, int rows, int max_new, int seqs, int H, int N, int P, int n_slots, int write_state, float out_scale, cudaStream_t s) {
+    constexpr size_t NEEDS = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
+    static_assert(NEEDS <= CHUNK_ALONE, "shared memory of one block");
+    // Where the longest sequence's chain is as long as all SMs' work, an SM to itself for every block of it (and for the others one at a time, through
+    // the shared memory a block asks for): 16 heads of 128 x 256, sequences of 2,000 and three of 100 rows 351 -> 249 us the whole call, 8 heads, 400, 1,100 and 1,800 rows 310 -> 251;
+    // not for 16 heads of the latter, half as much again for all SMs as for the longest (354 and 346), nor for two of 2,048 (382 and 452).
+    const long long work = (long long)((P + 31) / 32) * H * rows;
+    const size_t SMEM = seqs > 1 && work * 7 <= (long long)bc_sm_count() * max_new * 8 ? CHUNK_ALONE : NEEDS;
     if (cudaError_t e = bc_allow_shared<chunk_scan_kernel<DL, DELTA>>(SMEM); e != cudaSuccess) return e;
     return bc_launch(chunk_scan_kernel<DL, DELTA>, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H,
                      N, P, n_slots, write_state, out_scale);

@@ -333,7 +333,7 @@ extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t,
                                  key_eps, seqs, n_slots, run, (int)places);
             },
             [&](const ChunkSpan& span) {
-                return chunk_scan_launch<DLC_D / 32, true>(span, pack, proj + 2 * H * D, stride, state, seq_rows, seq_slot, out, seqs, H, D, D, n_slots, write_state, 1.0f, s);
+                return chunk_scan_launch<DLC_D / 32, true>(span, pack, proj + 2 * H * D, stride, state, seq_rows, seq_slot, out, rows, max_new, seqs, H, D, D, n_slots, write_state, 1.0f, s);
             });
     if (e != cudaSuccess) {
         bc_set_error("delta_chunked: %s", cudaGetErrorString(e));

@@ -139,7 +139,7 @@ static int gla_chunked(const float* proj, int stride, int q_at, int k_at, int v_
                              w2t, b, rank, seq_rows, seq_slot, pack, H, N, inv_tau, seqs, n_slots);
         },
         [&](const ChunkSpan& span) {
-            return chunk_scan_launch<D / 32, false>(span, pack, proj + v_at, stride, state, seq_rows, seq_slot, out, seqs, H, N, P, n_slots, write_state, f, s);
+            return chunk_scan_launch<D / 32, false>(span, pack, proj + v_at, stride, state, seq_rows, seq_slot, out, rows, max_new, seqs, H, N, P, n_slots, write_state, f, s);
         });
     if (e != cudaSuccess) {
         bc_set_error("gla_chunked: %s", cudaGetErrorString(e));
