@@ -582,7 +582,8 @@ talk_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
 // the raw ones have been read.  The next keys and this tile's values arrive between them, while the mix runs, so one stage of each suffices.
 // (Thirty-two heads as a cluster of two blocks of sixteen rows handed every raw score to the other block's memory: the release of those stores, twice
 // a tile, and the registers of their addresses left a scheduler idle 62 % of the time.)
-// One prompt of 2,048, window 1,024, 32 heads of 128 on 8: 392 us; as a cluster 569, with the kernel above 769.  Of 64 on 16: 304, as a cluster 391.
+// One prompt of 2,048, window 1,024, 32 heads of 128 on 8: 343 us; with masks worked out and accumulators rescaled in every tile, not only where a row's bound
+// or a risen maximum asks for it, 392; as a cluster 569, with the kernel above 769.  Of 64 on 16: 304, as a cluster 391.
 // 8 rows that see 4,000 positions: 73, as a cluster 159.  Sixteen heads of 128 on 4, one prompt: 200, with two stages and the cluster's order 236.
 #define TM_PAGES_KEPT 256
 #define TP_WARPS 16
@@ -775,15 +776,27 @@ talk_by_rows_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, con
                 s[2 * half][2 * i] = v.x, s[2 * half][2 * i + 1] = v.y, s[2 * half + 1][2 * i] = v.z, s[2 * half + 1][2 * i + 1] = v.w;
             }
         float tmax[2] = {-INFINITY, -INFINITY};
+        // Tiles that every row of the block sees whole have nothing to mask (rows past the sequence are never written).
+        const bool whole = page_ok && tile * TT_KEYS + TT_KEYS - 1 <= p_first && tile * TT_KEYS >= first_seen(p_last);
+        if (whole) {
 #pragma unroll
-        for (int nb = 0; nb < 4; nb++)
+            for (int nb = 0; nb < 4; nb++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int i = e >> 1, t = tile * TT_KEYS + nb * 8 + 2 * tq + (e & 1);
-                const bool seen = page_ok && live[i] && t <= pos[i] && (t >= lo[i] || t < keep_first);
-                s[nb][e] = seen ? s[nb][e] * LOG2E : -INFINITY;
-                tmax[i] = fmaxf(tmax[i], s[nb][e]);
-            }
+                for (int e = 0; e < 4; e++) {
+                    s[nb][e] *= LOG2E;
+                    tmax[e >> 1] = fmaxf(tmax[e >> 1], s[nb][e]);
+                }
+        } else {
+#pragma unroll
+            for (int nb = 0; nb < 4; nb++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int i = e >> 1, t = tile * TT_KEYS + nb * 8 + 2 * tq + (e & 1);
+                    const bool seen = page_ok && live[i] && t <= pos[i] && (t >= lo[i] || t < keep_first);
+                    s[nb][e] = seen ? s[nb][e] * LOG2E : -INFINITY;
+                    tmax[i] = fmaxf(tmax[i], s[nb][e]);
+                }
+        }
         float corr[2], base[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
@@ -820,8 +833,9 @@ talk_by_rows_kernel(const bf16* q, const bf16* k_cache, const bf16* v_cache, con
             __syncthreads();
         }
         if (page_ok) {                                     // the product with the values
+            if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f))        // a maximum rose
 #pragma unroll
-            for (int nd = 0; nd < ND; nd++) o[nd][0] *= corr[0], o[nd][1] *= corr[0], o[nd][2] *= corr[1], o[nd][3] *= corr[1];
+                for (int nd = 0; nd < ND; nd++) o[nd][0] *= corr[0], o[nd][1] *= corr[0], o[nd][2] *= corr[1], o[nd][3] *= corr[1];
 #pragma unroll
             for (int kk = 0; kk < 2; kk++)
 #pragma unroll
