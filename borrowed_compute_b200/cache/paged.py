@@ -18,8 +18,10 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Dict, List, Mapping, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
+from .. import ops
 from ..parts.base import CacheNeed, RunMemory, Runtime, StateNeed
 from .slots import PAGE, GroupPlan, SlotTable, pages_for
 
@@ -31,6 +33,7 @@ class _Group:
     planes: Optional[List[torch.Tensor]] = None
     table: Optional[torch.Tensor] = None
     host_table: Optional[torch.Tensor] = None
+    host_rows: Optional[np.ndarray] = None      # host_table's memory
 
 
 class PagedCache:
@@ -64,6 +67,7 @@ class PagedCache:
                         for heads, width in g.need.planes]
             g.host_table = torch.full((n_slots, self.slots.max_pages), -1, dtype=torch.int32).pin_memory() \
                 if rt.device.type == "cuda" else torch.full((n_slots, self.slots.max_pages), -1, dtype=torch.int32)
+            g.host_rows = g.host_table.numpy()
             g.table = torch.full((n_slots, self.slots.max_pages), -1, dtype=torch.int32, device=rt.device)
         self._copied: Optional[torch.cuda.Event] = None
         self.state: Dict[int, torch.Tensor] = {}
@@ -99,7 +103,7 @@ class PagedCache:
         if self._copied is not None:
             self._copied.synchronize()   # the last copy out of the pinned tables is done
         for g, slot in self.slots.dirty:
-            self.groups[g].host_table[slot] = torch.tensor(self.slots.tables[g][slot], dtype=torch.int32)
+            self.groups[g].host_rows[slot] = self.slots.tables[g][slot]
             touched.add(g)
         self.slots.dirty.clear()
         for g in touched:
@@ -107,7 +111,7 @@ class PagedCache:
         if self.rt.device.type == "cuda":
             if self._copied is None:
                 self._copied = torch.cuda.Event()
-            self._copied.record()
+            self._copied.record(ops.current_stream())
         return sum(self.groups[g].host_table.numel() * 4 for g in touched)
 
     # -- what a run sees

@@ -159,10 +159,16 @@ class SlotTable:
             if more > self.pools[g].available + self._releasable(g, pages, new_len, rows):
                 raise CacheError(f"the cache is full: slot {slot} needs {more} more pages of {PAGE} tokens in group {g}, "
                                  f"{self.pools[g].available} are free")
+        self._take(st, slot, need, new_len, rows)
+
+    def _take(self, st: _Slot, slot: int, need: int, new_len: int, rows: int) -> None:
+        """Moves the pages of a reservation that has been counted."""
         for g, pages in enumerate(st.pages):
-            first = self._first_needed_page(g, new_len, rows)
-            kept = self._kept_pages(g)
-            dropped = [p for p in pages[kept:first] if p >= 0]
+            dropped = []
+            if self._lets_go(g):
+                first = self._first_needed_page(g, new_len, rows)
+                kept = self._kept_pages(g)
+                dropped = [p for p in pages[kept:first] if p >= 0]
             if dropped:
                 self.pools[g].give_back(dropped)
                 for i in range(kept, min(first, len(pages))):
@@ -191,9 +197,15 @@ class SlotTable:
                 raise CacheError(f"the cache is full: this step needs {n} more pages of {PAGE} tokens in group {g}, "
                                  f"{self.pools[g].available} are free")
         for slot, new_len, rows in requests:
-            self.reserve(slot, new_len, rows)
+            self._take(self._slots[slot], slot, pages_for(new_len), new_len, rows)
+
+    def _lets_go(self, g: int) -> bool:
+        """Whether the group's sequences let pages go as they grow."""
+        return self.groups[g].window > 0 or self.groups[g].chunk > 0
 
     def _releasable(self, g: int, pages: List[int], new_len: int, rows: int) -> int:
+        if not self._lets_go(g):
+            return 0
         first = self._first_needed_page(g, new_len, rows)
         return sum(1 for p in pages[self._kept_pages(g):first] if p >= 0)
 

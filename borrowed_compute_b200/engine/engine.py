@@ -57,35 +57,34 @@ class _DecodeGraph:
         total = sum(n for _, n in self.sizes)
         self.ints = torch.zeros(total, dtype=torch.int32, device=dev)
         self.host = torch.zeros(total, dtype=torch.int32).pin_memory()
+        self.host_ints = self.host.numpy()
         self.copied: Optional[torch.cuda.Event] = None
-        self.views, at = {}, 0
+        self.views, self.at, at = {}, {}, 0
         for name, n in self.sizes:
             self.views[name] = self.ints[at:at + n]
+            self.at[name] = at
             at += n
+        # A step of padding rows alone: what pack() starts from.
+        self.blank = np.zeros(total, dtype=np.int32)
+        for name in ("row_slot", "seq_slot"):
+            self.blank[self.at[name]:self.at[name] + rows] = -1
+        self.blank[self.at["seq_rows"]:self.at["seq_rows"] + rows + 1] = np.arange(rows + 1)
+        self.blank[self.at["want_rows"]:self.at["want_rows"] + rows] = np.arange(rows)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.scores: Optional[torch.Tensor] = None
 
     def pack(self, tokens, row_pos, row_slot, rows_used: int) -> np.ndarray:
         """The step's integers in the layout of ``sizes``: one row a sequence, padding rows
         (slot -1) after them.  ``tokens`` may be None and filled into [:rows_used] later."""
-        rows, n = self.rows, rows_used
-        out = np.zeros(sum(size for _, size in self.sizes), dtype=np.int32)
-        at = {}
-        o = 0
-        for name, size in self.sizes:
-            at[name] = o
-            o += size
+        rows, n, at = self.rows, rows_used, self.at
+        out = self.blank.copy()
         if tokens is not None:
             out[at["tokens"]:at["tokens"] + n] = tokens
         out[at["row_pos"]:at["row_pos"] + n] = row_pos
-        out[at["row_slot"]:at["row_slot"] + rows] = -1
         out[at["row_slot"]:at["row_slot"] + n] = row_slot
-        out[at["seq_rows"]:at["seq_rows"] + rows + 1] = n
-        out[at["seq_rows"]:at["seq_rows"] + n + 1] = np.arange(n + 1, dtype=np.int32)
-        out[at["seq_slot"]:at["seq_slot"] + rows] = -1
+        out[at["seq_rows"] + n:at["seq_rows"] + rows + 1] = n
         out[at["seq_slot"]:at["seq_slot"] + n] = row_slot
         out[at["seq_start"]:at["seq_start"] + n] = row_pos
-        out[at["want_rows"]:at["want_rows"] + rows] = np.arange(rows, dtype=np.int32)
         return out
 
     def _upload(self, packed: np.ndarray, keep_tokens: bool = False) -> None:
@@ -94,12 +93,15 @@ class _DecodeGraph:
         if self.copied is not None:
             self.copied.synchronize()   # the last copy out of the pinned buffer is done
         first = self.rows if keep_tokens else 0     # the tokens come first in the layout
-        self.host[first:].copy_(torch.from_numpy(packed[first:]))
-        self.ints[first:].copy_(self.host[first:], non_blocking=True)
-        count_traffic("h2d", 4 * (self.host.numel() - first), True)
+        self.host_ints[first:] = packed[first:]
+        if first:
+            self.ints[first:].copy_(self.host[first:], non_blocking=True)
+        else:
+            self.ints.copy_(self.host, non_blocking=True)
+        count_traffic("h2d", 4 * (packed.size - first), True)
         if self.copied is None:
             self.copied = torch.cuda.Event()
-        self.copied.record()
+        self.copied.record(ops.current_stream())
 
     @property
     def engine(self) -> "Engine":
@@ -315,17 +317,15 @@ class Engine:
             self._staged = None
         if self._staged is not None:
             self._staged.synchronize()   # the last copy out of the pinned buffer is done
-        self._host_ints[:n].copy_(torch.from_numpy(packed))
-        self._ints[:n].copy_(self._host_ints[:n], non_blocking=True)
+        self._host_ints.numpy()[:n] = packed
+        ints = self._ints[:n]
+        ints.copy_(self._host_ints[:n], non_blocking=True)
         count_traffic("h2d", 4 * n, plan.decode)
         if self._staged is None:
             self._staged = torch.cuda.Event()
-        self._staged.record()
-        views, at = {}, 0
-        for name, size in plan.layout():
-            views[name] = self._ints[at:at + size]
-            at += size
-        return views
+        self._staged.record(ops.current_stream())
+        names, sizes = zip(*plan.layout())
+        return dict(zip(names, torch.split(ints, sizes)))
 
     def check_entries(self, entries: Sequence[StepEntry]) -> List[int]:
         """The guards of a step; returns every entry's start position."""
@@ -458,8 +458,8 @@ class Engine:
         ctx = StepContext(
             rows=plan.padded_rows, seqs=plan.seqs, tokens=v["tokens"], row_pos=v["row_pos"], row_slot=v["row_slot"],
             seq_rows=v["seq_rows"], seq_slot=v["seq_slot"], seq_start=v["seq_start"], max_new=plan.max_new,
-            max_total=plan.max_total, decode=plan.decode, host_seq_rows=tuple(int(x) for x in plan.seq_rows),
-            host_seq_slot=tuple(int(x) for x in plan.seq_slot), host_seq_start=tuple(int(x) for x in plan.seq_start))
+            max_total=plan.max_total, decode=plan.decode, host_seq_rows=tuple(plan.seq_rows.tolist()),
+            host_seq_slot=tuple(plan.seq_slot.tolist()), host_seq_start=tuple(plan.seq_start.tolist()))
         scores = self.model.forward(ctx, self.cache, v["want_rows"], len(plan.want_rows))
         for e, start in zip(entries, starts):
             self.cache.slots.commit(e.slot, start + len(e.tokens))

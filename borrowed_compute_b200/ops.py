@@ -76,6 +76,21 @@ def _stream() -> _c_void_p:
     return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
+_streams = {}
+
+
+def current_stream() -> torch.cuda.Stream:
+    """torch.cuda.current_stream() without building its object anew: 3 microseconds of Python less wherever an event is recorded."""
+    device = torch._C._cuda_getDevice()
+    key = (device, torch._C._cuda_getCurrentRawStream(device))
+    stream = _streams.get(key)
+    if stream is None:
+        if len(_streams) > 64:
+            _streams.clear()
+        stream = _streams[key] = torch.cuda.current_stream()
+    return stream
+
+
 def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
     return _c_void_p(0 if t is None else t.data_ptr())
 
@@ -206,9 +221,15 @@ def _call(fn, *args) -> None:
         raise KernelError(f"{fn.__name__} failed ({status}): {msg.decode() if msg else ''}")
 
 
+_fns = {}
+
+
 def _fn(name: str):
-    f = getattr(lib(), name)
-    f.restype = _c_int
+    f = _fns.get(name)
+    if f is None:
+        f = getattr(lib(), name)
+        f.restype = _c_int
+        _fns[name] = f
     return f
 
 
