@@ -52,7 +52,8 @@ struct TcParams {
     int k_iters_per_split;
     int clustered;      // split-K: the splits of a tile are one thread-block cluster and add up through shared memory
     int n_tiles, t_tiles;   // blocks along the weight rows and along the tokens
-    int pair_tokens;        // the paired kernel: tokens a tile (64, 128, 192 or 256)
+    int pair_tokens;        // the paired kernel: tokens a tile (64, 128, 192 or 256),
+    int staged;             // and whether tensor copies take the output's rows (16-byte strides): results then go through shared memory
     int starve;             // test hook: the first stage expects 16 bytes that never come, so a bounded wait runs out
     float act_a, act_b;     // EPI_XIELU: its two numbers
     int act_cols;           // EPI_SILU_F32: output columns below this one are gated by their own sigmoid
@@ -450,10 +451,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // barrier.  No load is multicast.
 #define TCP_THREADS 320        // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 #define TCP_STAGES_MAX 8
+// Which results go out through shared memory and tensor copies, a few thousand bytes at a time: bfloat16, whose 64 bytes a warp and token
+// are half a line a store, and sums added to floats, one reduction a box instead of one a value.  Floats that are stored go straight from the registers, a
+// whole line a warp and token.  A round of tiles costs, beside its products and the memory's share (K 1,024 to 8,192, four rounds), us: bfloat16 7.8 before
+// and 6.3 through shared memory, adding 19 and 15, floats 9 and 10.
+#define TCP_STAGED(EPI) (EPI_TO_BF16(EPI) || (EPI) == EPI_ADD_F32)
+#define TCP_OUT_BYTES 8192     // a buffer of results on their way out: 32 tokens of 128 bfloat16 outputs, or 16 of floats; two for each half of the epilogue warps
 
 template <int EPI>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcParams p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out, const TcParams p) {
     constexpr int BN = 256;                               // token columns of an accumulator in TMEM; a pair's tile takes p.pair_tokens <= BN
     constexpr int TILE = TC_BM * TC_BK * 2;               // 16 KB: 128 rows of 64 k
     constexpr int STAGE_BYTES = 3 * TILE;                 // two weight tiles and this block's half of the tokens
@@ -584,12 +591,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const uint32_t pair_acc_empty = map_to_rank(acc_empty, 0);
         bool ok = true;
         pdl_wait();   // the output may still be in use by the preceding kernel
+        // Results on their way out: PT tokens of 128 outputs, [token][output], two buffers a set.
+        constexpr bool TO_BF16 = EPI_TO_BF16(EPI);
+        constexpr int PT = TCP_OUT_BYTES / (TC_BM * (TO_BF16 ? 2 : 4));
+        uint8_t* out_smem = smem + (size_t)stages * STAGE_BYTES + set * 2 * TCP_OUT_BYTES;
+        const bool issuer = q == 2 && lane == 0;              // warps 2 and 6, the sets' first
+        int buffer = 0;
         int n = 0;
         for (int tile = pair; tile < total_tiles; tile += n_pairs, n++) {
             int tile_n, tile_t;
             place(tile, tile_n, tile_t);
             const int t0 = tile_t * bn;
-            ok = mbar_wait_warp(acc_full, n & 1, 3);
+            // (A warp whose wait ran out still meets its set, and all of it stops: nobody waits at a barrier without end.)
+            ok = named_barrier_all(1 + set, 128, mbar_wait_warp(acc_full, n & 1, 3));
             if (!ok) break;
             tc_fence_after();
             const int out_n = tile_n * 2 * OUT_ROWS + (int)rank * OUT_ROWS + 32 * q + lane + (EPI == EPI_SWIGLU ? 0 : TC_BM * set);
@@ -617,6 +631,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int COLS = EPI == EPI_SWIGLU ? bn / 2 : bn;              // token columns this warp writes (a multiple of 32)
             const int c_first = EPI == EPI_SWIGLU ? set * COLS : 0;
             const uint32_t src = lanes + (EPI == EPI_SWIGLU ? c_first : set * BN);   // SwiGLU: the gate accumulator; up is BN columns on
+            // Through shared memory: sixteen columns into this thread's place of the buffer; at a buffer's end one thread sends it off, once the buffer
+            // before has been read, so that all may go on into that one behind the barrier.
+            const int n_first = out_n - 32 * q - lane;
+            auto put = [&](const uint32_t* v, const uint32_t* u, int c0) {
+                uint8_t* to = out_smem + buffer * TCP_OUT_BYTES;
+                const int at = ((c0 - c_first) % PT) * TC_BM + 32 * q + lane;
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float r = EPI == EPI_SWIGLU ? glu_mul(__uint_as_float(v[j]), __uint_as_float(u[j]), p.glu_limit, p.glu_alpha) : epi_plain<EPI>(__uint_as_float(v[j]), p.act_a, p.act_b, out_n, p.act_cols);
+                    if (TO_BF16) reinterpret_cast<bf16*>(to)[at + j * TC_BM] = __float2bfloat16_rn(r);
+                    else reinterpret_cast<float*>(to)[at + j * TC_BM] = r;
+                }
+                if ((c0 - c_first + 16) % PT) return;
+                fence_proxy_async();
+                if (issuer) bulk_wait_read();
+                named_barrier(1 + set, 128);
+                const int t_first = t0 + c0 + 16 - PT;
+                if (issuer && t_first < p.T && n_first < p.N) {     // past the output's edges nothing is written
+                    if (EPI == EPI_ADD_F32) tma_add_2d(&map_out, smem_u32(to), n_first, t_first);
+                    else tma_store_2d(&map_out, smem_u32(to), n_first, t_first);
+                    bulk_commit();
+                }
+                buffer ^= 1;
+            };
+            auto give = [&](const uint32_t* v, const uint32_t* u, int c0) {
+                if (TCP_STAGED(EPI) && p.staged) put(v, u, c0);
+                else emit(v, u, c0);
+            };
             uint32_t va[16], vb[16], ua[16], ub[16];
             tmem_load16(src, va);
             if (EPI == EPI_SWIGLU) tmem_load16(src + BN, ua);
@@ -625,20 +667,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 tmem_load_wait();
                 tmem_load16(src + cc + 16, vb);
                 if (EPI == EPI_SWIGLU) tmem_load16(src + BN + cc + 16, ub);
-                emit(va, ua, c_first + cc);
+                give(va, ua, c_first + cc);
                 tmem_load_wait();
                 if (cc + 32 < COLS) {
                     tmem_load16(src + cc + 32, va);
                     if (EPI == EPI_SWIGLU) tmem_load16(src + BN + cc + 32, ua);
                 }
-                emit(vb, ub, c_first + cc + 16);
+                give(vb, ub, c_first + cc + 16);
             }
             // This warp has read its share of the accumulators: tell the MMA thread of the even block.
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(pair_acc_empty);
         }
+        if (issuer) bulk_wait();          // what is on its way out of this block's shared memory
     }
+    __syncwarp();
     tc_fence_before();
     cl.sync();   // neither block leaves, or frees TMEM, while the pair's MMAs or arrivals may still touch it
     if (warp == 1) {
@@ -679,6 +723,22 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int K, int box
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         bc_set_error("gemm_tc: cuTensorMapEncodeTiled failed (%d) for a [%d, %d] matrix, box %d x %d", (int)r, rows, K, box_rows, TC_BK);
+        return BC_ERR_DRIVER;
+    }
+    return BC_OK;
+}
+
+// An output [rows, N] of bfloat16 or floats cut into what a buffer of results holds (see the paired kernel), no swizzle.
+static int out_map(CUtensorMap* map, const void* base, int rows, int N, bool to_bf16) {
+    const int size = to_bf16 ? 2 : 4;
+    cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)N * size};
+    cuuint32_t box[2] = {TC_BM, (cuuint32_t)(TCP_OUT_BYTES / (TC_BM * size))};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = encode_fn()(map, to_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        bc_set_error("gemm_tc: cuTensorMapEncodeTiled failed (%d) for an output [%d, %d]", (int)r, rows, N);
         return BC_ERR_DRIVER;
     }
     return BC_OK;
@@ -768,19 +828,26 @@ static int g_tc_pair = 1;
 static int g_tc_pair_tokens = 0;   // 0: the launcher chooses the tokens a paired tile takes; 64, 128, 192, 256 force it
 extern "C" void bc_gemm_tc_set_pair_tokens(int n) { g_tc_pair_tokens = (n == 64 || n == 128 || n == 192 || n == 256) ? n : 0; }
 extern "C" void bc_gemm_tc_set_pair(int on) { g_tc_pair = on != 0; }
+static int g_tc_pair_staged = 1;   // whether its results may go out through shared memory; for measurements and tests
+extern "C" void bc_gemm_tc_set_pair_staged(int on) { g_tc_pair_staged = on != 0; }
 
 template <int EPI>
 static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcParams p, cudaStream_t s) {
     constexpr int STAGE_BYTES = 3 * TC_BM * TC_BK * 2;
     const int k_iters = (p.K + TC_BK - 1) / TC_BK;
-    int stages = (TC_SMEM_LIMIT - 1024) / STAGE_BYTES;
+    constexpr int OUT_BYTES = TCP_STAGED(EPI) ? 4 * TCP_OUT_BYTES : 0;
+    int stages = (TC_SMEM_LIMIT - 1024 - OUT_BYTES) / STAGE_BYTES;
     if (stages > TCP_STAGES_MAX) stages = TCP_STAGES_MAX;
     if (g_tc_stage_cap > 0 && stages > g_tc_stage_cap) stages = g_tc_stage_cap;
     if (stages < 2) stages = 2;
     p.stages = stages;
     p.clustered = 0;
     p.k_iters_per_split = k_iters;
-    const int smem = stages * STAGE_BYTES + 1024;
+    const int smem = stages * STAGE_BYTES + OUT_BYTES + 1024;
+    CUtensorMap mo;
+    p.staged = TCP_STAGED(EPI) && (uintptr_t)p.out % 16 == 0 && (long long)p.N * (EPI_TO_BF16(EPI) ? 2 : 4) % 16 == 0 && g_tc_pair_staged;
+    if (int st = p.staged ? out_map(&mo, p.out, p.T, p.N, EPI_TO_BF16(EPI)) : BC_OK; st != BC_OK) return st;
+    if (!p.staged) mo = mx;
     if (cudaError_t e = bc_allow_shared<gemm_tc_pair_kernel<EPI>>(TC_SMEM_LIMIT); e != cudaSuccess) {
         bc_set_error("gemm_tc: cannot raise the shared memory limit: %s", cudaGetErrorString(e));
         return (int)e;
@@ -807,7 +874,7 @@ static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcParams p,
     const long long tiles = (long long)p.n_tiles * p.t_tiles;
     const int pairs = tiles < pairs_on_device ? (int)tiles : pairs_on_device;   // persistent: a pair walks over tiles
     dim3 grid(2 * pairs, 1, 1);
-    cudaError_t e = bc_launch_clustered(gemm_tc_pair_kernel<EPI>, grid, dim3(TCP_THREADS), (size_t)smem, s, dim3(2, 1, 1), mw, mx, p);
+    cudaError_t e = bc_launch_clustered(gemm_tc_pair_kernel<EPI>, grid, dim3(TCP_THREADS), (size_t)smem, s, dim3(2, 1, 1), mw, mx, mo, p);
     if (e != cudaSuccess) {
         bc_set_error("gemm_tc: launch of the paired kernel failed: %s", cudaGetErrorString(e));
         return (int)e;

@@ -144,6 +144,33 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
                  "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
                  : "memory");
 }
+// A box of shared memory to global memory, or added to the floats there; it counts in the issuing thread's open group of such copies.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Until all of this thread's groups have read their shared memory; until they are wholly done.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// A barrier of `threads` threads of the block (whole warps), and whether all of them said yes.
+__device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ bool named_barrier_all(int id, int threads, bool yes) {
+    uint32_t all;
+    asm volatile(
+        "{\n"
+        ".reg .pred p, r;\n"
+        "setp.ne.u32 p, %1, 0;\n"
+        "barrier.cta.red.and.pred r, %2, %3, p;\n"
+        "selp.u32 %0, 1, 0, r;\n"
+        "}\n"
+        : "=r"(all)
+        : "r"((uint32_t)yes), "r"(id), "r"(threads)
+        : "memory");
+    return all != 0;
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
