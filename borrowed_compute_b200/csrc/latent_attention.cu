@@ -36,44 +36,93 @@ __device__ __forceinline__ float2 lat_load2(const bf16* p) {
 // ------------------------------------------------------------------------------------ prepare
 // One block a row.  proj: [rows, P] float; the q part starts at 0 and is QR wide, the c part at kv_at (R wide, then
 // ROT values of r; kv_at < 0: the mixer reads another layer's cache and has no such part), the gate part at g_at (H wide).
-template <class T>
-__global__ void __launch_bounds__(128)
+// What bounds it is the chain of one row's waits, not its bytes, so with QUADS (every part and row on a 16-byte border, whole
+// quads, QR <= LP_Q_MOST) a row is read once, all of it asked for before the first sum, and both sums are taken over one
+// barrier.  2,048 rows of 1,536 + 512 + 64 + 32 values: 9.4 us (read twice by single values, one sum after the other: 14.3).
+#define LP_THREADS 128
+#define LP_QUADS 4                                   // quads of the q part that a thread keeps
+#define LP_Q_MOST (4 * LP_THREADS * LP_QUADS)
+static_assert(LAT_MAX_R <= 4 * LP_THREADS, "a thread keeps one quad of the c part");
+
+__device__ __forceinline__ void lat_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void lat_store4(bf16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(reinterpret_cast<const unsigned&>(a), reinterpret_cast<const unsigned&>(b));
+}
+__device__ __forceinline__ float lat_squares(float4 v, float s) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, s)))); }
+__device__ __forceinline__ float4 lat_scaled(float4 v, float by, float4 w) { return make_float4(v.x * by * w.x, v.y * by * w.y, v.z * by * w.z, v.w * by * w.w); }
+
+template <class T, bool QUADS>
+__global__ void __launch_bounds__(LP_THREADS)
 latent_prepare_kernel(const float* proj, int P, int QR, int kv_at, int R, int ROT, int g_at, int H, const float* __restrict__ q_w,
                       const float* __restrict__ kv_w, const float* __restrict__ cos_sin, int table_positions, const int* __restrict__ row_pos,
                       const int* __restrict__ row_slot, const int* __restrict__ page_table, int max_pages, int n_pages, T* c_pages, T* r_pages,
                       T* __restrict__ cq, float* __restrict__ gate, float eps, int write) {
-    __shared__ float scratch[32];
+    __shared__ float scratch[2][LP_THREADS / 32];
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(proj);
     const int r = blockIdx.x;
     const float* x = proj + (size_t)r * P;
-    float s = 0.0f;
+    const bool keeps = kv_at >= 0 && write;
+    const float* z = x + kv_at;          // (only read if the row keeps a position)
+    int slot = -1, pos = -1;
+    if (keeps) slot = row_slot[r], pos = row_pos[r];
+    float4 q[LP_QUADS], c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float s = 0.0f, t = 0.0f;
+    if constexpr (QUADS) {
+#pragma unroll
+        for (int e = 0; e < LP_QUADS; e++) {
+            const int i = 4 * (threadIdx.x + LP_THREADS * e);
+            q[e] = i < QR ? lat_load4(x + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        if (keeps && 4 * threadIdx.x < R) c = lat_load4(z + 4 * threadIdx.x);
+#pragma unroll
+        for (int e = 0; e < LP_QUADS; e++) s = lat_squares(q[e], s);
+        t = lat_squares(c, t);
+    } else {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < QR; i += blockDim.x) s = fmaf(x[i], x[i], s);
-    s = block_sum(s, scratch);
-    const float qs = 1.0f / sqrtf(s / (float)QR + eps);
+        for (int i = threadIdx.x; i < QR; i += LP_THREADS) s = fmaf(x[i], x[i], s);
+        if (keeps) {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < QR; i += blockDim.x) cq[(size_t)r * QR + i] = from_f32<T>(x[i] * qs * q_w[i]);
-    for (int i = threadIdx.x; i < H; i += blockDim.x) gate[(size_t)r * H + i] = 1.0f / (1.0f + expf(-x[g_at + i]));
-    if (kv_at < 0 || !write) return;
-    const int slot = row_slot[r], pos = row_pos[r];
-    if (slot < 0 || pos < 0) return;
+            for (int i = threadIdx.x; i < R; i += LP_THREADS) t = fmaf(z[i], z[i], t);
+        }
+    }
+    for (int i = threadIdx.x; i < H; i += LP_THREADS) gate[(size_t)r * H + i] = 1.0f / (1.0f + expf(-x[g_at + i]));
     const int pi = pos / BC_PAGE;
-    const int page = pi < max_pages ? page_table[(size_t)slot * max_pages + pi] : -1;
-    const float* z = x + kv_at;
-    float t = 0.0f;
+    const int page = slot >= 0 && pos >= 0 && pi < max_pages ? page_table[(size_t)slot * max_pages + pi] : -1;
+    s = warp_sum(s);
+    t = warp_sum(t);
+    if (threadIdx.x % 32 == 0) scratch[0][threadIdx.x / 32] = s, scratch[1][threadIdx.x / 32] = t;
+    __syncthreads();
+    s = t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < LP_THREADS / 32; w++) s += scratch[0][w], t += scratch[1][w];
+    const float qs = 1.0f / sqrtf(s / (float)QR + eps);
+    T* to = cq + (size_t)r * QR;
+    if constexpr (QUADS) {
+#pragma unroll
+        for (int e = 0; e < LP_QUADS; e++) {
+            const int i = 4 * (threadIdx.x + LP_THREADS * e);
+            if (i < QR) lat_store4(to + i, lat_scaled(q[e], qs, lat_load4(q_w + i)));
+        }
+    } else {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < R; i += blockDim.x) t = fmaf(z[i], z[i], t);
-    t = block_sum(t, scratch);
+        for (int i = threadIdx.x; i < QR; i += LP_THREADS) to[i] = from_f32<T>(x[i] * qs * q_w[i]);
+    }
     if (page < 0 || page >= n_pages) return;
     const float cs = 1.0f / sqrtf(t / (float)R + eps);
     const size_t at = (size_t)page * BC_PAGE + pos % BC_PAGE;
+    if constexpr (QUADS) {
+        const int i = 4 * threadIdx.x;
+        if (i < R) lat_store4(c_pages + at * R + i, lat_scaled(c, cs, lat_load4(kv_w + i)));
+    } else {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < R; i += blockDim.x) c_pages[at * R + i] = from_f32<T>(z[i] * cs * kv_w[i]);
+        for (int i = threadIdx.x; i < R; i += LP_THREADS) c_pages[at * R + i] = from_f32<T>(z[i] * cs * kv_w[i]);
+    }
     if (ROT > 0 && pos < table_positions) {
         const int half = ROT / 2;
-        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        for (int i = threadIdx.x; i < half; i += LP_THREADS) {
             const float2 f = *reinterpret_cast<const float2*>(cos_sin + ((size_t)pos * half + i) * 2);
             const float u = z[R + i], v = z[R + half + i];
             r_pages[at * ROT + i] = from_f32<T>(u * f.x - v * f.y);
@@ -339,8 +388,12 @@ static int prepare(const float* proj, int rows, int P, int QR, int kv_at, int R,
     BC_CHECK_ARG(QR <= P && g_at >= 0 && g_at + H <= P && (kv_at < 0 || kv_at + R + ROT <= P), "latent_prepare: the parts do not fit a row of %d", P);
     BC_CHECK_ARG(kv_at < 0 || !write || (c_pages && page_table && (ROT == 0 || (r_pages && cos_sin))), "latent_prepare: a cache to write is missing");
     if (rows == 0) return BC_OK;
-    bc_launch(latent_prepare_kernel<T>, dim3(rows), dim3(128), 0, s, proj, P, QR, kv_at, R, ROT, g_at, H, q_w, kv_w, cos_sin, table_positions, row_pos,
-              row_slot, page_table, max_pages, n_pages, (T*)c_pages, (T*)r_pages, (T*)cq, gate, eps, write);
+    auto on_border = [](const void* p) { return (uintptr_t)p % 16 == 0; };
+    const bool keeps = kv_at >= 0 && write;
+    const bool quads = P % 4 == 0 && QR % 4 == 0 && QR <= LP_Q_MOST && on_border(proj) && on_border(cq) && on_border(q_w) &&
+                       (!keeps || (kv_at % 4 == 0 && R % 4 == 0 && R <= LAT_MAX_R && on_border(c_pages) && on_border(kv_w)));
+    bc_launch(quads ? latent_prepare_kernel<T, true> : latent_prepare_kernel<T, false>, dim3(rows), dim3(LP_THREADS), 0, s, proj, P, QR, kv_at, R, ROT, g_at, H,
+              q_w, kv_w, cos_sin, table_positions, row_pos, row_slot, page_table, max_pages, n_pages, (T*)c_pages, (T*)r_pages, (T*)cq, gate, eps, write);
     BC_LAUNCH_STATUS();
 }
 extern "C" int bc_latent_prepare_f32(const float* proj, int rows, int P, int QR, int kv_at, int R, int ROT, int g_at, int H, const float* q_w,
