@@ -16,7 +16,7 @@
 // of the decays after them.  With all of it in float the results were 1.1 to 1.9 times as far from 64-bit sums as the row scan's; so they
 // are 0.80 to 1.00 times as far (outputs) and 0.95 to 1.00 (state): 1.1e-7 and 0.9e-7 at a decay_scale of exp(-1/2), the scan 1.2e-7 and 1.0e-7.
 // Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
-// of 2,048 rows, 64 heads of 64, decay rank 64: 450 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
+// of 2,048 rows, 64 heads of 64, decay rank 64: 407 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
 // The first two are bound by their instructions; the last walks 128 chunks, one warp a scheduler, each chunk's products waiting for the state of
 // the one before (half warps or warps a row, four or eight value channels a warp, sums across lanes or through shared memory: all within
 // 3 % of one another).
@@ -117,20 +117,28 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
 
 // ------------------------------------------------------------------------------------- packs
 #define DLC_D 64
-#define DLC_YP 34             // numbers a channel of the 32 rows [r W; u W] and [b / W; k / W]: a gap, so that 16-byte writes of eight channels meet no bank twice
+// Where channel d's number for row t of the 32 rows [r W; u W] (and [b / W; k / W]) lies, in doubles: pairs of rows are turned about by the channel, so
+// that neither the 16-byte writes of eight neighbouring channels nor the reads of four rows by four channels meet a bank twice.
+__device__ __forceinline__ int dlc_at(int d, int t) { return d * 2 * CHUNK + (t ^ (4 * (d & 3)) ^ (2 * (d >> 2 & 1))); }
+// c += a b: an 8 x 4 and a 4 x 8 tile of doubles, one number of each a lane (a: row lane / 4, column lane % 4; b: row lane % 4, column lane / 4;
+// c: row lane / 4, columns 2 (lane % 4) and the next).
+__device__ __forceinline__ void dlc_mma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
 #define DLC_RUN 4             // places of chunks a block takes one after another, the next one's rows on their way
 
 // A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
 // columns through the same substitutions.  Chains of dependent steps, so what counts is how many blocks an SM holds: one stage of rows, refilled as soon as
-// they are in registers, leaves room for four (two stages: three; with them and a square root a channel instead of a row 488 us the whole call, now 450).
+// they are in registers, leaves room for four (two stages: three; with them and a square root a channel instead of a row 488 us
+// the whole call, now 407).
 __global__ void __launch_bounds__(DLC_D + 32, 4)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
                     const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
     constexpr int PACK = chunk_pack_floats(DLC_D, true), THREADS = DLC_D + 32, ROW_SET = CHUNK * DLC_D;
     extern __shared__ __align__(16) float delta_smem[];
     float (*in)[CHUNK][DLC_D] = reinterpret_cast<float (*)[CHUNK][DLC_D]>(delta_smem);                  // a chunk's decays, r, k, a
-    double *Y = reinterpret_cast<double*>(delta_smem + 4 * ROW_SET), *X = Y + DLC_D * DLC_YP, *M = Y;      // (M [16][16] where Y was, once that has been used)
-    float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * DLC_YP);    // A, Bm, H, Gm
+    double *Y = reinterpret_cast<double*>(delta_smem + 4 * ROW_SET), *X = Y + DLC_D * 2 * CHUNK, *M = Y;      // (M [16][16] where Y was, once that has been used)
+    float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * 2 * CHUNK);    // A, Bm, H, Gm
     __shared__ float part[2][CHUNK], norm[CHUNK];
     __shared__ ChunkAt todo[DLC_RUN];
     __shared__ int todo_place[DLC_RUN], n_todo;
@@ -172,6 +180,8 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
     };
     issue(0);
     cp_async_commit();
+    // What lies above the diagonals by whole tiles stays zero.
+    for (int i = threadIdx.x; i < 4 * 64; i += THREADS) lower[i / 64][i / 8 % 8][8 + i % 8] = 0.0f;
     const float (*sw)[DLC_D] = in[0], (*sr)[DLC_D] = in[1], (*sk)[DLC_D] = in[2], (*sa)[DLC_D] = in[3];
     for (int c = 0; c < n; c++) {
         cp_async_wait<0>();
@@ -218,11 +228,11 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
                 z1[t] = rate * u;
                 zk[t] = k;
                 if (t & 1) {
-                    double *y = Y + d * DLC_YP + t - 1, *x = X + d * DLC_YP + t - 1;
-                    *reinterpret_cast<double2*>(y) = make_double2(own[t - 1], own[t]);
-                    *reinterpret_cast<double2*>(y + CHUNK) = make_double2(U[t - 1], U[t]);
-                    *reinterpret_cast<double2*>(x) = make_double2(xb_even, xb);
-                    *reinterpret_cast<double2*>(x + CHUNK) = make_double2(xk_even, xk);
+                    const int first = dlc_at(d, t - 1), second = dlc_at(d, CHUNK + t - 1);
+                    *reinterpret_cast<double2*>(Y + first) = make_double2(own[t - 1], own[t]);
+                    *reinterpret_cast<double2*>(Y + second) = make_double2(U[t - 1], U[t]);
+                    *reinterpret_cast<double2*>(X + first) = make_double2(xb_even, xb);
+                    *reinterpret_cast<double2*>(X + second) = make_double2(xk_even, xk);
                 }
                 xb_even = xb;
                 xk_even = xk;
@@ -241,28 +251,38 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         __syncthreads();
         if (c + 1 < n) issue(c + 1);              // these rows are in registers and in Y and X: the next ones may take their place
         cp_async_commit();
-        // [r W; u W] [b / W; k / W]^T over the channels in double: 32 x 32 sums, four rows by two of b and two of k a thread; those above the
-        // diagonals are left out.
-        if (channel) {
-            const int ty = d >> 3, tx = d & 7;
-            double acc[4][4] = {};
-#pragma unroll 4
-            for (int i = 0; i < DLC_D; i++) {
-                const double2 ya = *reinterpret_cast<const double2*>(Y + i * DLC_YP + 4 * ty), yb = *reinterpret_cast<const double2*>(Y + i * DLC_YP + 4 * ty + 2);
-                const double2 xb = *reinterpret_cast<const double2*>(X + i * DLC_YP + 2 * tx), xk = *reinterpret_cast<const double2*>(X + i * DLC_YP + CHUNK + 2 * tx);
-                const double ys[4] = {ya.x, ya.y, yb.x, yb.y}, xs[4] = {xb.x, xb.y, xk.x, xk.y};
+        // [r W; u W] [b / W; k / W]^T over the channels in double, 8 x 8 numbers a tile: the twelve tiles that reach below a diagonal, four a
+        // warp, which share one tile of rows (the last eight rows: all four) or two.  One prompt of 2,048 rows, 64 heads: 407 us the whole call
+        // (a number at a time, sixteen a thread of two warps, the halves above the diagonals too: 433).
+        {
+            const bool last = warp < 2;                     // of r W, then of u W; the third warp takes the first eight rows of both
+            const int g = lane >> 2, e = lane & 3;
+            double acc[4][2] = {};
+            const int of_y = last ? 8 + CHUNK * warp : 0;
+            auto tiles = [&](auto both) {
+                constexpr bool BOTH = decltype(both)::value;
+#pragma unroll 8
+                for (int i = 0; i < DLC_D; i += 4) {
+                    const int d0 = i + e;
+                    const double y0 = Y[dlc_at(d0, of_y + g)], b0 = X[dlc_at(d0, g)], k0 = X[dlc_at(d0, CHUNK + g)];
+                    if (BOTH) {
+                        const double y1 = Y[dlc_at(d0, CHUNK + g)];
+                        dlc_mma(acc[0], y0, b0), dlc_mma(acc[1], y0, k0), dlc_mma(acc[2], y1, b0), dlc_mma(acc[3], y1, k0);
+                    } else {
+                        const double b1 = X[dlc_at(d0, 8 + g)], k1 = X[dlc_at(d0, CHUNK + 8 + g)];
+                        dlc_mma(acc[0], y0, b0), dlc_mma(acc[1], y0, k0), dlc_mma(acc[2], y0, b1), dlc_mma(acc[3], y0, k1);
+                    }
+                }
+            };
+            if (last) tiles(std::false_type());
+            else tiles(std::true_type());
 #pragma unroll
-                for (int a = 0; a < 4; a++)
+            for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) acc[a][e] = fma(ys[a], xs[e], acc[a][e]);
-            }
-            const int t0 = 4 * (ty & 3);
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int t = t0 + a, s = 2 * tx + (e & 1), most = ty >= 4 ? t - 1 : t;      // s < t in A and Bm, or s <= t
-                    lower[(ty >= 4 ? 0 : 2) + (e >> 1)][t][s] = s <= most ? (float)acc[a][e] : 0.0f;
+                for (int j = 0; j < 2; j++) {
+                    const bool of_u = last ? warp == 1 : i >= 2;                 // A and Bm (s < t), or H and Gm (s <= t)
+                    const int t = last ? 8 + g : g, s = (last && i >= 2 ? 8 : 0) + 2 * e + j, most = of_u ? t - 1 : t;
+                    lower[(of_u ? 0 : 2) + (i & 1)][t][s] = s <= most ? (float)acc[i][j] : 0.0f;
                 }
         }
         __syncthreads();
@@ -319,7 +339,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         __syncthreads();          // the next chunk writes Y, X and the triangles
     }
 }
-#define DLC_SMEM ((4 * CHUNK * DLC_D + 4 * CHUNK * CHUNK_G) * sizeof(float) + 2 * DLC_D * DLC_YP * sizeof(double))
+#define DLC_SMEM ((4 * CHUNK * DLC_D + 4 * CHUNK * CHUNK_G) * sizeof(float) + 4 * CHUNK * DLC_D * sizeof(double))
 
 // Whether heads of D channels run in chunks, and the floats of scratch that `rows` rows of `seqs` sequences take (0: they do not), of which those of
 // fewer than min_rows rows are left alone.
