@@ -16,11 +16,26 @@
 // of the decays after them.  With all of it in float the results were 1.1 to 1.9 times as far from 64-bit sums as the row scan's; so they
 // are 0.80 to 1.00 times as far (outputs) and 0.95 to 1.00 (state): 1.1e-7 and 0.9e-7 at a decay_scale of exp(-1/2), the scan 1.2e-7 and 1.0e-7.
 // Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
-// of 2,048 rows, 64 heads of 64, decay rank 64: 407 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
+// of 2,048 rows, 64 heads of 64, decay rank 64: 363 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
 // The first two are bound by their instructions; the last walks 128 chunks, one warp a scheduler, each chunk's products waiting for the state of
 // the one before (half warps or warps a row, four or eight value channels a warp, sums across lanes or through shared memory: all within
 // 3 % of one another).
 #include "chunks.cuh"
+
+// 1 / x for x in [2^-126, 2^126] (or not a number), without the branch for all others that a division brings, so that many go on side by side: the
+// hardware's approximation and one step of Newton's iteration, r + r (1 - x r), whose own error is far below its last rounding.  With divisions a row of a
+// chunk's pack took 520 clocks of dependent steps, now 170; the results' distance from 64-bit sums is the same to five digits.
+__device__ __forceinline__ float dlc_reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+// 1 / (1 + exp(-x)).  Below -87 the divisor is held at 2^126.
+__device__ __forceinline__ float dlc_sigmoid(float x) {
+    float y = 1.0f + expf(-x);
+    asm("min.NaN.f32 %0, %0, 0f7E800000;" : "+f"(y));
+    return dlc_reciprocal(y);
+}
 
 // ------------------------------------------------------------------------------------ decays
 // decay[r, c] = exp(-decay_scale * sigmoid(z + w0[c])) with z = sum_j w2t[j, c] tanh(inner[r, j]): a product of 64 rows x 128 channels a block,
@@ -110,7 +125,7 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
         unpack_f32x2(z[r][0], v[0], v[1]);
         unpack_f32x2(z[r][1], v[2], v[3]);
 #pragma unroll
-        for (int e = 0; e < 4; e++) v[e] = expf(-decay_scale * (1.0f / (1.0f + expf(-(v[e] + b[e])))));
+        for (int e = 0; e < 4; e++) v[e] = expf(-decay_scale * dlc_sigmoid(v[e] + b[e]));
         *reinterpret_cast<float4*>(decay + (size_t)row * HD + c) = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
@@ -130,7 +145,7 @@ __device__ __forceinline__ void dlc_mma(double (&c)[2], double a, double b) {
 // A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
 // columns through the same substitutions.  Chains of dependent steps, so what counts is how many blocks an SM holds: one stage of rows, refilled as soon as
 // they are in registers, leaves room for four (two stages: three; with them and a square root a channel instead of a row 488 us
-// the whole call, now 407).
+// the whole call, now 363).
 __global__ void __launch_bounds__(DLC_D + 32, 4)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
                     const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
@@ -139,7 +154,8 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
     float (*in)[CHUNK][DLC_D] = reinterpret_cast<float (*)[CHUNK][DLC_D]>(delta_smem);                  // a chunk's decays, r, k, a
     double *Y = reinterpret_cast<double*>(delta_smem + 4 * ROW_SET), *X = Y + DLC_D * 2 * CHUNK, *M = Y;      // (M [16][16] where Y was, once that has been used)
     float (*lower)[CHUNK][CHUNK_G] = reinterpret_cast<float (*)[CHUNK][CHUNK_G]>(X + DLC_D * 2 * CHUNK);    // A, Bm, H, Gm
-    __shared__ float part[2][CHUNK], norm[CHUNK];
+    __shared__ float part[2][CHUNK];
+    __shared__ float2 norm[CHUNK];            // and its reciprocal
     __shared__ ChunkAt todo[DLC_RUN];
     __shared__ int todo_place[DLC_RUN], n_todo;
     pdl_launch_dependents_if_resident();
@@ -208,7 +224,10 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             if (lane < CHUNK) part[warp][lane] = kk[0];
         }
         __syncthreads();
-        if (d < CHUNK) norm[d] = sqrtf(part[0][d] + part[1][d] + key_eps);      // once a row, not once a channel
+        if (d < CHUNK) {                          // once a row, not once a channel; an infinity's quotients are its reciprocal's products, nothing more
+            const float of = sqrtf(part[0][d] + part[1][d] + key_eps);
+            norm[d] = make_float2(isinf(of) ? 0.0f : of, 1.0f / of);
+        }
         __syncthreads();
         float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
@@ -219,12 +238,14 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             for (int t = 0; t < CHUNK; t++) {
                 const bool ok = mine && t < rows;
                 const float k = ok ? sk[t][d] : 0.0f;
-                const float rate = 1.0f / (1.0f + expf(-((ok ? sa[t][d] : 0.0f) + bias)));
-                const float u = ok ? k / norm[t] : 0.0f;      // zero in rows and channels that do not exist
+                const float rate = dlc_sigmoid((ok ? sa[t][d] : 0.0f) + bias);
+                // k / norm: the product with the reciprocal, and once what that leaves over (Markstein's quotient).  Zero in rows and channels that do not exist.
+                const float2 by = norm[t];
+                const float quotient = k * by.y, u = ok ? fmaf(fmaf(-quotient, by.x, k), by.y, quotient) : 0.0f;
                 U[t] = u * run;
                 run *= ok ? sw[t][d] : 1.0f;
                 own[t] = (ok ? sr[t][d] : 0.0f) * run;
-                const float over = 1.0f / run, xb = rate * u * over, xk = k * over;
+                const float over = dlc_reciprocal(run), xb = rate * u * over, xk = k * over;
                 z1[t] = rate * u;
                 zk[t] = k;
                 if (t & 1) {
@@ -252,8 +273,8 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         if (c + 1 < n) issue(c + 1);              // these rows are in registers and in Y and X: the next ones may take their place
         cp_async_commit();
         // [r W; u W] [b / W; k / W]^T over the channels in double, 8 x 8 numbers a tile: the twelve tiles that reach below a diagonal, four a
-        // warp, which share one tile of rows (the last eight rows: all four) or two.  One prompt of 2,048 rows, 64 heads: 407 us the whole call
-        // (a number at a time, sixteen a thread of two warps, the halves above the diagonals too: 433).
+        // warp, which share one tile of rows (the last eight rows: all four) or two.  One prompt of 2,048 rows, 64 heads: 433 -> 407 us the
+        // whole call (a number at a time, sixteen a thread of two warps, the halves above the diagonals too).
         {
             const bool last = warp < 2;                     // of r W, then of u W; the third warp takes the first eight rows of both
             const int g = lane >> 2, e = lane & 3;

@@ -28,3 +28,34 @@ def test_decays(rows, heads, inner, offset):
     want = torch.exp(-scale * torch.sigmoid(z))
     # z is off by at most (inner + 3) U of its terms' sizes (tanhf 2 U); a decay moves by at most scale / 4 of that; two exponentials, a sum, a quotient and a product.
     assert ((decay.double() - want).abs() <= 2.0 ** -24 * ((inner + 3) * size * scale / 4 + 12) * want).all()
+
+
+@pytest.mark.parametrize("gate,key", [(0.0, 1.0), (300.0, 1.0), (-300.0, 1.0), (-87.5, 1e-25), (0.0, 1e25)])
+def test_removals_at_the_ends_of_the_range(gate, key):
+    """A last row whose removal gate is shut or open all the way, whose key is nearly nothing or whose key's norm is an infinity (its unit key is then zero)."""
+    from borrowed_compute_b200 import ops
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    rows, H, D, inner = 19, 2, 64, 8
+    HD = H * D
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    proj, w2t, w0, bias, before = rnd(rows, 5 * HD + inner), rnd(inner, HD), rnd(HD), torch.zeros(HD, device="cuda"), rnd(1, H, D, D)
+    proj[-1, HD:2 * HD] *= key
+    proj[-1, 4 * HD:5 * HD] = gate
+    state, out, decay = before.clone(), torch.empty((rows, HD), device="cuda"), torch.empty((rows, HD), device="cuda")
+    pack = torch.empty((ops.delta_chunked_scratch(rows, 1, H, D, inner, 0.6),), device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    ops.delta_chunked(proj, w2t, w0, bias, decay, pack, state, i32([0, rows]), i32([0]), out, 1, rows, H, D, 0.6, 1e-6)
+    P = proj.double()
+    r, k, v, _, a = (P[:, i * HD:(i + 1) * HD].view(rows, H, D) for i in range(5))
+    w = decay.double().view(rows, H, D)
+    u = k / torch.sqrt((proj[:, HD:2 * HD].view(rows, H, D) ** 2).sum(-1, keepdim=True) + 1e-6).double()
+    S, size = before[0].double(), None
+    for t in range(rows):
+        e = (S * u[t][:, None]).sum(-1, keepdim=True)
+        size = S.abs() + (e * u[t][:, None]).abs() + (v[t][..., None] * k[t][:, None]).abs()
+        S = S * w[t][:, None] - e * (torch.sigmoid(a[t]) * u[t])[:, None] + v[t][..., None] * k[t][:, None]
+    # Errors grow along the chain of removals; 1e-5 of the largest summand is far below what a gate or a unit key that is off by a part in a thousand gives.
+    assert ((state[0].double() - S).abs() <= 1e-5 * size.amax()).all()
+    assert ((out[-1].double().view(H, D) - (S * r[-1][:, None]).sum(-1)).abs() <= 1e-5 * (size * r[-1][:, None].abs()).sum(-1).amax()).all()
