@@ -151,20 +151,29 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
     // whose place may have held another's: rows of zeros in Z0, times an infinity, would be none.)
     for (int i = threadIdx.x; i < CHUNK_STAGES * CHUNK * 32; i += CHUNK_THREADS) chunk_smem[(i / (CHUNK * 32)) * STAGE + V_AT + i % (CHUNK * 32)] = 0.0f;
     __syncthreads();
-    auto issue = [&](int c) {
-        const float* src = pack + (chunk_place(span, row0, seq, c) * H + h) * PACK;
-        const uint32_t dst = ad_smem(chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < PACK / 4; i += CHUNK_THREADS) cp_async16(dst + 16 * i, src + 4 * i);
-        const int rows = min(CHUNK, n_rows - c * CHUNK), t = threadIdx.x >> 3, at = 4 * (threadIdx.x & 7);
-        if (t < rows && at < pv) cp_async16(dst + 4 * (V_AT + t * 32 + at), v + (size_t)(row0 + c * CHUNK + t) * v_stride + (size_t)h * P + p0 + at);
-        if (t >= rows) *reinterpret_cast<float4*>(chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE + V_AT + t * 32 + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // The chunk that is asked for next (a sequence's chunks lie at neighbouring places): where this thread's first quads come from, the rows from there on, its stage.
+    const int t = threadIdx.x >> 3, at = 4 * (threadIdx.x & 7);
+    const float* next = pack + (chunk_place(span, row0, seq, span.first) * H + h) * PACK + 4 * threadIdx.x;
+    const float* next_v = v + (size_t)(row0 + span.first * CHUNK + t) * v_stride + (size_t)h * P + p0 + at;
+    int next_rows = min(n_rows, (span.first + span.count) * CHUNK) - span.first * CHUNK, next_at = 0;
+    auto issue = [&] {
+        if (next_rows > 0) {
+            float* stage = chunk_smem + next_at;
+            const uint32_t dst = ad_smem(stage) + 16 * threadIdx.x;
+#pragma unroll
+            for (int i = 0; i < PACK / 4 / CHUNK_THREADS; i++) cp_async16(dst + 16 * CHUNK_THREADS * i, next + 4 * CHUNK_THREADS * i);
+            if (threadIdx.x < PACK / 4 % CHUNK_THREADS) cp_async16(dst + 4 * (PACK - PACK % (4 * CHUNK_THREADS)), next + (PACK - PACK % (4 * CHUNK_THREADS)));
+            if (t >= next_rows) *reinterpret_cast<float4*>(stage + V_AT + t * 32 + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            else if (at < pv) cp_async16(ad_smem(stage) + 4 * (V_AT + t * 32 + at), next_v);
+        }
+        cp_async_commit();
+        next += (size_t)H * PACK;
+        next_v += (size_t)CHUNK * v_stride;
+        next_rows -= CHUNK;
+        next_at = next_at == (CHUNK_STAGES - 1) * STAGE ? 0 : next_at + STAGE;
     };
 #pragma unroll
-    for (int i = 0; i < CHUNK_STAGES - 1; i++) {
-        if (span.first + i < n_chunks) issue(span.first + i);
-        cp_async_commit();
-    }
+    for (int i = 0; i < CHUNK_STAGES - 1; i++) issue();
     uint64_t S[DT / 2][PT];
     const bool p_ok = pg * PT < pv;
     float* st = state + (((size_t)slot * H + h) * P + p0 + (p_ok ? pg * PT : 0)) * N + 4 * dg;
@@ -177,12 +186,13 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
             S[2 * m][p] = pack_f32x2(x.x, x.y);
             S[2 * m + 1][p] = pack_f32x2(x.z, x.w);
         }
+    int now_at = 0;               // the stage worked on
     for (int c = span.first; c < n_chunks; c++) {
         cp_async_wait<CHUNK_STAGES - 2>();
         __syncthreads();          // the chunk is there for all, and all have left the one whose stage is filled next
-        if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
-        cp_async_commit();
-        const float* sx = chunk_smem + ((c - span.first) % CHUNK_STAGES) * STAGE;
+        issue();
+        const float* sx = chunk_smem + now_at;
+        now_at = now_at == (CHUNK_STAGES - 1) * STAGE ? 0 : now_at + STAGE;
         const float *x0 = sx + 4 * dg, *z0 = x0 + (DELTA ? 2 : 1) * CHUNK * D, *z1 = z0 + CHUNK * D, *g = sx + MATS * CHUNK * D, *tot = g + CHUNK * CHUNK_G;
         const float* sv = sx + V_AT + pg * PT;
         float vr[CHUNK][PT];      // sixteen rows of this half warp's values
@@ -191,7 +201,7 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
             const float4 x = *reinterpret_cast<const float4*>(sv + t * 32);
             vr[t][0] = x.x, vr[t][1] = x.y, vr[t][2] = x.z, vr[t][3] = x.w;
         }
-        float o[PT], of_group[4][PT];
+        float o[PT], removed[PT], of_group[4][PT];
         ChunkRows<DT> rows_now, rows_next;
         rows_now.load(DELTA ? x0 + CHUNK * D : x0, 0, dg);
         if (DELTA) {
@@ -201,11 +211,7 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
                 rows_now.template times<PT>(S, of_group[i]);
                 rows_now = rows_next;
             }
-            float e[PT];
-            chunk_groups<PT>(of_group, e);
-            __syncwarp();
-            *reinterpret_cast<float4*>(mine + dg * PT) = make_float4(-e[0], -e[1], -e[2], -e[3]);
-            __syncwarp();
+            chunk_groups<PT>(of_group, removed);
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -233,6 +239,10 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
         }
         if (p_ok && c * CHUNK + dg < n_rows)
             *reinterpret_cast<float4*>(out + (size_t)(row0 + c * CHUNK + dg) * H * P + (size_t)h * P + p0 + pg * PT) = make_float4(out_scale * o[0], out_scale * o[1], out_scale * o[2], out_scale * o[3]);
+        if (DELTA) {              // (handed over no sooner than it is needed: what is removed is still being summed while O is begun)
+            *reinterpret_cast<float4*>(mine + dg * PT) = make_float4(-removed[0], -removed[1], -removed[2], -removed[3]);
+            __syncwarp();
+        }
         // The state after the chunk.  Of a delta rule: what was, less what is removed, then what is added (removed last, the sums carry parts that
         // cancel: 1.8 times as far from 64-bit sums).  Else: twelve rows' sum from nothing, what was, the last four rows (what was first: 1.1 times
         // as far where decays are slow; what was last: 1.2 times where they are fast).
