@@ -128,8 +128,43 @@ template <int PT> __device__ __forceinline__ void chunk_groups(const float (*g)[
 // through a ring of asynchronous copies.
 #define CHUNK_THREADS 128
 #define CHUNK_STAGES 3         // chunks on their way or worked on
+#define CHUNK_SORTED 64        // sequences of a step that are put in order (two a lane)
 #define CHUNK_ALONE (120 * 1024)      // bytes of shared memory of which an SM holds one block's
-template <int DL, bool DELTA>      // D = 32 DL
+// A sequence, the step's row it starts at, its rows and its slot.  Of at most 64 the one that comes z-th when the longest come first, by eighths of the
+// longest's rows (of those alike the earlier); every warp works it out for itself, two sequences a lane.
+struct ChunkSequence {
+    int seq, row0, rows, slot;
+};
+__device__ __forceinline__ ChunkSequence chunk_long_first(int z, const int* seq_rows, const int* seq_slot, int seqs) {
+    const int lane = threadIdx.x & 31;
+    int row0[2], rows[2], slot[2], eighth[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int seq = lane + 32 * i;
+        row0[i] = seq < seqs ? seq_rows[seq] : 0;
+        rows[i] = seq < seqs ? seq_rows[seq + 1] - row0[i] : -1;
+        slot[i] = seq < seqs ? seq_slot[seq] : -1;
+    }
+    const int longest = max(__reduce_max_sync(0xffffffffu, max(rows[0], rows[1])), 1);
+#pragma unroll
+    for (int i = 0; i < 2; i++) eighth[i] = rows[i] < 0 ? -1 : (int)min(7ll, 8ll * rows[i] / longest);
+    int before = 0;
+    for (int e = 7; e >= 0; e--) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const unsigned here = __ballot_sync(0xffffffffu, eighth[i] == e);
+            if (z < before + __popc(here)) {
+                const unsigned found = __ballot_sync(0xffffffffu, eighth[i] == e && before + __popc(here & ((1u << lane) - 1u)) == z);
+                const int from = __ffs(found) - 1;
+                return {from + 32 * i, __shfl_sync(0xffffffffu, row0[i], from), __shfl_sync(0xffffffffu, rows[i], from), __shfl_sync(0xffffffffu, slot[i], from)};
+            }
+            before += __popc(here);
+        }
+    }
+    return {z, 0, 0, -1};
+}
+
+template <int DL, bool DELTA, bool LONG_FIRST>      // D = 32 DL
 __global__ void __launch_bounds__(CHUNK_THREADS)
 chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v_stride, float* __restrict__ state, const int* __restrict__ seq_rows,
                   const int* __restrict__ seq_slot, float* __restrict__ out, int H, int N, int P, int n_slots, int write_state, float out_scale) {
@@ -140,9 +175,16 @@ chunk_scan_kernel(const ChunkSpan span, const float* pack, const float* v, int v
     pdl_launch_dependents_if_resident();
     pdl_wait();
     PDL_FRESH(pack); PDL_FRESH(v);
-    const int seq = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * 32;
-    const int slot = seq_slot[seq];
-    const int row0 = seq_rows[seq], n_rows = seq_rows[seq + 1] - row0;
+    const int h = blockIdx.y, p0 = blockIdx.x * 32;
+    int seq = blockIdx.z, row0, n_rows, slot;
+    if constexpr (LONG_FIRST) {
+        const ChunkSequence of = chunk_long_first(seq, seq_rows, seq_slot, gridDim.z);
+        seq = of.seq, row0 = of.row0, n_rows = of.rows, slot = of.slot;
+    } else {
+        slot = seq_slot[seq];
+        row0 = seq_rows[seq];
+        n_rows = seq_rows[seq + 1] - row0;
+    }
     if (slot < 0 || slot >= n_slots || n_rows <= 0 || n_rows < span.min_rows) return;
     const int n_chunks = min(span.first + span.count, (n_rows + CHUNK - 1) / CHUNK);
     if (span.first >= n_chunks) return;
@@ -318,14 +360,22 @@ static cudaError_t chunk_scan_launch(const ChunkSpan& span, const float* pack, c
                                      float* out, int rows, int max_new, int seqs, int H, int N, int P, int n_slots, int write_state, float out_scale, cudaStream_t s) {
     constexpr size_t NEEDS = (CHUNK_STAGES * (chunk_pack_floats(32 * DL, DELTA) + CHUNK * 32) + (DELTA ? 32 * CHUNK : 0)) * sizeof(float);
     static_assert(NEEDS <= CHUNK_ALONE, "shared memory of one block");
+    // Sequences of several lengths go longest first: the first blocks get an SM each and, being the oldest there, its schedulers; in the order they came, the
+    // longest may share an SM with its like.  16 heads of 128 x 256, 400 + 1,100 + 1,800 rows: 403 -> 351 us the whole call (before, the longest's blocks
+    // alone 168 to 308 us), 64 heads of a delta rule 580 -> 528.
     // Where the longest sequence's chain is as long as all SMs' work, an SM to itself for every block of it (and for the others one at a time, through
-    // the shared memory a block asks for): 16 heads of 128 x 256, sequences of 2,000 and three of 100 rows 351 -> 249 us the whole call, 8 heads, 400, 1,100 and 1,800 rows 310 -> 251;
-    // not for 16 heads of the latter, half as much again for all SMs as for the longest (354 and 346), nor for two of 2,048 (382 and 452).
+    // the shared memory a block asks for): 16 heads of 128 x 256, sequences of 2,000 and three of 100 rows 347 -> 243 us the whole call, 8 heads, 400, 1,100 and 1,800 rows 227 -> 208;
+    // not for 16 heads of the latter, half as much again for all SMs as for the longest, nor for two of 2,048 (382 and 452).
     const long long work = (long long)((P + 31) / 32) * H * rows;
     const size_t SMEM = seqs > 1 && work * 7 <= (long long)bc_sm_count() * max_new * 8 ? CHUNK_ALONE : NEEDS;
-    if (cudaError_t e = bc_allow_shared<chunk_scan_kernel<DL, DELTA>>(SMEM); e != cudaSuccess) return e;
-    return bc_launch(chunk_scan_kernel<DL, DELTA>, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H,
-                     N, P, n_slots, write_state, out_scale);
+    auto launch = [&](auto long_first) {
+        constexpr auto* kernel = chunk_scan_kernel<DL, DELTA, decltype(long_first)::value>;
+        if (cudaError_t e = bc_allow_shared<kernel>(SMEM); e != cudaSuccess) return e;
+        return bc_launch(kernel, dim3((P + 31) / 32, H, seqs), dim3(CHUNK_THREADS), SMEM, s, span, pack, v, v_stride, state, seq_rows, seq_slot, out, H, N, P, n_slots,
+                         write_state, out_scale);
+    };
+    const bool mixed = seqs > 1 && seqs <= CHUNK_SORTED && (long long)rows < (long long)seqs * max_new;
+    return mixed ? launch(std::true_type()) : launch(std::false_type());
 }
 
 // A step's chunks through `prepare` (the kernel that fills the pack) and the scan: at once where `capacity` chunks of scratch hold them, else

@@ -16,7 +16,7 @@
 // of the decays after them.  With all of it in float the results were 1.1 to 1.9 times as far from 64-bit sums as the row scan's; so they
 // are 0.80 to 1.00 times as far (outputs) and 0.95 to 1.00 (state): 1.1e-7 and 0.9e-7 at a decay_scale of exp(-1/2), the scan 1.2e-7 and 1.0e-7.
 // Three kernels: the decays of all rows, a product of its own; the chunks' packs, all side by side; the chunks in time order.  One sequence
-// of 2,048 rows, 64 heads of 64, decay rank 64: 363 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
+// of 2,048 rows, 64 heads of 64, decay rank 64: 350 us with the launches, where the kernels that prepare the rows and scan them one by one take 172 + 614 without.
 // The first two are bound by their instructions; the last walks 128 chunks, one warp a scheduler, each chunk's products waiting for the state of
 // the one before (half warps or warps a row, four or eight value channels a warp, sums across lanes or through shared memory: all within
 // 3 % of one another).
@@ -145,7 +145,7 @@ __device__ __forceinline__ void dlc_mma(double (&c)[2], double a, double b) {
 // A block takes the chunks at `run` neighbouring places, of one head: 64 threads a key channel each, and a warp whose first lanes take M's sixteen
 // columns through the same substitutions.  Chains of dependent steps, so what counts is how many blocks an SM holds: one stage of rows, refilled as soon as
 // they are in registers, leaves room for four (two stages: three; with them and a square root a channel instead of a row 488 us
-// the whole call, now 363).
+// the whole call, now 350).
 __global__ void __launch_bounds__(DLC_D + 32, 4)
 delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const float* decay, const float* __restrict__ a_bias, const int* __restrict__ seq_rows,
                     const int* __restrict__ seq_slot, float* __restrict__ pack, int H, int D, float key_eps, int seqs, int n_slots, int run, int places) {
