@@ -154,6 +154,20 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// 1 / x for x in [2^-126, 2^126] (or not a number), without the branch for all others that a division brings, so that many go on side by side: the
+// hardware's approximation and one step of Newton's iteration, r + r (1 - x r), whose own error is far below its last rounding.
+__device__ __forceinline__ float reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+// 1 / (1 + exp(-x)).  Where x is below -87 the divisor is held at 2^126.
+__device__ __forceinline__ float sigmoid_f(float x) {
+    float y = 1.0f + expf(-x);
+    asm("min.NaN.f32 %0, %0, 0f7E800000;" : "+f"(y));
+    return reciprocal(y);
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.  `scratch` holds
 // 32 floats of shared memory.  The order of the additions is fixed by the thread layout.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

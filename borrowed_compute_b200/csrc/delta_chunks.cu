@@ -22,25 +22,10 @@
 // 3 % of one another).
 #include "chunks.cuh"
 
-// 1 / x for x in [2^-126, 2^126] (or not a number), without the branch for all others that a division brings, so that many go on side by side: the
-// hardware's approximation and one step of Newton's iteration, r + r (1 - x r), whose own error is far below its last rounding.  With divisions a row of a
-// chunk's pack took 520 clocks of dependent steps, now 170; the results' distance from 64-bit sums is the same to five digits.
-__device__ __forceinline__ float dlc_reciprocal(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
-// 1 / (1 + exp(-x)).  Below -87 the divisor is held at 2^126.
-__device__ __forceinline__ float dlc_sigmoid(float x) {
-    float y = 1.0f + expf(-x);
-    asm("min.NaN.f32 %0, %0, 0f7E800000;" : "+f"(y));
-    return dlc_reciprocal(y);
-}
-
 // ------------------------------------------------------------------------------------ decays
 // decay[r, c] = exp(-decay_scale * sigmoid(z + w0[c])) with z = sum_j w2t[j, c] tanh(inner[r, j]): a product of 64 rows x 128 channels a block,
 // eight rows by four channels a thread, 64 inner channels at a time, all asked for at once, sixteen bytes a load.
-// 2,048 rows x 4,096 channels, rank 64: 40 us (32 inner channels at a time, four bytes a load: 56).
+// 2,048 rows x 4,096 channels, rank 64: 38 us (32 inner channels at a time, four bytes a load: 56).
 #define DLC_ROWS 64
 #define DLC_COLS 128
 #define DLC_K 64
@@ -125,7 +110,7 @@ delta_decay_kernel(const float* proj, int stride, int inner_at, const float* __r
         unpack_f32x2(z[r][0], v[0], v[1]);
         unpack_f32x2(z[r][1], v[2], v[3]);
 #pragma unroll
-        for (int e = 0; e < 4; e++) v[e] = expf(-decay_scale * dlc_sigmoid(v[e] + b[e]));
+        for (int e = 0; e < 4; e++) v[e] = expf(-decay_scale * sigmoid_f(v[e] + b[e]));
         *reinterpret_cast<float4*>(decay + (size_t)row * HD + c) = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
@@ -232,20 +217,21 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
         float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
         float z1[CHUNK], zk[CHUNK];               // b_t and k_t, then times the decays after row t
+        // (With divisions and their branches a row took 520 clocks of dependent steps, now 170; the results' distance from 64-bit sums is the same to five digits.)
         if (channel) {
             float run = 1.0f, xb_even = 0.0f, xk_even = 0.0f;
 #pragma unroll
             for (int t = 0; t < CHUNK; t++) {
                 const bool ok = mine && t < rows;
                 const float k = ok ? sk[t][d] : 0.0f;
-                const float rate = dlc_sigmoid((ok ? sa[t][d] : 0.0f) + bias);
+                const float rate = sigmoid_f((ok ? sa[t][d] : 0.0f) + bias);
                 // k / norm: the product with the reciprocal, and once what that leaves over (Markstein's quotient).  Zero in rows and channels that do not exist.
                 const float2 by = norm[t];
                 const float quotient = k * by.y, u = ok ? fmaf(fmaf(-quotient, by.x, k), by.y, quotient) : 0.0f;
                 U[t] = u * run;
                 run *= ok ? sw[t][d] : 1.0f;
                 own[t] = (ok ? sr[t][d] : 0.0f) * run;
-                const float over = dlc_reciprocal(run), xb = rate * u * over, xk = k * over;
+                const float over = reciprocal(run), xb = rate * u * over, xk = k * over;
                 z1[t] = rate * u;
                 zk[t] = k;
                 if (t & 1) {

@@ -31,8 +31,6 @@
 #define DR_BLOCK_COLS (DR_COLS * DR_CJ)
 #define DR_MAX_D 256
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-
 // The eight threads that share a value channel hold the key channels in runs of four neighbours, the eight threads'
 // runs side by side (a load of 16 bytes a thread then covers 128 bytes without a gap) and the next runs 32 channels
 // on: thread `lane` holds channels 32 m + 4 lane .. + 3 for m = 0 .. R/4 - 1.  Heads of at most 16 channels: two
@@ -268,7 +266,8 @@ delta_scan_kernel(const float* __restrict__ proj, int stride, const float* __res
 // out[row, c] = o[row, c] / rms(o[row, head(c)]) * weight[c] * sigmoid(gate[row, c]), in the activation type.
 // A warp takes DF_HEADS heads of a row, all their loads asked for together (a block a head with two block sums a row: 47 us for 2,048 rows of 64
 // heads of 64, against 14 us of bytes).  Lane L holds channels L, L + 32, .. of a head; the sums are those of block_sum over a thread a
-// channel, in the same order, so that delta_step_kernel below gives the same bits.
+// channel, in the same order, so that delta_step_kernel below gives the same bits.  2,048 rows of 64 heads of 64: 33 us (a sum a run, a root a head and lane,
+// gates with a division's branch: 39).
 #define DF_HEADS 4
 template <int NW, class T>      // runs of 32 channels a head: D <= 32 NW
 __global__ void __launch_bounds__(256)
@@ -292,15 +291,41 @@ delta_finish_kernel(const float* o, const float* gate, int gate_stride, const fl
             v[e][i] = ok ? o[row * HD + c] : 0.0f;
             g[e][i] = ok ? gate[row * gate_stride + c] : 0.0f;
         }
+    float mine = 0.0f;
+    if constexpr (HEADS > 1) {
+        // All heads' sums at once, halved among the lanes: lanes 8 e .. 8 e + 7 are left with head e's (of each of its two runs four of them).
+        static_assert(HEADS == 4 && NW == 2, "eight sums: two bits of a lane's number for the head, one for the run");
+        float s[HEADS * NW];
+#pragma unroll
+        for (int i = 0; i < HEADS * NW; i++) s[i] = v[i / NW][i % NW] * v[i / NW][i % NW];
+#pragma unroll
+        for (int n = HEADS * NW / 2; n > 0; n >>= 1) {
+            const bool up = lane & 4 * n;
+#pragma unroll
+            for (int i = 0; i < n; i++) {
+                const float keep = up ? s[i + n] : s[i], send = up ? s[i] : s[i + n];
+                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * n);
+            }
+        }
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 4);        // the two runs'
+        mine = 1.0f / sqrtf(s[0] / (float)D + eps);
+    }
 #pragma unroll
     for (int e = 0; e < HEADS; e++) {
-        float part = 0.0f;
+        float scale;
+        if constexpr (HEADS > 1) {
+            scale = __shfl_sync(0xffffffffu, mine, 8 * e);
+        } else {
+            float part = 0.0f;
 #pragma unroll
-        for (int i = 0; i < NW; i++) {
-            const float sum = warp_sum(v[e][i] * v[e][i]);
-            part = lane == i ? sum : part;
+            for (int i = 0; i < NW; i++) {
+                const float sum = warp_sum(v[e][i] * v[e][i]);
+                part = lane == i ? sum : part;
+            }
+            scale = 1.0f / sqrtf(warp_sum(part) / (float)D + eps);
         }
-        const float scale = 1.0f / sqrtf(warp_sum(part) / (float)D + eps);
 #pragma unroll
         for (int i = 0; i < NW; i++) {
             const int c = (h0 + e) * D + lane + 32 * i;
