@@ -36,23 +36,16 @@ __device__ __forceinline__ float2 lat_load2(const bf16* p) {
 // ------------------------------------------------------------------------------------ prepare
 // One block a row.  proj: [rows, P] float; the q part starts at 0 and is QR wide, the c part at kv_at (R wide, then
 // ROT values of r; kv_at < 0: the mixer reads another layer's cache and has no such part), the gate part at g_at (H wide).
-// What bounds it is the chain of one row's waits, not its bytes, so with QUADS (every part and row on a 16-byte border, whole
-// quads, QR <= LP_Q_MOST) a row is read once, all of it asked for before the first sum, and both sums are taken over one
-// barrier.  2,048 rows of 1,536 + 512 + 64 + 32 values: 9.4 us (read twice by single values, one sum after the other: 14.3).
+// What bounds it is the chain of one row's waits, not its bytes, so a row whose parts fit the threads' registers (KEPT: QR <= LP_Q_MOST) is
+// read once, all of it asked for before the first sum, and both sums are taken over one barrier.  Either way a thread adds up every
+// LP_THREADS-th value and the warps' sums are added as block_sum adds them, so the two ways give the same bits.
 #define LP_THREADS 128
-#define LP_QUADS 4                                   // quads of the q part that a thread keeps
-#define LP_Q_MOST (4 * LP_THREADS * LP_QUADS)
-static_assert(LAT_MAX_R <= 4 * LP_THREADS, "a thread keeps one quad of the c part");
+#define LP_Q_KEPT 16                                 // values of the q part that a thread keeps, and of the c part
+#define LP_C_KEPT 4
+#define LP_Q_MOST (LP_THREADS * LP_Q_KEPT)
+static_assert(LAT_MAX_R <= LP_THREADS * LP_C_KEPT, "a thread keeps its share of the c part");
 
-__device__ __forceinline__ void lat_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void lat_store4(bf16* p, float4 v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = make_uint2(reinterpret_cast<const unsigned&>(a), reinterpret_cast<const unsigned&>(b));
-}
-__device__ __forceinline__ float lat_squares(float4 v, float s) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, s)))); }
-__device__ __forceinline__ float4 lat_scaled(float4 v, float by, float4 w) { return make_float4(v.x * by * w.x, v.y * by * w.y, v.z * by * w.z, v.w * by * w.w); }
-
-template <class T, bool QUADS>
+template <class T, bool KEPT>
 __global__ void __launch_bounds__(LP_THREADS)
 latent_prepare_kernel(const float* proj, int P, int QR, int kv_at, int R, int ROT, int g_at, int H, const float* __restrict__ q_w,
                       const float* __restrict__ kv_w, const float* __restrict__ cos_sin, int table_positions, const int* __restrict__ row_pos,
@@ -68,18 +61,23 @@ latent_prepare_kernel(const float* proj, int P, int QR, int kv_at, int R, int RO
     const float* z = x + kv_at;          // (only read if the row keeps a position)
     int slot = -1, pos = -1;
     if (keeps) slot = row_slot[r], pos = row_pos[r];
-    float4 q[LP_QUADS], c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float q[LP_Q_KEPT], c[LP_C_KEPT];
     float s = 0.0f, t = 0.0f;
-    if constexpr (QUADS) {
+    if constexpr (KEPT) {
 #pragma unroll
-        for (int e = 0; e < LP_QUADS; e++) {
-            const int i = 4 * (threadIdx.x + LP_THREADS * e);
-            q[e] = i < QR ? lat_load4(x + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int e = 0; e < LP_Q_KEPT; e++) {
+            const int i = threadIdx.x + LP_THREADS * e;
+            q[e] = i < QR ? x[i] : 0.0f;
         }
-        if (keeps && 4 * threadIdx.x < R) c = lat_load4(z + 4 * threadIdx.x);
 #pragma unroll
-        for (int e = 0; e < LP_QUADS; e++) s = lat_squares(q[e], s);
-        t = lat_squares(c, t);
+        for (int e = 0; e < LP_C_KEPT; e++) {
+            const int i = threadIdx.x + LP_THREADS * e;
+            c[e] = keeps && i < R ? z[i] : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < LP_Q_KEPT; e++) s = fmaf(q[e], q[e], s);
+#pragma unroll
+        for (int e = 0; e < LP_C_KEPT; e++) t = fmaf(c[e], c[e], t);
     } else {
 #pragma unroll 4
         for (int i = threadIdx.x; i < QR; i += LP_THREADS) s = fmaf(x[i], x[i], s);
@@ -95,27 +93,29 @@ latent_prepare_kernel(const float* proj, int P, int QR, int kv_at, int R, int RO
     t = warp_sum(t);
     if (threadIdx.x % 32 == 0) scratch[0][threadIdx.x / 32] = s, scratch[1][threadIdx.x / 32] = t;
     __syncthreads();
-    s = t = 0.0f;
-#pragma unroll
-    for (int w = 0; w < LP_THREADS / 32; w++) s += scratch[0][w], t += scratch[1][w];
-    const float qs = 1.0f / sqrtf(s / (float)QR + eps);
+    auto of_warps = [](const float* part) { return (part[0] + part[2]) + (part[1] + part[3]); };
+    static_assert(LP_THREADS == 128, "four warps' sums");
+    const float qs = 1.0f / sqrtf(of_warps(scratch[0]) / (float)QR + eps);
     T* to = cq + (size_t)r * QR;
-    if constexpr (QUADS) {
+    if constexpr (KEPT) {
 #pragma unroll
-        for (int e = 0; e < LP_QUADS; e++) {
-            const int i = 4 * (threadIdx.x + LP_THREADS * e);
-            if (i < QR) lat_store4(to + i, lat_scaled(q[e], qs, lat_load4(q_w + i)));
+        for (int e = 0; e < LP_Q_KEPT; e++) {
+            const int i = threadIdx.x + LP_THREADS * e;
+            if (i < QR) to[i] = from_f32<T>(q[e] * qs * q_w[i]);
         }
     } else {
 #pragma unroll 4
         for (int i = threadIdx.x; i < QR; i += LP_THREADS) to[i] = from_f32<T>(x[i] * qs * q_w[i]);
     }
     if (page < 0 || page >= n_pages) return;
-    const float cs = 1.0f / sqrtf(t / (float)R + eps);
+    const float cs = 1.0f / sqrtf(of_warps(scratch[1]) / (float)R + eps);
     const size_t at = (size_t)page * BC_PAGE + pos % BC_PAGE;
-    if constexpr (QUADS) {
-        const int i = 4 * threadIdx.x;
-        if (i < R) lat_store4(c_pages + at * R + i, lat_scaled(c, cs, lat_load4(kv_w + i)));
+    if constexpr (KEPT) {
+#pragma unroll
+        for (int e = 0; e < LP_C_KEPT; e++) {
+            const int i = threadIdx.x + LP_THREADS * e;
+            if (i < R) c_pages[at * R + i] = from_f32<T>(c[e] * cs * kv_w[i]);
+        }
     } else {
 #pragma unroll 4
         for (int i = threadIdx.x; i < R; i += LP_THREADS) c_pages[at * R + i] = from_f32<T>(z[i] * cs * kv_w[i]);
@@ -388,11 +388,8 @@ static int prepare(const float* proj, int rows, int P, int QR, int kv_at, int R,
     BC_CHECK_ARG(QR <= P && g_at >= 0 && g_at + H <= P && (kv_at < 0 || kv_at + R + ROT <= P), "latent_prepare: the parts do not fit a row of %d", P);
     BC_CHECK_ARG(kv_at < 0 || !write || (c_pages && page_table && (ROT == 0 || (r_pages && cos_sin))), "latent_prepare: a cache to write is missing");
     if (rows == 0) return BC_OK;
-    auto on_border = [](const void* p) { return (uintptr_t)p % 16 == 0; };
-    const bool keeps = kv_at >= 0 && write;
-    const bool quads = P % 4 == 0 && QR % 4 == 0 && QR <= LP_Q_MOST && on_border(proj) && on_border(cq) && on_border(q_w) &&
-                       (!keeps || (kv_at % 4 == 0 && R % 4 == 0 && R <= LAT_MAX_R && on_border(c_pages) && on_border(kv_w)));
-    bc_launch(quads ? latent_prepare_kernel<T, true> : latent_prepare_kernel<T, false>, dim3(rows), dim3(LP_THREADS), 0, s, proj, P, QR, kv_at, R, ROT, g_at, H,
+    const bool kept = QR <= LP_Q_MOST && (kv_at < 0 || !write || R <= LAT_MAX_R);
+    bc_launch(kept ? latent_prepare_kernel<T, true> : latent_prepare_kernel<T, false>, dim3(rows), dim3(LP_THREADS), 0, s, proj, P, QR, kv_at, R, ROT, g_at, H,
               q_w, kv_w, cos_sin, table_positions, row_pos, row_slot, page_table, max_pages, n_pages, (T*)c_pages, (T*)r_pages, (T*)cq, gate, eps, write);
     BC_LAUNCH_STATUS();
 }
