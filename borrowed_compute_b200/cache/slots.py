@@ -159,30 +159,36 @@ class SlotTable:
             if more > self.pools[g].available + self._releasable(g, pages, new_len, rows):
                 raise CacheError(f"the cache is full: slot {slot} needs {more} more pages of {PAGE} tokens in group {g}, "
                                  f"{self.pools[g].available} are free")
-        self._take(st, slot, need, new_len, rows)
+        self._let_go(st, slot, new_len, rows)
+        self._take(st, slot, need)
 
-    def _take(self, st: _Slot, slot: int, need: int, new_len: int, rows: int) -> None:
-        """Moves the pages of a reservation that has been counted."""
+    def _let_go(self, st: _Slot, slot: int, new_len: int, rows: int) -> None:
+        """Gives back the pages that a counted reservation no longer reads."""
         for g, pages in enumerate(st.pages):
-            dropped = []
-            if self._lets_go(g):
-                first = self._first_needed_page(g, new_len, rows)
-                kept = self._kept_pages(g)
-                dropped = [p for p in pages[kept:first] if p >= 0]
+            if not self._lets_go(g):
+                continue
+            first = self._first_needed_page(g, new_len, rows)
+            kept = self._kept_pages(g)
+            dropped = [p for p in pages[kept:first] if p >= 0]
             if dropped:
                 self.pools[g].give_back(dropped)
                 for i in range(kept, min(first, len(pages))):
                     pages[i] = -1
+                self._write_row(g, slot, pages)
+
+    def _take(self, st: _Slot, slot: int, need: int) -> None:
+        """Takes what a counted reservation lacks of ``need`` pages a group."""
+        for g, pages in enumerate(st.pages):
             more = need - len(pages)
             if more > 0:
                 pages.extend(self.pools[g].take(more))
-            if dropped or more > 0:
                 self._write_row(g, slot, pages)
 
     def reserve_many(self, requests: Sequence[tuple]) -> None:
         """``reserve`` for several slots, all or nothing: ``requests`` holds (slot, new_len,
-        rows) of distinct slots; what all of them need together is counted against every
-        pool before any page moves, so a refusal leaves the bookkeeping as it was."""
+        rows) of distinct slots; what all of them need together, less what they let go, is
+        counted against every pool before any page moves, so a refusal leaves the bookkeeping
+        as it was.  All let go before any takes, so what has been counted is there."""
         need = [0] * len(self.groups)
         for slot, new_len, rows in requests:
             st = self._held(slot)
@@ -191,13 +197,16 @@ class SlotTable:
             if new_len < st.length:
                 raise CacheError(f"slot {slot} holds {st.length} positions, reserve cannot shrink it to {new_len}")
             for g, pages in enumerate(st.pages):
-                need[g] += pages_for(new_len) - len(pages) - self._releasable(g, pages, new_len, rows)
+                # (Pages that a slot holds beyond its need are no other slot's.)
+                need[g] += max(0, pages_for(new_len) - len(pages)) - self._releasable(g, pages, new_len, rows)
         for g, n in enumerate(need):
             if n > self.pools[g].available:
                 raise CacheError(f"the cache is full: this step needs {n} more pages of {PAGE} tokens in group {g}, "
                                  f"{self.pools[g].available} are free")
         for slot, new_len, rows in requests:
-            self._take(self._slots[slot], slot, pages_for(new_len), new_len, rows)
+            self._let_go(self._slots[slot], slot, new_len, rows)
+        for slot, new_len, _ in requests:
+            self._take(self._slots[slot], slot, pages_for(new_len))
 
     def _lets_go(self, g: int) -> bool:
         """Whether the group's sequences let pages go as they grow."""

@@ -162,6 +162,52 @@ def test_reserving_for_several_slots_is_all_or_nothing():
     t.check()
 
 
+def _everything(t):
+    return ([[list(r) for r in rows] for rows in t.tables], set(t.dirty), [list(p._free) for p in t.pools], [list(p._held) for p in t.pools],
+            {s: (st.length, [list(p) for p in st.pages]) for s, st in t._slots.items()})
+
+
+@pytest.mark.parametrize("groups", [[GroupPlan(window=64)], [GroupPlan(window=64), GroupPlan(window=64)], [GroupPlan(window=64), GroupPlan(chunk=256)]])
+def test_what_one_slot_lets_go_pays_for_another_whatever_their_order(groups):
+    for order in (0, 1):
+        t = SlotTable(n_slots=2, n_pages=8, max_seq=1024, groups=groups)
+        a, b = t.acquire(), t.acquire()
+        t.reserve_many([(a, 256, 256), (b, 256, 256)])
+        t.commit(a, 256), t.commit(b, 256)
+        requests = [(a, 576, 320), (b, 257, 1)]      # 5 pages and 1 a group; both let go what lies before position 193 or 256
+        t.reserve_many(requests[::-1] if order else requests)
+        t.commit(a, 576), t.commit(b, 257)
+        t.check()
+        assert all(t.tables[g][s][:n] == t._slots[s].pages[g] for g in range(len(groups)) for s, n in ((a, 9), (b, 5)))
+
+
+@pytest.mark.parametrize("groups", [[GroupPlan(window=64)], [GroupPlan(window=64), GroupPlan()], [GroupPlan(chunk=128, keep_first=4), GroupPlan(window=200)]])
+def test_a_refused_request_of_several_slots_changes_nothing(groups):
+    rnd = random.Random(5)
+    refused = 0
+    for _ in range(600):
+        t = SlotTable(n_slots=3, n_pages=rnd.randrange(6, 12), max_seq=1024, groups=groups)
+        slots = [t.acquire() for _ in range(3)]
+        for step in range(8):
+            live = rnd.sample(slots, rnd.randrange(1, 4))
+            requests = []
+            for s in live:
+                rows = rnd.choice([1, 1, 40, 90, 150, 320])
+                requests.append((s, min(t.length(s) + rows, 1024), rows))
+            before = _everything(t)
+            try:
+                t.reserve_many(requests)
+            except CacheError:
+                refused += 1
+                assert _everything(t) == before
+                continue
+            for s, n, _ in requests:
+                if rnd.random() < 0.8:               # else: reserved, but never filled
+                    t.commit(s, n)
+            t.check()
+    assert refused > 100
+
+
 def test_check_rollback_changes_nothing():
     t = SlotTable(n_slots=1, n_pages=8, max_seq=512, groups=[GroupPlan(), GroupPlan(window=70)])
     s = t.acquire()
