@@ -161,11 +161,10 @@ __device__ __forceinline__ float reciprocal(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return fmaf(r, fmaf(-x, r, 1.0f), r);
 }
-// 1 / (1 + exp(-x)).  Where x is below -87 the divisor is held at 2^126.
+// 1 / (1 + exp(-x)), a quarter of the divisor's reciprocal taken: the divisor may reach 2^128.  Where exp(-x) is infinite (x below -88.7) it is zero.
 __device__ __forceinline__ float sigmoid_f(float x) {
-    float y = 1.0f + expf(-x);
-    asm("min.NaN.f32 %0, %0, 0f7E800000;" : "+f"(y));
-    return reciprocal(y);
+    const float e = expf(-x), r = 0.25f * reciprocal(fmaf(0.25f, e, 0.25f));
+    return e == INFINITY ? 0.0f : r;
 }
 
 // Sum over a block of up to 1024 threads; every thread gets the result.  `scratch` holds

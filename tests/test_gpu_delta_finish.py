@@ -25,7 +25,16 @@ def test_finish(dtype, rows, heads, dim):
     x = o.double().view(rows, heads, dim)
     want = (x / (x.square().mean(-1, keepdim=True) + eps).sqrt()).view(rows, HD) * weight.double() * torch.sigmoid(proj[:, 8:].double())
     # Seven additions of positive numbers and a square, halved by the root; a quotient, a root and two products; an exponential (2 ulp), a sum and a
-    # reciprocal; the rounding to the result's type.  A gate's divisor past 2^126 is held there.
+    # reciprocal; the rounding to the result's type.  A gate below 2^-126 is off by the smallest float, below 2^-128 (its exponential overflows) it is
+    # zero; a result is off by half the smallest of its type.
     u = 2.0 ** -24
-    store = u if dtype == torch.float32 else 2.0 ** -8
-    assert ((out.double() - want).abs() <= (16 * u + store) * want.abs() + 2.0 ** -122).all()
+    store, least = (u, 2.0 ** -150) if dtype == torch.float32 else (2.0 ** -8, 2.0 ** -134)
+    gate = torch.sigmoid(proj[:, 8:].double())
+    size = (want / gate).abs().nan_to_num(0.0, 0.0, 0.0)
+    gate_off = torch.where(gate < 2.0 ** -127.9, 2.0 ** -127.9, 2.0 ** -149)
+    assert ((out.double() - want).abs() <= (16 * u + store) * want.abs() + gate_off * (size + 1) + least).all()
+    assert (out[0, :n][gates[:n] < -89.0] == 0.0).all(), "a gate that is shut lets nothing through"
+    # With an infinity behind it the result is not a number: zero times infinity.
+    weight[0], proj[0, 8] = float("inf"), -100.0
+    ops.delta_finish(o, proj, 8, weight, out, heads, dim, eps)
+    assert out[0, 0].isnan()
