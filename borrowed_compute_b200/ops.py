@@ -597,62 +597,63 @@ _self_checked = set()
 
 
 def self_check(device: torch.device) -> None:
-    """Once a device and process: every epilogue of the tensor-core product, and the CUDA-core
-    product, on a 37 x 512 weight with one row and with three, against float64 sums, as the
+    """Once a device and process: every epilogue of the tensor-core product, of the CUDA-core product and of the float32 product on the
+    tensor cores against float64 sums, on a 37 x 512 weight with one row and with three, as the
     reference checks its products before it trusts a GPU (crates/bc-infer/src/gpu/mod.rs:
     181-206, same sizes, same inputs rule, same 1e-3 (1 + |want|) bound; there a failure means
-    the CPU serves, here there is no other path, so it raises)."""
+    the CPU serves, here there is no other path, so it raises).  The float32 product on the tensor cores takes sums of more than 512 products:
+    1,028 of them, two pieces, with three rows and with 130, which go different ways.  One multiply-add after another is off by 8e-6 (1 + |want|) at most on
+    these inputs, sums without the operands' last eight bits by 1e-4, so the bound there is 2e-5 (1 + |want|)."""
     import numpy as np
 
     index = device.index if device.index is not None else torch.cuda.current_device()
     if index in _self_checked:
         return
-    rows_w, cols = 37, 512
+    rows_w = 37
     rng = np.random.default_rng(7)
-    w = rng.standard_normal((2 * rows_w, cols)).astype(np.float32) * 0.5
-    wb = torch.from_numpy(w).to(device=device, dtype=torch.bfloat16)
-    w64 = wb.float().cpu().numpy().astype(np.float64)
 
-    def bad(got: torch.Tensor, want: np.ndarray, rel: float = 1e-3) -> bool:
-        g = got.float().cpu().numpy().astype(np.float64)
-        return (not np.isfinite(g).all()) or bool((np.abs(g - want) > rel * (1.0 + np.abs(want))).any())
+    def inputs(n: int, cols: int) -> np.ndarray:
+        return (((np.arange(n * cols) * 31 % 97).astype(np.float32) - 48.0) / 50.0).reshape(n, cols)
 
-    rounded = 2.0 ** -7    # an output that is itself rounded to bfloat16 carries half an ulp of 2^-8 besides
-    for n in (1, 3):       # one row and a batch take different paths
-        x = (((np.arange(n * cols) * 31 % 97).astype(np.float32) - 48.0) / 50.0).reshape(n, cols)
-        xb = torch.from_numpy(x).to(device=device, dtype=torch.bfloat16)
-        x64 = xb.float().cpu().numpy().astype(np.float64)
-        full = x64 @ w64.T                                                    # [n, 74]: gate rows, then up rows
+    def weight(cols: int) -> np.ndarray:
+        return rng.standard_normal((2 * rows_w, cols)).astype(np.float32) * 0.5
+
+    def check(name: str, product, x: torch.Tensor, w: torch.Tensor, rel: float = 1e-3) -> None:
+        n, act = x.shape[0], x.dtype
+        rounded = 2.0 ** -7 if act == torch.bfloat16 else rel    # an output that is itself rounded to bfloat16 carries half an ulp of 2^-8 besides
+        full = x.float().cpu().numpy().astype(np.float64) @ w.float().cpu().numpy().astype(np.float64).T      # [n, 74]: gate rows, then up rows
         gate, up = full[:, :rows_w], full[:, rows_w:]
+        wrong = []
+
+        def one(what: str, epilogue: int, want: np.ndarray, stored: torch.dtype, within: float, base: float = 0.0, **numbers) -> None:
+            out = torch.full(want.shape, base, dtype=stored, device=device)
+            product(x, w, out, epilogue, **numbers)
+            g = out.float().cpu().numpy().astype(np.float64)
+            if not np.isfinite(g).all() or bool((np.abs(g - want) > within * (1.0 + np.abs(want))).any()):
+                wrong.append(what)
+
+        below = np.minimum(full, 0.0)
+        one("store", EPI_STORE, full, act, rounded)
+        one("store_f32", EPI_STORE_F32, full, torch.float32, rel)
+        one("add_f32", EPI_ADD_F32, full + 0.25, torch.float32, rel, base=0.25)
+        one("swiglu", EPI_SWIGLU, gate / (1.0 + np.exp(-gate)) * up, act, rounded)
+        one("relu2", EPI_RELU2, np.maximum(full, 0.0) ** 2, act, rounded)
+        one("xielu", EPI_XIELU, np.where(full > 0, 0.75 * full * full, 1.25 * (np.expm1(below) - below)) + 0.5 * full, act, rounded, act=(0.75, 1.25))
+        one("silu_f32", EPI_SILU_F32, np.where(np.arange(2 * rows_w) < 41, full / (1.0 + np.exp(-full)), full), torch.float32, rel, cols=41)
+        if wrong:
+            raise KernelError(f"self-check: the {name} product with {n} row(s) is wrong for the epilogue(s) {wrong} on a "
+                              f"{rows_w} x {x.shape[1]} weight; this device or this build of the kernels cannot be trusted")
+
+    def on_device(a: np.ndarray, dtype: torch.dtype = torch.float32) -> torch.Tensor:
+        return torch.from_numpy(a).to(device=device, dtype=dtype)
+
+    w, long_w = weight(512), weight(1028)
+    for n in (1, 3):       # one row and a batch take different paths
         for name, product in (("tensor-core", gemm_tc), ("CUDA-core", gemm_simt)):
-            stored = torch.empty((n, 2 * rows_w), dtype=torch.bfloat16, device=device)
-            product(xb, wb, stored, EPI_STORE)
-            scores = torch.empty((n, 2 * rows_w), dtype=torch.float32, device=device)
-            product(xb, wb, scores, EPI_STORE_F32)
-            added = torch.full((n, 2 * rows_w), 0.25, dtype=torch.float32, device=device)
-            product(xb, wb, added, EPI_ADD_F32)
-            gated = torch.empty((n, rows_w), dtype=torch.bfloat16, device=device)
-            product(xb, wb, gated, EPI_SWIGLU)
-            squared = torch.empty((n, 2 * rows_w), dtype=torch.bfloat16, device=device)
-            product(xb, wb, squared, EPI_RELU2)
-            curved = torch.empty((n, 2 * rows_w), dtype=torch.bfloat16, device=device)
-            product(xb, wb, curved, EPI_XIELU, act=(0.75, 1.25))
-            curve = np.where(full > 0, 0.75 * full * full, 1.25 * (np.expm1(np.minimum(full, 0.0)) - np.minimum(full, 0.0))) + 0.5 * full
-            gated_cols = torch.empty((n, 2 * rows_w), dtype=torch.float32, device=device)
-            product(xb, wb, gated_cols, EPI_SILU_F32, cols=41)
-            partly = np.where(np.arange(2 * rows_w) < 41, full / (1.0 + np.exp(-full)), full)
-            checks = {"store": bad(stored, full, rounded), "store_f32": bad(scores, full), "add_f32": bad(added, full + 0.25),
-                      "swiglu": bad(gated, gate / (1.0 + np.exp(-gate)) * up, rounded), "relu2": bad(squared, np.maximum(full, 0.0) ** 2, rounded),
-                      "xielu": bad(curved, curve, rounded), "silu_f32": bad(gated_cols, partly)}
-            wrong = [k for k, v in checks.items() if v]
-            if wrong:
-                raise KernelError(f"self-check: the {name} product with {n} row(s) is wrong for the epilogue(s) {wrong} on a "
-                                  f"{rows_w} x {cols} weight; this device or this build of the kernels cannot be trusted")
-    x = (((np.arange(3 * cols) * 31 % 97).astype(np.float32) - 48.0) / 50.0).reshape(3, cols)
-    scores = torch.empty((3, 2 * rows_w), dtype=torch.float32, device=device)
-    gemm_simt(torch.from_numpy(x).to(device), torch.from_numpy(w).to(device), scores, EPI_STORE_F32)
-    if bad(scores, x.astype(np.float64) @ w.astype(np.float64).T):
-        raise KernelError("self-check: the float32 CUDA-core product is wrong; this device or this build of the kernels cannot be trusted")
+            check(name, product, on_device(inputs(n, 512), torch.bfloat16), on_device(w, torch.bfloat16))
+    check("float32 CUDA-core", gemm_simt, on_device(inputs(3, 512)), on_device(w))
+    for n in (3, 130):
+        check("float32 tensor-core", gemm_simt, on_device(inputs(n, 1028)), on_device(long_w), rel=2e-5)
     torch.cuda.synchronize(device)
     check_status(device)
     _self_checked.add(index)

@@ -93,3 +93,26 @@ def test_the_start_up_check_passes_and_catches_a_wrong_product(monkeypatch):
         ops.self_check(dev)
     monkeypatch.undo()
     ops.self_check(dev)
+
+
+@pytest.mark.parametrize("rows", [3, 130])
+@pytest.mark.parametrize("lost", ["middle", "low"])
+def test_the_start_up_check_sees_the_float32_product(monkeypatch, rows, lost):
+    """A float32 product of long sums that drops a part of its operands, as a product of fewer bfloat16 parts would, is not trusted."""
+    from borrowed_compute_b200 import ops
+
+    dev = torch.device("cuda:0")
+    real = ops.gemm_simt
+
+    def without_a_part(x, w, out, epilogue, **numbers):
+        if x.dtype == torch.float32 and x.shape[1] > 512 and x.shape[0] == rows:
+            bits = 16 if lost == "middle" else 8
+            x = (x.contiguous().view(torch.int32) >> bits << bits).view(torch.float32)
+        real(x, w, out, epilogue, **numbers)
+
+    ops._self_checked.discard(0)
+    monkeypatch.setattr(ops, "gemm_simt", without_a_part)
+    with pytest.raises(ops.KernelError, match=f"self-check: the float32 tensor-core product with {rows} row"):
+        ops.self_check(dev)
+    monkeypatch.undo()
+    ops.self_check(dev)
