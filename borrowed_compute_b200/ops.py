@@ -375,10 +375,10 @@ def _split_scratch(M: int, K: int) -> int:
 
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, act: Optional[Tuple[float, float]] = None,
-              cols: Optional[int] = None) -> None:
+              cols: Optional[int] = None, cores: bool = False) -> None:
     """out = x @ w.T with float accumulation, k ascending in one piece or in up to eight that are added in order: on the CUDA cores, or,
-    for float32 sums of more than 512 products, on the tensor cores with every operand whole, as three bfloat16 parts (csrc/gemm_split.cu).
-    Both operands are read after the kernels before this launch have ended.
+    for float32 sums of more than 512 products, on the tensor cores with every operand whole, as three bfloat16 parts (csrc/gemm_split.cu);
+    ``cores``: on the CUDA cores whatever the sizes, that kernel's checked twin.  Both operands are read after the kernels before this launch have ended.
     EPI_STORE: out in x's type; EPI_STORE_F32: float32; EPI_ADD_F32: out += (float32);
     EPI_SWIGLU: w stacks gate rows on up rows, out[:, j] = silu(g_j) * u_j in x's type;
     EPI_RELU2: out = max(sum, 0)^2 in x's type, squared in float and rounded once;
@@ -395,7 +395,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int
     if tuple(out.shape) != (M, N):
         raise KernelError(f"gemm: out is {tuple(out.shape)}, wanted {(M, N)}")
     numbers = _act_numbers("gemm_simt", epilogue, act, cols)
-    if x.dtype == torch.float32 and K > 512 and _fn("bc_gemm_split_takes")(_ptr(x), _ptr(w), _c_int(n_w), _c_int(K)):
+    if x.dtype == torch.float32 and K > 512 and not cores and _fn("bc_gemm_split_takes")(_ptr(x), _ptr(w), _c_int(n_w), _c_int(K)):
         a, b, n_cols = numbers or (0.0, 0.0, 0)
         scratch = None
         if M <= SPLIT_FEW:

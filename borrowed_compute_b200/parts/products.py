@@ -3,8 +3,8 @@
 ``linear(x, w, out, epilogue)`` computes ``x @ w.T`` with float accumulation.  On the
 32-bit path ``ops.gemm_simt`` chooses: every operand whole as three bfloat16 parts on the tensor
 cores, or, for short sums, the CUDA-core kernel; never tf32.  For
-bfloat16 it is the tcgen05 tensor-core kernel; the CUDA-core kernel on the same operands is
-its checked twin and can be forced for a test with ``force_simt``.
+bfloat16 it is the tcgen05 tensor-core kernel.  The CUDA-core kernel on the same operands is
+the checked twin of both and can be forced for a test with ``force_simt``.
 """
 
 from __future__ import annotations
@@ -38,4 +38,4 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, w
     elif glu is not None:
         raise ops.KernelError("a bounded gate in the epilogue comes with the tensor-core product")
     else:
-        ops.gemm_simt(x, w, out, epilogue, act=act, cols=cols)
+        ops.gemm_simt(x, w, out, epilogue, act=act, cols=cols, cores=force_simt)

@@ -1,4 +1,4 @@
-"""The CUDA-core product where its kernels change over: short sums of few outputs, tiles of 16 and of 64 rows, sums over K in one
+"""The CUDA-core product (``cores``: also where float32 sums go to the tensor cores by themselves) where its kernels change over: short sums of few outputs, tiles of 16 and of 64 rows, sums over K in one
 piece and in clusters of two to eight, widths with and without 16-byte loads.
 
 Tolerance: a float sum of K products in any order is off by at most K 2^-24 sum |x w| (plus the roundings of what follows it)."""
@@ -28,15 +28,15 @@ def test_products_around_the_edges_of_their_kernels(dtype, M, N, K):
     full, bound = x.double() @ w.double().T, (K + 4) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     wn = w[:N].contiguous()
     out = torch.full((M, N), float("nan"), device="cuda")
-    ops.gemm_simt(x, wn, out, ops.EPI_STORE_F32)
+    ops.gemm_simt(x, wn, out, ops.EPI_STORE_F32, cores=True)
     assert ((out.double() - full[:, :N]).abs() <= bound[:, :N]).all()
     base = torch.randn(M, N, generator=g, device="cuda")
     acc = base.clone()
-    ops.gemm_simt(x, wn, acc, ops.EPI_ADD_F32)
+    ops.gemm_simt(x, wn, acc, ops.EPI_ADD_F32, cores=True)
     ref = base.double() + full[:, :N]
     assert ((acc.double() - ref).abs() <= bound[:, :N] + 2.0 ** -23 * ref.abs()).all()
     glu = torch.empty((M, N), dtype=dtype, device="cuda")
-    ops.gemm_simt(x, w, glu, ops.EPI_SWIGLU)
+    ops.gemm_simt(x, w, glu, ops.EPI_SWIGLU, cores=True)
     gate, up = full[:, :N], full[:, N:]
     act = gate * torch.sigmoid(gate)
     unit = 2.0 ** -21 if dtype == torch.float32 else 2.0 ** -8                                 # the quotient's few roundings, or bf16's one
@@ -46,25 +46,25 @@ def test_products_around_the_edges_of_their_kernels(dtype, M, N, K):
     # A row alone, and a few of them, give the bits that they give among all.
     for rows in (slice(M - 1, M), slice(0, min(M, 20)), slice(0, min(M, 60))):
         few = torch.empty((rows.stop - rows.start, N), device="cuda")
-        ops.gemm_simt(x[rows].contiguous(), wn, few, ops.EPI_STORE_F32)
+        ops.gemm_simt(x[rows].contiguous(), wn, few, ops.EPI_STORE_F32, cores=True)
         assert torch.equal(few, out[rows])
 
 
 def test_an_infinity_stays_in_its_row():
     from borrowed_compute_b200 import ops
 
-    for M, N, K in ((5, 33, 70), (40, 140, 1030), (70, 140, 520)):
+    for M, N, K in ((5, 33, 70), (40, 140, 1030), (70, 140, 520), (5, 140, 1032)):
         x, w = torch.ones((M, K), device="cuda"), torch.ones((N, K), device="cuda")
         x[2, K - 1], x[3, 0] = float("inf"), float("nan")
         out = torch.empty((M, N), device="cuda")
-        ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+        ops.gemm_simt(x, w, out, ops.EPI_STORE_F32, cores=True)
         assert torch.isinf(out[2]).all() and torch.isnan(out[3]).all()
         assert (out[[0, 1, 4]] == K).all() and np.isfinite(out[4:].cpu().numpy()).all()
 
 
 @pytest.mark.parametrize("epilogue", ["store", "glu"])
-@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (16, 512, 512), (70, 130, 520)])
-def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K, epilogue):
+@pytest.mark.parametrize("M,N,K,cores", [(1, 64, 64, True), (16, 512, 512, True), (70, 130, 520, True), (70, 130, 520, False), (130, 130, 1032, False)])
+def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K, cores, epilogue):
     """Kernels may start while the one before still runs; no operand is read before that one's end.  Sums of ones: exact."""
     from borrowed_compute_b200 import ops
 
@@ -73,7 +73,7 @@ def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K, epilogue):
     outs = [torch.empty((M, N), device="cuda") for _ in range(12)]
     for out in outs:
         ops.scale_scores(w, 2.0)
-        ops.gemm_simt(x, w, out, ops.EPI_SWIGLU if glu else ops.EPI_STORE_F32)
+        ops.gemm_simt(x, w, out, ops.EPI_SWIGLU if glu else ops.EPI_STORE_F32, cores=cores)
     for i, out in enumerate(outs):
         s = K * 2.0 ** (i + 1 - 10)
         want = s * s / (1.0 + np.exp(-s)) if glu else s
