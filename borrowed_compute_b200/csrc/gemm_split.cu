@@ -1,20 +1,23 @@
 // The true 32-bit matrix product on the tensor cores: Y[m, n] = sum_k X[m, k] W[n, k] for float operands, every operand taken whole.
 //
 // A float's 24 bits are three bfloat16 numbers: h, its first 8 bits (truncated, so that no finite number becomes an infinity), m, the
-// next, rounded, and l, what is left, exactly.  Of the nine products of two such triples six are summed: h h, h m, m h, m m, h l, l h; the
-// others lie below 2^-22 of the whole product.  The products are exact and the tensor core adds them in float, but it truncates: sums
+// next, rounded, and l, what is left, exactly.  Of the nine products of two such triples all but l l are summed, which lies below 2^-32 of the
+// whole product.  (Without m l and l m, 2^-22 together, sums of one or a few products were further from 64 bits than a multiply-add; with them the tensor
+// core's time is still hidden, a feed-forward of 300 rows 270 us against 267.)
+// The products are exact and the tensor core adds them in float, but it truncates: sums
 // of h h alone (the accumulator D1) are therefore taken out of tensor memory every 64 k and added up in registers, rounded, in ascending
-// order; the five smaller products, at most 2^-7 of the first, go into an accumulator of their own (D2) that stays until the end.
-// Measured against 64 bits (2-norm of the error over that of the result, normal operands): 300 x 8,192 x 2,048 1.7e-7, one multiply-add after another
-// (gemm_simt.cu) 8.1e-7; 300 x 2,048 x 8,192 in eight pieces 1.4e-7 and 5.8e-7; 3 x 2,816 x 1,024 1.1e-7 and 4.0e-7.
+// order; the seven smaller products, at most 2^-6 of the first, go into an accumulator of their own (D2) that stays until the end.
+// Measured against 64 bits (2-norm of the error over that of the result, normal operands): 130 x 2,048 x 12,416 1.9e-7, one multiply-add after another
+// (gemm_simt.cu) 8.1e-7; 130 x 8,192 x 128 in eight pieces 1.4e-7 and 5.7e-7; 7 x 1,024 x 128 1.1e-7 and 4.2e-7; rows with one number 2.5e-8 and 2.5e-8, with
+// two 3.4e-8 and 3.5e-8.
 // Operands below 2^-110 lose their last bits (bfloat16 ends at 2^-133).
 // An operand that is infinite or not a number has no m and l: where the sum of h h is either, it is the result by itself.
 //
 // Two ways, the same sums in the same order and so the same bits:
 //
 //   rows   Every block splits its weights, into tensor memory (the MMA's A operand, so that shared memory is free for the other), and its tokens, into
-//          shared memory.  What bounds it: six tensor-core products a multiply-add, 32 k (a chunk) of 128 weight rows by N tokens in some 1,000 clocks of an SM
-//          at N 112, and the rounds of wait, split, store and fence of its warps, 1,425 clocks a chunk.
+//          shared memory.  What bounds it: eight tensor-core products a multiply-add (six: 32 k, a chunk, of 128 weight rows by N tokens in some 1,000 clocks of an SM
+//          at N 112), and the rounds of wait, split, store and fence of its warps, 1,425 clocks a chunk.
 //   few    Up to a tile of rows, where weights are what there is to read: a kernel splits the tokens once, into planes of bfloat16 in scratch memory; they
 //          come by TMA as they are multiplied and all sixteen warps split weights.  742 clocks a chunk at one token, most of them the weights' way from memory.
 //          With more rows the planes' six bytes instead of four a value through the L2, in every block, cost more than the splits: 300 rows of 16,384 x 2,048
@@ -270,6 +273,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     mma_bf16_a_tmem(tmem + SPL_D2, a + 16, m, idesc, 1);
                     mma_bf16_a_tmem(tmem + SPL_D2, a + 32, h, idesc, 1);
                     mma_bf16_a_tmem(tmem + SPL_D2, a, l, idesc, 1);
+                    mma_bf16_a_tmem(tmem + SPL_D2, a + 32, m, idesc, 1);
+                    mma_bf16_a_tmem(tmem + SPL_D2, a + 16, l, idesc, 1);
                 }
                 mma_commit(done + 8 * (j & 3));
                 if ((j & 1) || j + 1 == chunks) mma_commit(d1_full + 8 * b);
@@ -473,6 +478,8 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     mma_bf16_a_tmem(tmem + d2_at, a + 16, m, idesc, 1);
                     mma_bf16_a_tmem(tmem + d2_at, a + 32, h, idesc, 1);
                     mma_bf16_a_tmem(tmem + d2_at, a, l, idesc, 1);
+                    mma_bf16_a_tmem(tmem + d2_at, a + 32, m, idesc, 1);
+                    mma_bf16_a_tmem(tmem + d2_at, a + 16, l, idesc, 1);
                 }
                 mma_commit(done + 8 * (j & 3));
                 if (last) {
