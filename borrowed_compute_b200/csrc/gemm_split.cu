@@ -10,8 +10,10 @@
 // Measured against 64 bits (2-norm of the error over that of the result, normal operands): 130 x 2,048 x 12,416 1.9e-7, one multiply-add after another
 // (gemm_simt.cu) 8.1e-7; 130 x 8,192 x 128 in eight pieces 1.4e-7 and 5.7e-7; 7 x 1,024 x 128 1.1e-7 and 4.2e-7; rows with one number 2.5e-8 and 2.5e-8, with
 // two 3.4e-8 and 3.5e-8.
-// Operands below 2^-110 lose their last bits (bfloat16 ends at 2^-133).
-// An operand that is infinite or not a number has no m and l: where the sum of h h is either, it is the result by itself.
+// What is left after h and m is l only down to bfloat16's last bit, 2^-133: floats below 2^-110 may have bits past it, and an infinity or a not-a-number has
+// no parts at all.  Every row in which a block meets one (the bits that l drops are collected on the way, an instruction for two floats) is remembered, and
+// that block's sums of it are taken anew, one multiply-add after another from the operands themselves (split_redo): slow, but whole.
+// (The collecting costs that feed-forward 275 us against 270; a row taken anew of its 300 some 50 us more, a row of a single one 1.4 to 1.8 times its time.)
 //
 // Two ways, the same sums in the same order and so the same bits:
 //
@@ -58,12 +60,15 @@ struct SplitParams {
     int M, N, K;
     int second_row;              // SwiGLU: the matrix row where the up rows start
     int bn, stages, x_stages, piece;
+    const float *X, *W;          // the operands themselves
+    const int* lost;             // the second way: [row][slice], whether three parts do not hold one of that slice's floats; slices a row and a piece of K
+    int row_slices, piece_slices;
     float act_a, act_b;
     int act_cols;
 };
 
-// Four floats as triples of bfloat16, two to a register.
-__device__ __forceinline__ void split4(const float4 v, uint32_t* h, uint32_t* m, uint32_t* l) {
+// Four floats as triples of bfloat16, two to a register.  The last 16 bits of `lost` collect what the third parts drop: zero where they are exact.
+__device__ __forceinline__ void split4(const float4 v, uint32_t* h, uint32_t* m, uint32_t* l, uint32_t& lost) {
     const uint64_t minus = pack_f32x2(-1.0f, -1.0f);
     auto two = [&](float a, float b, uint32_t& h2, uint32_t& m2, uint32_t& l2) {
         asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(h2) : "f"(b), "f"(a));
@@ -73,24 +78,58 @@ __device__ __forceinline__ void split4(const float4 v, uint32_t* h, uint32_t* m,
         m2 = pack_bf16(r0, r1);
         unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(m2 << 16), __uint_as_float(m2 & 0xffff0000u)), minus, rest), r0, r1);
         l2 = pack_bf16(r0, r1);
+        lost |= __float_as_uint(r0) | __float_as_uint(r1);
     };
     two(v.x, v.y, h[0], m[0], l[0]);
     two(v.z, v.w, h[1], m[1], l[1]);
 }
 
+// This block's sums of the rows (bits of lost: four words of weight rows, four of tokens) whose floats three parts do not hold, a warp a sum.
+template <int EPI>
+__device__ __noinline__ void split_redo(const SplitParams& p, float* tile, const uint32_t* lost, int t0, int n0) {
+    constexpr int HALF_N = TC_BM / 2;
+    const float *X = p.X, *W = p.W;
+    PDL_FRESH(X); PDL_FRESH(W);
+    const int lane = threadIdx.x & 31, rows = min(p.bn, p.M - t0);
+    const int k_begin = blockIdx.z * p.piece, k_end = min(p.K, k_begin + p.piece);
+    const bool weights = lost[0] | lost[1] | lost[2] | lost[3];
+    for (int r = 0; r < rows; r++) {
+        const bool all = lost[4 + (r >> 5)] >> (r & 31) & 1;
+        if (!all && !weights) continue;
+        const float* x = X + (size_t)(t0 + r) * p.K;
+        for (int c = threadIdx.x >> 5; c < TC_BM; c += SPL_THREADS / 32) {
+            const int n = n0 + (EPI == EPI_SWIGLU ? c % HALF_N : c);
+            if (n >= p.N || !(all || (lost[c >> 5] >> (c & 31) & 1))) continue;
+            const float* w = W + ((size_t)(EPI == EPI_SWIGLU && c >= HALF_N ? p.second_row : 0) + n) * p.K;
+            float sum = 0.0f;
+#pragma unroll 4
+            for (int k = k_begin + 4 * lane; k < k_end; k += 128) {
+                const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+                sum = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum))));
+            }
+            sum = warp_sum(sum);
+            if (lane == 0) tile[r * TC_BM + c] = sum;
+        }
+    }
+}
+
 // The end of both: the sums of the pieces of K, in ascending order out of the cluster's blocks, and the epilogue.
 template <int EPI>
-__device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, const int* gave_up, int t0, int n0) {
+__device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, const int* gave_up, const uint32_t* lost, int t0, int n0) {
     constexpr int HALF_N = TC_BM / 2, OUT_COLS = EPI == EPI_SWIGLU ? HALF_N : TC_BM;
     const int S = gridDim.z;
     __syncwarp();
     tc_fence_before();
-    if (S > 1) cg::this_cluster().sync();
-    else __syncthreads();
+    __syncthreads();
     if (dealloc) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
+    const uint4 of_w = *reinterpret_cast<const uint4*>(lost), of_x = *reinterpret_cast<const uint4*>(lost + 4);
+    const bool redo = (of_w.x | of_w.y | of_w.z | of_w.w | of_x.x | of_x.y | of_x.z | of_x.w) && !*reinterpret_cast<const volatile int*>(gave_up);
+    if (redo) split_redo<EPI>(p, tile, lost, t0, n0);
+    if (S > 1) cg::this_cluster().sync();
+    else if (redo) __syncthreads();
     if (!*reinterpret_cast<const volatile int*>(gave_up)) {
         const int rows = min(p.bn, p.M - t0);
         for (int e = blockIdx.z * SPL_THREADS + threadIdx.x; e < rows * OUT_COLS; e += S * SPL_THREADS) {
@@ -112,13 +151,14 @@ __device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, 
 // swizzle); 17 issues the products.
 template <int EPI>
 __global__ void __launch_bounds__(SPL_THREADS, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SplitParams p) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitParams p) {
     constexpr int HALF_N = TC_BM / 2, OUT_COLS = EPI == EPI_SWIGLU ? HALF_N : TC_BM;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * SPL_STAGES + 4 + 4 + 2 + 2];
     __shared__ uint32_t tmem_slot;
     __shared__ int gave_up;
+    __shared__ __align__(16) uint32_t lost[8];      // rows whose floats three parts do not hold, a bit each: weight rows, tokens
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int bn = p.bn, stages = p.stages;
     const int plane = bn * 128, stage_bytes = SPL_W_BYTES + plane;      // a plane: bn rows of 64 k of one part; two stages of three planes behind the raw ring
@@ -128,6 +168,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int chunks = (k_end - k_begin + SPL_K - 1) / SPL_K, periods = (chunks + 1) / 2;
     const uint32_t raw_full = smem_u32(bars), raw_empty = raw_full + 8 * SPL_STAGES, ready = raw_empty + 8 * SPL_STAGES, done = ready + 32, d1_full = done + 32,
                    d1_empty = d1_full + 16;
+    if (threadIdx.x < 8) lost[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         gave_up = 0;
         for (int s = 0; s < stages; s++) {
@@ -161,6 +202,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int row = 32 * (warp & 3) + lane;
         const uint32_t a_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + SPL_A;
         const int back = weights ? 2 : 4;
+        uint32_t dropped = 0;
         for (int j = 0, s = 0, round = 0; j < chunks; j++) {
             if (!wait(raw_full + 8 * s, round, 1)) break;
             const uint8_t* src = smem + (size_t)s * stage_bytes + (weights ? 0 : SPL_W_BYTES) + row * 128;
@@ -170,7 +212,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (int c = 0; c < 8; c++) v[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
 #pragma unroll
-                for (int c = 0; c < 8; c++) split4(v[c], h + 2 * c, m + 2 * c, l + 2 * c);
+                for (int c = 0; c < 8; c++) split4(v[c], h + 2 * c, m + 2 * c, l + 2 * c, dropped);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(raw_empty + 8 * s);
@@ -199,6 +241,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             mbar_arrive(ready + 8 * (j & 3));
         }
+        const uint32_t rows = __ballot_sync(0xffffffffu, dropped & 0xffffu);
+        if (lane == 0) lost[warp] = rows;
     } else if (warp < 16) {
         // Two warps a quarter of the lanes: every other sixteen of the token columns each.
         const int q = warp & 3, half = (warp - 8) >> 2;
@@ -234,8 +278,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     float a0, a1;
                     unpack_f32x2(acc[c][e], a0, a1);
                     float* to = tile + (32 * c + 16 * half + 2 * e) * TC_BM + 32 * q + lane;
-                    to[0] = fabsf(a0) < INFINITY ? a0 + __uint_as_float(v[2 * e]) : a0;
-                    to[TC_BM] = fabsf(a1) < INFINITY ? a1 + __uint_as_float(v[2 * e + 1]) : a1;
+                    to[0] = a0 + __uint_as_float(v[2 * e]);
+                    to[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
                 }
             }
         }
@@ -283,38 +327,43 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
     }
     if (!ok) *reinterpret_cast<volatile int*>(&gave_up) = 1;
-    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, t0, n0);
+    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, lost, t0, n0);
 }
 
-// planes[part][row][k_row] = the parts of x[row][k], four k a thread.
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* x, bf16* __restrict__ planes, int rows, int K, int k_row) {
+// planes[part][row][k_row] = the parts of x[row][k], four k a thread; lost[row][slice]: whether they do not hold one of the slice's floats.  Block (x, y): row y's
+// slice x, of at most SPL_SLICE k of one piece.
+#define SPL_SLICE 1024
+__global__ void __launch_bounds__(SPL_SLICE / 4) split_rows_kernel(const float* x, bf16* __restrict__ planes, int* __restrict__ lost, int rows, int K, int k_row, int piece, int piece_slices) {
     pdl_wait();                        // before the next kernel may start: it reads its weights at once
     pdl_launch_dependents();
     PDL_FRESH(x);
-    const int quads = K / 4;
     const size_t part = (size_t)rows * k_row;
-    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < (long long)rows * quads; i += 256ll * gridDim.x) {
-        const int r = (int)(i / quads), k = 4 * (int)(i - (long long)r * quads);
+    const int r = blockIdx.y, begin = blockIdx.x / piece_slices * piece, k = begin + blockIdx.x % piece_slices * SPL_SLICE + 4 * threadIdx.x;
+    uint32_t dropped = 0;
+    if (k < min(K, begin + piece)) {
         uint32_t h[2], m[2], l[2];
-        split4(*reinterpret_cast<const float4*>(x + (size_t)r * K + k), h, m, l);
+        split4(*reinterpret_cast<const float4*>(x + (size_t)r * K + k), h, m, l, dropped);
         bf16* to = planes + (size_t)r * k_row + k;
         *reinterpret_cast<uint2*>(to) = make_uint2(h[0], h[1]);
         *reinterpret_cast<uint2*>(to + part) = make_uint2(m[0], m[1]);
         *reinterpret_cast<uint2*>(to + 2 * part) = make_uint2(l[0], l[1]);
     }
+    const int any = __syncthreads_or(dropped & 0xffffu);
+    if (threadIdx.x == 0) lost[(size_t)r * gridDim.x + blockIdx.x] = any;
 }
 
 // Warps: 0-15 split the weights of every fourth chunk, four warps a chunk, a row a thread, and take D1 out, a share of the columns each; 16 asks for tiles; 17
 // issues the products.
 template <int EPI>
 __global__ void __launch_bounds__(SPL_THREADS, 1)
-gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SplitParams p) {
+gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SplitParams p) {
     constexpr int HALF_N = TC_BM / 2;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * SPL_STAGES + 2 * SPL_X_STAGES + 4 + 4 + 2 + 2];
     __shared__ uint32_t tmem_slot;
     __shared__ int gave_up;
+    __shared__ __align__(16) uint32_t lost[8];      // rows whose floats three parts do not hold, a bit each: weight rows, tokens
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int bn = p.bn, stages = p.stages, x_stages = p.x_stages;
     const int buffers = split_buffers(bn), d2_at = 2 * bn, a_at = 3 * bn;
@@ -325,6 +374,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int chunks = (k_end - k_begin + SPL_K - 1) / SPL_K, periods = (chunks + 1) / 2;
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * SPL_STAGES, x_full = w_empty + 8 * SPL_STAGES, x_empty = x_full + 8 * SPL_X_STAGES,
                    ready = x_empty + 8 * SPL_X_STAGES, done = ready + 32, d1_full = done + 32, d1_empty = d1_full + 16;
+    if (threadIdx.x < 8) lost[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         gave_up = 0;
         for (int i = 0; i < SPL_STAGES; i++) {
@@ -361,6 +411,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int row = 32 * q + lane;
         const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16);
         uint64_t acc[2][8] = {};                             // token columns 16 part .. and 64 + 16 part ..
+        uint32_t dropped = 0;
         int taken = 0;
         auto take_out_before = [&](int end) {
             for (; taken < end; taken++) {
@@ -389,7 +440,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 #pragma unroll
             for (int c = 0; c < 8; c++) v[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
 #pragma unroll
-            for (int c = 0; c < 8; c++) split4(v[c], h + 2 * c, m + 2 * c, l + 2 * c);
+            for (int c = 0; c < 8; c++) split4(v[c], h + 2 * c, m + 2 * c, l + 2 * c, dropped);
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * s);
             if ((s += 4) >= stages) s -= stages, round++;
@@ -407,6 +458,8 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             take_out_before(j / 2);       // all but the stretch under way: the products of the next one but one wait for this one's sums
             if (!ok) break;
         }
+        const uint32_t rows = __ballot_sync(0xffffffffu, dropped & 0xffffu);
+        if (lane == 0 && rows) atomicOr(&lost[q], rows);     // (four warps a quarter)
         if (ok) take_out_before(periods);
         if (ok) {
             // D1's last sums came after the last product, D2's with them.  No tile is on its way and none is read any more.
@@ -421,8 +474,8 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     float a0, a1;
                     unpack_f32x2(acc[c][e], a0, a1);
                     float* to = tile + (64 * c + 16 * part + 2 * e) * TC_BM + 32 * q + lane;
-                    to[0] = fabsf(a0) < INFINITY ? a0 + __uint_as_float(v[2 * e]) : a0;
-                    to[TC_BM] = fabsf(a1) < INFINITY ? a1 + __uint_as_float(v[2 * e + 1]) : a1;
+                    to[0] = a0 + __uint_as_float(v[2 * e]);
+                    to[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
                 }
             }
         }
@@ -453,6 +506,19 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
                 if (++s == stages) s = 0, round++;
             }
+        }
+        __syncwarp();
+        // The last tiles are on their way: time to look which of the tokens' rows need their sums anew.
+        pdl_wait();
+        const int* flags = p.lost;
+        PDL_FRESH(flags);
+        for (int i = 0; 32 * i < bn; i++) {
+            const int r = t0 + 32 * i + lane;
+            int any = 0;
+            if (r < p.M)
+                for (int c = 0; c < p.piece_slices; c++) any |= flags[(size_t)r * p.row_slices + blockIdx.z * p.piece_slices + c];
+            const uint32_t rows = __ballot_sync(0xffffffffu, any);
+            if (lane == 0) lost[4 + i] = rows;
         }
     } else {
         const uint32_t idesc = instr_desc(bn);
@@ -494,7 +560,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
     pdl_wait();       // the output may still be in use by a kernel before
     if (!ok) *reinterpret_cast<volatile int*>(&gave_up) = 1;
-    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, t0, n0);
+    split_finish<EPI>(p, tile, tmem, warp == 17, &gave_up, lost, t0, n0);
 }
 
 // -------------------------------------------------------------------------------- the host
@@ -538,8 +604,8 @@ extern "C" int bc_gemm_split_takes(const void* X, const void* W, int cols, int K
 }
 
 static int split_k_row(int K) { return (K + 7) / 8 * 8; }
-// Bytes of scratch: three planes of the rows that go the second way.
-extern "C" long long bc_gemm_split_scratch(int M, int K) { return M <= SPL_FEW ? 6ll * M * split_k_row(K) : 0; }
+// Bytes of scratch: three planes of the rows that go the second way, and a word a row and slice of K (the pieces' slices, at most K / SPL_SLICE and ten more).
+extern "C" long long bc_gemm_split_scratch(int M, int K) { return M <= SPL_FEW ? 6ll * M * split_k_row(K) + 4ll * M * (K / SPL_SLICE + 10) : 0; }
 
 template <int EPI>
 static int launch(const void* X, const void* W, void* out, int M, int N, int K, float a, float b, int cols, void* scratch, cudaStream_t s) {
@@ -551,6 +617,10 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
     p.bn = ((M + t_tiles - 1) / t_tiles + 15) / 16 * 16;
     const int splits = split_pieces(w_rows, K);
     p.piece = ((K + splits - 1) / splits + 2 * SPL_K - 1) / (2 * SPL_K) * (2 * SPL_K);
+    p.X = (const float*)X, p.W = (const float*)W;
+    p.piece_slices = (p.piece + SPL_SLICE - 1) / SPL_SLICE, p.row_slices = splits * p.piece_slices;
+    int* lost = few ? (int*)((char*)scratch + 6ll * M * split_k_row(K)) : nullptr;
+    p.lost = lost;
     // A ring of chunks, both operands' raw tiles or the weights' alone, and stages of 64 k of the tokens' planes.
     p.x_stages = !few || p.bn > 64 ? 2 : SPL_X_STAGES;
     const int stage = SPL_W_BYTES + (few ? 0 : p.bn * 128), planes = p.x_stages * 3 * p.bn * 128;
@@ -562,10 +632,8 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
     if (st == BC_OK) st = few ? planes_map(&mx, scratch, M, K, split_k_row(K), p.bn) : float_map(&mx, X, M, K, p.bn);
     if (st != BC_OK) return st;
     cudaError_t e = few ? bc_allow_shared<gemm_split_few_kernel<EPI>>(TC_SMEM_LIMIT) : bc_allow_shared<gemm_split_kernel<EPI>>(TC_SMEM_LIMIT);
-    if (e == cudaSuccess && few) {
-        const int quads = M * (K / 4), most = 8 * bc_sm_count();
-        e = bc_launch(split_rows_kernel, dim3((quads + 255) / 256 < most ? (quads + 255) / 256 : most), dim3(256), 0, s, (const float*)X, (bf16*)scratch, M, K, split_k_row(K));
-    }
+    if (e == cudaSuccess && few)
+        e = bc_launch(split_rows_kernel, dim3(p.row_slices, M), dim3(SPL_SLICE / 4), 0, s, (const float*)X, (bf16*)scratch, lost, M, K, split_k_row(K), p.piece, p.piece_slices);
     // Token tiles fastest: the blocks that read the same weights run side by side.
     const dim3 grid((M + p.bn - 1) / p.bn, (N + out_cols - 1) / out_cols, splits);
     auto go = [&](auto kernel) {

@@ -111,6 +111,49 @@ def test_numbers_at_the_ends_of_the_range():
     assert got.isnan().all()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 70, 1028), (40, 130, 516), (112, 64, 2100), (113, 130, 1028), (300, 64, 2100)])
+@pytest.mark.parametrize("of_x,of_w", [(-108, 90), (-115, 100), (-125, 100), (-135, 110), (-147, 120), (110, -135), (100, -115), (-60, -60), (-70, -65), (-75, -70)])
+def test_small_floats_are_whole(M, N, K, of_x, of_w):
+    """Floats whose last bits bfloat16 does not reach, subnormal ones among them, and results down to the last bit of a float."""
+    from borrowed_compute_b200 import ops
+
+    x, w = operands(M, N, K, 3)
+    x, w = x * 2.0 ** of_x, w * K ** 0.5 * 2.0 ** of_w
+    out = torch.empty((M, N), device="cuda")
+    ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+    full, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # Eight products of sixteen k and two additions a stretch may each drop what lies below 2^-149.
+    assert ((out.double() - full).abs() <= bound(K) * size + (K / 2 + K / 32 + 8) * 2.0 ** -149).all()
+    few = torch.empty((1, N), device="cuda")
+    ops.gemm_simt(x[M - 1:].contiguous(), w, few, ops.EPI_STORE_F32)
+    assert torch.equal(few, out[M - 1:])
+
+
+@pytest.mark.parametrize("M", [40, 130])
+def test_rows_with_small_floats_leave_the_others_alone(M):
+    from borrowed_compute_b200 import ops
+
+    N, K, inf = 200, 1032, float("inf")
+    x, w = operands(M, N, K, 4)
+    plain, gated = torch.empty((M, N), device="cuda"), torch.empty((M, N // 2), device="cuda")
+    ops.gemm_simt(x, w, plain, ops.EPI_STORE_F32)
+    x[3, 5], x[M - 1, K - 1], w[7, 600], w[150, 0] = 2.0 ** -149, 2.0 ** -120 * (1 + 2.0 ** -23), 2.0 ** -130 * 1.9, -2.0 ** -140
+    x[9, 600], x[11, 2] = inf, inf
+    w[8, 2], w[20, 2], w[21, 2], w[21, 1] = 2.0 ** -148, -2.0 ** -148, 0.0, 1.0
+    out = torch.empty((M, N), device="cuda")
+    ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+    rows, cols = [m for m in range(M) if m not in (3, 9, 11, M - 1)], [n for n in range(N) if n not in (7, 8, 20, 21, 150)]
+    assert torch.equal(out[rows][:, cols], plain[rows][:, cols])
+    full, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    near = (out.double() - full).abs() <= bound(K) * size
+    assert (near | (out.double() == full) | (out.isnan() & full.isnan())).all()      # an infinity times a small float is one, times zero it is no number
+    assert out[9, 7] == inf and out[11, 8] == inf and out[11, 20] == -inf and out[11, 21].isnan()
+    ops.gemm_simt(x, w, gated, ops.EPI_SWIGLU)
+    up = full[:, N // 2:]
+    want = full[:, :N // 2] * torch.sigmoid(full[:, :N // 2]) * up
+    assert (((gated.double() - want).abs() <= 2.0 ** -14 * (1 + size[:, :N // 2]) * (1 + up.abs())) | (gated.double() == want) | (gated.isnan() & want.isnan())).all()
+
+
 def test_operands_that_tensor_copies_cannot_take_go_the_other_way():
     """K no multiple of four, or operands off their 16 bytes: the CUDA-core kernel, as before."""
     from borrowed_compute_b200 import ops
