@@ -1,17 +1,20 @@
 // The true 32-bit matrix product on the tensor cores: Y[m, n] = sum_k X[m, k] W[n, k] for float operands, every operand taken whole.
 //
-// A float's 24 bits are three bfloat16 numbers: h, its first 8 bits (truncated, so that no finite number becomes an infinity), m, the
-// next, rounded, and l, what is left, exactly.  Of the nine products of two such triples all but l l are summed, which lies below 2^-32 of the
+// A float's 24 bits are three bfloat16 numbers: h, the nearest of 8 bits, m, the nearest to what is left, and l, the rest, exactly.
+// Of the nine products of two such triples all but l l are summed, which lies below 2^-33 of the
 // whole product.  (Without m l and l m, 2^-22 together, sums of one or a few products were further from 64 bits than a multiply-add; with them the tensor
 // core's time is still hidden, a feed-forward of 300 rows 270 us against 267.)
 // The products are exact and the tensor core adds them in float, but it truncates: sums
 // of h h alone (the accumulator D1) are therefore taken out of tensor memory every 64 k and added up in registers, rounded, in ascending
-// order; the seven smaller products, at most 2^-6 of the first, go into an accumulator of their own (D2) that stays until the end.
-// Measured against 64 bits (2-norm of the error over that of the result, normal operands): 130 x 2,048 x 12,416 1.9e-7, one multiply-add after another
-// (gemm_simt.cu) 8.1e-7; 130 x 8,192 x 128 in eight pieces 1.4e-7 and 5.7e-7; 7 x 1,024 x 128 1.1e-7 and 4.2e-7; rows with one number 2.5e-8 and 2.5e-8, with
-// two 3.4e-8 and 3.5e-8.
+// order; the seven smaller products, below 2^-6 of the first, go into an accumulator of their own (D2) that stays until the end.  Their signs
+// are as good as random whatever the operands': h truncated, they had those of the operands, and where all of these are positive, a long D2, truncated
+// at every addition, was off by more than the first sums (K 8,192 in eight pieces, squares by absolute values 2.1e-7, 16,384 uniform numbers 1.7e-6).
+// Measured against 64 bits (2-norm of the error over that of the result), here and one multiply-add after another (gemm_simt.cu): normal operands
+// 130 x 2,048 x 12,416 1.3e-7 and 8.1e-7, 130 x 8,192 x 128 in eight pieces 1.2e-7 and 5.7e-7, 7 x 1,024 x 128 0.9e-7 and 4.2e-7; uniform ones of one sign
+// 130 x 8,192 x 128 0.8e-7 and 1.6e-7, 20 x 16,384 x 12,416 2.2e-7 and 1.7e-6; squares by absolute values 1.3e-7 and 1.8e-7, 2.6e-7 and 2.4e-6; rows of one
+// number 2.5e-8 and 2.5e-8, of two 3.4e-8 and 3.5e-8.
 // What is left after h and m is l only down to bfloat16's last bit, 2^-133: floats below 2^-110 may have bits past it, and an infinity or a not-a-number has
-// no parts at all.  Every row in which a block meets one (the bits that l drops are collected on the way, an instruction for two floats) is remembered, and
+// no parts at all, nor has a float that would round to one.  Every row in which a block meets one (the bits that l drops are collected on the way, an instruction for two floats) is remembered, and
 // that block's sums of it are taken anew, one multiply-add after another from the operands themselves (split_redo): slow, but whole.
 // (The collecting costs that feed-forward 275 us against 270; a row taken anew of its 300 some 50 us more, a row of a single one 1.4 to 1.8 times its time.)
 //
@@ -71,8 +74,8 @@ struct SplitParams {
 __device__ __forceinline__ void split4(const float4 v, uint32_t* h, uint32_t* m, uint32_t* l, uint32_t& lost) {
     const uint64_t minus = pack_f32x2(-1.0f, -1.0f);
     auto two = [&](float a, float b, uint32_t& h2, uint32_t& m2, uint32_t& l2) {
-        asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(h2) : "f"(b), "f"(a));
         float r0, r1;
+        h2 = pack_bf16(a, b);
         const uint64_t rest = fma_f32x2(pack_f32x2(__uint_as_float(h2 << 16), __uint_as_float(h2 & 0xffff0000u)), minus, pack_f32x2(a, b));
         unpack_f32x2(rest, r0, r1);
         m2 = pack_bf16(r0, r1);
