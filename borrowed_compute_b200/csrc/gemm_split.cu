@@ -66,6 +66,7 @@ struct SplitParams {
     const float *X, *W;          // the operands themselves
     const int* lost;             // the second way: [row][slice], whether three parts do not hold one of that slice's floats; slices a row and a piece of K
     int row_slices, piece_slices;
+    int starve;                  // test hook: the last piece's first tile expects 16 bytes that never come, so that a bounded wait runs out
     float act_a, act_b;
     int act_cols;
 };
@@ -129,11 +130,14 @@ __device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, 
         tmem_dealloc(tmem, 512);
     }
     const uint4 of_w = *reinterpret_cast<const uint4*>(lost), of_x = *reinterpret_cast<const uint4*>(lost + 4);
-    const bool redo = (of_w.x | of_w.y | of_w.z | of_w.w | of_x.x | of_x.y | of_x.z | of_x.w) && !*reinterpret_cast<const volatile int*>(gave_up);
+    int failed = *reinterpret_cast<const volatile int*>(gave_up);
+    const bool redo = (of_w.x | of_w.y | of_w.z | of_w.w | of_x.x | of_x.y | of_x.z | of_x.w) && !failed;
     if (redo) split_redo<EPI>(p, tile, lost, t0, n0);
-    if (S > 1) cg::this_cluster().sync();
-    else if (redo) __syncthreads();
-    if (!*reinterpret_cast<const volatile int*>(gave_up)) {
+    if (S > 1) {
+        cg::this_cluster().sync();
+        for (int z = 0; z < S; z++) failed |= *cg::this_cluster().map_shared_rank(gave_up, z);      // what one gave up, no other writes
+    } else if (redo) __syncthreads();
+    if (!failed) {
         const int rows = min(p.bn, p.M - t0);
         for (int e = blockIdx.z * SPL_THREADS + threadIdx.x; e < rows * OUT_COLS; e += S * SPL_THREADS) {
             const int r = e / OUT_COLS, c = e % OUT_COLS, n = n0 + c;
@@ -289,11 +293,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     } else if (warp == 16) {
         if (elect_one()) {
             const int second = EPI == EPI_SWIGLU ? p.second_row + n0 : n0 + HALF_N;
+            const bool starve = p.starve && blockIdx.z + 1 == gridDim.z;
             for (int j = 0, s = 0, round = 0; j < chunks; j++) {
                 const int k = k_begin + j * SPL_K;
                 if (round && !(ok = mbar_wait(raw_empty + 8 * s, (round - 1) & 1, 4))) break;
                 const uint32_t dst = smem_u32(smem + (size_t)s * stage_bytes), bar = raw_full + 8 * s;
-                mbar_expect_tx(bar, (uint32_t)stage_bytes);
+                mbar_expect_tx(bar, (uint32_t)stage_bytes + (j == 0 && starve ? 16 : 0));
                 tma_load_2d(dst, &map_w, bar, k, n0);
                 tma_load_2d(dst + SPL_W_BYTES / 2, &map_w, bar, k, second);
                 tma_load_2d(dst + SPL_W_BYTES, &map_x, bar, k, t0);
@@ -485,9 +490,10 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     } else if (warp == 16) {
         if (elect_one()) {
             const int second = EPI == EPI_SWIGLU ? p.second_row + n0 : n0 + HALF_N;
+            const bool starve = p.starve && blockIdx.z + 1 == gridDim.z;
             auto load_w = [&](int j, int s) {
                 const uint32_t dst = smem_u32(smem + s * SPL_W_BYTES), bar = w_full + 8 * s;
-                mbar_expect_tx(bar, SPL_W_BYTES);
+                mbar_expect_tx(bar, SPL_W_BYTES + (j == 0 && starve ? 16 : 0));
                 tma_load_2d(dst, &map_w, bar, k_begin + j * SPL_K, n0);
                 tma_load_2d(dst + SPL_W_BYTES / 2, &map_w, bar, k_begin + j * SPL_K, second);
             };
@@ -606,6 +612,9 @@ extern "C" int bc_gemm_split_takes(const void* X, const void* W, int cols, int K
     return K > 512 && K % 4 == 0 && (uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0 && (long long)cols <= 65535ll * 64 && bc_encode_tiled_fn() != nullptr;
 }
 
+static int g_split_starve = 0;
+extern "C" void bc_gemm_split_test_starve_next_launch() { g_split_starve = 1; }
+
 static int split_k_row(int K) { return (K + 7) / 8 * 8; }
 // Bytes of scratch: three planes of the rows that go the second way, and a word a row and slice of K (the pieces' slices, at most K / SPL_SLICE and ten more).
 extern "C" long long bc_gemm_split_scratch(int M, int K) { return M <= SPL_FEW ? 6ll * M * split_k_row(K) + 4ll * M * (K / SPL_SLICE + 10) : 0; }
@@ -624,6 +633,8 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
     p.piece_slices = (p.piece + SPL_SLICE - 1) / SPL_SLICE, p.row_slices = splits * p.piece_slices;
     int* lost = few ? (int*)((char*)scratch + 6ll * M * split_k_row(K)) : nullptr;
     p.lost = lost;
+    p.starve = g_split_starve;
+    g_split_starve = 0;
     // A ring of chunks, both operands' raw tiles or the weights' alone, and stages of 64 k of the tokens' planes.
     p.x_stages = !few || p.bn > 64 ? 2 : SPL_X_STAGES;
     const int stage = SPL_W_BYTES + (few ? 0 : p.bn * 128), planes = p.x_stages * 3 * p.bn * 128;

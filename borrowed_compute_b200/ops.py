@@ -544,6 +544,11 @@ def gemm_tc_test_starve_next_launch() -> None:
     lib().bc_gemm_tc_test_starve_next_launch()
 
 
+def gemm_split_test_starve_next_launch() -> None:
+    """The same for the next float32 product on the tensor cores (csrc/gemm_split.cu): of its pieces of K the last."""
+    lib().bc_gemm_split_test_starve_next_launch()
+
+
 # ------------------------------------------------------------ errors that reach the caller
 
 _STATUS_UNITS = ("the tensor-core product (gemm_tc)", "the tcgen05 prompt attention (attention_prefill_tc)", "the decode attention (attention_decode)",

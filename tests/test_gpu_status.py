@@ -52,6 +52,35 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_launch_is_right():
     ops.check_status()
 
 
+@pytest.mark.parametrize("M,K", [(8, 520), (8, 2100), (130, 520), (130, 1028)])       # the two ways, in one piece of K, in two and in four
+def test_a_float32_product_that_gives_up_is_reported_and_the_next_is_right(M, K):
+    from borrowed_compute_b200 import ops
+
+    ops.bind_status()
+    torch.cuda.synchronize()
+    ops.check_status()
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(300, K, generator=g, device="cuda")
+    want = x.double() @ w.double().T
+    ops.set_wait_cycles(2_000_000)
+    try:
+        for _ in range(3):                                  # every time with all of the SMs' tensor memory
+            out = torch.full((M, 300), 7.0, device="cuda")
+            ops.gemm_split_test_starve_next_launch()
+            ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+            torch.cuda.synchronize()
+            with pytest.raises(ops.KernelError, match="true 32-bit product.*ran out"):
+                ops.check_status()
+            assert bool((out == 7.0).all()), "a block that gave up writes nothing, and no block that adds its piece"
+            ops.check_status()
+    finally:
+        ops.set_wait_cycles(0)
+    ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert ((out.double() - want).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)).all()
+
+
 def test_the_entry_point_raises_when_a_kernel_gave_up(model_folders):
     from borrowed_compute_b200 import Local, ops
 
