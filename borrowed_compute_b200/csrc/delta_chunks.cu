@@ -209,10 +209,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
             if (lane < CHUNK) part[warp][lane] = kk[0];
         }
         __syncthreads();
-        if (d < CHUNK) {                          // once a row, not once a channel; an infinity's quotients are its reciprocal's products, nothing more
-            const float of = sqrtf(part[0][d] + part[1][d] + key_eps);
-            norm[d] = make_float2(isinf(of) ? 0.0f : of, 1.0f / of);
-        }
+        if (d < CHUNK) norm[d] = divisor(sqrtf(part[0][d] + part[1][d] + key_eps));      // once a row, not once a channel
         __syncthreads();
         float* dst = pack + ((size_t)todo_place[c] * H + h) * PACK;
         float U[CHUNK], own[CHUNK];               // u_t W_(t-1), then P, and r_t W_t, then X0; in the last warp columns of Bm, then M, and of Gm, then G
@@ -225,9 +222,7 @@ delta_chunks_kernel(const ChunkSpan span, const float* proj, int stride, const f
                 const bool ok = mine && t < rows;
                 const float k = ok ? sk[t][d] : 0.0f;
                 const float rate = sigmoid_f((ok ? sa[t][d] : 0.0f) + bias);
-                // k / norm: the product with the reciprocal, and once what that leaves over (Markstein's quotient).  Zero in rows and channels that do not exist.
-                const float2 by = norm[t];
-                const float quotient = k * by.y, u = ok ? fmaf(fmaf(-quotient, by.x, k), by.y, quotient) : 0.0f;
+                const float u = ok ? quotient(k, norm[t]) : 0.0f;      // zero in rows and channels that do not exist
                 U[t] = u * run;
                 run *= ok ? sw[t][d] : 1.0f;
                 own[t] = (ok ? sr[t][d] : 0.0f) * run;
@@ -399,5 +394,18 @@ extern "C" int bc_delta_chunked(const float* proj, int stride, const float* w2t,
         bc_set_error("delta_chunked: %s", cudaGetErrorString(e));
         return (int)e;
     }
+    BC_LAUNCH_STATUS();
+}
+
+// out[i] = 1 / a[i], its sigmoid, or a[i] / b[i], as the kernels above work them out.  For tests.
+__global__ void delta_arithmetic_kernel(const float* a, const float* b, float* out, int what, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    out[i] = what == 0 ? reciprocal(a[i]) : what == 1 ? sigmoid_f(a[i]) : quotient(a[i], divisor(b[i]));
+}
+extern "C" int bc_delta_arithmetic(const float* a, const float* b, float* out, int what, int n, cudaStream_t s) {
+    BC_CHECK_ARG(n >= 0 && what >= 0 && what <= 2 && (what < 2 || b != nullptr), "delta_arithmetic: bad arguments n=%d what=%d", n, what);
+    if (n == 0) return BC_OK;
+    delta_arithmetic_kernel<<<(n + 255) / 256, 256, 0, s>>>(a, b, out, what, n);
     BC_LAUNCH_STATUS();
 }
