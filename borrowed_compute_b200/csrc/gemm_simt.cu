@@ -1,7 +1,7 @@
 // Matrix product on the CUDA cores: Y[m, n] = sum_k X[m, k] * W[n, k], float accumulation
 // in ascending k, one fused multiply-add a term.  This is the product of the true 32-bit
 // path where K is short (at most 512) or the operands are not laid out for tensor copies (the others: gemm_split.cu, by the
-// matrix alone) and the checked twin of the tensor-core kernel for bf16 operands.  Reference: the same contraction is k_matmul,
+// matrix alone) and the checked twin of the tensor-core kernels, for bf16 operands and for those others.  Reference: the same contraction is k_matmul,
 // crates/bc-infer/src/gpu/kernels.h:204-223, one warp a weight row.  An output's sum never depends on how many other rows
 // share the launch: k is walked in ascending order, in one piece or in two to eight equal ones whose sums are added in
 // ascending order (simt_splits, by the matrix alone), whichever of the kernels below takes the launch.

@@ -80,8 +80,10 @@ moe_logits_kernel(const T* __restrict__ h, const float* __restrict__ router, flo
 // The same sums where rows are many: sixteen rows by sixteen experts a block, four by eight a warp, both operands through shared memory 256 k at a time,
 // the next ones on their way.  A lane's share of a row's sum and the order of the shares are those of the kernel above, so are the bits.
 // What bounds that one at many rows are its reads (two 16-byte loads for eight multiply-adds); here twelve serve 128.
-// Logits and choice, us, that kernel and this: bfloat16, K 2,048, 64 experts: 4,096 rows 81 and 54, 2,048 48 and 34, 500 24 and 17, 256 17 and 17, 64 17 and 17; 64 rows of
-// 32 experts, K 4,096 26 and 24; 600 of 17, K 1,000 17 and 13; but of 8 experts, half a tile, 9,000 rows 36 and 38, 2,048, K 4,096 24 and 26.
+// Logits and choice behind a kernel that writes the rows, its time in them, router cold, us, that kernel and this: bfloat16, K 2,048, 64 experts: 4,096 rows 83 and 56,
+// 2,048 48 and 34, 512 24 and 16, 64 16 and 15, 1 16 and 14; K 4,096, 32 experts: 2,048 rows 54 and 35, 64 24 and 22, 1 23 and 21; K 7,168, 256 experts: 512 rows
+// 131 and 89, 64 46 and 34, 1 36 and 32.  Sixteen experts: K 2,048 4,096 rows 36 and 25, 64 and one the same; K 4,096 64 to 1,024 rows 21 and 22.  But of 8 experts, half a
+// tile, 9,000 rows 36 and 38, 2,048, K 4,096 24 and 26, so from sixteen on at any number of rows.
 #define RT_ROWS 16
 #define RT_EXPERTS 16
 #define RT_K 256

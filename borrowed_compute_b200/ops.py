@@ -377,7 +377,8 @@ def _split_scratch(M: int, K: int) -> int:
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, act: Optional[Tuple[float, float]] = None,
               cols: Optional[int] = None, cores: bool = False) -> None:
     """out = x @ w.T with float accumulation, k ascending in one piece or in up to eight that are added in order: on the CUDA cores, or,
-    for float32 sums of more than 512 products, on the tensor cores with every operand whole, as three bfloat16 parts (csrc/gemm_split.cu);
+    for float32 sums of more than 512 products, on the tensor cores, every operand as the three bfloat16 parts that make it up and all products of
+    parts summed but those of two lowest ones, 2^-33 (csrc/gemm_split.cu);
     ``cores``: on the CUDA cores whatever the sizes, that kernel's checked twin.  Both operands are read after the kernels before this launch have ended.
     EPI_STORE: out in x's type; EPI_STORE_F32: float32; EPI_ADD_F32: out += (float32);
     EPI_SWIGLU: w stacks gate rows on up rows, out[:, j] = silu(g_j) * u_j in x's type;

@@ -1,8 +1,8 @@
 """The one place that decides which kernel multiplies matrices.
 
 ``linear(x, w, out, epilogue)`` computes ``x @ w.T`` with float accumulation.  On the
-32-bit path ``ops.gemm_simt`` chooses: every operand whole as three bfloat16 parts on the tensor
-cores, or, for short sums, the CUDA-core kernel; never tf32.  For
+32-bit path ``ops.gemm_simt`` chooses: every operand as three bfloat16 parts on the tensor
+cores (all products of parts but those of two lowest, 2^-33 of the whole), or, for short sums, the CUDA-core kernel; never tf32.  For
 bfloat16 it is the tcgen05 tensor-core kernel.  The CUDA-core kernel on the same operands is
 the checked twin of both and can be forced for a test with ``force_simt``.
 """
