@@ -23,13 +23,14 @@
 //   rows   Every block splits its weights, into tensor memory (the MMA's A operand, so that shared memory is free for the other), and its tokens, into
 //          shared memory.  What bounds it: eight tensor-core products a multiply-add (six: 32 k, a chunk, of 128 weight rows by N tokens in some 1,000 clocks of an SM
 //          at N 112), and the rounds of wait, split, store and fence of its warps, 1,425 clocks a chunk.
-//   few    Up to a tile of rows, where weights are what there is to read: a kernel splits the tokens once, into planes of bfloat16 in scratch memory; they
-//          come by TMA as they are multiplied and all sixteen warps split weights.  742 clocks a chunk at one token, most of them the weights' way from memory.
-//          With more rows the planes' six bytes instead of four a value through the L2, in every block, cost more than the splits: 300 rows of 16,384 x 2,048
-//          173 us against 158, 2,000 of 4,096 x 4,096 529 against 481; 130 of 1,024 x 2,816 34 against 31; 64 of 16,384 x 2,048 48 against 54, 128 of 512 x 1,024 21 against 27.
+//   few    Up to 64 rows, where weights are what there is to read: a kernel splits the tokens once, into planes of bfloat16 in scratch memory; they
+//          come by TMA as they are multiplied and all sixteen warps split weights, four buffers of triples on their way.
+//          With more rows the planes' six bytes instead of four a value through the L2, in every block, cost more than the splits.  Us, this way and the other:
+//          4,096 x 4,096 one row 21 and 27, 64 rows 28 and 31, 80 36 and 32, 112 40 and 33; 16,384 x 2,048 34 and 48, 47 and 54, 63 and 56, 70 and 59;
+//          2,048 x 8,192 36 and 50, 49 and 56, 63 and 57, 70 and 60; 512 x 1,024 11 and 13, 16 and 16, 19 and 17, 21 and 18.
 //
-// Times, caches cold, against gemm_simt.cu's: 300 rows of a feed-forward of 2,048 x 8,192 157 + 126 us, 544 + 303; 3 rows 44 + 44, 126 + 78;
-// 2,000 x 4,096 x 4,096 481, 1,574; one row of 2 x 14,336 x 4,096 126, 260, of 4,096 x 14,336 64, 219; 5 x 64 x 2,048 15, 35.
+// Times, caches cold, against gemm_simt.cu's: 300 rows of a feed-forward of 2,048 x 8,192 158 + 118 us, 544 + 303; 3 rows 32 + 37, 126 + 78;
+// 2,000 x 4,096 x 4,096 481, 1,574; one row of 2 x 14,336 x 4,096 110, 260, of 4,096 x 14,336 53, 219; 5 x 64 x 2,048 11, 35.
 // (Tried for many rows, none faster: sixteen warps that split and take sums out, three and four buffers of triples, two thirds of the products, 80 and 96 tokens a tile.)
 //
 // Every wait is bounded.
@@ -49,20 +50,21 @@ namespace cg = cooperative_groups;
 #define SPL_BN 128               // tokens a tile at most
 #define SPL_W_BYTES (TC_BM * SPL_K * 4)
 #define SPL_STAGES 8
-#define SPL_FEW 112              // rows at most that go the second way, in one tile
-#define SPL_X_STAGES 4           // stages of 64 k of their planes on their way at most
+#define SPL_FEW 64               // rows at most that go the second way, in one tile
+#define SPL_X_STAGES 4           // stages of 64 k of their planes on their way
 #define SPL_D2 256               // tensor memory of the first way: D1 at 0 and 128, D2, then two buffers of the weights' triples, 16 columns a part
 #define SPL_A 384
 
-// The second way: D1 (two of bn columns), D2, then the triples' buffers, three at 112 tokens, four below.
+// The second way: D1 (two of bn columns), D2, then the triples' buffers, one for each four of its warps.
 #define SPL_A_COLS 48
-__host__ __device__ constexpr int split_buffers(int bn) { return (512 - 3 * bn) / SPL_A_COLS > 4 ? 4 : (512 - 3 * bn) / SPL_A_COLS; }
+#define SPL_BUFFERS 4
+static_assert(3 * SPL_FEW + SPL_BUFFERS * SPL_A_COLS <= 512, "tensor memory");
 
 struct SplitParams {
     float* out;
     int M, N, K;
     int second_row;              // SwiGLU: the matrix row where the up rows start
-    int bn, stages, x_stages, piece;
+    int bn, stages, piece;
     const float *X, *W;          // the operands themselves
     const int* lost;             // the second way: [row][slice], whether three parts do not hold one of that slice's floats; slices a row and a piece of K
     int row_slices, piece_slices;
@@ -119,7 +121,7 @@ __device__ __noinline__ void split_redo(const SplitParams& p, float* tile, const
 
 // The end of both: the sums of the pieces of K, in ascending order out of the cluster's blocks, and the epilogue.
 template <int EPI>
-__device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, const int* gave_up, const uint32_t* lost, int t0, int n0) {
+__device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, int* gave_up, const uint32_t* lost, int t0, int n0) {
     constexpr int HALF_N = TC_BM / 2, OUT_COLS = EPI == EPI_SWIGLU ? HALF_N : TC_BM;
     const int S = gridDim.z;
     __syncwarp();
@@ -130,14 +132,15 @@ __device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, 
         tmem_dealloc(tmem, 512);
     }
     const uint4 of_w = *reinterpret_cast<const uint4*>(lost), of_x = *reinterpret_cast<const uint4*>(lost + 4);
-    int failed = *reinterpret_cast<const volatile int*>(gave_up);
-    const bool redo = (of_w.x | of_w.y | of_w.z | of_w.w | of_x.x | of_x.y | of_x.z | of_x.w) && !failed;
+    const bool failed_here = *reinterpret_cast<volatile int*>(gave_up);
+    const bool redo = (of_w.x | of_w.y | of_w.z | of_w.w | of_x.x | of_x.y | of_x.z | of_x.w) && !failed_here;
     if (redo) split_redo<EPI>(p, tile, lost, t0, n0);
     if (S > 1) {
+        cg::this_cluster().barrier_wait();                   // of the start: all blocks' words are there
+        if (failed_here && threadIdx.x < S) *cg::this_cluster().map_shared_rank(gave_up, threadIdx.x) = 1;      // what one gives up, no other writes
         cg::this_cluster().sync();
-        for (int z = 0; z < S; z++) failed |= *cg::this_cluster().map_shared_rank(gave_up, z);      // what one gave up, no other writes
     } else if (redo) __syncthreads();
-    if (!failed) {
+    if (!*reinterpret_cast<volatile int*>(gave_up)) {
         const int rows = min(p.bn, p.M - t0);
         for (int e = blockIdx.z * SPL_THREADS + threadIdx.x; e < rows * OUT_COLS; e += S * SPL_THREADS) {
             const int r = e / OUT_COLS, c = e % OUT_COLS, n = n0 + c;
@@ -195,6 +198,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (warp == 17) tmem_alloc(smem_u32(&tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
+    if (gridDim.z > 1) cg::this_cluster().barrier_arrive();      // (split_finish waits for it)
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     float* tile = reinterpret_cast<float*>(smem);        // [bn][128]: the result, over the raw ring once that is drained
@@ -373,8 +377,8 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __shared__ int gave_up;
     __shared__ __align__(16) uint32_t lost[8];      // rows whose floats three parts do not hold, a bit each: weight rows, tokens
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
-    const int bn = p.bn, stages = p.stages, x_stages = p.x_stages;
-    const int buffers = split_buffers(bn), d2_at = 2 * bn, a_at = 3 * bn;
+    const int bn = p.bn, stages = p.stages;
+    const int d2_at = 2 * bn, a_at = 3 * bn;
     const int plane = bn * 128;                              // bn rows of 64 k of one part; stages of three behind the ring of weights
     uint8_t* planes = smem + stages * SPL_W_BYTES;
     const int t0 = blockIdx.x * bn, n0 = blockIdx.y * (EPI == EPI_SWIGLU ? HALF_N : TC_BM);
@@ -406,6 +410,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (warp == 17) tmem_alloc(smem_u32(&tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
+    if (gridDim.z > 1) cg::this_cluster().barrier_arrive();      // (split_finish waits for it)
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     float* tile = reinterpret_cast<float*>(smem);        // [bn][128]: the result, over the ring of weights once that is drained
@@ -413,12 +418,12 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     auto wait = [&](uint32_t bar, int phase, int code) { return ok = mbar_wait_warp(bar, phase & 1, code); };   // the whole warp
     pdl_launch_dependents();
     if (warp < 16) {
-        // Chunk j is four warps' (j % 4): out of ring stage j % stages into tensor memory buffer j % buffers, free when the products of chunk j - buffers
+        // Chunk j is four warps' (j % 4): out of ring stage j % stages into tensor memory buffer j % 4, free when the products of chunk j - 4
         // are done.  After its chunk every warp takes its share of the stretches (two chunks each) before out of D1.
         const int q = warp & 3, part = warp >> 2;
         const int row = 32 * q + lane;
         const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16);
-        uint64_t acc[2][8] = {};                             // token columns 16 part .. and 64 + 16 part ..
+        uint64_t acc[8] = {};                                // token columns 16 part ..
         uint32_t dropped = 0;
         int taken = 0;
         auto take_out_before = [&](int end) {
@@ -426,21 +431,20 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 const int b = taken & 1;
                 if (!wait(d1_full + 8 * b, taken >> 1, 3)) return;
                 tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    if (64 * c + 16 * part >= bn) break;
+                if (16 * part < bn) {
                     uint32_t v[16];
-                    tmem_load16(lanes + bn * b + 64 * c + 16 * part, v);
+                    tmem_load16(lanes + bn * b + 16 * part, v);
                     tmem_load_wait();
 #pragma unroll
-                    for (int e = 0; e < 8; e++) acc[c][e] = add_f32x2(acc[c][e], pack_f32x2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
+                    for (int e = 0; e < 8; e++) acc[e] = add_f32x2(acc[e], pack_f32x2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(d1_empty + 8 * b);
             }
         };
-        for (int j = part, s = part % stages, round = part / stages, buffer = part % buffers; j < chunks; j += 4) {
+        const uint32_t to = lanes + a_at + part * SPL_A_COLS;
+        for (int j = part, s = part % stages, round = part / stages; j < chunks; j += 4) {
             if (!wait(w_full + 8 * s, round, 1)) break;
             const uint8_t* src = smem + s * SPL_W_BYTES + row * 128;
             uint32_t h[16], m[16], l[16];
@@ -452,17 +456,15 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * s);
             if ((s += 4) >= stages) s -= stages, round++;
-            if (j >= buffers && !wait(done + 8 * ((j - buffers) & 3), (j - buffers) >> 2, 2)) break;
+            if (j >= 4 && !wait(done + 8 * part, (j >> 2) - 1, 2)) break;
             tc_fence_after();
-            const uint32_t to = lanes + a_at + buffer * SPL_A_COLS;
             tmem_store16(to, h);
             tmem_store16(to + 16, m);
             tmem_store16(to + 32, l);
             tmem_store_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready + 8 * (j & 3));
-            if ((buffer += 4 % buffers) >= buffers) buffer -= buffers;
+            if (lane == 0) mbar_arrive(ready + 8 * part);
             take_out_before(j / 2);       // all but the stretch under way: the products of the next one but one wait for this one's sums
             if (!ok) break;
         }
@@ -471,19 +473,17 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         if (ok) take_out_before(periods);
         if (ok) {
             // D1's last sums came after the last product, D2's with them.  No tile is on its way and none is read any more.
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                if (64 * c + 16 * part >= bn) break;
+            if (16 * part < bn) {
                 uint32_t v[16];
-                tmem_load16(lanes + d2_at + 64 * c + 16 * part, v);
+                tmem_load16(lanes + d2_at + 16 * part, v);
                 tmem_load_wait();
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
                     float a0, a1;
-                    unpack_f32x2(acc[c][e], a0, a1);
-                    float* to = tile + (64 * c + 16 * part + 2 * e) * TC_BM + 32 * q + lane;
-                    to[0] = a0 + __uint_as_float(v[2 * e]);
-                    to[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
+                    unpack_f32x2(acc[e], a0, a1);
+                    float* at = tile + (16 * part + 2 * e) * TC_BM + 32 * q + lane;
+                    at[0] = a0 + __uint_as_float(v[2 * e]);
+                    at[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
                 }
             }
         }
@@ -507,7 +507,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     const uint32_t dst = smem_u32(planes + xs * 3 * plane), bar = x_full + 8 * xs;
                     mbar_expect_tx(bar, (uint32_t)(3 * plane));
                     for (int i = 0; i < 3; i++) tma_load_3d(dst + i * plane, &map_x, bar, k_begin + j * SPL_K, t0, i);
-                    if (++xs == x_stages) xs = 0, x_round++;
+                    if (++xs == SPL_X_STAGES) xs = 0, x_round++;
                 }
                 if (round) {
                     if (!(ok = mbar_wait(w_empty + 8 * s, (round - 1) & 1, 4))) break;
@@ -533,7 +533,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const uint32_t idesc = instr_desc(bn);
         const uint64_t b_desc = smem_desc(smem_u32(planes));
         const uint32_t part = (uint32_t)plane >> 4;
-        for (int j = 0, buffer = 0, xs = 0, x_round = 0; j < chunks; j++) {
+        for (int j = 0, xs = 0, x_round = 0; j < chunks; j++) {
             const int b = (j >> 1) & 1;
             const bool last = (j & 1) || j + 1 == chunks;     // of its stretch and its stage of tokens
             if (!(j & 1)) {
@@ -545,7 +545,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < SPL_K / 16; kk++) {
-                    const uint32_t a = tmem + a_at + buffer * SPL_A_COLS + 8 * kk;
+                    const uint32_t a = tmem + a_at + (j & 3) * SPL_A_COLS + 8 * kk;
                     const uint64_t h = b_desc + (uint64_t)(xs * 3 * part + (j & 1) * 4 + 2 * kk), m = h + part, l = m + part;
                     mma_bf16_a_tmem(tmem + bn * b, a, h, idesc, (j & 1) | kk);
                     mma_bf16_a_tmem(tmem + d2_at, a + 16, h, idesc, j | kk);
@@ -563,8 +563,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
             __syncwarp();
-            if (last && ++xs == x_stages) xs = 0, x_round++;
-            if (++buffer == buffers) buffer = 0;
+            if (last && ++xs == SPL_X_STAGES) xs = 0, x_round++;
         }
     }
     pdl_wait();       // the output may still be in use by a kernel before
@@ -636,8 +635,7 @@ static int launch(const void* X, const void* W, void* out, int M, int N, int K, 
     p.starve = g_split_starve;
     g_split_starve = 0;
     // A ring of chunks, both operands' raw tiles or the weights' alone, and stages of 64 k of the tokens' planes.
-    p.x_stages = !few || p.bn > 64 ? 2 : SPL_X_STAGES;
-    const int stage = SPL_W_BYTES + (few ? 0 : p.bn * 128), planes = p.x_stages * 3 * p.bn * 128;
+    const int stage = SPL_W_BYTES + (few ? 0 : p.bn * 128), planes = (few ? SPL_X_STAGES : 2) * 3 * p.bn * 128;
     p.stages = (TC_SMEM_LIMIT - 1024 - planes) / stage;
     if (p.stages > SPL_STAGES) p.stages = SPL_STAGES;
     const int smem = p.stages * stage + planes + 1024;

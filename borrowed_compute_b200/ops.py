@@ -365,7 +365,7 @@ def _act_numbers(who: str, epilogue: int, act: Optional[Tuple[float, float]], co
     return (0.0, 0.0, int(cols)) if act is None else (float(act[0]), float(act[1]), 0)
 
 
-SPLIT_FEW = 112     # rows at most whose parts the float32 product on the tensor cores keeps in scratch memory (csrc/gemm_split.cu)
+SPLIT_FEW = 64     # rows at most whose parts the float32 product on the tensor cores keeps in scratch memory (csrc/gemm_split.cu)
 
 
 def _split_scratch(M: int, K: int) -> int:
