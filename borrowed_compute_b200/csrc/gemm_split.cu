@@ -119,6 +119,20 @@ __device__ __noinline__ void split_redo(const SplitParams& p, float* tile, const
     }
 }
 
+// Two tokens' sums of a weight row into the tile; `largest`: of their bits without the sign.
+__device__ __forceinline__ void split_put(float* at, float s0, float s1, uint32_t& largest) {
+    at[0] = s0;
+    at[TC_BM] = s1;
+    largest = max(largest, max(__float_as_uint(s0) << 1, __float_as_uint(s1) << 1));
+}
+// A sum that is not finite may be the parts' doing (first parts rounded up, their product past the largest float): its token's sums are taken anew as well.
+// This thread's sums: of `tokens` tokens from token0 on.
+__device__ __forceinline__ void split_overflow(const float* at, int token0, int tokens, uint32_t* lost, uint32_t largest) {
+    if (largest < 0xff000000u) return;
+    for (int t = 0; t < tokens; t++)
+        if (!(fabsf(at[t * TC_BM]) < INFINITY)) atomicOr(&lost[4 + ((token0 + t) >> 5)], 1u << ((token0 + t) & 31));
+}
+
 // The end of both: the sums of the pieces of K, in ascending order out of the cluster's blocks, and the epilogue.
 template <int EPI>
 __device__ __forceinline__ void split_finish(const SplitParams& p, float* tile, uint32_t tmem, bool dealloc, int* gave_up, const uint32_t* lost, int t0, int n0) {
@@ -253,7 +267,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             mbar_arrive(ready + 8 * (j & 3));
         }
         const uint32_t rows = __ballot_sync(0xffffffffu, dropped & 0xffffu);
-        if (lane == 0) lost[warp] = rows;
+        if (lane == 0 && rows) atomicOr(&lost[warp], rows);
     } else if (warp < 16) {
         // Two warps a quarter of the lanes: every other sixteen of the token columns each.
         const int q = warp & 3, half = (warp - 8) >> 2;
@@ -281,17 +295,17 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 if (32 * c + 16 * half >= bn) break;
-                uint32_t v[16];
+                float* at = tile + (32 * c + 16 * half) * TC_BM + 32 * q + lane;
+                uint32_t v[16], largest = 0;
                 tmem_load16(lanes + SPL_D2 + 32 * c, v);
                 tmem_load_wait();
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
                     float a0, a1;
                     unpack_f32x2(acc[c][e], a0, a1);
-                    float* to = tile + (32 * c + 16 * half + 2 * e) * TC_BM + 32 * q + lane;
-                    to[0] = a0 + __uint_as_float(v[2 * e]);
-                    to[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
+                    split_put(at + 2 * e * TC_BM, a0 + __uint_as_float(v[2 * e]), a1 + __uint_as_float(v[2 * e + 1]), largest);
                 }
+                split_overflow(at, 32 * c + 16 * half, 16, lost, largest);
             }
         }
     } else if (warp == 16) {
@@ -474,17 +488,17 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         if (ok) {
             // D1's last sums came after the last product, D2's with them.  No tile is on its way and none is read any more.
             if (16 * part < bn) {
-                uint32_t v[16];
+                float* at = tile + 16 * part * TC_BM + 32 * q + lane;
+                uint32_t v[16], largest = 0;
                 tmem_load16(lanes + d2_at + 16 * part, v);
                 tmem_load_wait();
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
                     float a0, a1;
                     unpack_f32x2(acc[e], a0, a1);
-                    float* at = tile + (16 * part + 2 * e) * TC_BM + 32 * q + lane;
-                    at[0] = a0 + __uint_as_float(v[2 * e]);
-                    at[TC_BM] = a1 + __uint_as_float(v[2 * e + 1]);
+                    split_put(at + 2 * e * TC_BM, a0 + __uint_as_float(v[2 * e]), a1 + __uint_as_float(v[2 * e + 1]), largest);
                 }
+                split_overflow(at, 16 * part, 16, lost, largest);
             }
         }
     } else if (warp == 16) {
@@ -527,7 +541,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (r < p.M)
                 for (int c = 0; c < p.piece_slices; c++) any |= flags[(size_t)r * p.row_slices + blockIdx.z * p.piece_slices + c];
             const uint32_t rows = __ballot_sync(0xffffffffu, any);
-            if (lane == 0) lost[4 + i] = rows;
+            if (lane == 0 && rows) atomicOr(&lost[4 + i], rows);
         }
     } else {
         const uint32_t idesc = instr_desc(bn);

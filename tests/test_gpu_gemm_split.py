@@ -94,11 +94,12 @@ def test_rows_of_few_numbers(M, kept):
         assert most <= 2.0 ** -24 + 2.0 ** -26 and most_there <= 2.0 ** -24, (most, most_there)
 
 
-def test_numbers_at_the_ends_of_the_range():
+@pytest.mark.parametrize("M", [40, 130])
+def test_numbers_at_the_ends_of_the_range(M):
     """Infinities and not-a-numbers reach every output of their row and column and no other; the largest floats and small ones keep their bits."""
     from borrowed_compute_b200 import ops
 
-    M, N, K = 40, 140, 1032
+    N, K = 140, 1032
     inf, biggest = float("inf"), 3.4028234663852886e38
     x, w = torch.ones((M, K), device="cuda"), torch.ones((N, K), device="cuda")
     x[2, K - 1], x[3, 0], x[5, 7], w[9, 40] = inf, float("nan"), -inf, inf
@@ -112,6 +113,14 @@ def test_numbers_at_the_ends_of_the_range():
     assert (out[4][others] == biggest).all() and out[4, 9].isnan()
     assert (out[[0, 1, 8]][:, others] == K).all() and (out[[0, 1, 8], 9] == inf).all()
     assert ((out[6][others].double() / (K * 2.0 ** -100 * (1 + 2.0 ** -23)) - 1).abs() <= bound(K)).all() and (out[7][others] == 0).all()
+    # Results within a rounded first part of the largest float, and sums that are larger.
+    x[8, 1:], x[9, 2:], w[20, :], w[20, 0] = 0.0, 0.0, 0.0, 2.0 ** 64
+    x[8, 0], x[9, 0], x[9, 1], w[21, 1] = (2 - 2.0 ** -9) * 2.0 ** 63, biggest, biggest, 1.0
+    ops.gemm_simt(x, w, out, ops.EPI_STORE_F32)
+    assert out[8, 20] == (2 - 2.0 ** -9) * 2.0 ** 127 and (out[8][[n for n in others if n != 20]] == (2 - 2.0 ** -9) * 2.0 ** 63).all() and out[9, 21] == inf
+    alone = torch.empty((1, N), device="cuda")
+    ops.gemm_simt(x[8:9].contiguous(), w, alone, ops.EPI_STORE_F32)
+    assert torch.equal(alone[0][others], out[8][others])
     # A payload below bfloat16's bits is still not a number.
     odd = torch.full((1, K), 1.0, device="cuda")
     odd.view(torch.int32)[0, 3] = 0x7F800001
